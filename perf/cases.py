@@ -174,6 +174,98 @@ def work(case):
             "flops": 3.0 * flops}
 
 
+_GATED = {
+    "swiglu": torch.nn.functional.silu,
+    "geglu": lambda g: torch.nn.functional.gelu(g, approximate="tanh"),
+    "geglu_erf": torch.nn.functional.gelu,
+    "relu_squared": lambda g: torch.relu(g).square(),
+}
+
+
+def exact(case, seed):
+    """What run() returns, evaluated in 64 bits on the operands the layer computes with: parameters and tokens as bf16
+    values, router logits rounded to bf16 (the layer's contract: experts are chosen on them, ties to the lower index),
+    everything after that unrounded."""
+    state = prepare(case, seed)
+    train = case["kind"] == "train"
+    if "layer" in state:
+        names = [n for n, _ in state["layer"].named_parameters()]
+    else:
+        names = ["gate.weight", "w_up", "w_down"]
+    given = dict(zip(names, state["weights"]))
+    k, e, act = case["top_k"], case["experts"], case["activation"]
+    h = case["ffn_dim"] // 2
+
+    def wide(t):
+        return t.detach().to(torch.bfloat16).double()
+
+    x = wide(state["x"])
+    n = x.shape[0]
+    logits = (x @ wide(given["gate.weight"]).T).to(torch.bfloat16).double()
+    value = logits if case["gating"] == "softmax" else torch.sigmoid(logits)
+    select = value.float() + state["bias"] if "bias" in state else value
+    idx = torch.sort(select, dim=1, descending=True, stable=True).indices[:, :k]
+    leaf = logits.requires_grad_(train)
+    picked = (leaf if case["gating"] == "softmax" else torch.sigmoid(leaf)).gather(1, idx)
+    weight = torch.softmax(picked, 1) if case["gating"] == "softmax" else picked / (picked.sum(1, keepdim=True) + 1e-6)
+    losses = []
+    if train and case["aux"] > 0:
+        f = torch.bincount(idx.reshape(-1), minlength=e).double() / n
+        if case["gating"] == "softmax":
+            share = torch.zeros(e, dtype=torch.float64, device=x.device).scatter_add(0, idx.reshape(-1), weight.reshape(-1)) / n
+        else:
+            share = torch.sigmoid(leaf).mean(0)
+        losses.append(case["aux"] * e * (f * share).sum())
+    if train and case["z"] > 0:
+        losses.append(case["z"] * torch.logsumexp(leaf, 1).square().mean())
+    out, go = torch.zeros_like(x), wide(state["grad_out"]) if train else None
+    dx, dweight, grads = torch.zeros_like(x), torch.zeros_like(weight), {}
+
+    def glu(rows, w_gate, w_up, w_down, g_rows, scale, activation):
+        """GLU feed-forward of `rows`; with g_rows, the gradient of its scaled output, also every gradient."""
+        a, u = rows @ w_gate.T, rows @ w_up.T
+        if g_rows is None:
+            return (_GATED[activation](a) * u) @ w_down.T, None
+        a.requires_grad_(True)
+        gated = _GATED[activation](a)
+        hidden = (gated * u).detach()
+        y = hidden @ w_down.T
+        dy = g_rows * scale
+        dhid = dy @ w_down
+        da = torch.autograd.grad(gated, a, dhid * u)[0]
+        du = dhid * gated.detach()
+        return y, (da @ w_gate + du @ w_up, da.T @ rows, du.T @ rows, dy.T @ hidden)
+
+    if train:
+        grads["w_up"] = torch.zeros(given["w_up"].shape, dtype=torch.float64, device=x.device)
+        grads["w_down"] = torch.zeros(given["w_down"].shape, dtype=torch.float64, device=x.device)
+    for i in range(e):
+        token, slot = torch.nonzero(idx == i, as_tuple=True)
+        if token.numel() == 0:
+            continue
+        w = wide(given["w_up"][i])
+        scale = weight.detach()[token, slot].unsqueeze(1)
+        y, g = glu(x[token], w[:h], w[h:], wide(given["w_down"][i]), go[token] if train else None, scale, act)
+        out.index_add_(0, token, y * scale)
+        if train:
+            dweight[token, slot] = (go[token] * y).sum(1)
+            dx.index_add_(0, token, g[0])
+            grads["w_up"][i, :h], grads["w_up"][i, h:], grads["w_down"][i] = g[1], g[2], g[3]
+    if "shared_expert.w_gate.weight" in given:
+        own = ["shared_expert.%s.weight" % m for m in ("w_gate", "w_up", "w_down")]
+        y, g = glu(x, *(wide(given[m]) for m in own), go, 1.0, "geglu_erf" if act == "geglu" else act)
+        out += y
+        if train:
+            dx += g[0]
+            grads.update(zip(own, g[1:]))
+    if not train:
+        return out
+    dlogits = torch.autograd.grad([(weight * dweight).sum(), *losses], leaf)[0]
+    grads["gate.weight"] = dlogits.T @ x
+    dx += dlogits @ wide(given["gate.weight"])
+    return [out, *[t.detach() for t in losses], dx, *[grads[m] for m in names]]
+
+
 def tolerance(case):
     # Against an fp32 evaluation with the same expert choice every output and gradient of the bf16 path lies within
     # rel 4.9e-3 and max 5.1e-2 (bf16 roundings of the pre-activations, activations, expert outputs and gradients in
