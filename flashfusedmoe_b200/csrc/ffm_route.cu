@@ -429,8 +429,8 @@ route_gate_topk(const bf16* __restrict__ hidden, const bf16* __restrict__ gate_w
       m += s_mass[w][e];
       c += s_cnt[w][e];
     }
-    block_mass[static_cast<long long>(blockIdx.x) * E + e] = m;
-    block_hist[static_cast<long long>(blockIdx.x) * E + e] = c;
+    block_mass[static_cast<long long>(e) * gridDim.x + blockIdx.x] = m;
+    block_hist[static_cast<long long>(e) * gridDim.x + blockIdx.x] = c;
   }
   if (threadIdx.x == 0) {
     float z = 0.0f;
@@ -490,8 +490,8 @@ route_from_logits(const bf16* __restrict__ logits, const float* __restrict__ bia
       m += s_mass[w][e];
       c += s_cnt[w][e];
     }
-    block_mass[static_cast<long long>(blockIdx.x) * E + e] = m;
-    block_hist[static_cast<long long>(blockIdx.x) * E + e] = c;
+    block_mass[static_cast<long long>(e) * gridDim.x + blockIdx.x] = m;
+    block_hist[static_cast<long long>(e) * gridDim.x + blockIdx.x] = c;
   }
   if (threadIdx.x == 0) {
     float z = 0.0f;
@@ -519,13 +519,52 @@ route_hist_ids(const int32_t* __restrict__ ids, long long T, int E, int slots_pe
     }
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < E; e += ROUTE_THREADS) block_hist[static_cast<long long>(blockIdx.x) * E + e] = s_cnt[e];
+  for (int e = threadIdx.x; e < E; e += ROUTE_THREADS) block_hist[static_cast<long long>(e) * gridDim.x + blockIdx.x] = s_cnt[e];
 }
 
-// One block. block_off[b][e] = sum_{b' < b} hist[b'][e]; counts; tile_start; stats.
-// One warp per expert: the lanes sweep the block histograms 32 at a time (independent loads, a shuffle scan and a
-// carry), so the kernel costs a few dozen dependent steps instead of one per block. All sums keep a fixed order.
-__global__ void __launch_bounds__(ROUTE_THREADS)
+// Segment starts (in 128-row tiles, always even) and the dot product of counts and probability masses, from per-expert
+// totals in shared memory. One warp, eight consecutive experts per lane: a fixed order of sums.
+__device__ __forceinline__ void finish_counts(const int* s_counts, const float* s_mass, float zsum, int E, int lane,
+                                              int32_t* __restrict__ tile_start, float* __restrict__ stats) {
+  constexpr int PER = MAX_E / 32;
+  int tiles[PER];
+  int mine = 0;
+  float dot = 0.0f;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int e = lane * PER + i;
+    const int c = e < E ? s_counts[e] : 0;
+    tiles[i] = ((c + 255) >> 8) << 1;  // segments start on multiples of 256 rows
+    mine += tiles[i];
+    if (e < E) dot += static_cast<float>(c) * s_mass[e];
+  }
+  int incl = mine;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += t;
+  }
+  int run = incl - mine;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int e = lane * PER + i;
+    if (e < E) tile_start[e] = run;
+    run += tiles[i];
+    if (e + 1 == E) tile_start[E] = run;
+  }
+  dot = warp_sum(dot);
+  if (lane == 0 && stats != nullptr) {
+    stats[E] = zsum;
+    stats[E + 1] = dot;
+  }
+}
+
+// One block of 32 warps. block_off[e][b] = sum_{b' < b} hist[e][b']; counts; tile_start; stats.
+// One warp per expert, the lanes sweep its block histograms 32 at a time: the histograms are stored expert-major, so a
+// sweep reads one 128-byte line (block-major, each lane touched its own line: with eight warps the kernel took 73 us at
+// 512 blocks x 64 experts and 49 us at 64 x 256; now 15 us and, on the path for few tokens, part of route_finish_small). All sums keep a fixed order.
+constexpr int SCAN_THREADS = 1024;
+__global__ void __launch_bounds__(SCAN_THREADS)
 route_scan(const int32_t* __restrict__ block_hist, const float* __restrict__ block_mass,
            const float* __restrict__ block_z, int blocks, int E, int32_t* __restrict__ block_off,
            int32_t* __restrict__ counts, int32_t* __restrict__ tile_start, float* __restrict__ stats) {
@@ -534,22 +573,22 @@ route_scan(const int32_t* __restrict__ block_hist, const float* __restrict__ blo
   __shared__ float s_zsum;
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  for (int e = warp; e < E; e += ROUTE_WARPS) {
+  for (int e = warp; e < E; e += SCAN_THREADS / 32) {
+    const long long row = static_cast<long long>(e) * blocks;
     int carry = 0;
     float m = 0.0f;
 #pragma unroll 4
     for (int b0 = 0; b0 < blocks; b0 += 32) {
       const int b = b0 + lane;
-      const long long o = static_cast<long long>(b) * E + e;
-      const int v = (b < blocks) ? block_hist[o] : 0;
-      if (block_mass != nullptr && b < blocks) m += block_mass[o];
+      const int v = (b < blocks) ? block_hist[row + b] : 0;
+      if (block_mass != nullptr && b < blocks) m += block_mass[row + b];
       int x = v;
 #pragma unroll
       for (int d = 1; d < 32; d <<= 1) {
         const int t = __shfl_up_sync(0xffffffffu, x, d);
         if (lane >= d) x += t;
       }
-      if (b < blocks) block_off[o] = carry + x - v;
+      if (b < blocks) block_off[row + b] = carry + x - v;
       carry += __shfl_sync(0xffffffffu, x, 31);
     }
     m = warp_sum(m);
@@ -560,7 +599,7 @@ route_scan(const int32_t* __restrict__ block_hist, const float* __restrict__ blo
       if (stats != nullptr) stats[e] = m;
     }
   }
-  if (warp == ROUTE_WARPS - 1) {
+  if (warp == SCAN_THREADS / 32 - 1) {
     float z = 0.0f;
     if (block_z != nullptr) {
       for (int b = lane; b < blocks; b += 32) z += block_z[b];
@@ -569,20 +608,7 @@ route_scan(const int32_t* __restrict__ block_hist, const float* __restrict__ blo
     if (lane == 0) s_zsum = z;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int tiles = 0;
-    float dot = 0.0f;
-    tile_start[0] = 0;
-    for (int e = 0; e < E; ++e) {
-      tiles += ((s_counts[e] + 255) >> 8) << 1;  // segments start on multiples of 256 rows
-      tile_start[e + 1] = tiles;
-      dot += static_cast<float>(s_counts[e]) * s_mass[e];
-    }
-    if (stats != nullptr) {
-      stats[E] = s_zsum;
-      stats[E + 1] = dot;
-    }
-  }
+  if (warp == 0) finish_counts(s_counts, s_mass, s_zsum, E, lane, tile_start, stats);
 }
 
 // Stable rank inside each expert segment. Each warp owns a contiguous run of the block's slots.
@@ -612,7 +638,7 @@ route_rank(const int32_t* __restrict__ ids, long long T, int E, int slots_per_bl
   __syncthreads();
   // exclusive scan over warps, per expert, plus the block and segment bases
   for (int e = threadIdx.x; e < E; e += ROUTE_THREADS) {
-    int run = tile_start[e] * 128 + block_off[static_cast<long long>(blockIdx.x) * E + e];
+    int run = tile_start[e] * 128 + block_off[static_cast<long long>(e) * gridDim.x + blockIdx.x];
     for (int w = 0; w < ROUTE_WARPS; ++w) {
       const int c = s_run[w][e];
       s_run[w][e] = run;
@@ -644,6 +670,205 @@ route_rank(const int32_t* __restrict__ ids, long long T, int E, int slots_per_bl
       if (r < rows_cap) {
         pos[i] = static_cast<int32_t>(r);
         src[r] = static_cast<int32_t>(i);
+      } else {
+        atomicCAS(status, 0, FFM_STATUS_BAD_INDEX);
+      }
+    }
+  }
+}
+
+// ---- few tokens (decode) -----------------------------------------------------------------------
+// With a handful of tokens the kernels above leave the chip idle: one warp walks the whole row of a token pair (72 us
+// at 7 tokens, D = 4096, E = 8), or one CTA pair walks the whole contraction of the tensor-core gate GEMM (46 us at 128
+// tokens, D = 7168, E = 256), and scan and rank are two more launches. Here the gate product is spread over (token
+// group x expert group) blocks whose eight warps split D, and one cluster does the rest.
+constexpr int SMALL_TOKENS = 256;   // most tokens of this path
+constexpr int SMALL_SLOTS = 4096;   // most routed slots (one block ranks them all)
+constexpr int SMALL_TG = 4;         // tokens per gate block
+constexpr int SMALL_EG = 8;         // experts per gate block
+constexpr int FINISH_THREADS = 512;
+constexpr int FINISH_WARPS = FINISH_THREADS / 32;
+constexpr int FINISH_CLUSTER = 8;
+
+// logits[n, e] = bf16(hidden[n, :] . gate_w[e, :]) in fp32, SMALL_EG experts x SMALL_TG tokens per block; also
+// src[:] = -1. Sixteen experts per block read fewer bytes from L2 but take 165 registers, one block per SM, and leave
+// the load latency exposed (42 us at 128 tokens, E = 256, D = 7168).
+__global__ void __launch_bounds__(ROUTE_THREADS, 2)
+route_gate_small(const bf16* __restrict__ hidden, const bf16* __restrict__ gate_w, int N, int D, int E,
+                 bf16* __restrict__ logits, int32_t* __restrict__ src, long long rows_cap) {
+  constexpr int EG = SMALL_EG;
+  constexpr int ACC = EG * SMALL_TG;
+  __shared__ float s_part[ROUTE_WARPS][ACC];
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int n0 = blockIdx.x * SMALL_TG;
+  const int e0 = blockIdx.y * EG;
+  const int chunks = D >> 3;
+  {
+    const long long nthreads = static_cast<long long>(gridDim.x) * gridDim.y * ROUTE_THREADS;
+    const long long tid = (static_cast<long long>(blockIdx.y) * gridDim.x + blockIdx.x) * ROUTE_THREADS + threadIdx.x;
+    for (long long i = tid; i < rows_cap; i += nthreads) src[i] = -1;
+  }
+  float acc[ACC];
+#pragma unroll
+  for (int i = 0; i < ACC; ++i) acc[i] = 0.0f;
+  for (int c = threadIdx.x; c < chunks; c += ROUTE_THREADS) {
+    uint4 h[SMALL_TG];
+#pragma unroll
+    for (int t = 0; t < SMALL_TG; ++t) {
+      const int n = min(n0 + t, N - 1);  // rows past the last token repeat it; their logits are not stored
+      h[t] = __ldg(reinterpret_cast<const uint4*>(hidden + static_cast<long long>(n) * D) + c);
+    }
+#pragma unroll
+    for (int e = 0; e < EG; ++e) {
+      const int ee = min(e0 + e, E - 1);
+      const uint4 w = __ldg(reinterpret_cast<const uint4*>(gate_w + static_cast<long long>(ee) * D) + c);
+#pragma unroll
+      for (int t = 0; t < SMALL_TG; ++t) acc[t * EG + e] = dot8(h[t], w, acc[t * EG + e]);
+    }
+  }
+  static_assert(ACC == 32, "one total per lane");
+  transpose_reduce<ACC>(acc, lane);
+  s_part[warp][lane] = acc[0];
+  __syncthreads();
+  if (threadIdx.x < ACC) {
+    const int n = n0 + threadIdx.x / EG;
+    const int e = e0 + threadIdx.x % EG;
+    float t = 0.0f;
+#pragma unroll
+    for (int w = 0; w < ROUTE_WARPS; ++w) t += s_part[w][threadIdx.x];
+    if (n < N && e < E) logits[static_cast<long long>(n) * E + e] = __float2bfloat16_rn(t);
+  }
+}
+
+// Scoring, top-k and statistics of every token (one warp each, spread over the cluster), then counts, segment starts
+// and the stable rank of every slot in block 0. Launched as one cluster of gridDim.x blocks.
+template <int NG>
+__global__ void __launch_bounds__(FINISH_THREADS)
+route_finish_small(const bf16* __restrict__ logits, const float* __restrict__ bias, int N, int E, int top_k,
+                   RouteOpts opts, float* __restrict__ topk_w, int32_t* topk_idx, float* __restrict__ lse_out,
+                   int32_t* block_hist, float* block_mass, float* block_z, int32_t* __restrict__ counts,
+                   int32_t* __restrict__ tile_start, float* __restrict__ stats, long long rows_cap,
+                   int32_t* __restrict__ pos, int32_t* __restrict__ src, int32_t* __restrict__ status) {
+  __shared__ float s_mass[FINISH_WARPS][NG * 32];
+  __shared__ int s_cnt[FINISH_WARPS][NG * 32];
+  __shared__ float s_z[FINISH_WARPS];
+  __shared__ int s_counts[MAX_E];
+  __shared__ float s_tot[MAX_E];
+  __shared__ int s_start[MAX_E + 1];
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int blocks = gridDim.x;
+  const int per_block = (N + blocks - 1) / blocks;
+  const int begin = blockIdx.x * per_block;
+  const int end = min(begin + per_block, N);
+  float mass[NG];
+  int cnt[NG];
+#pragma unroll
+  for (int g = 0; g < NG; ++g) {
+    mass[g] = 0.0f;
+    cnt[g] = 0;
+  }
+  float zsum = 0.0f;
+  for (int n = begin + warp; n < end; n += FINISH_WARPS) {
+    float logit[NG];
+#pragma unroll
+    for (int g = 0; g < NG; ++g) {
+      const int e = g * 32 + lane;
+      logit[g] = (e < E) ? __bfloat162float(logits[static_cast<long long>(n) * E + e]) : 0.0f;
+    }
+    route_token<32, NG>(logit, n, lane, E, top_k, opts, bias, nullptr, topk_w, topk_idx, lse_out, mass, cnt, zsum);
+  }
+#pragma unroll
+  for (int g = 0; g < NG; ++g) {
+    s_mass[warp][g * 32 + lane] = mass[g];
+    s_cnt[warp][g * 32 + lane] = cnt[g];
+  }
+  if (lane == 0) s_z[warp] = zsum;
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += FINISH_THREADS) {
+    float m = 0.0f;
+    int c = 0;
+    for (int w = 0; w < FINISH_WARPS; ++w) {
+      m += s_mass[w][e];
+      c += s_cnt[w][e];
+    }
+    block_mass[static_cast<long long>(e) * blocks + blockIdx.x] = m;
+    block_hist[static_cast<long long>(e) * blocks + blockIdx.x] = c;
+  }
+  if (threadIdx.x == 0) {
+    float z = 0.0f;
+    for (int w = 0; w < FINISH_WARPS; ++w) z += s_z[w];
+    block_z[blockIdx.x] = z;
+  }
+  // what the other blocks of the cluster wrote (ids, statistics) is visible to block 0 after this barrier
+  __threadfence();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (blockIdx.x != 0) return;
+  for (int e = threadIdx.x; e < E; e += FINISH_THREADS) {
+    float m = 0.0f;
+    int c = 0;
+    for (int b = 0; b < blocks; ++b) {
+      m += __ldcg(block_mass + static_cast<long long>(e) * blocks + b);
+      c += __ldcg(block_hist + static_cast<long long>(e) * blocks + b);
+    }
+    s_counts[e] = c;
+    s_tot[e] = m;
+    counts[e] = c;
+    stats[e] = m;
+  }
+  for (int i = threadIdx.x; i < FINISH_WARPS * NG * 32; i += FINISH_THREADS) (&s_cnt[0][0])[i] = 0;
+  __syncthreads();
+  if (warp == 0) {
+    float z = 0.0f;
+    for (int b = 0; b < blocks; ++b) z += __ldcg(block_z + b);
+    finish_counts(s_counts, s_tot, z, E, lane, s_start, stats);
+  }
+  // per-warp runs of slots, as in route_rank
+  const int T = N * top_k;
+  const int per_warp = ((T + FINISH_WARPS - 1) / FINISH_WARPS + 31) / 32 * 32;
+  const int wb = warp * per_warp;
+  const int we = min(wb + per_warp, T);
+  for (int i = wb + lane; i < we; i += 32) {
+    const int e = __ldcg(topk_idx + i);
+    if (e >= 0 && e < E) atomicAdd(&s_cnt[warp][e], 1);
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e <= E; e += FINISH_THREADS) {
+    tile_start[e] = s_start[e];
+    if (e < E) {
+      int run = s_start[e] * 128;
+      for (int w = 0; w < FINISH_WARPS; ++w) {
+        const int c = s_cnt[w][e];
+        s_cnt[w][e] = run;
+        run += c;
+      }
+    }
+  }
+  __syncthreads();
+  for (int i0 = wb; i0 < we; i0 += 32) {
+    const int i = i0 + lane;
+    const bool active = i < we;
+    int e = active ? __ldcg(topk_idx + i) : -1;
+    if (active && (e < 0 || e >= E)) {
+      atomicCAS(status, 0, FFM_STATUS_BAD_INDEX);
+      e = -1;
+    }
+    const unsigned same = __match_any_sync(0xffffffffu, e);
+    const int leader = __ffs(same) - 1;
+    const int rank = __popc(same & ((1u << lane) - 1u));
+    int base = 0;
+    if (e >= 0 && lane == leader) {
+      base = s_cnt[warp][e];
+      s_cnt[warp][e] = base + __popc(same);
+    }
+    base = __shfl_sync(0xffffffffu, base, leader);
+    __syncwarp();
+    if (e >= 0) {
+      const int r = base + rank;
+      if (r < rows_cap) {
+        pos[i] = r;
+        src[r] = i;
       } else {
         atomicCAS(status, 0, FFM_STATUS_BAD_INDEX);
       }
@@ -701,6 +926,32 @@ void launch_route(int blocks, cudaStream_t s, const bf16* hidden, const bf16* ga
   route_gate_topk<GW, NG><<<blocks, ROUTE_THREADS, in_smem ? gate_bytes : 0, s>>>(
       hidden, gate_w, bias, N, D, E, top_k, opts, tpb, logits, topk_w, topk_idx, lse, w.block_hist, w.block_mass,
       w.block_z, in_smem ? 1 : 0);
+}
+
+template <int NG>
+int launch_finish_small(const bf16* logits, const float* bias, int N, int E, int top_k, const RouteOpts& opts,
+                        float* topk_w, int32_t* topk_idx, float* lse, const RouteWorkspace& w, int32_t* counts,
+                        int32_t* tile_start, float* stats, long long rows_cap, int32_t* pos, int32_t* src,
+                        int32_t* status, cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
+  // up to one token per warp, a single block is enough; beyond, the tokens are spread over a cluster
+  cfg.gridDim = dim3(N <= FINISH_WARPS ? 1 : FINISH_CLUSTER, 1, 1);
+  cfg.blockDim = dim3(FINISH_THREADS, 1, 1);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cfg.gridDim.x;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, route_finish_small<NG>, logits, bias, N, E, top_k, opts, topk_w, topk_idx, lse,
+                         w.block_hist, w.block_mass, w.block_z, counts, tile_start, stats, rows_cap, pos, src,
+                         status) != cudaSuccess) {
+    cudaGetLastError();
+    return FFM_ERR_LAUNCH;
+  }
+  return FFM_OK;
 }
 
 // Expert capacity: a routed slot whose rank inside its expert segment is >= capacity is dropped. One thread
@@ -778,6 +1029,7 @@ extern "C" size_t ffm_route_workspace_bytes(int64_t N, int E, int top_k) {
   RouteGrid g = route_grid(N > 0 ? N : 1, route_granule(E));
   RouteGrid g2 = route_grid(N > 0 ? N * (top_k > 0 ? top_k : 1) : 1);
   int blocks = g.blocks > g2.blocks ? g.blocks : g2.blocks;
+  if (blocks < FINISH_CLUSTER) blocks = FINISH_CLUSTER;
   return carve_workspace(nullptr, blocks, E).bytes;
 }
 
@@ -804,12 +1056,30 @@ extern "C" int ffm_route_forward(const void* hidden, const void* gate_w, const f
   opts.topk_group = topk_group;
   if (workspace_bytes < ffm_route_workspace_bytes(N, E, top_k)) return FFM_ERR_WORKSPACE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (cudaMemsetAsync(src, 0xFF, static_cast<size_t>(rows_cap) * 4, s) != cudaSuccess) return FFM_ERR_LAUNCH;
-  const RouteGrid g = route_grid(N > 0 ? N : 1, route_granule(E));
-  RouteWorkspace w = carve_workspace(workspace, g.blocks, E);
   const bf16* h = static_cast<const bf16*>(hidden);
   const bf16* gw = static_cast<const bf16*>(gate_w);
   bf16* lg = static_cast<bf16*>(logits);
+  // Few tokens: two launches. The line lies where the gate product on CUDA cores (N E D multiply-adds, 29 us at
+  // N = 128, E = 256, D = 7168) stops being cheaper than the tensor-core GEMM, whose one CTA pair takes 46 us for that
+  // contraction; 7 tokens, E = 8, D = 4096: 6 + 6 us against 72 + 3 + 3 with the kernels for many tokens.
+  if (N > 0 && N <= SMALL_TOKENS && N * top_k <= SMALL_SLOTS && lg != nullptr) {
+    const RouteWorkspace w = carve_workspace(workspace, FINISH_CLUSTER, E);
+    const int n = static_cast<int>(N);
+    const dim3 grid((n + SMALL_TG - 1) / SMALL_TG, (E + SMALL_EG - 1) / SMALL_EG, 1);
+    route_gate_small<<<grid, ROUTE_THREADS, 0, s>>>(h, gw, n, D, E, lg, src, rows_cap);
+    if (cudaGetLastError() != cudaSuccess) return FFM_ERR_LAUNCH;
+#define FFM_FINISH_CASE(NG)                                                                                            \
+  launch_finish_small<NG>(lg, expert_bias, n, E, top_k, opts, topk_w, topk_idx, lse, w, counts, tile_start, stats, \
+                          rows_cap, pos, src, status, s)
+    if (E <= 32) return FFM_FINISH_CASE(1);
+    if (E <= 64) return FFM_FINISH_CASE(2);
+    if (E <= 128) return FFM_FINISH_CASE(4);
+    return FFM_FINISH_CASE(8);
+#undef FFM_FINISH_CASE
+  }
+  if (cudaMemsetAsync(src, 0xFF, static_cast<size_t>(rows_cap) * 4, s) != cudaSuccess) return FFM_ERR_LAUNCH;
+  const RouteGrid g = route_grid(N > 0 ? N : 1, route_granule(E));
+  RouteWorkspace w = carve_workspace(workspace, g.blocks, E);
   // Many experts: gate GEMM on the tensor cores (dense tcgen05 GEMM, fp32 accumulate, bf16 logits), then one
   // scoring kernel. Few experts: everything in one warp-level kernel.
   // (E = 32 included: one warp owning 32 experts keeps 64 accumulators per lane and ran at 0.12 TB/s)
@@ -849,7 +1119,7 @@ extern "C" int ffm_route_forward(const void* hidden, const void* gate_w, const f
 #undef FFM_ROUTE_CASE
   }
   FFM_PREFER_MAX_SHARED(route_scan);
-  route_scan<<<1, ROUTE_THREADS, 0, s>>>(w.block_hist, w.block_mass, w.block_z, g.blocks, E, w.block_off, counts,
+  route_scan<<<1, SCAN_THREADS, 0, s>>>(w.block_hist, w.block_mass, w.block_z, g.blocks, E, w.block_off, counts,
                                          tile_start, stats);
   route_rank<<<g.blocks, ROUTE_THREADS, 0, s>>>(topk_idx, N * top_k, E, g.tokens_per_block * top_k, w.block_off,
                                                 tile_start, rows_cap, pos, src, status);
@@ -869,7 +1139,7 @@ extern "C" int ffm_group_rows(const int32_t* expert_ids, int64_t T, int E, int32
   if (cudaMemsetAsync(src, 0xFF, static_cast<size_t>(rows_cap) * 4, s) != cudaSuccess) return FFM_ERR_LAUNCH;
   RouteWorkspace w = carve_workspace(workspace, g.blocks, E);
   route_hist_ids<<<g.blocks, ROUTE_THREADS, 0, s>>>(expert_ids, T, E, g.tokens_per_block, w.block_hist, status);
-  route_scan<<<1, ROUTE_THREADS, 0, s>>>(w.block_hist, nullptr, nullptr, g.blocks, E, w.block_off, counts, tile_start,
+  route_scan<<<1, SCAN_THREADS, 0, s>>>(w.block_hist, nullptr, nullptr, g.blocks, E, w.block_off, counts, tile_start,
                                          nullptr);
   route_rank<<<g.blocks, ROUTE_THREADS, 0, s>>>(expert_ids, T, E, g.tokens_per_block, w.block_off, tile_start,
                                                 rows_cap, pos, src, status);
@@ -896,7 +1166,7 @@ extern "C" int ffm_group_rows_static(const int32_t* expert_ids, int64_t T, int E
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (cudaMemsetAsync(src, 0xFF, static_cast<size_t>(rows_cap) * 4, s) != cudaSuccess) return FFM_ERR_LAUNCH;
   route_hist_ids<<<g.blocks, ROUTE_THREADS, 0, s>>>(expert_ids, T, E, g.tokens_per_block, block_hist, status);
-  route_scan<<<1, ROUTE_THREADS, 0, s>>>(block_hist, nullptr, nullptr, g.blocks, E, block_off, counts, tile_start,
+  route_scan<<<1, SCAN_THREADS, 0, s>>>(block_hist, nullptr, nullptr, g.blocks, E, block_off, counts, tile_start,
                                          nullptr);
   route_rank<<<g.blocks, ROUTE_THREADS, 0, s>>>(expert_ids, T, E, g.tokens_per_block, block_off, tile_start, rows_cap,
                                                 pos, src, status);
