@@ -44,6 +44,8 @@ SIGNATURES = {
                                      c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p]),
     "ffm_grouped_gemm": (c_int, [c_void_p, c_void_p, c_int, c_int, c_void_p, c_int64, c_int, c_int, c_float,
                                  c_void_p, c_void_p, c_int, c_void_p, c_void_p]),
+    "ffm_dense_gemm_two": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_int64, c_int, c_int, c_void_p, c_void_p,
+                                   c_void_p]),
     "ffm_grouped_gemm_wgrad": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_int64, c_int, c_int, c_float,
                                        c_void_p, c_void_p, c_void_p]),
     "ffm_grouped_gemm_wgrad_glu_backward": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_int64, c_int, c_int, c_float,
@@ -59,6 +61,8 @@ SIGNATURES = {
                                      c_void_p, c_int, c_void_p, c_void_p]),
     "ffm_combine_forward": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_void_p,
                                     c_void_p]),
+    "ffm_combine_forward_add2": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_void_p,
+                                         c_void_p]),
     "ffm_combine_backward": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_void_p,
                                      c_void_p, c_void_p]),
     "ffm_glu_backward": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int64, c_int, c_int, c_void_p, c_void_p]),

@@ -127,7 +127,8 @@ struct GemmParams {
   int n_cols;              // output columns per group (GLU: H)
   int k_blocks;            // K / 64 (grouped-M / dense)
   long long b_group_rows;  // rows of the B tensor map per group
-  int b1_row_offset;       // row offset of the second 128-row half of a K-major B tile
+  int b1_row_offset;       // row offset of the second 128-row half of a K-major B tile; N-major plain GEMM: K row at which
+                           // the second B map takes over (0: one map)
   int has_c2;              // GLU: also store the pre-activations
   int glu_h;
   float scale;
@@ -660,12 +661,15 @@ ffm_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           if (B_MN) {
             const int krow = GROUPK ? (t.k_row0 + k0) : static_cast<int>(t.group * p.b_group_rows + k0);
             const int n0 = t.n_block * BN + (CTA2 ? static_cast<int>(rank) * 128 : 0);
+            const bool second = EPI == EPI_PLAIN && !GROUPK && p.b1_row_offset > 0 && krow >= p.b1_row_offset;
+            const CUtensorMap* mb = second ? &tmB1 : &tmB0;
+            const int kr = second ? krow - p.b1_row_offset : krow;
             if (CTA2) {
-              tma_load_2d_pair(b_dst, &tmB0, full, n0, krow);
-              tma_load_2d_pair(b_dst + 8192, &tmB0, full, n0 + 64, krow);
+              tma_load_2d_pair(b_dst, mb, full, n0, kr);
+              tma_load_2d_pair(b_dst + 8192, mb, full, n0 + 64, kr);
             } else {
 #pragma unroll
-              for (int j = 0; j < 4; ++j) tma_load_2d(b_dst + j * 8192, &tmB0, full, n0 + 64 * j, krow);
+              for (int j = 0; j < 4; ++j) tma_load_2d(b_dst + j * 8192, mb, full, n0 + 64 * j, kr);
             }
           } else {
             const int nrow = static_cast<int>(t.group * p.b_group_rows) + t.n_block * (EPI == EPI_GLU ? 128 : BN);
@@ -1270,6 +1274,33 @@ extern "C" int ffm_grouped_gemm(const void* A, const void* B, int b_major, int g
   if ((rc = make_map_2d(&tmB, B, static_cast<long long>(groups) * K, Nout, 64, 64)) != FFM_OK) return rc;
   p.b_group_rows = K;
   return launch_gemm<0, 1, EPI_PLAIN, 0>(tmA, tmB, tmB, tmC, tmC, p, m_tiles, p.n_tiles, s, tile_rows);
+}
+
+extern "C" int ffm_dense_gemm_two(const void* A, const void* B1, int K1, const void* B2, int64_t rows, int K, int Nout,
+                                  void* out, int32_t* status, ffm_stream_t stream) {
+  if (!A || !B1 || !B2 || !out || !status) return FFM_ERR_BAD_ARG;
+  if (rows < 0 || K <= 0 || K1 <= 0 || K1 >= K || Nout <= 0) return FFM_ERR_BAD_ARG;
+  if (K % 64 != 0 || K1 % 64 != 0 || Nout % 64 != 0) return FFM_ERR_UNSUPPORTED;
+  if (rows == 0) return FFM_OK;
+  CUtensorMap tmA, tmB, tmB2, tmC;
+  int rc;
+  if ((rc = make_map_2d(&tmA, A, rows, K, 64, 128)) != FFM_OK) return rc;
+  if ((rc = make_out_map(&tmC, out, 1, rows, Nout)) != FFM_OK) return rc;
+  if ((rc = make_map_2d(&tmB, B1, K1, Nout, 64, 64)) != FFM_OK) return rc;
+  if ((rc = make_map_2d(&tmB2, B2, K - K1, Nout, 64, 64)) != FFM_OK) return rc;
+  GemmParams p = {};
+  p.groups = 1;
+  p.dense_m_tiles = static_cast<int>((rows + BM - 1) / BM);
+  p.n_cols = Nout;
+  p.k_blocks = K / BK;
+  p.scale = 1.0f;
+  p.n_tiles = (Nout + BN - 1) / BN;
+  p.status = status;
+  p.wait_cycles = g_wait_cycles;
+  p.b_group_rows = K;
+  p.b1_row_offset = K1;
+  return launch_gemm<0, 1, EPI_PLAIN, 0>(tmA, tmB, tmB2, tmC, tmC, p, p.dense_m_tiles, p.n_tiles,
+                                         static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int ffm_grouped_gemm_wgrad(const void* A, const void* B, int groups, const int32_t* tile_start,

@@ -94,6 +94,7 @@ route_bwd_token(const float* __restrict__ gw, const float* __restrict__ topk_w, 
     }
 
     // ---- dH[n, :] (+)= sum_e gl[e] * gate_w[e, :] ----
+    if (dH == nullptr) continue;
     for (int c0 = 0; c0 < chunks; c0 += 32) {
       const int c = c0 + lane;
       const bool active = c < chunks;
@@ -323,9 +324,18 @@ extern "C" int ffm_route_backward(const float* gw, const float* topk_w, const in
     long long blocks = (N + RB_WARPS - 1) / RB_WARPS;
     if (blocks > 148LL * 16) blocks = 148LL * 16;
     FFM_PREFER_MAX_SHARED(route_bwd_token);
+    // A z-loss, or an aux loss on sigmoid scores, makes every entry of gl non-zero: dH = gl gate_w is then a GEMM with
+    // K = E, on the tensor cores where the shape allows (16384 tokens, E = 64, D = 2048: the token kernel ran 971 us beside
+    // the layer's GEMMs, which it slowed down). Otherwise a row has top_k entries and the token kernel adds their rows.
+    const bool dense = gz != nullptr || (gating == FFM_GATING_SIGMOID && gaux != nullptr);
+    const bool gemm_dh = dense && accumulate == 0 && E % 64 == 0 && D % 64 == 0;
     route_bwd_token<<<static_cast<int>(blocks), RB_THREADS, 0, s>>>(
         gw, topk_w, topk_idx, static_cast<const bf16*>(logits), lse, gaux, gz, static_cast<const bf16*>(gate_w), N, D,
-        E, top_k, gating, accumulate, gl, static_cast<bf16*>(dH));
+        E, top_k, gating, accumulate, gl, gemm_dh ? nullptr : static_cast<bf16*>(dH));
+    if (gemm_dh) {
+      const int rc = ffm_grouped_gemm(gl, gate_w, FFM_B_NMAJOR, 1, nullptr, N, E, D, 1.0f, dH, nullptr, 0, status, stream);
+      if (rc != FFM_OK) return rc;
+    }
   }
   if (dgate_on_tensor_cores(N, D, E)) {
     // gl is [N, E] contiguous here (E % 8 == 0). dGate[e, :] = sum_n gl[n, e] hidden[n, :]

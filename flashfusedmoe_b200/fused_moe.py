@@ -313,18 +313,16 @@ def _glu_ffn_backward(go, x, act, pre, w_gate, w_up, w_down, activation):
     cur, side = _fork_small(go)
     if side is None:
         d_wdown = d_wdown.sum(dim=0) if split == 2 else d_wdown[0]
-        w_cat = torch.cat([w_gate, w_up], dim=0)
-        dx = ops.grouped_gemm(gU, w_cat, _lib.B_NMAJOR, 1, None, 2 * Hs, D)
+        dx = ops.dense_gemm_two(gU, w_gate, w_up)
         d_wcat = ops.grouped_gemm_wgrad(gU, x, 1, ts)[0]
         return dx, d_wcat[:Hs], d_wcat[Hs:], d_wdown
     # the sum of the two partial products is needed only at the end: it runs as a side branch beside the next two
-    # GEMMs. The stacked [gate; up] weights of the dX GEMM are copied on the current stream (the GEMM needs them next).
+    # GEMMs
     parts = d_wdown
     parts.record_stream(side)  # freed below while the side stream may still read it
     with torch.cuda.stream(side):
         d_wdown = parts.sum(dim=0) if split == 2 else parts[0]
-    w_cat = torch.cat([w_gate, w_up], dim=0)
-    dx = ops.grouped_gemm(gU, w_cat, _lib.B_NMAJOR, 1, None, 2 * Hs, D)
+    dx = ops.dense_gemm_two(gU, w_gate, w_up)
     d_wcat = ops.grouped_gemm_wgrad(gU, x, 1, ts)[0]
     _join_small(cur, side, d_wdown)
     return dx, d_wcat[:Hs], d_wcat[Hs:], d_wdown
@@ -554,9 +552,11 @@ class _FusedMoEFunction(torch.autograd.Function):
                 join = torch.cuda.Event()
                 join.record(gemm)
             main.wait_event(route_done)
-            dH = ops.combine_forward(dXg, pos, None, N, k, addend=dH_route)
+            if shared_done is not None:
+                main.wait_event(shared_done)
+            dH = ops.combine_forward(dXg, pos, None, N, k, addend=dH_route, addend2=s_dx if ctx.has_shared else None)
             main.wait_event(join)
-            for t_side in (dH_route, d_gate, d_wu):
+            for t_side in (dH_route, d_gate, d_wu) + ((s_dx, s_dwg, s_dwu, s_dwd) if ctx.has_shared else ()):
                 t_side.record_stream(main)  # allocated on a side stream, consumed on the main one from here on
         else:
             d_act = ops.grouped_gemm(gYw, wd, _lib.B_NMAJOR, E, tile_start, D, H)
@@ -574,12 +574,8 @@ class _FusedMoEFunction(torch.autograd.Function):
             d_add = go.to(dt[4])
         s_grads = (None, None, None)
         if ctx.has_shared:
-            if shared_done is not None:
-                cur_s = torch.cuda.current_stream()
-                cur_s.wait_event(shared_done)
-                for t_side in (s_dx, s_dwg, s_dwu, s_dwd):
-                    t_side.record_stream(cur_s)
-            dH = dH + s_dx
+            if not _OVERLAP:
+                dH = dH + s_dx
             s_grads = (s_dwg.to(dt[5]), s_dwu.to(dt[6]), s_dwd.to(dt[7]))
         return (dH.to(dt[0]), d_gate.to(dt[1]), d_wu.to(dt[2]), d_wd.to(dt[3]), d_add) + s_grads + (None, None)
 

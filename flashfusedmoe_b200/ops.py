@@ -344,6 +344,20 @@ def grouped_gemm(A, B, b_major, groups, tile_start, K, n_out, scale=1.0, valid_r
     return out
 
 
+def dense_gemm_two(A, B1, B2):
+    """A [B1; B2] with the contraction's rows in two tensors (ffm_dense_gemm_two)."""
+    lib = _lib.load()
+    for name, t in (("A", A), ("B1", B1), ("B2", B2)):
+        _req(t, torch.bfloat16, name)
+    rows, K = A.shape
+    out = torch.empty(rows, B1.shape[1], dtype=torch.bfloat16, device=A.device)
+    with _Launch("gemm", 1):
+        rc = lib.ffm_dense_gemm_two(_ptr(A), _ptr(B1), B1.shape[0], _ptr(B2), rows, K, B1.shape[1], _ptr(out),
+                                    _ptr(status_tensor(A.device)), _stream())
+    _lib.check(rc, "ffm_dense_gemm_two")
+    return out
+
+
 def grouped_gemm_wgrad(A, B, groups, tile_start, scale=1.0):
     """dW[e] = scale * A[rows of e]^T B[rows of e]; A [rows_cap, M], B [rows_cap, N] -> [groups, M, N]."""
     lib = _lib.load()
@@ -456,15 +470,16 @@ def grouped_gemm_fp8(Aq, a_scale, Bq, b_scale, groups, tile_start, K, n_out, til
     return out
 
 
-def combine_forward(Y, pos, w, N, top_k, addend=None):
+def combine_forward(Y, pos, w, N, top_k, addend=None, addend2=None):
     lib = _lib.load()
     _req(Y, torch.bfloat16, "Y")
     _req(pos, torch.int32, "pos")
     D = Y.shape[1]
     out = torch.empty(N, D, dtype=torch.bfloat16, device=Y.device)
     with _Launch("combine_forward", 1):
-        rc = lib.ffm_combine_forward(_ptr(Y), _ptr(pos), _ptr(w), _ptr(addend), N, top_k, D, _ptr(out), _stream())
-    _lib.check(rc, "ffm_combine_forward")
+        rc = lib.ffm_combine_forward_add2(_ptr(Y), _ptr(pos), _ptr(w), _ptr(addend), _ptr(addend2), N, top_k, D, _ptr(out),
+                                          _stream())
+    _lib.check(rc, "ffm_combine_forward_add2")
     return out
 
 

@@ -193,6 +193,10 @@ int ffm_grouped_gemm_glu(const void* A, const void* w_gate, const void* w_up, in
 int ffm_grouped_gemm(const void* A, const void* B, int b_major, int groups, const int32_t* tile_start,
                      int64_t rows, int K, int Nout, float scale, void* out, const int32_t* valid_rows,
                      int tile_rows, int32_t* status, ffm_stream_t stream);
+/* out [rows, Nout] = A [rows, K] [B1; B2] with the K rows of B in two tensors, B1 [K1, Nout] and B2 [K - K1, Nout] (the
+ * input gradient of a GLU whose gate and up weights are separate). K, K1 and Nout multiples of 64. */
+int ffm_dense_gemm_two(const void* A, const void* B1, int K1, const void* B2, int64_t rows, int K, int Nout, void* out,
+                       int32_t* status, ffm_stream_t stream);
 int ffm_grouped_gemm_wgrad(const void* A, const void* B, int groups, const int32_t* tile_start, int64_t rows_cap,
                            int M, int Nout, float scale, void* dW, int32_t* status, ffm_stream_t stream);
 /* dAct GEMM with the GLU backward fused into its epilogue: gU [rows, 2H] = GLU backward of (gY Wd (N-major B, as
@@ -222,6 +226,9 @@ int ffm_grouped_gemm_wgrad_glu_backward(const void* A, const void* B, int groups
  * ------------------------------------------------------------------------------------------------- */
 int ffm_combine_forward(const void* Y, const int32_t* pos, const float* w, const void* addend, int64_t N,
                         int top_k, int D, void* out, ffm_stream_t stream);
+/* The same with a second addend, added after the first (each sum rounded to bf16); either may be NULL. */
+int ffm_combine_forward_add2(const void* Y, const int32_t* pos, const float* w, const void* addend, const void* addend2,
+                             int64_t N, int top_k, int D, void* out, ffm_stream_t stream);
 
 /* -------------------------------------------------------------------------------------------------
  * Combine backward, one pass over the grouped rows:
