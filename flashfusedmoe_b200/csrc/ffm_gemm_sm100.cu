@@ -37,6 +37,7 @@
 #include <stdlib.h>
 
 #include "ffm_common.cuh"
+#include "ffm_internal.h"
 
 namespace ffm {
 
@@ -591,9 +592,11 @@ ffm_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     }
   } else if (p.tile_start != nullptr) {
     for (int i = threadIdx.x; i <= p.groups; i += blockDim.x) ctrl->tile_start[i] = p.tile_start[i];
-  } else if (threadIdx.x == 0) {
-    ctrl->tile_start[0] = 0;
-    ctrl->tile_start[1] = p.dense_m_tiles;
+  } else {
+    // dense: one group, or (grouped-K) equal ranges of the rows
+    for (int i = threadIdx.x; i <= p.groups; i += blockDim.x) {
+      ctrl->tile_start[i] = static_cast<int>(static_cast<long long>(p.dense_m_tiles) * i / p.groups);
+    }
   }
   if (warp == 1) {
     if (CTA2) {
@@ -1303,10 +1306,9 @@ extern "C" int ffm_dense_gemm_two(const void* A, const void* B1, int K1, const v
                                          static_cast<cudaStream_t>(stream));
 }
 
-extern "C" int ffm_grouped_gemm_wgrad(const void* A, const void* B, int groups, const int32_t* tile_start,
-                                      int64_t rows_cap, int M, int Nout, float scale, void* dW, int32_t* status,
-                                      ffm_stream_t stream) {
-  if (!A || !B || !dW || !status || !tile_start) return FFM_ERR_BAD_ARG;
+int ffm::grouped_wgrad(const void* A, const void* B, int groups, const int32_t* tile_start, int64_t rows_cap, int M, int Nout,
+                       float scale, void* dW, int32_t* status, ffm_stream_t stream) {
+  if (!A || !B || !dW || !status) return FFM_ERR_BAD_ARG;
   if (groups < 1 || groups > MAX_GROUPS || rows_cap <= 0 || M <= 0 || Nout <= 0) return FFM_ERR_BAD_ARG;
   if (M % 64 != 0 || Nout % 64 != 0) return FFM_ERR_UNSUPPORTED;
   CUtensorMap tmA, tmB, tmC;
@@ -1317,6 +1319,7 @@ extern "C" int ffm_grouped_gemm_wgrad(const void* A, const void* B, int groups, 
   GemmParams p = {};
   p.tile_start = tile_start;
   p.groups = groups;
+  p.dense_m_tiles = static_cast<int>((rows_cap + BM - 1) / BM);
   p.n_cols = Nout;
   p.scale = scale;
   p.m_tiles_per_group = (M + BM - 1) / BM;
@@ -1326,6 +1329,13 @@ extern "C" int ffm_grouped_gemm_wgrad(const void* A, const void* B, int groups, 
   return launch_gemm<1, 1, EPI_PLAIN, 1>(tmA, tmB, tmB, tmC, tmC, p, p.m_tiles_per_group,
                                          static_cast<long long>(groups) * p.n_tiles,
                                          static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int ffm_grouped_gemm_wgrad(const void* A, const void* B, int groups, const int32_t* tile_start,
+                                      int64_t rows_cap, int M, int Nout, float scale, void* dW, int32_t* status,
+                                      ffm_stream_t stream) {
+  if (!tile_start) return FFM_ERR_BAD_ARG;
+  return ffm::grouped_wgrad(A, B, groups, tile_start, rows_cap, M, Nout, scale, dW, status, stream);
 }
 
 extern "C" int ffm_grouped_gemm_wgrad_glu_backward(const void* A, const void* B, int groups, const int32_t* tile_start,

@@ -13,6 +13,7 @@
 #include <atomic>
 
 #include "ffm_common.cuh"
+#include "ffm_internal.h"
 
 namespace ffm {
 
@@ -22,6 +23,16 @@ constexpr int ROUTE_THREADS = 256;
 constexpr int ROUTE_WARPS = ROUTE_THREADS / 32;
 constexpr int MAX_E = 256;
 constexpr int TPW = 2;  // tokens per warp pass
+
+// What the last routing kernel derives from the statistics: aux = aux_scale * sum_e counts[e] * mass[e],
+// z = z_scale * sum_n lse[n]^2, and a zeroed word (the count of dropped slots). Any pointer may be null.
+struct LossOut {
+  float* aux;
+  float* z;
+  int32_t* zero;
+  float aux_scale;
+  float z_scale;
+};
 
 struct RouteGrid {
   int blocks;
@@ -525,7 +536,8 @@ route_hist_ids(const int32_t* __restrict__ ids, long long T, int E, int slots_pe
 // Segment starts (in 128-row tiles, always even) and the dot product of counts and probability masses, from per-expert
 // totals in shared memory. One warp, eight consecutive experts per lane: a fixed order of sums.
 __device__ __forceinline__ void finish_counts(const int* s_counts, const float* s_mass, float zsum, int E, int lane,
-                                              int32_t* __restrict__ tile_start, float* __restrict__ stats) {
+                                              int32_t* __restrict__ tile_start, float* __restrict__ stats,
+                                              const LossOut& lo) {
   constexpr int PER = MAX_E / 32;
   int tiles[PER];
   int mine = 0;
@@ -557,6 +569,11 @@ __device__ __forceinline__ void finish_counts(const int* s_counts, const float* 
     stats[E] = zsum;
     stats[E + 1] = dot;
   }
+  if (lane == 0) {
+    if (lo.aux != nullptr) *lo.aux = dot * lo.aux_scale;
+    if (lo.z != nullptr) *lo.z = zsum * lo.z_scale;
+    if (lo.zero != nullptr) *lo.zero = 0;
+  }
 }
 
 // One block of 32 warps. block_off[e][b] = sum_{b' < b} hist[e][b']; counts; tile_start; stats.
@@ -567,7 +584,7 @@ constexpr int SCAN_THREADS = 1024;
 __global__ void __launch_bounds__(SCAN_THREADS)
 route_scan(const int32_t* __restrict__ block_hist, const float* __restrict__ block_mass,
            const float* __restrict__ block_z, int blocks, int E, int32_t* __restrict__ block_off,
-           int32_t* __restrict__ counts, int32_t* __restrict__ tile_start, float* __restrict__ stats) {
+           int32_t* __restrict__ counts, int32_t* __restrict__ tile_start, float* __restrict__ stats, LossOut lo) {
   __shared__ int s_counts[MAX_E];
   __shared__ float s_mass[MAX_E];
   __shared__ float s_zsum;
@@ -608,7 +625,7 @@ route_scan(const int32_t* __restrict__ block_hist, const float* __restrict__ blo
     if (lane == 0) s_zsum = z;
   }
   __syncthreads();
-  if (warp == 0) finish_counts(s_counts, s_mass, s_zsum, E, lane, tile_start, stats);
+  if (warp == 0) finish_counts(s_counts, s_mass, s_zsum, E, lane, tile_start, stats, lo);
 }
 
 // Stable rank inside each expert segment. Each warp owns a contiguous run of the block's slots.
@@ -749,7 +766,7 @@ route_finish_small(const bf16* __restrict__ logits, const float* __restrict__ bi
                    RouteOpts opts, float* __restrict__ topk_w, int32_t* topk_idx, float* __restrict__ lse_out,
                    int32_t* block_hist, float* block_mass, float* block_z, int32_t* __restrict__ counts,
                    int32_t* __restrict__ tile_start, float* __restrict__ stats, long long rows_cap,
-                   int32_t* __restrict__ pos, int32_t* __restrict__ src, int32_t* __restrict__ status) {
+                   int32_t* __restrict__ pos, int32_t* __restrict__ src, int32_t* __restrict__ status, LossOut lo) {
   __shared__ float s_mass[FINISH_WARPS][NG * 32];
   __shared__ int s_cnt[FINISH_WARPS][NG * 32];
   __shared__ float s_z[FINISH_WARPS];
@@ -822,7 +839,7 @@ route_finish_small(const bf16* __restrict__ logits, const float* __restrict__ bi
   if (warp == 0) {
     float z = 0.0f;
     for (int b = 0; b < blocks; ++b) z += __ldcg(block_z + b);
-    finish_counts(s_counts, s_tot, z, E, lane, s_start, stats);
+    finish_counts(s_counts, s_tot, z, E, lane, s_start, stats, lo);
   }
   // per-warp runs of slots, as in route_rank
   const int T = N * top_k;
@@ -932,7 +949,7 @@ template <int NG>
 int launch_finish_small(const bf16* logits, const float* bias, int N, int E, int top_k, const RouteOpts& opts,
                         float* topk_w, int32_t* topk_idx, float* lse, const RouteWorkspace& w, int32_t* counts,
                         int32_t* tile_start, float* stats, long long rows_cap, int32_t* pos, int32_t* src,
-                        int32_t* status, cudaStream_t s) {
+                        int32_t* status, const LossOut& lo, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   // up to one token per warp, a single block is enough; beyond, the tokens are spread over a cluster
   cfg.gridDim = dim3(N <= FINISH_WARPS ? 1 : FINISH_CLUSTER, 1, 1);
@@ -947,7 +964,7 @@ int launch_finish_small(const bf16* logits, const float* bias, int N, int E, int
   cfg.numAttrs = 1;
   if (cudaLaunchKernelEx(&cfg, route_finish_small<NG>, logits, bias, N, E, top_k, opts, topk_w, topk_idx, lse,
                          w.block_hist, w.block_mass, w.block_z, counts, tile_start, stats, rows_cap, pos, src,
-                         status) != cudaSuccess) {
+                         status, lo) != cudaSuccess) {
     cudaGetLastError();
     return FFM_ERR_LAUNCH;
   }
@@ -1033,12 +1050,13 @@ extern "C" size_t ffm_route_workspace_bytes(int64_t N, int E, int top_k) {
   return carve_workspace(nullptr, blocks, E).bytes;
 }
 
-extern "C" int ffm_route_forward(const void* hidden, const void* gate_w, const float* expert_bias, int64_t N, int D,
-                                 int E, int top_k, int gating, float weight_scale, int pre_softmax, int n_group,
-                                 int topk_group, void* logits, float* topk_w,
-                                 int32_t* topk_idx, float* lse, int32_t* counts, int32_t* tile_start, int32_t* pos,
-                                 int32_t* src, int64_t rows_cap, float* stats, void* workspace,
-                                 size_t workspace_bytes, int32_t* status, ffm_stream_t stream) {
+int ffm::route_forward_losses(const void* hidden, const void* gate_w, const float* expert_bias, int64_t N, int D, int E,
+                              int top_k, int gating, float weight_scale, int pre_softmax, int n_group, int topk_group,
+                              void* logits, float* topk_w, int32_t* topk_idx, float* lse, int32_t* counts,
+                              int32_t* tile_start, int32_t* pos, int32_t* src, int64_t rows_cap, float* stats,
+                              float* aux, float aux_scale, float* z, float z_scale, int32_t* zero, void* workspace,
+                              size_t workspace_bytes, int32_t* status, ffm_stream_t stream) {
+  const LossOut lo = {aux, z, zero, aux_scale, z_scale};
   if (!hidden || !gate_w || !topk_w || !topk_idx || !lse || !counts || !tile_start || !pos || !src || !stats ||
       !workspace || !status)
     return FFM_ERR_BAD_ARG;
@@ -1070,7 +1088,7 @@ extern "C" int ffm_route_forward(const void* hidden, const void* gate_w, const f
     if (cudaGetLastError() != cudaSuccess) return FFM_ERR_LAUNCH;
 #define FFM_FINISH_CASE(NG)                                                                                            \
   launch_finish_small<NG>(lg, expert_bias, n, E, top_k, opts, topk_w, topk_idx, lse, w, counts, tile_start, stats, \
-                          rows_cap, pos, src, status, s)
+                          rows_cap, pos, src, status, lo, s)
     if (E <= 32) return FFM_FINISH_CASE(1);
     if (E <= 64) return FFM_FINISH_CASE(2);
     if (E <= 128) return FFM_FINISH_CASE(4);
@@ -1120,10 +1138,22 @@ extern "C" int ffm_route_forward(const void* hidden, const void* gate_w, const f
   }
   FFM_PREFER_MAX_SHARED(route_scan);
   route_scan<<<1, SCAN_THREADS, 0, s>>>(w.block_hist, w.block_mass, w.block_z, g.blocks, E, w.block_off, counts,
-                                         tile_start, stats);
+                                         tile_start, stats, lo);
   route_rank<<<g.blocks, ROUTE_THREADS, 0, s>>>(topk_idx, N * top_k, E, g.tokens_per_block * top_k, w.block_off,
                                                 tile_start, rows_cap, pos, src, status);
   return cudaGetLastError() == cudaSuccess ? FFM_OK : FFM_ERR_LAUNCH;
+}
+
+extern "C" int ffm_route_forward(const void* hidden, const void* gate_w, const float* expert_bias, int64_t N, int D,
+                                 int E, int top_k, int gating, float weight_scale, int pre_softmax, int n_group,
+                                 int topk_group, void* logits, float* topk_w,
+                                 int32_t* topk_idx, float* lse, int32_t* counts, int32_t* tile_start, int32_t* pos,
+                                 int32_t* src, int64_t rows_cap, float* stats, void* workspace,
+                                 size_t workspace_bytes, int32_t* status, ffm_stream_t stream) {
+  return ffm::route_forward_losses(hidden, gate_w, expert_bias, N, D, E, top_k, gating, weight_scale, pre_softmax, n_group,
+                                   topk_group, logits, topk_w, topk_idx, lse, counts, tile_start, pos, src, rows_cap,
+                                   stats, nullptr, 0.0f, nullptr, 0.0f, nullptr, workspace, workspace_bytes, status,
+                                   stream);
 }
 
 extern "C" int ffm_group_rows(const int32_t* expert_ids, int64_t T, int E, int32_t* counts, int32_t* tile_start,
@@ -1140,7 +1170,7 @@ extern "C" int ffm_group_rows(const int32_t* expert_ids, int64_t T, int E, int32
   RouteWorkspace w = carve_workspace(workspace, g.blocks, E);
   route_hist_ids<<<g.blocks, ROUTE_THREADS, 0, s>>>(expert_ids, T, E, g.tokens_per_block, w.block_hist, status);
   route_scan<<<1, SCAN_THREADS, 0, s>>>(w.block_hist, nullptr, nullptr, g.blocks, E, w.block_off, counts, tile_start,
-                                         nullptr);
+                                         nullptr, LossOut{});
   route_rank<<<g.blocks, ROUTE_THREADS, 0, s>>>(expert_ids, T, E, g.tokens_per_block, w.block_off, tile_start,
                                                 rows_cap, pos, src, status);
   return cudaGetLastError() == cudaSuccess ? FFM_OK : FFM_ERR_LAUNCH;
@@ -1167,7 +1197,7 @@ extern "C" int ffm_group_rows_static(const int32_t* expert_ids, int64_t T, int E
   if (cudaMemsetAsync(src, 0xFF, static_cast<size_t>(rows_cap) * 4, s) != cudaSuccess) return FFM_ERR_LAUNCH;
   route_hist_ids<<<g.blocks, ROUTE_THREADS, 0, s>>>(expert_ids, T, E, g.tokens_per_block, block_hist, status);
   route_scan<<<1, SCAN_THREADS, 0, s>>>(block_hist, nullptr, nullptr, g.blocks, E, block_off, counts, tile_start,
-                                         nullptr);
+                                         nullptr, LossOut{});
   route_rank<<<g.blocks, ROUTE_THREADS, 0, s>>>(expert_ids, T, E, g.tokens_per_block, block_off, tile_start, rows_cap,
                                                 pos, src, status);
   return cudaGetLastError() == cudaSuccess ? FFM_OK : FFM_ERR_LAUNCH;

@@ -10,6 +10,7 @@
 // tokens, partial products in bf16, summed in fixed order by dgate_sum_splits); the dense CUDA-core reduction costs
 // N E D multiply-adds, 285 us at N = 16384, E = 64, D = 2048.
 #include "ffm_common.cuh"
+#include "ffm_internal.h"
 
 namespace ffm {
 
@@ -26,15 +27,20 @@ __device__ __forceinline__ int round_up8(int x) { return (x + 7) & ~7; }
 
 __global__ void __launch_bounds__(RB_THREADS)
 route_bwd_token(const float* __restrict__ gw, const float* __restrict__ topk_w, const int32_t* __restrict__ topk_idx,
-                const bf16* __restrict__ logits, const float* __restrict__ lse, const float* __restrict__ gaux,
-                const float* __restrict__ gz_ptr, const bf16* __restrict__ gate_w, long long N, int D, int E, int top_k, int gating,
+                const bf16* __restrict__ logits, const float* __restrict__ lse, LossGrads lg,
+                const bf16* __restrict__ gate_w, long long N, int D, int E, int top_k, int gating,
                 int accumulate, bf16* __restrict__ gl_out, bf16* __restrict__ dH) {
   const int lane = threadIdx.x & 31;
   const int chunks = D >> 3;
   const int groups = (E + 31) >> 5;
   const int ldg_ = round_up8(E);
   const float inv_n = 1.0f / static_cast<float>(N);
-  const float gz = (gz_ptr != nullptr) ? __ldg(gz_ptr) : 0.0f;
+  const float gz = lg.gz != nullptr ? __ldg(lg.gz) : (lg.grad_z != nullptr ? __ldg(lg.grad_z) * lg.z_coef : 0.0f);
+  const bool has_aux = lg.gaux != nullptr || lg.grad_aux != nullptr;
+  const float aux_up = lg.grad_aux != nullptr ? __ldg(lg.grad_aux) * lg.aux_coef : 0.0f;
+  auto gaux_of = [&](int e) {
+    return lg.gaux != nullptr ? __ldg(lg.gaux + e) : static_cast<float>(__ldg(lg.counts + e)) * aux_up;
+  };
 
   for (long long n = static_cast<long long>(blockIdx.x) * RB_WARPS + (threadIdx.x >> 5); n < N;
        n += static_cast<long long>(gridDim.x) * RB_WARPS) {
@@ -49,7 +55,7 @@ route_bwd_token(const float* __restrict__ gw, const float* __restrict__ topk_w, 
     }
     float gtl;
     if (gating == FFM_GATING_SOFTMAX) {
-      if (gaux != nullptr && idx >= 0) g += gaux[idx] * inv_n;
+      if (has_aux && idx >= 0) g += gaux_of(idx) * inv_n;
       const float sg = warp_sum(g * s);
       gtl = s * (g - sg);
     } else {
@@ -75,13 +81,13 @@ route_bwd_token(const float* __restrict__ gw, const float* __restrict__ topk_w, 
           if (ij == e) v += gj;
         }
         if (e < E) {
-          const bool need_logit = (gz != 0.0f) || (gating == FFM_GATING_SIGMOID && gaux != nullptr);
+          const bool need_logit = (gz != 0.0f) || (gating == FFM_GATING_SIGMOID && has_aux);
           if (need_logit) {
             const float l = __bfloat162float(logits[n * E + e]);
             if (gz != 0.0f) v += gz * 2.0f * lse_n * inv_n * __expf(l - lse_n);
-            if (gating == FFM_GATING_SIGMOID && gaux != nullptr) {
+            if (gating == FFM_GATING_SIGMOID && has_aux) {
               const float sc = sigmoidf_(l);
-              v += gaux[e] * sc * (1.0f - sc) * inv_n;
+              v += gaux_of(e) * sc * (1.0f - sc) * inv_n;
             }
           }
           const bf16 vb = __float2bfloat16_rn(v);
@@ -242,12 +248,6 @@ route_bwd_reduce(const float* __restrict__ partial, int chunks_n, int D, int E, 
 
 constexpr int DG_SPLITS = 8;
 
-// tile_start of DG_SPLITS equal ranges (whole tile pairs) over `pairs` pairs of 128-row tiles
-__global__ void dgate_split_tiles(int32_t* __restrict__ ts, int pairs) {
-  const int s = threadIdx.x;
-  if (s <= DG_SPLITS) ts[s] = 2 * static_cast<int>((static_cast<long long>(pairs) * s) / DG_SPLITS);
-}
-
 __global__ void __launch_bounds__(256) dgate_sum_splits(const bf16* __restrict__ part, long long total,
                                                         bf16* __restrict__ dGate) {
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
@@ -295,24 +295,25 @@ extern "C" size_t ffm_route_backward_workspace_bytes(int64_t N, int D, int E) {
   const int ldg_ = (E + 7) & ~7;
   const size_t gl_bytes = align256(static_cast<size_t>(N > 0 ? N : 1) * ldg_ * 2);
   if (dgate_on_tensor_cores(N, D, E)) {
-    return gl_bytes + align256(static_cast<size_t>(DG_SPLITS) * E * D * 2) + 256;  // partials (bf16) + tile_start
+    return gl_bytes + align256(static_cast<size_t>(DG_SPLITS) * E * D * 2);  // partials (bf16)
   }
   DgatePlan p = plan_dgate(N > 0 ? N : 1, D, E);
   return gl_bytes + align256(static_cast<size_t>(p.chunks_n) * ldg_ * D * 4);
 }
 
-extern "C" int ffm_route_backward(const float* gw, const float* topk_w, const int32_t* topk_idx, const void* logits,
-                                  const float* lse, const float* gaux, const float* gz, const void* hidden,
-                                  const void* gate_w, int64_t N, int D, int E, int top_k, int gating, int accumulate,
-                                  void* dH, void* dGate, void* workspace, size_t workspace_bytes, int32_t* status,
-                                  ffm_stream_t stream) {
+int ffm::route_backward_losses(const float* gw, const float* topk_w, const int32_t* topk_idx, const void* logits,
+                               const float* lse, const LossGrads& lg, const void* hidden, const void* gate_w, int64_t N,
+                               int D, int E, int top_k, int gating, int accumulate, void* dH, void* dGate,
+                               void* workspace, size_t workspace_bytes, int32_t* status, ffm_stream_t stream) {
+  const bool has_aux = lg.gaux != nullptr || lg.grad_aux != nullptr;
+  const bool has_z = lg.gz != nullptr || lg.grad_z != nullptr;
   if (!gw || !topk_w || !topk_idx || !hidden || !gate_w || !dH || !dGate || !workspace || !status) {
     return FFM_ERR_BAD_ARG;
   }
   if (N < 0 || D <= 0 || E < 1 || top_k < 1) return FFM_ERR_BAD_ARG;
   if (gating != FFM_GATING_SOFTMAX && gating != FFM_GATING_SIGMOID) return FFM_ERR_BAD_ARG;
-  const bool need_logits = gating == FFM_GATING_SIGMOID || gz != nullptr;
-  if (need_logits && (!logits || (gz != nullptr && !lse))) return FFM_ERR_BAD_ARG;
+  const bool need_logits = gating == FFM_GATING_SIGMOID || has_z;
+  if (need_logits && (!logits || (has_z && !lse))) return FFM_ERR_BAD_ARG;
   if (D % 8 != 0 || E > MAX_E || top_k > 32 || top_k > E) return FFM_ERR_UNSUPPORTED;
   if (workspace_bytes < ffm_route_backward_workspace_bytes(N, D, E)) return FFM_ERR_WORKSPACE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -327,10 +328,10 @@ extern "C" int ffm_route_backward(const float* gw, const float* topk_w, const in
     // A z-loss, or an aux loss on sigmoid scores, makes every entry of gl non-zero: dH = gl gate_w is then a GEMM with
     // K = E, on the tensor cores where the shape allows (16384 tokens, E = 64, D = 2048: the token kernel ran 971 us beside
     // the layer's GEMMs, which it slowed down). Otherwise a row has top_k entries and the token kernel adds their rows.
-    const bool dense = gz != nullptr || (gating == FFM_GATING_SIGMOID && gaux != nullptr);
+    const bool dense = has_z || (gating == FFM_GATING_SIGMOID && has_aux);
     const bool gemm_dh = dense && accumulate == 0 && E % 64 == 0 && D % 64 == 0;
     route_bwd_token<<<static_cast<int>(blocks), RB_THREADS, 0, s>>>(
-        gw, topk_w, topk_idx, static_cast<const bf16*>(logits), lse, gaux, gz, static_cast<const bf16*>(gate_w), N, D,
+        gw, topk_w, topk_idx, static_cast<const bf16*>(logits), lse, lg, static_cast<const bf16*>(gate_w), N, D,
         E, top_k, gating, accumulate, gl, gemm_dh ? nullptr : static_cast<bf16*>(dH));
     if (gemm_dh) {
       const int rc = ffm_grouped_gemm(gl, gate_w, FFM_B_NMAJOR, 1, nullptr, N, E, D, 1.0f, dH, nullptr, 0, status, stream);
@@ -341,10 +342,7 @@ extern "C" int ffm_route_backward(const float* gw, const float* topk_w, const in
     // gl is [N, E] contiguous here (E % 8 == 0). dGate[e, :] = sum_n gl[n, e] hidden[n, :]
     uint8_t* base = static_cast<uint8_t*>(workspace) + align256(static_cast<size_t>(N) * ldg_ * 2);
     bf16* part = reinterpret_cast<bf16*>(base);
-    int32_t* ts = reinterpret_cast<int32_t*>(base + align256(static_cast<size_t>(DG_SPLITS) * E * D * 2));
-    const int pairs = static_cast<int>((N + 255) / 256);
-    dgate_split_tiles<<<1, 32, 0, s>>>(ts, pairs);
-    const int rc = ffm_grouped_gemm_wgrad(gl, hidden, DG_SPLITS, ts, N, E, D, 1.0f, part, status, stream);
+    const int rc = grouped_wgrad(gl, hidden, DG_SPLITS, nullptr, N, E, D, 1.0f, part, status, stream);
     if (rc != FFM_OK) return rc;
     const long long total = static_cast<long long>(E) * D;
     long long blocks = (total + 255) / 256;
@@ -368,4 +366,14 @@ extern "C" int ffm_route_backward(const float* gw, const float* topk_w, const in
                                                               static_cast<bf16*>(dGate));
   }
   return cudaGetLastError() == cudaSuccess ? FFM_OK : FFM_ERR_LAUNCH;
+}
+
+extern "C" int ffm_route_backward(const float* gw, const float* topk_w, const int32_t* topk_idx, const void* logits,
+                                  const float* lse, const float* gaux, const float* gz, const void* hidden,
+                                  const void* gate_w, int64_t N, int D, int E, int top_k, int gating, int accumulate,
+                                  void* dH, void* dGate, void* workspace, size_t workspace_bytes, int32_t* status,
+                                  ffm_stream_t stream) {
+  const ffm::LossGrads lg = {gaux, gz, nullptr, nullptr, nullptr, 0.0f, 0.0f};
+  return ffm::route_backward_losses(gw, topk_w, topk_idx, logits, lse, lg, hidden, gate_w, N, D, E, top_k, gating,
+                                    accumulate, dH, dGate, workspace, workspace_bytes, status, stream);
 }

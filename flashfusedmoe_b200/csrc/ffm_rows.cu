@@ -1,6 +1,7 @@
 // HBM-bound row kernels: permute into grouped rows, weighted combine and its backward, GLU backward.
 // One warp per row, 16-byte vector accesses, fp32 arithmetic, bf16 storage.
 #include "ffm_common.cuh"
+#include "ffm_internal.h"
 
 namespace ffm {
 
@@ -169,6 +170,17 @@ glu_backward_kernel(const bf16* __restrict__ dAct, const bf16* __restrict__ prea
   }
 }
 
+__global__ void __launch_bounds__(ROW_THREADS)
+add_bf16_kernel(const uint4* __restrict__ a, const uint4* __restrict__ b, long long n8, uint4* __restrict__ out) {
+  for (long long i = static_cast<long long>(blockIdx.x) * ROW_THREADS + threadIdx.x; i < n8;
+       i += static_cast<long long>(gridDim.x) * ROW_THREADS) {
+    float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    fma8(s, __ldg(a + i), 1.0f);
+    fma8(s, __ldg(b + i), 1.0f);
+    out[i] = pack8(s);
+  }
+}
+
 int grid_for_rows(long long rows) {
   long long blocks = (rows + ROW_WARPS - 1) / ROW_WARPS;
   const long long cap = 148LL * 16;
@@ -182,6 +194,14 @@ int grid_for_rows(long long rows) {
 }  // namespace ffm
 
 using namespace ffm;
+
+int ffm::add_bf16(const void* a, const void* b, int64_t n, void* out, ffm_stream_t stream) {
+  if (n % 8 != 0) return FFM_ERR_UNSUPPORTED;
+  if (n == 0) return FFM_OK;
+  add_bf16_kernel<<<grid_for_rows(n / 256 + 1), ROW_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<const uint4*>(a), static_cast<const uint4*>(b), n / 8, static_cast<uint4*>(out));
+  return cudaGetLastError() == cudaSuccess ? FFM_OK : FFM_ERR_LAUNCH;
+}
 
 extern "C" int ffm_permute_rows(const void* x, const int32_t* src, int64_t rows_cap, int top_k, int D,
                                 int zero_padding, void* grouped, ffm_stream_t stream) {

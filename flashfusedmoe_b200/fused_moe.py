@@ -97,23 +97,6 @@ def _quantized_weight(owner, w):
     return q, sc
 
 
-def _expert_ffn_forward(Xg, wu, wd, E, tile_start, D, H, activation, keep, small, owners=None):
-    """Up-projection + GLU and down-projection of the routed experts over grouped rows: (act, pre, Y)."""
-    if _EXPERT_GEMM == "fp8" and D % 128 == 0 and H % 128 == 0 and not small:
-        xq, xs = ops.quantize_rows_e4m3(Xg)
-        own_u, own_d = owners if owners is not None else (wu, wd)
-        wuq, wus = _quantized_weight(own_u, wu)
-        act, pre = ops.grouped_gemm_glu_fp8(xq, xs, wuq, wus, E, tile_start, D, H, activation, want_preact=keep)
-        aq, as_ = ops.quantize_rows_e4m3(act)
-        wdq, wds = _quantized_weight(own_d, wd)
-        Y = ops.grouped_gemm_fp8(aq, as_, wdq, wds, E, tile_start, H, D)
-        return act, pre, Y
-    act, pre = ops.grouped_gemm_glu(Xg, wu, wu.view(-1, D)[H:], 2 * H, E, tile_start, D, H, activation,
-                                    want_preact=keep, **small)
-    Y = ops.grouped_gemm(act, wd, _lib.B_KMAJOR, E, tile_start, H, D, **small)
-    return act, pre, Y
-
-
 def set_ep_dry_exchange(enable):
     """Benchmark switch: skip the payload of the expert-parallel exchanges (results are then meaningless). In
     host-sync-free mode the row kernels then move local rows only and every barrier still runs; the host-planned
@@ -249,14 +232,28 @@ def _dense_ts(rows, device, split=1):
     return t
 
 
-def _route(h, g, cfg, training):
-    """Routing kernels for one call. With input_jitter the logits see h * U(1 - j, 1 + j) in training, exactly as
-    the reference draws it (fused_moe.py:329-332); everything downstream uses the clean h."""
-    h_route = h
+def _device_tensor(t, name):
+    return ops._req(t, torch.bfloat16, name)
+
+
+def _side_handle(name):
+    """cudaStream_t of a side stream. The shared expert's chain is the longest beside the routing kernels: its stream has
+    priority."""
+    return _get_side_stream(name, priority=-1 if name == "shared" else 0).cuda_stream
+
+
+def _jittered(h, cfg, training):
+    """What the router sees: with input_jitter h * U(1 - j, 1 + j) in training, exactly as the reference draws it
+    (fused_moe.py:329-332); everything downstream uses the clean h."""
     if cfg.input_jitter > 0.0 and training:
         noise = torch.empty_like(h).uniform_(1.0 - cfg.input_jitter, 1.0 + cfg.input_jitter)
-        h_route = h * noise
-    return ops.route_forward(h_route, g, cfg.top_k, cfg.gating, cfg.expert_bias, cfg.weight_scale,
+        return h * noise
+    return h
+
+
+def _route(h, g, cfg, training):
+    """Routing kernels for one call."""
+    return ops.route_forward(_jittered(h, cfg, training), g, cfg.top_k, cfg.gating, cfg.expert_bias, cfg.weight_scale,
                              pre_softmax=cfg.pre_softmax, n_group=cfg.n_group, topk_group=cfg.topk_group)
 
 
@@ -399,184 +396,178 @@ class _FusedMoEFunction(torch.autograd.Function):
         E = gate_weight.shape[0]
         H = w_up.shape[1] // 2
         k = cfg.top_k
-        h = _to(hidden_states, dtype)
+        h = _device_tensor(_to(hidden_states, dtype), "hidden")
         g = _to(gate_weight, dtype)
         wu = _to(w_up, dtype)
         wd = _to(w_down, dtype)
-        add = None if addend is None else _to(addend, dtype)
+        add = None if addend is None else _device_tensor(_to(addend, dtype), "addend")
         need_grad = cfg.wants_grad and any(ctx.needs_input_grad[:8])
+        keep = need_grad and not cfg.recompute
+        dev = h.device
         has_shared = sw_gate is not None
-        shared_ready = None
+        Hs = 0
+        swg = swu = swd = None
         if has_shared:
             assert add is None, "either an addend or shared expert weights"
-            swg, swu, swd = _to(sw_gate, dtype), _to(sw_up, dtype), _to(sw_down, dtype)
-            if _OVERLAP:
-                side = _get_side_stream("shared", priority=-1)
-                fork = torch.cuda.Event()
-                fork.record()
-                with torch.cuda.stream(side):
-                    side.wait_event(fork)
-                    add, s_act, s_pre = _glu_ffn_forward(h, swg, swu, swd, cfg.shared_activation, want_preact=need_grad)
-                    shared_ready = torch.cuda.Event()
-                    shared_ready.record(side)
-            else:
-                add, s_act, s_pre = _glu_ffn_forward(h, swg, swu, swd, cfg.shared_activation, want_preact=need_grad)
-
-        routing = _route(h, g, cfg, hidden_states.requires_grad)
-        cur, branch = (None, None) if cfg.capacity is not None else _fork_small(h)
-        if branch is None:
-            aux, z = _loss_tensors(routing, N, E, cfg)  # from the routing before any capacity dropping
-            if cfg.capacity is not None:
-                dropped = ops.route_apply_capacity(routing, cfg.capacity)
-            else:
-                dropped = torch.zeros(1, dtype=torch.int32, device=h.device)
-        else:
-            # three one-block kernels that nothing in the layer waits for: a side branch, joined before returning
-            with torch.cuda.stream(branch):
-                aux, z = _loss_tensors(routing, N, E, cfg)
-                dropped = torch.zeros(1, dtype=torch.int32, device=h.device)
-        # Without a backward pass nothing sums over the padding rows, so they are not zeroed -- except with capacity
-        # dropping: a dropped slot keeps its grouped row (now a padding row) with weight 0, and 0 * (whatever the
-        # GEMMs make of uninitialised memory, possibly NaN) would reach the output through the combine.
-        Xg = ops.permute_rows(h, routing.src, routing.rows_cap, k,
-                              zero_padding=need_grad or cfg.capacity is not None)
-        keep = need_grad and not cfg.recompute
+            swg, swu, swd = (_device_tensor(_to(w, dtype), "shared expert weight") for w in (sw_gate, sw_up, sw_down))
+            Hs = swg.shape[0]
+        h_route = _jittered(h, cfg, hidden_states.requires_grad)
+        bias = cfg.expert_bias
+        if bias is not None:
+            bias = ops._req(bias.to(torch.float32).contiguous(), torch.float32, "expert_bias")
+        fp8 = _EXPERT_GEMM == "fp8" and D % 128 == 0 and H % 128 == 0
         # inference with few rows per expert (decode): one CTA per 128-row tile and no work on tiles without rows
-        small = _small_m_kwargs(not need_grad and cfg.capacity is None and N * k < 128 * E, routing.counts)
-        act, pre, Y = _expert_ffn_forward(Xg, wu, wd, E, routing.tile_start, D, H, cfg.activation, keep, small,
-                                          owners=(w_up, w_down))
+        few = not need_grad and cfg.capacity is None and N * k < 128 * E
+        fp8 = fp8 and not few
+        if fp8:
+            (wuq, wus), (wdq, wds) = _quantized_weight(w_up, wu), _quantized_weight(w_down, wd)
+
+        rows, ws_bytes, _ = ops.layer_sizes(N, D, E, k)
+        rt_bytes, o_w, o_idx, o_lg, o_lse, o_ts, o_pos, o_src, o_stats = ops.routing_layout(N, E, k)
+        out = torch.empty(N, D, dtype=dtype, device=dev)
+        counts = torch.empty(E, dtype=torch.int32, device=dev)
+        aux = torch.empty((), dtype=torch.float32, device=dev)
+        z = torch.empty((), dtype=torch.float32, device=dev)
+        dropped = torch.empty(1, dtype=torch.int32, device=dev)
+        # kept for the backward pass: tensors of their own; everything else shares one scratch allocation. All of it is
+        # allocated on the current stream, which the side streams are forked from and joined to inside the call.
+        arena = ops.Arena()
+        routing = Xg = pre = act = Y = s_act = s_pre = None
+        if need_grad:
+            routing = torch.empty(rt_bytes, dtype=torch.uint8, device=dev)
+            Xg = torch.empty(rows, D, dtype=dtype, device=dev)
+            if has_shared:
+                s_act = torch.empty(N, Hs, dtype=dtype, device=dev)
+                s_pre = torch.empty(N, 2 * Hs, dtype=dtype, device=dev)
+        else:
+            o_rt, o_xg = arena.take(rt_bytes), arena.take(rows * D * 2)
+            if has_shared:
+                o_sact = arena.take(N * Hs * 2)
+        if keep:
+            pre = torch.empty(rows, 2 * H, dtype=dtype, device=dev)
+            act = torch.empty(rows, H, dtype=dtype, device=dev)
+            Y = torch.empty(rows, D, dtype=dtype, device=dev)
+        else:
+            o_act, o_y = arena.take(rows * H * 2), arena.take(rows * D * 2)
+        o_sout = arena.take(N * D * 2) if has_shared else 0
+        o_ws = arena.take(ws_bytes)
+        if fp8:
+            o_xq, o_xs, o_aq, o_as = (arena.take(n) for n in (rows * D, rows * 4, rows * H, rows * 4))
+        scratch = torch.empty(arena.size, dtype=torch.uint8, device=dev)
+        base = scratch.data_ptr()
+        rt = routing.data_ptr() if need_grad else base + o_rt
+        p = ops._ptr
+        block = ops.LAYER_FORWARD_ARGS.pack(
+            N, D, E, k, H, Hs, rows, _lib.GATING[cfg.gating], _lib.ACTIVATION[cfg.activation],
+            _lib.ACTIVATION[cfg.shared_activation], 1 if cfg.pre_softmax else 0, cfg.n_group, cfg.topk_group,
+            -1 if cfg.capacity is None else cfg.capacity, 1 if need_grad else 0, 1 if few else 0, 1 if fp8 else 0,
+            1 if _OVERLAP else 0,
+            cfg.weight_scale, cfg.aux_loss_coeff * E / (float(N) * float(N)), cfg.z_loss_coeff / float(N),
+            h.data_ptr(), h_route.data_ptr(), g.data_ptr(), wu.data_ptr(), wd.data_ptr(), p(bias), p(add), p(swg), p(swu),
+            p(swd), *((p(wuq), p(wus), p(wdq), p(wds)) if fp8 else (0, 0, 0, 0)),
+            rt + o_lg, rt + o_w, rt + o_idx, rt + o_lse, counts.data_ptr(), rt + o_ts, rt + o_pos, rt + o_src, rt + o_stats,
+            aux.data_ptr(), z.data_ptr(), dropped.data_ptr(), base + o_ws, ws_bytes,
+            Xg.data_ptr() if need_grad else base + o_xg, p(pre), act.data_ptr() if keep else base + o_act,
+            Y.data_ptr() if keep else base + o_y,
+            0 if not has_shared else (s_act.data_ptr() if need_grad else base + o_sact), p(s_pre), base + o_sout,
+            *((base + o_xq, base + o_xs, base + o_aq, base + o_as) if fp8 else (0, 0, 0, 0)), out.data_ptr(),
+            p(ops.status_tensor(dev)), ops._stream(), _side_handle("shared") if has_shared and _OVERLAP else 0,
+            0 if add is None or cfg.addend_ready is None else cfg.addend_ready.cuda_event)
+        ops.layer_call(_lib.load().ffm_layer_forward, block, ops.FORWARD_SITES)
         if add is not None and cfg.addend_ready is not None:
-            torch.cuda.current_stream().wait_event(cfg.addend_ready)
             add.record_stream(torch.cuda.current_stream())
-        if shared_ready is not None:
-            torch.cuda.current_stream().wait_event(shared_ready)
-            add.record_stream(torch.cuda.current_stream())
-        out = ops.combine_forward(Y, routing.pos, routing.topk_w, N, k, addend=add)
-        if branch is not None:
-            _join_small(cur, branch, aux, z, dropped)
 
         ctx.set_materialize_grads(False)
         ctx.cfg = cfg
-        ctx.shape = (N, D, E, H)
-        ctx.rows_cap = routing.rows_cap
+        ctx.shape = (N, D, E, H, Hs)
         ctx.in_dtypes = (hidden_states.dtype, gate_weight.dtype, w_up.dtype, w_down.dtype,
                          None if addend is None else addend.dtype) + tuple(
                              None if w is None else w.dtype for w in (sw_gate, sw_up, sw_down))
-        saved = [h, g, wu, wd, routing.topk_w, routing.topk_idx, routing.logits, routing.lse, routing.counts,
-                 routing.tile_start, routing.pos, routing.src, Xg]
-        if keep:
-            saved += [pre, act, Y]
         ctx.kept = keep
         ctx.has_shared = has_shared and need_grad
-        if ctx.has_shared:
-            saved += [s_act, s_pre, swg, swu, swd]
-        ctx.save_for_backward(*saved)
-        counts = routing.counts
+        if need_grad:
+            ctx.save_for_backward(h, g, wu, wd, routing, counts, Xg, pre, act, Y, s_act, s_pre, swg, swu, swd)
         ctx.mark_non_differentiable(counts, dropped)
         return out, aux, z, counts, dropped
 
     @staticmethod
     def backward(ctx, grad_out, grad_aux, grad_z, _grad_counts, _grad_dropped):
         cfg = ctx.cfg
-        N, D, E, H = ctx.shape
+        N, D, E, H, Hs = ctx.shape
         k = cfg.top_k
-        saved = ctx.saved_tensors
-        (h, g, wu, wd, topk_w, topk_idx, logits, lse, counts, tile_start, pos, src, Xg) = saved[:13]
-        if ctx.kept:
-            pre, act, Y = saved[13:16]
-        else:
-            # recompute the three large tensors with the same kernels: bit-identical to the forward pass
-            act, pre = ops.grouped_gemm_glu(Xg, wu, wu.view(-1, D)[H:], 2 * H, E, tile_start, D, H, cfg.activation,
-                                            want_preact=True)
-            Y = ops.grouped_gemm(act, wd, _lib.B_KMAJOR, E, tile_start, H, D)
-        routing = ops.Routing(topk_w, topk_idx, logits, lse, counts, tile_start, pos, src, None, ctx.rows_cap, k, E)
+        (h, g, wu, wd, routing, counts, Xg, pre, act, Y, s_act, s_pre, swg, swu, swd) = ctx.saved_tensors
+        dev, dtype = h.device, h.dtype
+        # saved-tensor hooks may have handed back other tensors than were saved
+        for t in (h, g, wu, wd, Xg, pre, act, Y, s_act, s_pre, swg, swu, swd):
+            if t is not None:
+                _device_tensor(t, "saved tensor")
+        ops._req(routing, torch.uint8, "saved tensor")
+        ops._req(counts, torch.int32, "saved tensor")
+        shared = ctx.has_shared
+        if not shared:
+            Hs = 0
+        rows, _, ws_bytes = ops.layer_sizes(N, D, E, k)
+        _, o_w, o_idx, o_lg, o_lse, o_ts, o_pos, o_src, _ = ops.routing_layout(N, E, k)
         if grad_out is None:
-            grad_out = torch.zeros(N, D, dtype=h.dtype, device=h.device)
-        go = _to(grad_out, h.dtype)  # also densifies expanded (stride-0) gradients
+            grad_out = torch.zeros(N, D, dtype=dtype, device=dev)
+        go = _device_tensor(_to(grad_out, dtype), "go")  # also densifies expanded (stride-0) gradients
+        # the softmax aux loss carries no gradient on the reference's fast path ("reference_cuda")
+        if not (cfg.aux_loss_coeff > 0.0 and (cfg.aux_grad == "analytic" or cfg.gating == "sigmoid")):
+            grad_aux = None
+        if cfg.z_loss_coeff <= 0.0:
+            grad_z = None
+        grad_aux, grad_z = (None if t is None else t.to(torch.float32) for t in (grad_aux, grad_z))
+        # [D, Hs] has few output tiles (32 CTA-pair tiles at D = 1024, Hs = 2048 for 74 pairs): split the token dimension
+        # in two halves, each accumulated in fp32, and add the two bf16 results
+        split = 2 if (N + 127) // 128 >= 64 and (D // 256) * ((Hs + 255) // 256) <= 40 else 1
 
-        shared_done = None
-        fork_s = None
-        if ctx.has_shared and _OVERLAP:
-            fork_s = torch.cuda.Event()
-            fork_s.record()
-        # first in launch order: the routed GEMMs wait for it, the shared expert's (launched next) do not
-        gYw, gw = ops.combine_backward(go, Y, topk_w, src, ctx.rows_cap, k)
-        if ctx.has_shared:
-            s_act, s_pre, swg, swu, swd = saved[-5:]
-            if _OVERLAP:
-                # the shared expert's backward depends on the output gradient alone: its GEMMs start with the backward
-                # pass, beside combine_backward, and the routed GEMMs follow them
-                side = _get_side_stream("shared", priority=-1)
-                with torch.cuda.stream(side):
-                    side.wait_event(fork_s)
-                    s_dx, s_dwg, s_dwu, s_dwd = _glu_ffn_backward(go, h, s_act, s_pre, swg, swu, swd,
-                                                                  cfg.shared_activation)
-                    shared_done = torch.cuda.Event()
-                    shared_done.record(side)
-                go.record_stream(side)
-            else:
-                s_dx, s_dwg, s_dwu, s_dwd = _glu_ffn_backward(go, h, s_act, s_pre, swg, swu, swd, cfg.shared_activation)
+        def empty(*shape):
+            return torch.empty(*shape, dtype=dtype, device=dev)
 
-        if _OVERLAP:
-            # Two GEMMs never share an SM, so the GEMMs stay in one chain and each HBM-bound kernel is paired with
-            # a GEMM that does not depend on it:
-            #   main:  dAct GEMM with the GLU backward in its epilogue -> dW_down GEMM -> dX GEMM -> un-permute (+ routing
-            #          term); with FFM_FUSED_GLU_BACKWARD=0: dAct GEMM -> dW_down GEMM carrying the GLU backward as passenger
-            #   gemm:  (after dX) dW_up GEMM
-            #   route: routing backward (fills the gaps between GEMMs)
-            main = torch.cuda.current_stream()
-            gemm = _get_side_stream("backward_gemm")
-            route = _get_side_stream("backward_route")
-            fork = torch.cuda.Event()
-            fork.record(main)
-            with torch.cuda.stream(route):
-                route.wait_event(fork)
-                gaux, gz = _loss_grads(routing, N, E, cfg, grad_aux, grad_z)
-                dH_route, d_gate = ops.route_backward(gw, routing, gaux, gz, h, g, cfg.gating, dH=None)
-                route_done = torch.cuda.Event()
-                route_done.record(route)
-            if _FUSED_GLU_BWD and H % 64 == 0 and D % 64 == 0:
-                # dAct GEMM with the GLU backward in its epilogue, then the plain dW_down GEMM
-                gU = ops.grouped_gemm_dact_glu_backward(gYw, wd, E, tile_start, D, H, pre, cfg.activation)
-                d_wd = ops.grouped_gemm_wgrad(gYw, act, E, tile_start)
-            else:
-                d_act = ops.grouped_gemm(gYw, wd, _lib.B_NMAJOR, E, tile_start, D, H)
-                # the GLU backward rides on extra warps of the dW_down GEMM (one launch)
-                d_wd, gU = ops.grouped_gemm_wgrad_glu_backward(gYw, act, E, tile_start, d_act, pre, cfg.activation)
-            dXg = ops.grouped_gemm(gU, wu, _lib.B_NMAJOR, E, tile_start, 2 * H, D)
-            dx_done = torch.cuda.Event()
-            dx_done.record(main)
-            with torch.cuda.stream(gemm):
-                gemm.wait_event(dx_done)
-                d_wu = ops.grouped_gemm_wgrad(gU, Xg, E, tile_start)
-                join = torch.cuda.Event()
-                join.record(gemm)
-            main.wait_event(route_done)
-            if shared_done is not None:
-                main.wait_event(shared_done)
-            dH = ops.combine_forward(dXg, pos, None, N, k, addend=dH_route, addend2=s_dx if ctx.has_shared else None)
-            main.wait_event(join)
-            for t_side in (dH_route, d_gate, d_wu) + ((s_dx, s_dwg, s_dwu, s_dwd) if ctx.has_shared else ()):
-                t_side.record_stream(main)  # allocated on a side stream, consumed on the main one from here on
-        else:
-            d_act = ops.grouped_gemm(gYw, wd, _lib.B_NMAJOR, E, tile_start, D, H)
-            gU = ops.glu_backward(d_act, pre, tile_start, E, cfg.activation)
-            dXg = ops.grouped_gemm(gU, wu, _lib.B_NMAJOR, E, tile_start, 2 * H, D)
-            dH = ops.combine_forward(dXg, pos, None, N, k)
-            d_wd = ops.grouped_gemm_wgrad(gYw, act, E, tile_start)
-            d_wu = ops.grouped_gemm_wgrad(gU, Xg, E, tile_start)
-            gaux, gz = _loss_grads(routing, N, E, cfg, grad_aux, grad_z)
-            dH, d_gate = ops.route_backward(gw, routing, gaux, gz, h, g, cfg.gating, dH=dH)
+        dH, d_gate, d_wu, d_wd = empty(N, D), empty(E, D), empty(E, 2 * H, D), empty(E, D, H)
+        s_dw = s_dwd = None
+        if shared:
+            s_dw, s_dwd = empty(2 * Hs, D), empty(D, Hs)
+        fused = 1 if _FUSED_GLU_BWD else 0
+        arena = ops.Arena()
+        take = arena.take
+        o_gyw, o_gw, o_gu = take(rows * D * 2), take(N * k * 4), take(rows * 4 * H)
+        o_dxg, o_dhr, o_ws = take(rows * D * 2), take(N * D * 2), take(ws_bytes)
+        o_dact = 0 if fused else take(rows * H * 2)
+        o_sgu = o_sdact = o_sdx = o_sparts = 0
+        if shared:
+            o_sgu, o_sdx = take(N * Hs * 4), take(N * D * 2)
+            o_sdact = 0 if fused else take(N * Hs * 2)
+            o_sparts = take(2 * D * Hs * 2) if split == 2 else 0
+        if not ctx.kept:
+            o_pre, o_act, o_y = take(rows * H * 4), take(rows * H * 2), take(rows * D * 2)
+        scratch = torch.empty(arena.size, dtype=torch.uint8, device=dev)
+        base = scratch.data_ptr()
+        rt = routing.data_ptr()
+        p = ops._ptr
+        names = ("shared", "backward_route", "backward_gemm", "small")
+        block = ops.LAYER_BACKWARD_ARGS.pack(
+            N, D, E, k, H, Hs, rows, _lib.GATING[cfg.gating], _lib.ACTIVATION[cfg.activation],
+            _lib.ACTIVATION[cfg.shared_activation], 0 if ctx.kept else 1, 0 if cfg.capacity is None else 1, fused,
+            1 if _OVERLAP else 0, split,
+            cfg.aux_loss_coeff * E / float(N), cfg.z_loss_coeff,
+            go.data_ptr(), h.data_ptr(), g.data_ptr(), wu.data_ptr(), wd.data_ptr(), p(swg), p(swu), p(swd), p(grad_aux),
+            p(grad_z), rt + o_w, rt + o_idx, rt + o_lg, rt + o_lse, counts.data_ptr(), rt + o_ts, rt + o_pos, rt + o_src,
+            Xg.data_ptr(), *((pre.data_ptr(), act.data_ptr(), Y.data_ptr()) if ctx.kept else
+                             (base + o_pre, base + o_act, base + o_y)), p(s_act), p(s_pre),
+            dH.data_ptr(), d_gate.data_ptr(), d_wu.data_ptr(), d_wd.data_ptr(), p(s_dw), p(s_dwd), base + o_gyw, base + o_gw,
+            base + o_gu, base + o_dxg, base + o_dhr, base + o_dact, base + o_sgu, base + o_sdact, base + o_sdx,
+            base + o_sparts, base + o_ws, ws_bytes,
+            p(ops.status_tensor(dev)), ops._stream(), *((_side_handle(n) if _OVERLAP else 0) for n in names))
+        ops.layer_call(_lib.load().ffm_layer_backward, block, ops.BACKWARD_SITES, fused_glu=bool(fused))
 
         dt = ctx.in_dtypes
         d_add = None
         if dt[4] is not None and ctx.needs_input_grad[4]:
             d_add = go.to(dt[4])
         s_grads = (None, None, None)
-        if ctx.has_shared:
-            if not _OVERLAP:
-                dH = dH + s_dx
-            s_grads = (s_dwg.to(dt[5]), s_dwu.to(dt[6]), s_dwd.to(dt[7]))
+        if shared:
+            s_grads = (s_dw[:Hs].to(dt[5]), s_dw[Hs:].to(dt[6]), s_dwd.to(dt[7]))
         return (dH.to(dt[0]), d_gate.to(dt[1]), d_wu.to(dt[2]), d_wd.to(dt[3]), d_add) + s_grads + (None, None)
 
 

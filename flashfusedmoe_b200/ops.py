@@ -5,7 +5,10 @@ and enqueues the kernels on the current CUDA stream. Nothing here computes on th
 or without the built library every call raises.
 """
 
+import ctypes
+import struct
 from dataclasses import dataclass
+from functools import lru_cache
 
 import torch
 
@@ -139,6 +142,19 @@ def check_status(device=None):
 _status_host = {}
 
 
+def _status_entry(dev, key):
+    """Pinned word, stream and events of one device's status copies; the events are recorded once so that their handles
+    exist."""
+    entry = {"host": torch.zeros(1, dtype=torch.int32).pin_memory(), "pending": False,
+             "stream": torch.cuda.Stream(device=dev), "ready": torch.cuda.Event(), "done": torch.cuda.Event()}
+    entry["ready"].record()
+    entry["done"].record(entry["stream"])
+    entry["args"] = (entry["host"].data_ptr(), entry["stream"].cuda_stream, entry["ready"].cuda_event,
+                     entry["done"].cuda_event)
+    _status_host[key] = entry
+    return entry
+
+
 def poll_status(device=None, enqueue=True):
     """Host-side check of the status word that never waits for the GPU.
 
@@ -153,9 +169,7 @@ def poll_status(device=None, enqueue=True):
     key = dev.index if dev.index is not None else torch.cuda.current_device()
     entry = _status_host.get(key)
     if entry is None:
-        entry = _status_host[key] = {"host": torch.zeros(1, dtype=torch.int32).pin_memory(), "pending": False,
-                                     "stream": torch.cuda.Stream(device=dev), "ready": torch.cuda.Event(),
-                                     "done": torch.cuda.Event()}
+        entry = _status_entry(dev, key)
     if entry["pending"]:
         if not entry["done"].query():
             return  # the last copy is still in flight: look again at the next call
@@ -167,12 +181,9 @@ def poll_status(device=None, enqueue=True):
             raise RuntimeError(f"libffmoe device status {code}: {_lib.error_string(code)} "
                                "(reported by a kernel of an earlier call; its results are not valid)")
     if enqueue:
-        side = entry["stream"]
-        entry["ready"].record()
-        side.wait_event(entry["ready"])
-        with torch.cuda.stream(side):
-            entry["host"].copy_(status_tensor(dev), non_blocking=True)
-            entry["done"].record(side)
+        host, side, ready, done = entry["args"]
+        _lib.check(_lib.load().ffm_status_copy(_ptr(status_tensor(dev)), host, _stream(), side, ready, done),
+                   "ffm_status_copy")
         entry["pending"] = True
 
 
@@ -529,3 +540,84 @@ def route_backward(gw, routing, gaux, gz, hidden, gate_w, gating, dH=None):
                                     _ptr(ws), ws.numel(), _ptr(status_tensor(dev)), _stream())
     _lib.check(rc, "ffm_route_backward")
     return dH, dGate
+
+
+# ----------------------------------------------------------------------------------------------
+# The single-GPU layer in one call each way (ffm_layer_forward / ffm_layer_backward)
+# ----------------------------------------------------------------------------------------------
+
+# argument blocks as include/ffmoe.h declares them (64-bit integers and pointers, doubles in between) without the last
+# two fields, timer and launched
+LAYER_FORWARD_ARGS = struct.Struct("=18q3d44q")
+LAYER_BACKWARD_ARGS = struct.Struct("=15q2d48q")
+
+# (timer bucket, second bucket, C call) of every launch site, in the order of the FFM_FWD_* and FFM_BWD_* enumerations
+_GLU, _GEMM, _WGRAD = ("gemm_up_glu", None, "ffm_grouped_gemm_glu"), ("gemm", None, "ffm_grouped_gemm"), \
+    ("gemm_wgrad", None, "ffm_grouped_gemm_wgrad")
+_DACT = ("gemm", "gemm_dact_glu_backward", "ffm_grouped_gemm_dact_glu_backward")
+FORWARD_SITES = (_GLU, _GEMM, ("route_forward", None, "ffm_route_forward"),
+                 ("route_capacity", None, "ffm_route_apply_capacity"), ("permute_rows", None, "ffm_permute_rows"),
+                 ("quantize_rows", None, "ffm_quantize_rows_e4m3"), _GLU,
+                 ("quantize_rows", None, "ffm_quantize_rows_e4m3"), _GEMM,
+                 ("combine_forward", None, "ffm_combine_forward"))
+BACKWARD_SITES = (_GLU, _GEMM, ("combine_backward", None, "ffm_combine_backward"), _DACT,
+                  ("glu_backward", None, "ffm_glu_backward"), _WGRAD, ("sum_splits", None, "add_bf16"), _GEMM, _WGRAD,
+                  ("route_backward", None, "ffm_route_backward"), _DACT, ("glu_backward", None, "ffm_glu_backward"),
+                  _WGRAD, _GEMM, _WGRAD, ("combine_forward", None, "ffm_combine_forward"))
+
+
+def layer_call(fn, block, sites, fused_glu=True):
+    """Run ffm_layer_forward / ffm_layer_backward on a packed argument block (all fields but the last two, timer and
+    launched). Counts its launches and, with a timer installed, files an event pair per launch site."""
+    global launch_count
+    launched = (ctypes.c_int64 * 3)()
+    pairs = handles = None
+    if _timer is not None:
+        pairs = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)) for _ in sites]
+        for a, b in pairs:
+            a.record()
+            b.record()
+        handles = (ctypes.c_int64 * (2 * len(sites)))(*(e.cuda_event for pair in pairs for e in pair))
+    tail = struct.pack("=2q", 0 if handles is None else ctypes.addressof(handles), ctypes.addressof(launched))
+    rc = fn(block + tail)
+    launch_count += launched[0]
+    if pairs is not None:
+        for i, (pair, (name, also, _)) in enumerate(zip(pairs, sites)):
+            if launched[1] >> i & 1:
+                _timer.events.setdefault(name, []).append(pair)
+                if also is not None and fused_glu:
+                    _timer.events.setdefault(also, []).append(pair)
+    if rc != _lib.FFM_OK:
+        site = launched[2]
+        _lib.check(rc, sites[site][2] if site >= 0 else "stream fork or join")
+
+
+class Arena:
+    """Byte offsets of buffers in one allocation, 256-byte aligned."""
+
+    def __init__(self):
+        self.size = 0
+
+    def take(self, nbytes):
+        offset = self.size
+        self.size += (int(nbytes) + 255) // 256 * 256
+        return offset
+
+
+@lru_cache(maxsize=1024)
+def layer_sizes(N, D, E, k):
+    """(rows_cap, forward workspace bytes, backward workspace bytes)."""
+    lib = _lib.load()
+    return (rows_capacity(N * k, E), int(lib.ffm_route_workspace_bytes(N, E, k)),
+            int(lib.ffm_route_backward_workspace_bytes(N, D, E)))
+
+
+@lru_cache(maxsize=1024)
+def routing_layout(N, E, k):
+    """Offsets of the routing results kept for the backward pass in one buffer: (size, topk_w, topk_idx, logits, lse,
+    tile_start, pos, src, stats)."""
+    a = Arena()
+    T = N * k
+    offsets = [a.take(n) for n in (T * 4, T * 4, N * E * 2, N * 4, (E + 1) * 4, T * 4, max(rows_capacity(T, E), 1) * 4,
+                                   (E + 2) * 4)]
+    return (max(a.size, 256), *offsets)

@@ -301,6 +301,91 @@ int ffm_grouped_gemm_fp8(const void* Aq, const float* a_scale, const void* Bq, c
                          int32_t* status, ffm_stream_t stream);
 
 /* -------------------------------------------------------------------------------------------------
+ * The single-GPU layer in one call each way: the launches of the forward and of the backward pass (_FusedMoEFunction of
+ * the reference, fused_moe.py:299-595) over caller-owned buffers, with the fork and join of the side streams. Nothing is
+ * allocated on the device and nothing is waited for on the host; with overlap != 0 every side stream is joined to
+ * `stream` before the call returns, so buffers may be freed in the order of `stream`, and a call can be captured.
+ *
+ * Forward: routing (aux = aux_scale * stats[E + 1] and z = z_scale * stats[E] when not null), capacity >= 0: dropping,
+ * permute, expert GEMMs, combine; Hs > 0: a shared expert (sw_*) beside the routing, its output added in the combine.
+ * need_grad: zero the padding rows and store preact / s_preact where given. few_rows: 128-row tiles that skip tiles
+ * without rows. fp8: e4m3 expert GEMMs (w_*_q, w_*_scale; xq, x_scale, aq, a_scale are scratch). addend_ready: a cudaEvent_t
+ * the combine waits for, or null.
+ *
+ * Backward: go [N, D] and the forward pass's buffers (recompute: preact, act and Y are written here first) -> dH, d_gate,
+ * d_w_up, d_w_down, and with Hs > 0 s_d_gate_up [2 Hs, D] and s_d_down [D, Hs]. Loss gradients: grad_aux, grad_z are device
+ * scalars or null; aux_coef = coefficient * E / N, z_coef = coefficient. zero_gw: slots may have no row (capacity).
+ * fused_glu: GLU backward inside the dAct GEMM; else d_act / s_d_act are scratch. shared_split: 1 or 2 ranges of the tokens
+ * for the shared down-projection's gradient (2: s_parts [2, D, Hs]).
+ *
+ * timer: null, or 2 cudaEvent_t per site (FFM_FWD_* / FFM_BWD_*), recorded around the launches of the sites that run.
+ * launched [3] out: kernels enqueued, bit mask of the sites that ran, the site a non-zero return code comes from.
+ * ------------------------------------------------------------------------------------------------- */
+enum { FFM_FWD_SHARED_UP, FFM_FWD_SHARED_DOWN, FFM_FWD_ROUTE, FFM_FWD_CAPACITY, FFM_FWD_PERMUTE, FFM_FWD_QUANT_X, FFM_FWD_UP,
+       FFM_FWD_QUANT_ACT, FFM_FWD_DOWN, FFM_FWD_COMBINE, FFM_FWD_SITES };
+enum { FFM_BWD_RE_UP, FFM_BWD_RE_DOWN, FFM_BWD_COMBINE, FFM_BWD_S_DACT, FFM_BWD_S_GLU, FFM_BWD_S_WDOWN, FFM_BWD_S_SUM,
+       FFM_BWD_S_DX, FFM_BWD_S_WUP, FFM_BWD_ROUTE, FFM_BWD_DACT, FFM_BWD_GLU, FFM_BWD_WDOWN, FFM_BWD_DX, FFM_BWD_WUP,
+       FFM_BWD_UNPERMUTE, FFM_BWD_SITES };
+typedef struct {
+  int64_t N, D, E, top_k, H, Hs, rows_cap, gating, activation, shared_activation, pre_softmax, n_group;
+  int64_t topk_group, capacity, need_grad, few_rows, fp8, overlap;
+  double weight_scale, aux_scale, z_scale;
+  const void *hidden, *hidden_route, *gate, *w_up, *w_down;
+  const float *expert_bias;
+  const void *addend, *sw_gate, *sw_up, *sw_down, *w_up_q;
+  const float *w_up_scale;
+  const void *w_down_q;
+  const float *w_down_scale;
+  void *logits;
+  float *topk_w;
+  int32_t *topk_idx;
+  float *lse;
+  int32_t *counts, *tile_start, *pos, *src;
+  float *stats, *aux, *z;
+  int32_t *dropped;
+  void *workspace;
+  int64_t workspace_bytes;
+  void *Xg, *preact, *act, *Y, *s_act, *s_preact, *s_out, *xq;
+  float *x_scale;
+  void *aq;
+  float *a_scale;
+  void *out;
+  int32_t *status;
+  ffm_stream_t stream, shared_stream;
+  void *addend_ready;
+  const int64_t *timer;
+  int64_t *launched;
+} ffm_layer_forward_args;
+typedef struct {
+  int64_t N, D, E, top_k, H, Hs, rows_cap, gating, activation, shared_activation, recompute, zero_gw;
+  int64_t fused_glu, overlap, shared_split;
+  double aux_coef, z_coef;
+  const void *go, *hidden, *gate, *w_up, *w_down, *sw_gate, *sw_up, *sw_down;
+  const float *grad_aux, *grad_z;
+  float *topk_w;
+  int32_t *topk_idx;
+  void *logits;
+  float *lse;
+  int32_t *counts, *tile_start, *pos, *src;
+  void *Xg, *preact, *act, *Y, *s_act, *s_preact;
+  void *dH, *d_gate, *d_w_up, *d_w_down, *s_d_gate_up, *s_d_down, *gYw;
+  float *gw;
+  void *gU, *dXg, *dH_route, *d_act, *s_gU, *s_d_act, *s_dx, *s_parts, *workspace;
+  int64_t workspace_bytes;
+  int32_t *status;
+  ffm_stream_t stream, shared_stream, route_stream, gemm_stream, small_stream;
+  const int64_t *timer;
+  int64_t *launched;
+} ffm_layer_backward_args;
+int ffm_layer_forward(const ffm_layer_forward_args* args);
+int ffm_layer_backward(const ffm_layer_backward_args* args);
+
+/* host[0] = *status by an asynchronous copy on side_stream, ordered after what `stream` holds: record `ready` on stream,
+ * side_stream waits for it, copies, records `done` (cudaEvent_t handles; host is pinned memory). */
+int ffm_status_copy(const int32_t* status, int32_t* host, ffm_stream_t stream, ffm_stream_t side_stream, void* ready,
+                    void* done);
+
+/* -------------------------------------------------------------------------------------------------
  * Expert-parallel exchange over NVLink with plain peer stores. Replaces the c10d all_to_all_single calls of the
  * reference's dispatcher (expert_parallel.py:253-258, :290-292; fused_moe.py:901-910).
  * The caller owns the receive buffers and the flag arrays, which must be mapped on every GPU of the group
