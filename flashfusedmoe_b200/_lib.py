@@ -48,6 +48,12 @@ SIGNATURES = {
                                    c_void_p]),
     "ffm_grouped_gemm_wgrad": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_int64, c_int, c_int, c_float,
                                        c_void_p, c_void_p, c_void_p]),
+    "ffm_grouped_gemm_wgrad_rows": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int64, c_int, c_int, c_float,
+                                            c_void_p, c_void_p, c_void_p]),
+    "ffm_decode_gemm_glu": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int, c_void_p, c_void_p, c_int64, c_int, c_int,
+                                    c_int, c_void_p, c_void_p, c_void_p]),
+    "ffm_decode_gemm": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int64, c_int, c_int, c_void_p, c_void_p,
+                                c_void_p]),
     "ffm_grouped_gemm_wgrad_glu_backward": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_int64, c_int, c_int, c_float,
                                                     c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_void_p,
                                                     c_void_p, c_void_p]),

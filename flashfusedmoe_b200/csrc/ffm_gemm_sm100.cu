@@ -36,7 +36,7 @@
 // tiles); the GLU epilogue fills three (activation, gate, up) per 64-column step.
 #include <stdlib.h>
 
-#include "ffm_common.cuh"
+#include "ffm_gemm_common.cuh"
 #include "ffm_internal.h"
 
 namespace ffm {
@@ -121,8 +121,9 @@ struct Shape {
 
 struct GemmParams {
   const int32_t* tile_start;  // [groups + 1] cumulative 128-row tiles, or null (dense)
-  const int32_t* group_rows;  // [groups] valid rows per group, or null: when given (grouped-M only) the tiles of a
-                              // group that hold no valid row are not computed
+  const int32_t* group_rows;  // [groups] valid rows per group, or null. Grouped-M: the tiles of a group that hold no
+                              // valid row are not computed. Grouped-K: K ends at the group's last valid row (rounded up
+                              // to 16) instead of its segment's end, up to 255 padding rows further
   int groups;
   int dense_m_tiles;
   int n_cols;              // output columns per group (GLU: H)
@@ -177,6 +178,7 @@ struct TileCoord {
   int n_block;   // BN-column block (GLU: 128-column block of H)
   int k_row0;    // grouped-K: first K row; else 0
   int k_blocks;  // 64-deep K blocks to accumulate
+  int k_tail;    // 16-deep MMA steps of the last K block (4 unless grouped-K rows are given)
 };
 
 // Walks the tiles of this CTA (or CTA pair) in launch order. The unit is one MMA tile: 128 rows, or with CTA2
@@ -187,6 +189,7 @@ template <int GROUPK, int CTA2>
 struct TileWalker {
   const int* ts;             // cumulative tiles to walk (shared memory)
   const int32_t* layout_ts;  // cumulative tiles of the memory layout when it differs from `ts` (global), else null
+  const int32_t* k_rows;     // grouped-K: valid rows per group, else null
   int groups, n_tiles, m_units_per_group, k_blocks, rank;
   long long total, cur, step;
   int g;
@@ -196,6 +199,7 @@ struct TileWalker {
   __device__ TileWalker(const GemmParams& p, const int* ts_smem, int cta_rank) {
     ts = ts_smem;
     layout_ts = (!GROUPK && p.group_rows != nullptr) ? p.tile_start : nullptr;
+    k_rows = GROUPK ? p.group_rows : nullptr;
     groups = p.groups;
     n_tiles = p.n_tiles;
     k_blocks = p.k_blocks;
@@ -222,6 +226,12 @@ struct TileWalker {
       t.n_block = r / m_units_per_group;
       t.k_row0 = ts[t.group] * BM;
       t.k_blocks = (ts[t.group + 1] - ts[t.group]) * (BM / BK);
+      t.k_tail = BK / UMMA_K;
+      if (k_rows != nullptr) {
+        const int steps = (__ldg(k_rows + t.group) + UMMA_K - 1) / UMMA_K;
+        t.k_blocks = (steps + BK / UMMA_K - 1) / (BK / UMMA_K);
+        t.k_tail = steps - (t.k_blocks - 1) * (BK / UMMA_K);
+      }
     } else {
       while (g < groups - 1 && cur >= static_cast<long long>(units(ts[g + 1])) * n_tiles) ++g;
       const int u0 = units(ts[g]);
@@ -238,135 +248,6 @@ struct TileWalker {
     return true;
   }
 };
-
-// ---- PTX used only by this kernel --------------------------------------------------------------
-
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-
-// shared::cluster address of the same shared-memory offset in CTA `rank` of this cluster
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
-  return r;
-}
-
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-
-// 2-D TMA load issued by either CTA of a pair into its own shared memory; the byte count completes on the
-// mbarrier at `bar`, a shared::cluster address that may belong to the other CTA of the pair.
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const void* map, uint32_t bar, int c0, int c1) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], "
-      "[%2];" ::"r"(dst),
-      "l"(map), "r"(bar), "r"(c0), "r"(c1)
-      : "memory");
-}
-
-// 3-D TMA load into this CTA's shared memory (no cluster broadcast), completing on one of its own mbarriers.
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const void* map, uint32_t bar, int c0, int c1, int c2) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-      ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
-      : "memory");
-}
-
-__device__ __forceinline__ void ld_shared_v4(uint32_t addr, uint4& v) {
-  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
-}
-
-__device__ __forceinline__ void tma_store_3d(const void* map, uint32_t src, int c0, int c1, int c2) {
-  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(map), "r"(src),
-               "r"(c0), "r"(c1), "r"(c2)
-               : "memory");
-}
-// Ask the TMA unit to bring one box of a tensor into L2 (nothing lands in shared memory, nothing to wait for).
-__device__ __forceinline__ void tma_prefetch_l2_2d(const void* map, int c0, int c1) {
-  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(c0), "r"(c1)
-               : "memory");
-}
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-// wait until at most N of this thread's bulk store groups have not finished reading shared memory
-template <int N>
-__device__ __forceinline__ void bulk_wait_read() {
-  asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
-}
-__device__ __forceinline__ void bulk_wait0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-
-__device__ __forceinline__ void tmem_alloc2(uint32_t slot_smem_addr, uint32_t cols) {
-  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot_smem_addr), "r"(cols)
-               : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish2() {
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc2(uint32_t taddr, uint32_t cols) {
-  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
-}
-
-__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                               uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
-      "}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// The same with 8-bit floating-point operands (e4m3 / e5m2 chosen by the instruction descriptor), 32 K elements per
-// instruction, fp32 accumulation.
-__device__ __forceinline__ void umma_f8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                        uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n"
-      "}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void umma_f8_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                             uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n"
-      "}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// Instruction descriptor for kind::f8f6f4 with e4m3 A and B (format code 0) and fp32 accumulation, K-major operands.
-__host__ __device__ constexpr uint32_t make_idesc_e4m3(int m, int n) {
-  return (1u << 4) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
-}
-
-// Arrive (once the pair's MMAs issued so far have completed) on one mbarrier given by shared::cluster address.
-__device__ __forceinline__ void umma_commit_pair(uint32_t cluster_bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cluster_bar)
-               : "memory");
-}
-
-// 16-byte chunk q (0..7) of row r inside a 32-row x 128-byte box with the 128-byte TMA swizzle
-__device__ __forceinline__ uint32_t box_offset(int r, int q) { return r * 128 + ((q ^ (r & 7)) << 4); }
-
-__device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
 
 // GLU backward over rows [0, rows): (d gate | d up)[r, :] from dAct[r, :] and the saved pre-activations. `rows` is
 // pz_rows cut at the end of the last group's tiles (buffers sized for a worst case hold far more rows than are used).
@@ -722,6 +603,7 @@ ffm_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           const uint32_t b_src = a_src + A_STAGE_BYTES;
 #pragma unroll
           for (int kk = 0; kk < BK / UMMA_K; ++kk) {
+            if (GROUPK && kb == t.k_blocks - 1 && kk >= t.k_tail) break;
             const uint64_t adesc = A_MN ? make_smem_desc_sw128(a_src + kk * 2048, 8192, 1024)
                                         : make_smem_desc_sw128(a_src + kk * 32, 16, 1024);
             const uint64_t bdesc = B_MN ? make_smem_desc_sw128(b_src + kk * 2048, 8192, 1024)
@@ -1013,88 +895,7 @@ ffm_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 // Host side
 // ---------------------------------------------------------------------------------------------
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn get_encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  static bool tried = false;
-  if (!tried) {
-    tried = true;
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) == cudaSuccess &&
-        qres == cudaDriverEntryPointSuccess) {
-      fn = reinterpret_cast<EncodeTiledFn>(ptr);
-    }
-  }
-  return fn;
-}
-
-// 2-D tensor map over a row-major [rows, cols] matrix of bf16 (elt_bytes 2) or bytes (elt_bytes 1: e4m3 operands),
-// 128-byte swizzle, zero fill out of bounds.
-int make_map_2d(CUtensorMap* map, const void* base, long long rows, long long cols, int box_cols, int box_rows,
-                int elt_bytes = 2) {
-  EncodeTiledFn fn = get_encode_fn();
-  if (fn == nullptr) return FFM_ERR_NO_DRIVER;
-  if (rows <= 0 || cols <= 0) return FFM_ERR_BAD_ARG;
-  if ((reinterpret_cast<uintptr_t>(base) & 15u) != 0 || (cols * elt_bytes) % 16 != 0) return FFM_ERR_UNSUPPORTED;
-  cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
-  cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * elt_bytes};
-  cuuint32_t box[2] = {static_cast<cuuint32_t>(box_cols), static_cast<cuuint32_t>(box_rows)};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, elt_bytes == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
-                  const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? FFM_OK : FFM_ERR_LAUNCH;
-}
-
-// 2-D bf16 map used only for L2 prefetches (cp.async.bulk.prefetch.tensor): box {256 columns, 128 rows}, no swizzle.
-int make_prefetch_map(CUtensorMap* map, const void* base, long long rows, long long cols) {
-  EncodeTiledFn fn = get_encode_fn();
-  if (fn == nullptr) return FFM_ERR_NO_DRIVER;
-  if (rows <= 0 || cols <= 0) return FFM_ERR_BAD_ARG;
-  if ((reinterpret_cast<uintptr_t>(base) & 15u) != 0 || (cols * 2) % 16 != 0) return FFM_ERR_UNSUPPORTED;
-  cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
-  cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * 2};
-  cuuint32_t box[2] = {static_cast<cuuint32_t>(cols < 256 ? cols : 256), static_cast<cuuint32_t>(rows < 128 ? rows : 128)};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? FFM_OK : FFM_ERR_LAUNCH;
-}
-
-// 3-D bf16 output map over [groups, rows, cols] (row-major, contiguous), 128-byte swizzle, box {64, 32, 1}.
-int make_out_map(CUtensorMap* map, void* base, long long groups, long long rows, long long cols) {
-  EncodeTiledFn fn = get_encode_fn();
-  if (fn == nullptr) return FFM_ERR_NO_DRIVER;
-  if (groups <= 0 || rows <= 0 || cols <= 0) return FFM_ERR_BAD_ARG;
-  if ((reinterpret_cast<uintptr_t>(base) & 15u) != 0 || (cols * 2) % 16 != 0) return FFM_ERR_UNSUPPORTED;
-  cuuint64_t dims[3] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(groups)};
-  cuuint64_t strides[2] = {static_cast<cuuint64_t>(cols) * 2, static_cast<cuuint64_t>(cols) * rows * 2};
-  cuuint32_t box[3] = {64, 32, 1};
-  cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, base, dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? FFM_OK : FFM_ERR_LAUNCH;
-}
-
-int num_sms() {
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (sms <= 0) sms = 148;
-  }
-  return sms;
-}
-
-long long g_wait_cycles = 2000000000LL;
+long long g_wait_cycles = 2000000000LL;  // see gemm_wait_cycles()
 int g_cta_pair = -1;  // -1: read FFM_GEMM_CTA_PAIR from the environment on first use (default on)
 
 bool use_cta_pair() {
@@ -1178,6 +979,8 @@ int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB0, const CUtensorM
 }
 
 }  // namespace
+
+long long gemm_wait_cycles() { return g_wait_cycles; }
 
 }  // namespace ffm
 
@@ -1306,8 +1109,8 @@ extern "C" int ffm_dense_gemm_two(const void* A, const void* B1, int K1, const v
                                          static_cast<cudaStream_t>(stream));
 }
 
-int ffm::grouped_wgrad(const void* A, const void* B, int groups, const int32_t* tile_start, int64_t rows_cap, int M, int Nout,
-                       float scale, void* dW, int32_t* status, ffm_stream_t stream) {
+int ffm::grouped_wgrad(const void* A, const void* B, int groups, const int32_t* tile_start, const int32_t* counts,
+                       int64_t rows_cap, int M, int Nout, float scale, void* dW, int32_t* status, ffm_stream_t stream) {
   if (!A || !B || !dW || !status) return FFM_ERR_BAD_ARG;
   if (groups < 1 || groups > MAX_GROUPS || rows_cap <= 0 || M <= 0 || Nout <= 0) return FFM_ERR_BAD_ARG;
   if (M % 64 != 0 || Nout % 64 != 0) return FFM_ERR_UNSUPPORTED;
@@ -1326,6 +1129,7 @@ int ffm::grouped_wgrad(const void* A, const void* B, int groups, const int32_t* 
   p.n_tiles = (Nout + BN - 1) / BN;
   p.status = status;
   p.wait_cycles = g_wait_cycles;
+  p.group_rows = counts;
   return launch_gemm<1, 1, EPI_PLAIN, 1>(tmA, tmB, tmB, tmC, tmC, p, p.m_tiles_per_group,
                                          static_cast<long long>(groups) * p.n_tiles,
                                          static_cast<cudaStream_t>(stream));
@@ -1335,7 +1139,14 @@ extern "C" int ffm_grouped_gemm_wgrad(const void* A, const void* B, int groups, 
                                       int64_t rows_cap, int M, int Nout, float scale, void* dW, int32_t* status,
                                       ffm_stream_t stream) {
   if (!tile_start) return FFM_ERR_BAD_ARG;
-  return ffm::grouped_wgrad(A, B, groups, tile_start, rows_cap, M, Nout, scale, dW, status, stream);
+  return ffm::grouped_wgrad(A, B, groups, tile_start, nullptr, rows_cap, M, Nout, scale, dW, status, stream);
+}
+
+extern "C" int ffm_grouped_gemm_wgrad_rows(const void* A, const void* B, int groups, const int32_t* tile_start,
+                                           const int32_t* counts, int64_t rows_cap, int M, int Nout, float scale, void* dW,
+                                           int32_t* status, ffm_stream_t stream) {
+  if (!tile_start) return FFM_ERR_BAD_ARG;
+  return ffm::grouped_wgrad(A, B, groups, tile_start, counts, rows_cap, M, Nout, scale, dW, status, stream);
 }
 
 extern "C" int ffm_grouped_gemm_wgrad_glu_backward(const void* A, const void* B, int groups, const int32_t* tile_start,

@@ -31,10 +31,10 @@ int route_backward_losses(const float* gw, const float* topk_w, const int32_t* t
                           int D, int E, int top_k, int gating, int accumulate, void* dH, void* dGate, void* workspace,
                           size_t workspace_bytes, int32_t* status, ffm_stream_t stream);
 
-// ffm_grouped_gemm_wgrad; with tile_start null the groups are equal ranges (in 128-row tiles) of the rows, a split of one
-// dense contraction.
-int grouped_wgrad(const void* A, const void* B, int groups, const int32_t* tile_start, int64_t rows_cap, int M, int Nout,
-                  float scale, void* dW, int32_t* status, ffm_stream_t stream);
+// ffm_grouped_gemm_wgrad_rows; with tile_start null the groups are equal ranges (in 128-row tiles) of the rows, a split of
+// one dense contraction.
+int grouped_wgrad(const void* A, const void* B, int groups, const int32_t* tile_start, const int32_t* counts,
+                  int64_t rows_cap, int M, int Nout, float scale, void* dW, int32_t* status, ffm_stream_t stream);
 
 // out = a + b, bf16 values added in fp32 (n elements, a multiple of 8)
 int add_bf16(const void* a, const void* b, int64_t n, void* out, ffm_stream_t stream);

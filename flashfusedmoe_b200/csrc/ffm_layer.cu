@@ -89,10 +89,17 @@ extern "C" int ffm_layer_forward(const ffm_layer_forward_args* args) {
   if (Hs > 0) {
     if (sh != st) sites.require(fork.order(st, sh));
     sites.run(FFM_FWD_SHARED_UP, 1, sh, [&] {
+      if (a.few_rows & FFM_FEW_DECODE_SHARED) {
+        return ffm_decode_gemm_glu(a.hidden, a.sw_gate, a.sw_up, Hs, 1, nullptr, nullptr, a.N, D, Hs,
+                                   static_cast<int>(a.shared_activation), a.s_act, a.status, sh);
+      }
       return ffm_grouped_gemm_glu(a.hidden, a.sw_gate, a.sw_up, Hs, 1, nullptr, a.N, D, Hs,
                                   static_cast<int>(a.shared_activation), a.s_act, a.s_preact, nullptr, 0, a.status, sh);
     });
     sites.run(FFM_FWD_SHARED_DOWN, 1, sh, [&] {
+      if (a.few_rows & FFM_FEW_DECODE_SHARED) {
+        return ffm_decode_gemm(a.s_act, a.sw_down, 1, nullptr, nullptr, a.N, Hs, D, a.s_out, a.status, sh);
+      }
       return ffm_grouped_gemm(a.s_act, a.sw_down, FFM_B_KMAJOR, 1, nullptr, a.N, Hs, D, 1.0f, a.s_out, nullptr, 0,
                               a.status, sh);
     });
@@ -119,8 +126,8 @@ extern "C" int ffm_layer_forward(const ffm_layer_forward_args* args) {
   sites.run(FFM_FWD_PERMUTE, 1, st, [&] {
     return ffm_permute_rows(a.hidden, a.src, a.rows_cap, k, D, a.need_grad || a.capacity >= 0 ? 1 : 0, a.Xg, st);
   });
-  const int32_t* valid = a.few_rows ? a.counts : nullptr;
-  const int tile_rows = a.few_rows ? 128 : 0;
+  const int32_t* valid = (a.few_rows & FFM_FEW_TILES) ? a.counts : nullptr;
+  const int tile_rows = (a.few_rows & FFM_FEW_TILES) ? 128 : 0;
   if (a.fp8) {
     sites.run(FFM_FWD_QUANT_X, 1, st, [&] { return ffm_quantize_rows_e4m3(a.Xg, a.rows_cap, D, a.xq, a.x_scale, st); });
     sites.run(FFM_FWD_UP, 1, st, [&] {
@@ -135,10 +142,17 @@ extern "C" int ffm_layer_forward(const ffm_layer_forward_args* args) {
   } else {
     const void* up_rows = static_cast<const char*>(a.w_up) + a.H * a.D * 2;
     sites.run(FFM_FWD_UP, 1, st, [&] {
+      if (a.few_rows & FFM_FEW_DECODE_UP) {
+        return ffm_decode_gemm_glu(a.Xg, a.w_up, up_rows, 2 * a.H, E, a.tile_start, a.counts, a.rows_cap, D, H, act, a.act,
+                                   a.status, st);
+      }
       return ffm_grouped_gemm_glu(a.Xg, a.w_up, up_rows, 2 * a.H, E, a.tile_start, a.rows_cap, D, H, act, a.act, a.preact,
                                   valid, tile_rows, a.status, st);
     });
     sites.run(FFM_FWD_DOWN, 1, st, [&] {
+      if (a.few_rows & FFM_FEW_DECODE_DOWN) {
+        return ffm_decode_gemm(a.act, a.w_down, E, a.tile_start, a.counts, a.rows_cap, H, D, a.Y, a.status, st);
+      }
       return ffm_grouped_gemm(a.act, a.w_down, FFM_B_KMAJOR, E, a.tile_start, a.rows_cap, H, D, 1.0f, a.Y, valid, tile_rows,
                               a.status, st);
     });
@@ -215,7 +229,7 @@ extern "C" int ffm_layer_backward(const ffm_layer_backward_args* args) {
       });
     }
     sites.run(FFM_BWD_S_WDOWN, 1, sh, [&] {
-      return grouped_wgrad(a.go, a.s_act, split, nullptr, a.N, D, Hs, 1.0f, parts, a.status, sh);
+      return grouped_wgrad(a.go, a.s_act, split, nullptr, nullptr, a.N, D, Hs, 1.0f, parts, a.status, sh);
     });
     if (split == 2) {
       if (overlap) sites.require(sum_fork.order(sh, sm));
@@ -227,7 +241,7 @@ extern "C" int ffm_layer_backward(const ffm_layer_backward_args* args) {
       return ffm_dense_gemm_two(a.s_gU, a.sw_gate, Hs, a.sw_up, a.N, 2 * Hs, D, a.s_dx, a.status, sh);
     });
     sites.run(FFM_BWD_S_WUP, 1, sh, [&] {
-      return grouped_wgrad(a.s_gU, a.hidden, 1, nullptr, a.N, 2 * Hs, D, 1.0f, a.s_d_gate_up, a.status, sh);
+      return grouped_wgrad(a.s_gU, a.hidden, 1, nullptr, nullptr, a.N, 2 * Hs, D, 1.0f, a.s_d_gate_up, a.status, sh);
     });
     if (overlap) {
       if (split == 2) sites.require(sum_done.wait(sh));
@@ -255,7 +269,7 @@ extern "C" int ffm_layer_backward(const ffm_layer_backward_args* args) {
                                                 a.status, st);
     });
     sites.run(FFM_BWD_WDOWN, 1, st, [&] {
-      return grouped_wgrad(a.gYw, a.act, E, a.tile_start, a.rows_cap, D, H, 1.0f, a.d_w_down, a.status, st);
+      return grouped_wgrad(a.gYw, a.act, E, a.tile_start, nullptr, a.rows_cap, D, H, 1.0f, a.d_w_down, a.status, st);
     });
   } else {
     sites.run(FFM_BWD_DACT, 1, st, [&] {
@@ -273,7 +287,7 @@ extern "C" int ffm_layer_backward(const ffm_layer_backward_args* args) {
         return ffm_glu_backward(a.d_act, a.preact, a.tile_start, E, a.rows_cap, H, act, a.gU, st);
       });
       sites.run(FFM_BWD_WDOWN, 1, st, [&] {
-        return grouped_wgrad(a.gYw, a.act, E, a.tile_start, a.rows_cap, D, H, 1.0f, a.d_w_down, a.status, st);
+        return grouped_wgrad(a.gYw, a.act, E, a.tile_start, nullptr, a.rows_cap, D, H, 1.0f, a.d_w_down, a.status, st);
       });
     }
   }
@@ -283,7 +297,7 @@ extern "C" int ffm_layer_backward(const ffm_layer_backward_args* args) {
   });
   if (overlap) sites.require(dx_done.order(st, gm));
   sites.run(FFM_BWD_WUP, 1, gm, [&] {
-    return grouped_wgrad(a.gU, a.Xg, E, a.tile_start, a.rows_cap, 2 * H, D, 1.0f, a.d_w_up, a.status, gm);
+    return grouped_wgrad(a.gU, a.Xg, E, a.tile_start, nullptr, a.rows_cap, 2 * H, D, 1.0f, a.d_w_up, a.status, gm);
   });
   if (overlap) {
     sites.require(join.record(gm));

@@ -342,7 +342,7 @@ int ffm::route_backward_losses(const float* gw, const float* topk_w, const int32
     // gl is [N, E] contiguous here (E % 8 == 0). dGate[e, :] = sum_n gl[n, e] hidden[n, :]
     uint8_t* base = static_cast<uint8_t*>(workspace) + align256(static_cast<size_t>(N) * ldg_ * 2);
     bf16* part = reinterpret_cast<bf16*>(base);
-    const int rc = grouped_wgrad(gl, hidden, DG_SPLITS, nullptr, N, E, D, 1.0f, part, status, stream);
+    const int rc = grouped_wgrad(gl, hidden, DG_SPLITS, nullptr, nullptr, N, E, D, 1.0f, part, status, stream);
     if (rc != FFM_OK) return rc;
     const long long total = static_cast<long long>(E) * D;
     long long blocks = (total + 255) / 256;

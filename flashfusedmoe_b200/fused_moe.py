@@ -384,6 +384,40 @@ def _require_bf16(dtype):
 # Single-GPU layer
 # ----------------------------------------------------------------------------------------------
 
+# Decode-sized calls without gradients. The GEMMs that stream weights past a few tokens (ffm_decode_gemm*) take over up to
+# this many routed rows per expert. Measured at 64 experts, K = 2048, H = 1408, up + down in us against the 128-row tiles:
+# 4 rows 131 + 75 -> 121 + 64, 32 rows 132 + 75 -> 126 + 67, 64 rows (many experts past one 64-token tile) 131 + 75 ->
+# 170 + 97.
+_DECODE_ROWS = 32
+# The shared expert as one dense group: up to one 64-token tile.
+_DECODE_SHARED_TOKENS = 64
+_FEW_TILES, _FEW_DECODE_UP, _FEW_DECODE_DOWN, _FEW_DECODE_SHARED = 1, 2, 4, 8   # FFM_FEW_*
+
+
+def _streams_weights(groups, K, n_out):
+    """Where the decode GEMM is the faster one: contractions up to 2304 and projections up to 1 GB. Beyond, its times
+    scatter with where the weights lie in memory (256 experts, 15.0 and 7.5 GB: 2415 and 1203 us with 128-row tiles, 2190 to
+    2760 and 1111 to 1600 here; 8 experts, K = 4096 and 14336: 333 and 156, here 300 to 375 and 155 to 205)."""
+    return K <= 2304 and groups * n_out * K * 2 <= 1 << 30
+
+
+def _few_rows(N, D, E, k, H, capacity, w_gate, w_up):
+    """FFM_FEW_* bits of a call without gradients: 128-row tiles that skip tiles without rows below 128 routed rows per
+    expert, decode GEMMs for a handful. (With capacity dropping the counts do not bound the rows in use.)"""
+    bits = 0
+    if w_gate is not None and N <= _DECODE_SHARED_TOKENS:
+        gap = abs(w_gate.data_ptr() - w_up.data_ptr())   # one tensor map holds both matrices
+        if 0 < gap < 1 << 40 and gap % 16 == 0:
+            bits |= _FEW_DECODE_SHARED
+    if capacity or N * k >= 128 * E:
+        return bits
+    bits |= _FEW_TILES
+    if N * k <= _DECODE_ROWS * E:
+        bits |= _FEW_DECODE_UP if _streams_weights(E, D, 2 * H) else 0
+        bits |= _FEW_DECODE_DOWN if _streams_weights(E, H, D) else 0
+    return bits
+
+
 class _FusedMoEFunction(torch.autograd.Function):
     """Routed experts on one GPU, optionally with the layer's shared expert (sw_*: its gate, up and down weights):
     its forward GEMMs run on a side stream beside routing and permute and its output is added inside the combine
@@ -416,9 +450,8 @@ class _FusedMoEFunction(torch.autograd.Function):
         if bias is not None:
             bias = ops._req(bias.to(torch.float32).contiguous(), torch.float32, "expert_bias")
         fp8 = _EXPERT_GEMM == "fp8" and D % 128 == 0 and H % 128 == 0
-        # inference with few rows per expert (decode): one CTA per 128-row tile and no work on tiles without rows
-        few = not need_grad and cfg.capacity is None and N * k < 128 * E
-        fp8 = fp8 and not few
+        few = 0 if need_grad else _few_rows(N, D, E, k, H, cfg.capacity is not None, swg, swu)
+        fp8 = fp8 and not few & _FEW_TILES
         if fp8:
             (wuq, wus), (wdq, wds) = _quantized_weight(w_up, wu), _quantized_weight(w_down, wd)
 
@@ -460,7 +493,7 @@ class _FusedMoEFunction(torch.autograd.Function):
         block = ops.LAYER_FORWARD_ARGS.pack(
             N, D, E, k, H, Hs, rows, _lib.GATING[cfg.gating], _lib.ACTIVATION[cfg.activation],
             _lib.ACTIVATION[cfg.shared_activation], 1 if cfg.pre_softmax else 0, cfg.n_group, cfg.topk_group,
-            -1 if cfg.capacity is None else cfg.capacity, 1 if need_grad else 0, 1 if few else 0, 1 if fp8 else 0,
+            -1 if cfg.capacity is None else cfg.capacity, 1 if need_grad else 0, few, 1 if fp8 else 0,
             1 if _OVERLAP else 0,
             cfg.weight_scale, cfg.aux_loss_coeff * E / (float(N) * float(N)), cfg.z_loss_coeff / float(N),
             h.data_ptr(), h_route.data_ptr(), g.data_ptr(), wu.data_ptr(), wd.data_ptr(), p(bias), p(add), p(swg), p(swu),

@@ -369,8 +369,38 @@ def dense_gemm_two(A, B1, B2):
     return out
 
 
-def grouped_gemm_wgrad(A, B, groups, tile_start, scale=1.0):
-    """dW[e] = scale * A[rows of e]^T B[rows of e]; A [rows_cap, M], B [rows_cap, N] -> [groups, M, N]."""
+def decode_gemm_glu(X, w_gate, w_up, group_rows_, groups, tile_start, counts, K, H, activation):
+    """act = glu(X Wg^T, X Wu^T) for a handful of rows per group (ffm_decode_gemm_glu); weights as in grouped_gemm_glu,
+    tile_start and counts None: one dense group."""
+    lib = _lib.load()
+    _req(X, torch.bfloat16, "X")
+    rows = X.shape[0]
+    act = torch.empty(rows, H, dtype=torch.bfloat16, device=X.device)
+    with _Launch("gemm_up_glu", 1):
+        rc = lib.ffm_decode_gemm_glu(_ptr(X), _ptr(w_gate), _ptr(w_up), group_rows_, groups, _ptr(tile_start),
+                                     _ptr(counts), rows, K, H, _lib.ACTIVATION[activation], _ptr(act),
+                                     _ptr(status_tensor(X.device)), _stream())
+    _lib.check(rc, "ffm_decode_gemm_glu")
+    return act
+
+
+def decode_gemm(X, W, groups, tile_start, counts, K, n_out):
+    """X W^T for a handful of rows per group (ffm_decode_gemm); W [groups, n_out, K]."""
+    lib = _lib.load()
+    _req(X, torch.bfloat16, "X")
+    _req(W, torch.bfloat16, "W")
+    rows = X.shape[0]
+    out = torch.empty(rows, n_out, dtype=torch.bfloat16, device=X.device)
+    with _Launch("gemm", 1):
+        rc = lib.ffm_decode_gemm(_ptr(X), _ptr(W), groups, _ptr(tile_start), _ptr(counts), rows, K, n_out, _ptr(out),
+                                 _ptr(status_tensor(X.device)), _stream())
+    _lib.check(rc, "ffm_decode_gemm")
+    return out
+
+
+def grouped_gemm_wgrad(A, B, groups, tile_start, scale=1.0, counts=None):
+    """dW[e] = scale * A[rows of e]^T B[rows of e]; A [rows_cap, M], B [rows_cap, N] -> [groups, M, N]. With counts (int32
+    [groups]) the sum ends at the last valid row, rounded up to 16, instead of the segment's end."""
     lib = _lib.load()
     _req(A, torch.bfloat16, "A")
     _req(B, torch.bfloat16, "B")
@@ -378,9 +408,9 @@ def grouped_gemm_wgrad(A, B, groups, tile_start, scale=1.0):
     n_out = B.shape[1]
     out = torch.empty(groups, M, n_out, dtype=torch.bfloat16, device=A.device)
     with _Launch("gemm_wgrad", 1):
-        rc = lib.ffm_grouped_gemm_wgrad(_ptr(A), _ptr(B), groups, _ptr(tile_start), rows_cap, M, n_out, float(scale),
-                                        _ptr(out), _ptr(status_tensor(A.device)), _stream())
-    _lib.check(rc, "ffm_grouped_gemm_wgrad")
+        rc = lib.ffm_grouped_gemm_wgrad_rows(_ptr(A), _ptr(B), groups, _ptr(tile_start), _ptr(counts), rows_cap, M, n_out,
+                                             float(scale), _ptr(out), _ptr(status_tensor(A.device)), _stream())
+    _lib.check(rc, "ffm_grouped_gemm_wgrad_rows")
     return out
 
 

@@ -199,6 +199,24 @@ int ffm_dense_gemm_two(const void* A, const void* B1, int K1, const void* B2, in
                        int32_t* status, ffm_stream_t stream);
 int ffm_grouped_gemm_wgrad(const void* A, const void* B, int groups, const int32_t* tile_start, int64_t rows_cap,
                            int M, int Nout, float scale, void* dW, int32_t* status, ffm_stream_t stream);
+/* The same with counts [groups]: the sum over a group's rows ends at its last valid row (rounded up to 16; those rows must
+ * be zero in both operands) instead of running over the padding up to the segment's end. counts may be null. */
+int ffm_grouped_gemm_wgrad_rows(const void* A, const void* B, int groups, const int32_t* tile_start,
+                                const int32_t* counts, int64_t rows_cap, int M, int Nout, float scale, void* dW,
+                                int32_t* status, ffm_stream_t stream);
+
+/* Grouped GEMMs for a handful of rows per group (decode): the launch streams the weights of the groups that hold rows and
+ * touches no others. Rows of group g are tile_start[g] * 128 ... + counts[g] (both null: one group of `rows`
+ * rows); output rows beyond counts[g] rounded up to 8 are left untouched.
+ *   _glu:     act [rows, H] = GLU(X Wg^T, X Wu^T), weights as ffm_grouped_gemm_glu; FFM_ERR_UNSUPPORTED also when w_gate and
+ *             w_up lie 2^40 bytes or more apart
+ *   (plain):  out [rows, Nout] = X W^T, W [groups, Nout, K]
+ * K % 64 == 0, H % 64 == 0, Nout % 32 == 0. */
+int ffm_decode_gemm_glu(const void* X, const void* w_gate, const void* w_up, int64_t group_rows, int groups,
+                        const int32_t* tile_start, const int32_t* counts, int64_t rows, int K, int H, int activation,
+                        void* act, int32_t* status, ffm_stream_t stream);
+int ffm_decode_gemm(const void* X, const void* W, int groups, const int32_t* tile_start, const int32_t* counts,
+                    int64_t rows, int K, int Nout, void* out, int32_t* status, ffm_stream_t stream);
 /* dAct GEMM with the GLU backward fused into its epilogue: gU [rows, 2H] = GLU backward of (gY Wd (N-major B, as
  * ffm_grouped_gemm with FFM_B_NMAJOR) rounded to bf16, preact [rows, 2H]), bit-identical to ffm_grouped_gemm followed by
  * ffm_glu_backward (reference: the bmm + activation_backward pair, fused_moe.py:520-531); dAct is never written. The
@@ -308,8 +326,8 @@ int ffm_grouped_gemm_fp8(const void* Aq, const float* a_scale, const void* Bq, c
  *
  * Forward: routing (aux = aux_scale * stats[E + 1] and z = z_scale * stats[E] when not null), capacity >= 0: dropping,
  * permute, expert GEMMs, combine; Hs > 0: a shared expert (sw_*) beside the routing, its output added in the combine.
- * need_grad: zero the padding rows and store preact / s_preact where given. few_rows: 128-row tiles that skip tiles
- * without rows. fp8: e4m3 expert GEMMs (w_*_q, w_*_scale; xq, x_scale, aq, a_scale are scratch). addend_ready: a cudaEvent_t
+ * need_grad: zero the padding rows and store preact / s_preact where given. few_rows: FFM_FEW_* bits,
+ * 128-row tiles that skip tiles without rows, and which GEMMs run as ffm_decode_gemm* (no preact then). fp8: e4m3 expert GEMMs (w_*_q, w_*_scale; xq, x_scale, aq, a_scale are scratch). addend_ready: a cudaEvent_t
  * the combine waits for, or null.
  *
  * Backward: go [N, D] and the forward pass's buffers (recompute: preact, act and Y are written here first) -> dH, d_gate,
@@ -326,6 +344,10 @@ enum { FFM_FWD_SHARED_UP, FFM_FWD_SHARED_DOWN, FFM_FWD_ROUTE, FFM_FWD_CAPACITY, 
 enum { FFM_BWD_RE_UP, FFM_BWD_RE_DOWN, FFM_BWD_COMBINE, FFM_BWD_S_DACT, FFM_BWD_S_GLU, FFM_BWD_S_WDOWN, FFM_BWD_S_SUM,
        FFM_BWD_S_DX, FFM_BWD_S_WUP, FFM_BWD_ROUTE, FFM_BWD_DACT, FFM_BWD_GLU, FFM_BWD_WDOWN, FFM_BWD_DX, FFM_BWD_WUP,
        FFM_BWD_UNPERMUTE, FFM_BWD_SITES };
+#define FFM_FEW_TILES 1
+#define FFM_FEW_DECODE_UP 2
+#define FFM_FEW_DECODE_DOWN 4
+#define FFM_FEW_DECODE_SHARED 8
 typedef struct {
   int64_t N, D, E, top_k, H, Hs, rows_cap, gating, activation, shared_activation, pre_softmax, n_group;
   int64_t topk_group, capacity, need_grad, few_rows, fp8, overlap;
