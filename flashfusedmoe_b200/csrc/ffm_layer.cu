@@ -269,7 +269,7 @@ extern "C" int ffm_layer_backward(const ffm_layer_backward_args* args) {
                                                 a.status, st);
     });
     sites.run(FFM_BWD_WDOWN, 1, st, [&] {
-      return grouped_wgrad(a.gYw, a.act, E, a.tile_start, nullptr, a.rows_cap, D, H, 1.0f, a.d_w_down, a.status, st);
+      return grouped_wgrad(a.gYw, a.act, E, a.tile_start, a.counts, a.rows_cap, D, H, 1.0f, a.d_w_down, a.status, st);
     });
   } else {
     sites.run(FFM_BWD_DACT, 1, st, [&] {
@@ -287,7 +287,7 @@ extern "C" int ffm_layer_backward(const ffm_layer_backward_args* args) {
         return ffm_glu_backward(a.d_act, a.preact, a.tile_start, E, a.rows_cap, H, act, a.gU, st);
       });
       sites.run(FFM_BWD_WDOWN, 1, st, [&] {
-        return grouped_wgrad(a.gYw, a.act, E, a.tile_start, nullptr, a.rows_cap, D, H, 1.0f, a.d_w_down, a.status, st);
+        return grouped_wgrad(a.gYw, a.act, E, a.tile_start, a.counts, a.rows_cap, D, H, 1.0f, a.d_w_down, a.status, st);
       });
     }
   }
@@ -297,7 +297,7 @@ extern "C" int ffm_layer_backward(const ffm_layer_backward_args* args) {
   });
   if (overlap) sites.require(dx_done.order(st, gm));
   sites.run(FFM_BWD_WUP, 1, gm, [&] {
-    return grouped_wgrad(a.gU, a.Xg, E, a.tile_start, nullptr, a.rows_cap, 2 * H, D, 1.0f, a.d_w_up, a.status, gm);
+    return grouped_wgrad(a.gU, a.Xg, E, a.tile_start, a.counts, a.rows_cap, 2 * H, D, 1.0f, a.d_w_up, a.status, gm);
   });
   if (overlap) {
     sites.require(join.record(gm));
