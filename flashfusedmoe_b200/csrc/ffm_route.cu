@@ -1,8 +1,8 @@
 // Routing forward for sm_100a.
 //
-//   route_gate_topk   one warp per pair of tokens: gate GEMM (fp32 accumulate, bf16 round), scoring,
-//                     iterative-argmax top-k (lowest index wins ties), renormalisation, logsumexp,
-//                     per-block expert histogram and probability-mass partial sums.
+//   route_gate_topk   gate product (fp32 accumulate, bf16 round), scoring, iterative-argmax top-k (lowest index
+//                     wins ties), renormalisation, logsumexp, per-block expert histogram and
+//                     probability-mass partial sums.
 //   route_scan        one block: per-expert exclusive scan of the block histograms, expert counts,
 //                     128-row-aligned segment starts (tile_start) and the loss statistics, all summed in a
 //                     fixed order so results do not depend on scheduling.
@@ -22,7 +22,6 @@ namespace {
 constexpr int ROUTE_THREADS = 256;
 constexpr int ROUTE_WARPS = ROUTE_THREADS / 32;
 constexpr int MAX_E = 256;
-constexpr int TPW = 2;  // tokens per warp pass
 
 // What the last routing kernel derives from the statistics: aux = aux_scale * sum_e counts[e] * mass[e],
 // z = z_scale * sum_n lse[n]^2, and a zeroed word (the count of dropped slots). Any pointer may be null.
@@ -39,9 +38,9 @@ struct RouteGrid {
   int tokens_per_block;
 };
 
-// Tokens a block of the gate kernel handles per iteration: 8 warps x 2 tokens when a warp owns all experts
-// (E <= 32), 16 / NG when the warps of a block share NG groups of 32 experts.
-int route_granule(int E) { return E <= 32 ? 16 : (E <= 64 ? 8 : (E <= 128 ? 4 : 2)); }
+// Tokens a block of the gate kernel handles per iteration, at least: 32 / slices of D with up to 32 experts, 16 / NG when
+// the warps of a block share NG groups of 32 experts.
+int route_granule(int E) { return E <= 32 ? 4 : (E <= 64 ? 8 : (E <= 128 ? 4 : 2)); }
 
 RouteGrid route_grid(long long N, int granule = 16) {
   // Contiguous token chunks, a multiple of the granule, about four blocks per SM.
@@ -98,10 +97,11 @@ struct RouteOpts {
   int topk_group;   // groups kept per token
 };
 
-// Warp arg-max of (value, expert) pairs: greater value wins, equal values go to the lower expert index.
-__device__ __forceinline__ void warp_argmax(float& best, int& best_e) {
+// Arg-max of (value, expert) pairs over W lanes: greater value wins, equal values go to the lower expert index.
+template <int W>
+__device__ __forceinline__ void lanes_argmax(float& best, int& best_e) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
+  for (int o = W / 2; o > 0; o >>= 1) {
     const float ov = __shfl_xor_sync(0xffffffffu, best, o);
     const int oe = __shfl_xor_sync(0xffffffffu, best_e, o);
     if (ov > best || (ov == best && oe < best_e)) {
@@ -111,38 +111,46 @@ __device__ __forceinline__ void warp_argmax(float& best, int& best_e) {
   }
 }
 
-// Scoring, selection, weights and statistics of one token whose bf16-rounded logits are spread over the warp:
-// lane holds expert g * 32 + lane for NG > 1 (GW == 32), expert lane % GW for NG == 1 (lanes >= GW replicate).
-template <int GW, int NG>
-__device__ __forceinline__ void route_token(const float (&logit)[NG], long long n, int lane, int E, int top_k,
+template <int W>
+__device__ __forceinline__ float lanes_sum(float v) {
+#pragma unroll
+  for (int o = W / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// Scoring, selection, weights and statistics of one token by W lanes (8, 16 or 32; 32 / W tokens per warp side by side),
+// whose bf16-rounded logits they hold: lane holds expert g * 32 + lane for NG > 1 (W == 32), expert lane % W for
+// NG == 1 (E <= W). `lane` counts within the W lanes; lanes whose token does not exist take part in the shuffles with
+// active == false and leave no trace.
+template <int W, int NG>
+__device__ __forceinline__ void route_token(const float (&logit)[NG], long long n, int lane, bool active, int E, int top_k,
                                             const RouteOpts& o, const float* __restrict__ bias,
                                             bf16* __restrict__ logits_out, float* __restrict__ topk_w,
                                             int32_t* __restrict__ topk_idx, float* __restrict__ lse_out,
                                             float (&mass)[NG], int (&cnt)[NG], float& zsum) {
-  const bool holder_lane = (NG > 1) || (lane < GW);
-  const int lane_e = (NG > 1) ? lane : (lane % GW);
+  static_assert(NG == 1 || W == 32, "one expert per lane with fewer than 32 lanes");
 
   // logsumexp over all experts (z-loss, and the normaliser of pre-softmax scoring)
   float lmax = -INFINITY;
 #pragma unroll
   for (int g = 0; g < NG; ++g) {
-    const int e = g * GW + lane_e;
-    if (holder_lane && e < E) {
+    const int e = g * 32 + lane;
+    if (e < E) {
       lmax = fmaxf(lmax, logit[g]);
-      if (logits_out != nullptr) logits_out[n * E + e] = __float2bfloat16_rn(logit[g]);
+      if (logits_out != nullptr && active) logits_out[n * E + e] = __float2bfloat16_rn(logit[g]);
     }
   }
 #pragma unroll
-  for (int s = 16; s > 0; s >>= 1) lmax = fmaxf(lmax, __shfl_xor_sync(0xffffffffu, lmax, s));
+  for (int s = W / 2; s > 0; s >>= 1) lmax = fmaxf(lmax, __shfl_xor_sync(0xffffffffu, lmax, s));
   float esum = 0.0f;
 #pragma unroll
   for (int g = 0; g < NG; ++g) {
-    const int e = g * GW + lane_e;
-    if (holder_lane && e < E) esum += __expf(logit[g] - lmax);
+    const int e = g * 32 + lane;
+    if (e < E) esum += __expf(logit[g] - lmax);
   }
-  esum = warp_sum(esum);
+  esum = lanes_sum<W>(esum);
   const float lse = lmax + __logf(esum);
-  if (lane == 0) {
+  if (lane == 0 && active) {
     lse_out[n] = lse;
     zsum += lse * lse;
   }
@@ -151,8 +159,8 @@ __device__ __forceinline__ void route_token(const float (&logit)[NG], long long 
   float val[NG];  // unbiased value that becomes the weight (logit, probability or sigmoid score)
 #pragma unroll
   for (int g = 0; g < NG; ++g) {
-    const int e = g * GW + lane_e;
-    const bool valid = holder_lane && e < E;
+    const int e = g * 32 + lane;
+    const bool valid = e < E;
     const float lg = logit[g];
     float v;
     if (o.gating == FFM_GATING_SIGMOID) {
@@ -169,7 +177,7 @@ __device__ __forceinline__ void route_token(const float (&logit)[NG], long long 
   }
   if (o.gating == FFM_GATING_SIGMOID) {
 #pragma unroll
-    for (int g = 0; g < NG; ++g) mass[g] += val[g];
+    for (int g = 0; g < NG; ++g) mass[g] += active ? val[g] : 0.0f;
   }
 
   // ---- group-limited selection: keep the topk_group groups with the best sum of their top scores ----
@@ -183,7 +191,7 @@ __device__ __forceinline__ void route_token(const float (&logit)[NG], long long 
       float tmp[NG];
 #pragma unroll
       for (int g = 0; g < NG; ++g) {
-        const int e = g * GW + lane_e;
+        const int e = g * 32 + lane;
         tmp[g] = (e / epg == gi) ? sel[g] : -INFINITY;
       }
       float score = 0.0f;
@@ -194,14 +202,14 @@ __device__ __forceinline__ void route_token(const float (&logit)[NG], long long 
         for (int g = 0; g < NG; ++g) {
           if (tmp[g] > best) {
             best = tmp[g];
-            best_e = g * GW + lane_e;
+            best_e = g * 32 + lane;
           }
         }
-        warp_argmax(best, best_e);
+        lanes_argmax<W>(best, best_e);
         score = (r == 0) ? best : score + best;
 #pragma unroll
         for (int g = 0; g < NG; ++g) {
-          if (holder_lane && g * GW + lane_e == best_e) tmp[g] = -INFINITY;
+          if (g * 32 + lane == best_e) tmp[g] = -INFINITY;
         }
       }
       if (lane == gi) my_gscore = score;
@@ -211,13 +219,13 @@ __device__ __forceinline__ void route_token(const float (&logit)[NG], long long 
     for (int r = 0; r < o.topk_group; ++r) {
       float best = gs;
       int best_l = (gs == -INFINITY) ? 0x7fffffff : lane;
-      warp_argmax(best, best_l);
+      lanes_argmax<W>(best, best_l);
       if (best_l < 32) keep |= 1u << best_l;
       if (lane == best_l) gs = -INFINITY;
     }
 #pragma unroll
     for (int g = 0; g < NG; ++g) {
-      const int e = g * GW + lane_e;
+      const int e = g * 32 + lane;
       if (!((keep >> ((e / epg) & 31)) & 1u)) sel[g] = -INFINITY;
     }
   }
@@ -232,20 +240,20 @@ __device__ __forceinline__ void route_token(const float (&logit)[NG], long long 
     for (int g = 0; g < NG; ++g) {
       if (sel[g] > best) {
         best = sel[g];
-        best_e = g * GW + lane_e;
+        best_e = g * 32 + lane;
       }
     }
-    warp_argmax(best, best_e);
+    lanes_argmax<W>(best, best_e);
     // the holder of best_e publishes the unbiased value and retires the expert
     float v_pub = 0.0f;
 #pragma unroll
     for (int g = 0; g < NG; ++g) {
-      if (holder_lane && g * GW + lane_e == best_e) {
+      if (g * 32 + lane == best_e) {
         v_pub = val[g];
         sel[g] = -INFINITY;
       }
     }
-    v_pub = __shfl_sync(0xffffffffu, v_pub, best_e & 31);
+    v_pub = __shfl_sync(0xffffffffu, v_pub, best_e & (W - 1), W);
     if (lane == j) {
       my_val = v_pub;
       my_idx = best_e;
@@ -257,28 +265,28 @@ __device__ __forceinline__ void route_token(const float (&logit)[NG], long long 
   if (o.gating == FFM_GATING_SOFTMAX && !o.pre_softmax) {
     float m = (lane < top_k) ? my_val : -INFINITY;
 #pragma unroll
-    for (int s = 16; s > 0; s >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s));
+    for (int s = W / 2; s > 0; s >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s));
     const float ex = (lane < top_k) ? __expf(my_val - m) : 0.0f;
-    const float den = warp_sum(ex);
+    const float den = lanes_sum<W>(ex);
     w = ex / den;
   } else {
     const float sc = (lane < top_k) ? my_val : 0.0f;
-    const float den = warp_sum(sc) + 1e-6f;
+    const float den = lanes_sum<W>(sc) + 1e-6f;
     w = sc / den;
   }
   w *= o.weight_scale;
-  if (lane < top_k) {
+  if (lane < top_k && active) {
     topk_w[n * top_k + lane] = w;
     topk_idx[n * top_k + lane] = my_idx;
   }
-  // ---- per-warp statistics: lane (e % 32) owns expert e ----
+  // ---- statistics: lane (e % 32) owns expert e ----
   for (int j = 0; j < top_k; ++j) {
-    const int ej = __shfl_sync(0xffffffffu, my_idx, j);
-    const float wj = __shfl_sync(0xffffffffu, w, j);
+    const int ej = __shfl_sync(0xffffffffu, my_idx, j, W);
+    const float wj = __shfl_sync(0xffffffffu, w, j, W);
     const int own_lane = (NG > 1) ? (ej & 31) : ej;
 #pragma unroll
     for (int g = 0; g < NG; ++g) {
-      if (lane == own_lane && g == ((NG > 1) ? (ej >> 5) : 0)) {
+      if (active && lane == own_lane && g == ((NG > 1) ? (ej >> 5) : 0)) {
         cnt[g] += 1;
         if (o.gating == FFM_GATING_SOFTMAX) mass[g] += wj;
       }
@@ -286,150 +294,24 @@ __device__ __forceinline__ void route_token(const float (&logit)[NG], long long 
   }
 }
 
-// Expert e = g * 32 + lane for NG > 1 (GW == 32); e = lane % GW for NG == 1.
-template <int GW, int NG>
-__global__ void __launch_bounds__(ROUTE_THREADS, (GW <= 8 ? 4 : (GW <= 16 ? 2 : 1)))
-route_gate_topk(const bf16* __restrict__ hidden, const bf16* __restrict__ gate_w, const float* __restrict__ bias,
-                long long N, int D, int E, int top_k, RouteOpts opts, int tokens_per_block,
-                bf16* __restrict__ logits_out, float* __restrict__ topk_w, int32_t* __restrict__ topk_idx,
-                float* __restrict__ lse_out, int32_t* __restrict__ block_hist, float* __restrict__ block_mass,
-                float* __restrict__ block_z, int gate_in_smem) {
-  // sized for the experts this instantiation can see, so that the few-expert variants fit beside a resident GEMM
-  __shared__ float s_mass[ROUTE_WARPS][GW * NG];
-  __shared__ int s_cnt[ROUTE_WARPS][GW * NG];
-  __shared__ float s_z[ROUTE_WARPS];
+// src[:] = -1 (padding), spread over the grid: the rank kernel later writes the rows in use.
+__device__ __forceinline__ void fill_src(int32_t* __restrict__ src, long long rows_cap) {
+  const long long step = static_cast<long long>(gridDim.x) * blockDim.x;
+  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < rows_cap; i += step) src[i] = -1;
+}
 
+// Statistics of one block, summed over its warps in warp order. Lane l holds experts g * 32 + l.
+template <int NG>
+__device__ __forceinline__ void block_statistics(float (&s_mass)[ROUTE_WARPS][NG * 32], int (&s_cnt)[ROUTE_WARPS][NG * 32],
+                                                 float (&s_z)[ROUTE_WARPS], const float (&mass)[NG],
+                                                 const int (&cnt)[NG], float zsum, int E, int32_t* __restrict__ block_hist,
+                                                 float* __restrict__ block_mass, float* __restrict__ block_z) {
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const long long tok_begin = static_cast<long long>(blockIdx.x) * tokens_per_block;
-  long long tok_end = tok_begin + tokens_per_block;
-  if (tok_end > N) tok_end = N;
-  const int chunks = D >> 3;  // 16-byte chunks per row
-
-  // Few experts (a warp owns them all): the block copies the gate matrix into shared memory once and every token's
-  // dot products read it from there. Read from global memory instead, each lane re-loads E 16-byte chunks per chunk
-  // of the token, far more loads than the 64 registers of this occupancy can keep in flight, and the kernel ran at
-  // an eighth of HBM speed.
-  extern __shared__ uint4 s_gate[];
-  if (NG == 1 && gate_in_smem) {
-    const uint4* gsrc = reinterpret_cast<const uint4*>(gate_w);
-    for (int i = threadIdx.x; i < E * chunks; i += ROUTE_THREADS) s_gate[i] = __ldg(gsrc + i);
-    __syncthreads();
-  }
-
-  float mass[NG];
-  int cnt[NG];
 #pragma unroll
   for (int g = 0; g < NG; ++g) {
-    mass[g] = 0.0f;
-    cnt[g] = 0;
-  }
-  float zsum = 0.0f;
-
-  if constexpr (NG > 1) {
-    // Many experts: the warps of a block share the gate GEMM of a few token pairs. Warp w computes the 32 experts
-    // of group (w % NG) for pair (w / NG) and leaves the logits in shared memory; then warp t routes token t of the
-    // iteration. 8 / NG pairs per iteration keep every warp busy in the GEMM phase for any NG in {2, 4, 8}.
-    constexpr int PAIRS = ROUTE_WARPS / NG;
-    __shared__ float s_logit[2 * PAIRS][NG * 32];
-    const int my_pair = warp / NG;
-    const int my_group = warp % NG;
-    for (long long it0 = tok_begin; it0 < tok_end; it0 += 2 * PAIRS) {
-      const long long t0 = it0 + 2 * my_pair;
-      if (t0 < tok_end) {
-        const bool has1 = (t0 + 1) < tok_end;
-        const uint4* h0p = reinterpret_cast<const uint4*>(hidden + t0 * D);
-        const uint4* h1p = reinterpret_cast<const uint4*>(hidden + (has1 ? t0 + 1 : t0) * D);
-        float acc0[32], acc1[32];
-#pragma unroll
-        for (int e = 0; e < 32; ++e) {
-          acc0[e] = 0.0f;
-          acc1[e] = 0.0f;
-        }
-        for (int c = lane; c < chunks; c += 32) {
-          const uint4 a0 = __ldg(h0p + c);
-          const uint4 a1 = __ldg(h1p + c);
-#pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            const int ee = my_group * 32 + e;
-            if (ee < E) {
-              const uint4 w = __ldg(reinterpret_cast<const uint4*>(gate_w + static_cast<long long>(ee) * D) + c);
-              acc0[e] = dot8(a0, w, acc0[e]);
-              acc1[e] = dot8(a1, w, acc1[e]);
-            }
-          }
-        }
-        transpose_reduce<32>(acc0, lane);
-        transpose_reduce<32>(acc1, lane);
-        s_logit[2 * my_pair][my_group * 32 + lane] = bf16_round(acc0[0]);
-        s_logit[2 * my_pair + 1][my_group * 32 + lane] = bf16_round(acc1[0]);
-      }
-      __syncthreads();
-      if (warp < 2 * PAIRS && it0 + warp < tok_end) {
-        float logit[NG];
-#pragma unroll
-        for (int g = 0; g < NG; ++g) logit[g] = s_logit[warp][g * 32 + lane];
-        route_token<GW, NG>(logit, it0 + warp, lane, E, top_k, opts, bias, logits_out, topk_w, topk_idx, lse_out, mass,
-                            cnt, zsum);
-      }
-      __syncthreads();
-    }
-  } else {
-    for (long long t0 = tok_begin + warp * TPW; t0 < tok_end; t0 += ROUTE_WARPS * TPW) {
-      const bool has1 = (t0 + 1) < tok_end;
-      const uint4* h0p = reinterpret_cast<const uint4*>(hidden + t0 * D);
-      const uint4* h1p = reinterpret_cast<const uint4*>(hidden + (has1 ? t0 + 1 : t0) * D);
-
-      // ---- gate GEMM: logit[tk][g] for expert g * 32 + lane (or lane % GW) ----
-      float logit0[NG], logit1[NG];
-  #pragma unroll
-      for (int g = 0; g < NG; ++g) {
-        float acc0[GW], acc1[GW];
-  #pragma unroll
-        for (int e = 0; e < GW; ++e) {
-          acc0[e] = 0.0f;
-          acc1[e] = 0.0f;
-        }
-        // unrolled so that the loads of several chunks are in flight together (the kernel is latency-bound)
-  #pragma unroll(GW <= 16 ? 4 : 1)
-        for (int c = lane; c < chunks; c += 32) {
-          const uint4 a0 = __ldg(h0p + c);
-          const uint4 a1 = __ldg(h1p + c);
-  #pragma unroll
-          for (int e = 0; e < GW; ++e) {
-            const int ee = g * GW + e;
-            if (ee < E) {
-              const uint4 w = gate_in_smem
-                                  ? s_gate[ee * chunks + c]
-                                  : __ldg(reinterpret_cast<const uint4*>(gate_w + static_cast<long long>(ee) * D) + c);
-              acc0[e] = dot8(a0, w, acc0[e]);
-              acc1[e] = dot8(a1, w, acc1[e]);
-            }
-          }
-        }
-        transpose_reduce<GW>(acc0, lane);
-        transpose_reduce<GW>(acc1, lane);
-        logit0[g] = bf16_round(acc0[0]);
-        logit1[g] = bf16_round(acc1[0]);
-      }
-
-      route_token<GW, NG>(logit0, t0, lane, E, top_k, opts, bias, logits_out, topk_w, topk_idx, lse_out, mass, cnt, zsum);
-      if (has1) {
-        route_token<GW, NG>(logit1, t0 + 1, lane, E, top_k, opts, bias, logits_out, topk_w, topk_idx, lse_out, mass, cnt,
-                            zsum);
-      }
-    }
-  }
-
-  // ---- block reduction in fixed warp order ----
-#pragma unroll
-  for (int g = 0; g < NG; ++g) {
-    const int e = g * GW + (NG > 1 ? lane : (lane % GW));
-    const bool holder_lane = (NG > 1) || (lane < GW);
-    if (holder_lane && e < E) {
-      s_mass[warp][e] = mass[g];
-      s_cnt[warp][e] = cnt[g];
-    }
+    s_mass[warp][g * 32 + lane] = mass[g];
+    s_cnt[warp][g * 32 + lane] = cnt[g];
   }
   if (lane == 0) s_z[warp] = zsum;
   __syncthreads();
@@ -450,6 +332,186 @@ route_gate_topk(const bf16* __restrict__ hidden, const bf16* __restrict__ gate_w
   }
 }
 
+// Up to 32 experts: gate product, scoring and top-k in one kernel. `slices` warps (1, 2, 4 or 8, by the width of a row)
+// split D for four tokens x eight experts, so that a row's chunks are all in flight at once and a block holds
+// 32 / slices tokens; the slices are summed in order, and then W lanes (E <= W) route a token, 32 / W tokens per warp side
+// by side, since that chain of shuffles is the longest part. With a token pair per warp (each lane walking a quarter to
+// a sixteenth of the row) the kernel waited for memory. Before and after: 36 -> 31 us at 16384 tokens, E = 8, D = 1024;
+// 13 -> 7 at 1999; 55 -> 48 at 8192, D = 4096; 17 -> 14 at 3001, E = 16; each with a memset of src less.
+// Registers: with 64 (E <= 8) a block fits beside a CTA of the shared expert's GEMM; at 128, four tokens per pass, it is a
+// little faster alone and 1 % slower in a layer with a shared expert.
+constexpr int GATE_TG = 4;
+constexpr int GATE_EG = 8;
+constexpr int GATE_PASS = 2;  // tokens per pass: 16 accumulators, so that the kernel also fits beside a GEMM CTA
+template <int W>
+__global__ void __launch_bounds__(ROUTE_THREADS, W == 8 ? 4 : 3)
+route_gate_topk(const bf16* __restrict__ hidden, const bf16* __restrict__ gate_w, const float* __restrict__ bias,
+                long long N, int D, int E, int top_k, RouteOpts opts, int tokens_per_block, int slices,
+                bf16* __restrict__ logits_out, float* __restrict__ topk_w, int32_t* __restrict__ topk_idx,
+                float* __restrict__ lse_out, int32_t* __restrict__ block_hist, float* __restrict__ block_mass,
+                float* __restrict__ block_z, int32_t* __restrict__ src, long long rows_cap) {
+  __shared__ float s_mass[ROUTE_WARPS][32];
+  __shared__ int s_cnt[ROUTE_WARPS][32];
+  __shared__ float s_z[ROUTE_WARPS];
+  __shared__ float s_part[ROUTE_WARPS][GATE_TG * GATE_EG];
+  __shared__ float s_logit[ROUTE_WARPS * GATE_TG][33];
+  static_assert(GATE_TG * GATE_EG <= 32, "one total per lane");
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const long long tok_begin = static_cast<long long>(blockIdx.x) * tokens_per_block;
+  long long tok_end = tok_begin + tokens_per_block;
+  if (tok_end > N) tok_end = N;
+  const int chunks = D >> 3;  // 16-byte chunks per row
+  const int groups = ROUTE_WARPS / slices;       // token groups of four per trip
+  const int slice = warp % slices;
+  const int tg = warp / slices;
+  fill_src(src, rows_cap);
+
+  float mass[1] = {0.0f};
+  int cnt[1] = {0};
+  float zsum = 0.0f;
+  for (long long it0 = tok_begin; it0 < tok_end; it0 += groups * GATE_TG) {
+    for (int e0 = 0; e0 < E; e0 += GATE_EG) {
+#pragma unroll 1
+      for (int p0 = 0; p0 < GATE_TG; p0 += GATE_PASS) {
+        const bf16* h[GATE_PASS];
+#pragma unroll
+        for (int t = 0; t < GATE_PASS; ++t) {
+          long long n = it0 + tg * GATE_TG + p0 + t;
+          if (n >= tok_end) n = tok_end - 1;  // tokens past the end repeat the last one; their logits are not used
+          h[t] = hidden + n * D;
+        }
+        float acc[GATE_PASS * GATE_EG];
+#pragma unroll
+        for (int i = 0; i < GATE_PASS * GATE_EG; ++i) acc[i] = 0.0f;
+        for (int c = slice * 32 + lane; c < chunks; c += slices * 32) {
+          uint4 hv[GATE_PASS];
+#pragma unroll
+          for (int t = 0; t < GATE_PASS; ++t) hv[t] = __ldg(reinterpret_cast<const uint4*>(h[t]) + c);
+#pragma unroll
+          for (int e = 0; e < GATE_EG; ++e) {
+            const int ee = min(e0 + e, E - 1);
+            const uint4 w = __ldg(reinterpret_cast<const uint4*>(gate_w + static_cast<long long>(ee) * D) + c);
+#pragma unroll
+            for (int t = 0; t < GATE_PASS; ++t) acc[t * GATE_EG + e] = dot8(hv[t], w, acc[t * GATE_EG + e]);
+          }
+        }
+        transpose_reduce<GATE_PASS * GATE_EG>(acc, lane);
+        if (lane < GATE_PASS * GATE_EG) s_part[warp][p0 * GATE_EG + lane] = acc[0];
+      }
+      __syncthreads();
+      if (warp < groups) {
+        float t = 0.0f;
+        for (int i = 0; i < slices; ++i) t += s_part[warp * slices + i][lane];
+        s_logit[warp * GATE_TG + lane / GATE_EG][e0 + lane % GATE_EG] = bf16_round(t);
+      }
+      __syncthreads();
+    }
+    constexpr int TPW = 32 / W;
+    const int sub = lane % W;
+    for (int t0 = warp * TPW; t0 < groups * GATE_TG && it0 + t0 < tok_end; t0 += ROUTE_WARPS * TPW) {
+      const int t = t0 + lane / W;
+      const float logit[1] = {sub < E ? s_logit[t][sub] : 0.0f};
+      route_token<W, 1>(logit, it0 + t, sub, it0 + t < tok_end, E, top_k, opts, bias, logits_out, topk_w, topk_idx, lse_out,
+                        mass, cnt, zsum);
+    }
+    __syncthreads();  // the logits are overwritten by the next trip
+  }
+  // lanes of the side-by-side tokens hold statistics of the same experts
+#pragma unroll
+  for (int o = W; o < 32; o <<= 1) {
+    mass[0] += __shfl_xor_sync(0xffffffffu, mass[0], o);
+    cnt[0] += __shfl_xor_sync(0xffffffffu, cnt[0], o);
+    zsum += __shfl_xor_sync(0xffffffffu, zsum, o);
+  }
+  block_statistics<1>(s_mass, s_cnt, s_z, mass, cnt, zsum, E, block_hist, block_mass, block_z);
+}
+
+// Slices of D for rows of D elements: one 32-lane sweep of 16-byte chunks each, at most one per warp.
+int gate_slices(int D) {
+  const int chunks = D >> 3;
+  return chunks <= 32 ? 1 : (chunks <= 64 ? 2 : (chunks <= 128 ? 4 : 8));
+}
+
+// More than 32 experts where the tensor-core gate GEMM does not apply: the warps of a block share the gate GEMM of a few
+// token pairs. Warp w computes the 32 experts of group (w % NG) for pair (w / NG) and leaves the logits in shared
+// memory; then warp t routes token t of the iteration. 8 / NG pairs per iteration keep every warp busy in the GEMM phase
+// for any NG in {2, 4, 8}. Expert e = g * 32 + lane.
+template <int NG>
+__global__ void __launch_bounds__(ROUTE_THREADS, 1)
+route_gate_topk_many(const bf16* __restrict__ hidden, const bf16* __restrict__ gate_w, const float* __restrict__ bias,
+                     long long N, int D, int E, int top_k, RouteOpts opts, int tokens_per_block,
+                     bf16* __restrict__ logits_out, float* __restrict__ topk_w, int32_t* __restrict__ topk_idx,
+                     float* __restrict__ lse_out, int32_t* __restrict__ block_hist, float* __restrict__ block_mass,
+                     float* __restrict__ block_z, int32_t* __restrict__ src, long long rows_cap) {
+  __shared__ float s_mass[ROUTE_WARPS][NG * 32];
+  __shared__ int s_cnt[ROUTE_WARPS][NG * 32];
+  __shared__ float s_z[ROUTE_WARPS];
+  constexpr int PAIRS = ROUTE_WARPS / NG;
+  __shared__ float s_logit[2 * PAIRS][NG * 32];
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const long long tok_begin = static_cast<long long>(blockIdx.x) * tokens_per_block;
+  long long tok_end = tok_begin + tokens_per_block;
+  if (tok_end > N) tok_end = N;
+  const int chunks = D >> 3;  // 16-byte chunks per row
+  fill_src(src, rows_cap);
+
+  float mass[NG];
+  int cnt[NG];
+#pragma unroll
+  for (int g = 0; g < NG; ++g) {
+    mass[g] = 0.0f;
+    cnt[g] = 0;
+  }
+  float zsum = 0.0f;
+  const int my_pair = warp / NG;
+  const int my_group = warp % NG;
+  for (long long it0 = tok_begin; it0 < tok_end; it0 += 2 * PAIRS) {
+    const long long t0 = it0 + 2 * my_pair;
+    if (t0 < tok_end) {
+      const bool has1 = (t0 + 1) < tok_end;
+      const uint4* h0p = reinterpret_cast<const uint4*>(hidden + t0 * D);
+      const uint4* h1p = reinterpret_cast<const uint4*>(hidden + (has1 ? t0 + 1 : t0) * D);
+      float acc0[32], acc1[32];
+#pragma unroll
+      for (int e = 0; e < 32; ++e) {
+        acc0[e] = 0.0f;
+        acc1[e] = 0.0f;
+      }
+      for (int c = lane; c < chunks; c += 32) {
+        const uint4 a0 = __ldg(h0p + c);
+        const uint4 a1 = __ldg(h1p + c);
+#pragma unroll
+        for (int e = 0; e < 32; ++e) {
+          const int ee = my_group * 32 + e;
+          if (ee < E) {
+            const uint4 w = __ldg(reinterpret_cast<const uint4*>(gate_w + static_cast<long long>(ee) * D) + c);
+            acc0[e] = dot8(a0, w, acc0[e]);
+            acc1[e] = dot8(a1, w, acc1[e]);
+          }
+        }
+      }
+      transpose_reduce<32>(acc0, lane);
+      transpose_reduce<32>(acc1, lane);
+      s_logit[2 * my_pair][my_group * 32 + lane] = bf16_round(acc0[0]);
+      s_logit[2 * my_pair + 1][my_group * 32 + lane] = bf16_round(acc1[0]);
+    }
+    __syncthreads();
+    if (warp < 2 * PAIRS && it0 + warp < tok_end) {
+      float logit[NG];
+#pragma unroll
+      for (int g = 0; g < NG; ++g) logit[g] = s_logit[warp][g * 32 + lane];
+      route_token<32, NG>(logit, it0 + warp, lane, true, E, top_k, opts, bias, logits_out, topk_w, topk_idx, lse_out, mass,
+                          cnt, zsum);
+    }
+    __syncthreads();
+  }
+  block_statistics<NG>(s_mass, s_cnt, s_z, mass, cnt, zsum, E, block_hist, block_mass, block_z);
+}
+
 // Scoring / top-k / statistics from logits that a GEMM already wrote (bf16 [N, E]): one warp per token, lane holds
 // experts g * 32 + lane. Used when the gate GEMM runs on the tensor cores (many experts), where a CUDA-core dot
 // product per (token, expert) would dominate the routing time.
@@ -458,15 +520,16 @@ __global__ void __launch_bounds__(ROUTE_THREADS)
 route_from_logits(const bf16* __restrict__ logits, const float* __restrict__ bias, long long N, int E, int top_k,
                   RouteOpts opts, int tokens_per_block, float* __restrict__ topk_w, int32_t* __restrict__ topk_idx,
                   float* __restrict__ lse_out, int32_t* __restrict__ block_hist, float* __restrict__ block_mass,
-                  float* __restrict__ block_z) {
-  __shared__ float s_mass[ROUTE_WARPS][MAX_E];
-  __shared__ int s_cnt[ROUTE_WARPS][MAX_E];
+                  float* __restrict__ block_z, int32_t* __restrict__ src, long long rows_cap) {
+  __shared__ float s_mass[ROUTE_WARPS][NG * 32];
+  __shared__ int s_cnt[ROUTE_WARPS][NG * 32];
   __shared__ float s_z[ROUTE_WARPS];
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const long long tok_begin = static_cast<long long>(blockIdx.x) * tokens_per_block;
   long long tok_end = tok_begin + tokens_per_block;
   if (tok_end > N) tok_end = N;
+  fill_src(src, rows_cap);
   float mass[NG];
   int cnt[NG];
 #pragma unroll
@@ -482,33 +545,9 @@ route_from_logits(const bf16* __restrict__ logits, const float* __restrict__ bia
       const int e = g * 32 + lane;
       logit[g] = (e < E) ? __bfloat162float(logits[n * E + e]) : 0.0f;
     }
-    route_token<32, NG>(logit, n, lane, E, top_k, opts, bias, nullptr, topk_w, topk_idx, lse_out, mass, cnt, zsum);
+    route_token<32, NG>(logit, n, lane, true, E, top_k, opts, bias, nullptr, topk_w, topk_idx, lse_out, mass, cnt, zsum);
   }
-#pragma unroll
-  for (int g = 0; g < NG; ++g) {
-    const int e = g * 32 + lane;
-    if (e < E) {
-      s_mass[warp][e] = mass[g];
-      s_cnt[warp][e] = cnt[g];
-    }
-  }
-  if (lane == 0) s_z[warp] = zsum;
-  __syncthreads();
-  for (int e = threadIdx.x; e < E; e += ROUTE_THREADS) {
-    float m = 0.0f;
-    int c = 0;
-    for (int w = 0; w < ROUTE_WARPS; ++w) {
-      m += s_mass[w][e];
-      c += s_cnt[w][e];
-    }
-    block_mass[static_cast<long long>(e) * gridDim.x + blockIdx.x] = m;
-    block_hist[static_cast<long long>(e) * gridDim.x + blockIdx.x] = c;
-  }
-  if (threadIdx.x == 0) {
-    float z = 0.0f;
-    for (int w = 0; w < ROUTE_WARPS; ++w) z += s_z[w];
-    block_z[blockIdx.x] = z;
-  }
+  block_statistics<NG>(s_mass, s_cnt, s_z, mass, cnt, zsum, E, block_hist, block_mass, block_z);
 }
 
 // Histogram of given expert ids with the same block chunking (expert-parallel receive side).
@@ -794,7 +833,7 @@ route_finish_small(const bf16* __restrict__ logits, const float* __restrict__ bi
       const int e = g * 32 + lane;
       logit[g] = (e < E) ? __bfloat162float(logits[static_cast<long long>(n) * E + e]) : 0.0f;
     }
-    route_token<32, NG>(logit, n, lane, E, top_k, opts, bias, nullptr, topk_w, topk_idx, lse_out, mass, cnt, zsum);
+    route_token<32, NG>(logit, n, lane, true, E, top_k, opts, bias, nullptr, topk_w, topk_idx, lse_out, mass, cnt, zsum);
   }
 #pragma unroll
   for (int g = 0; g < NG; ++g) {
@@ -918,31 +957,6 @@ RouteWorkspace carve_workspace(void* base, int blocks, int E) {
   w.block_z = reinterpret_cast<float*>(b + o_z);
   w.bytes = off;
   return w;
-}
-
-template <int GW, int NG>
-void launch_route(int blocks, cudaStream_t s, const bf16* hidden, const bf16* gate_w, const float* bias, long long N,
-                  int D, int E, int top_k, const RouteOpts& opts, int tpb, bf16* logits, float* topk_w,
-                  int32_t* topk_idx, float* lse, const RouteWorkspace& w) {
-  auto kernel = route_gate_topk<GW, NG>;
-  FFM_PREFER_MAX_SHARED(kernel);
-  // gate matrix in shared memory when a warp owns all experts, E x D bf16 fits in 64 KiB and E > 8: with up to eight
-  // experts staging gains nothing (the matrix stays hot in L1), and without it a block needs 2 KiB of shared memory
-  // and can run on an SM that holds a GEMM CTA (the shared expert's GEMMs run beside the routing kernels)
-  constexpr size_t kGateSmemMax = 64 * 1024;
-  const size_t gate_bytes = static_cast<size_t>(E) * D * sizeof(bf16);
-  static bool smem_ok = false, smem_tried = false;
-  if (NG == 1 && !smem_tried) {
-    smem_tried = true;
-    smem_ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(kGateSmemMax)) == cudaSuccess;
-    if (!smem_ok) cudaGetLastError();
-  }
-  const bool in_smem =
-      NG == 1 && E > 8 && gate_bytes <= kGateSmemMax && (gate_bytes <= 48 * 1024 || smem_ok) && D % 8 == 0;
-  route_gate_topk<GW, NG><<<blocks, ROUTE_THREADS, in_smem ? gate_bytes : 0, s>>>(
-      hidden, gate_w, bias, N, D, E, top_k, opts, tpb, logits, topk_w, topk_idx, lse, w.block_hist, w.block_mass,
-      w.block_z, in_smem ? 1 : 0);
 }
 
 template <int NG>
@@ -1095,20 +1109,20 @@ int ffm::route_forward_losses(const void* hidden, const void* gate_w, const floa
     return FFM_FINISH_CASE(8);
 #undef FFM_FINISH_CASE
   }
-  if (cudaMemsetAsync(src, 0xFF, static_cast<size_t>(rows_cap) * 4, s) != cudaSuccess) return FFM_ERR_LAUNCH;
-  const RouteGrid g = route_grid(N > 0 ? N : 1, route_granule(E));
-  RouteWorkspace w = carve_workspace(workspace, g.blocks, E);
   // Many experts: gate GEMM on the tensor cores (dense tcgen05 GEMM, fp32 accumulate, bf16 logits), then one
   // scoring kernel. Few experts: everything in one warp-level kernel.
   // (E = 32 included: one warp owning 32 experts keeps 64 accumulators per lane and ran at 0.12 TB/s)
   const bool tensor_gate = E >= 32 && D % 64 == 0 && E % 32 == 0 && logits != nullptr;
+  const RouteGrid g = route_grid(N > 0 ? N : 1, tensor_gate || E > 32 ? route_granule(E) : 32 / gate_slices(D));
+  RouteWorkspace w = carve_workspace(workspace, g.blocks, E);
   if (tensor_gate) {
     const int rc = ffm_grouped_gemm(hidden, gate_w, FFM_B_KMAJOR, 1, nullptr, N, D, E, 1.0f, logits, nullptr, 0, status,
                                     stream);
     if (rc != FFM_OK) return rc;
 #define FFM_LOGIT_CASE(NG)                                                                                      \
   route_from_logits<NG><<<g.blocks, ROUTE_THREADS, 0, s>>>(lg, expert_bias, N, E, top_k, opts, g.tokens_per_block, \
-                                                           topk_w, topk_idx, lse, w.block_hist, w.block_mass, w.block_z)
+                                                           topk_w, topk_idx, lse, w.block_hist, w.block_mass, w.block_z,  \
+                                                           src, rows_cap)
     if (E <= 64) {
       FFM_LOGIT_CASE(2);
     } else if (E <= 128) {
@@ -1118,22 +1132,31 @@ int ffm::route_forward_losses(const void* hidden, const void* gate_w, const floa
     }
 #undef FFM_LOGIT_CASE
   } else {
-#define FFM_ROUTE_CASE(GW, NG)                                                                                 \
-  launch_route<GW, NG>(g.blocks, s, h, gw, expert_bias, N, D, E, top_k, opts, g.tokens_per_block, lg, topk_w, \
-                       topk_idx, lse, w)
-  if (E <= 8) {
-    FFM_ROUTE_CASE(8, 1);
-  } else if (E <= 16) {
-    FFM_ROUTE_CASE(16, 1);
-  } else if (E <= 32) {
-    FFM_ROUTE_CASE(32, 1);
-  } else if (E <= 64) {
-    FFM_ROUTE_CASE(32, 2);
-  } else if (E <= 128) {
-    FFM_ROUTE_CASE(32, 4);
-  } else {
-    FFM_ROUTE_CASE(32, 8);
-  }
+#define FFM_ROUTE_CASE(NG)                                                                                          \
+  route_gate_topk_many<NG><<<g.blocks, ROUTE_THREADS, 0, s>>>(h, gw, expert_bias, N, D, E, top_k, opts,             \
+                                                              g.tokens_per_block, lg, topk_w, topk_idx, lse,       \
+                                                              w.block_hist, w.block_mass, w.block_z, src, rows_cap)
+    if (E <= 32) {
+#define FFM_GATE_CASE(W)                                                                                              \
+  FFM_PREFER_MAX_SHARED(route_gate_topk<W>);                                                                          \
+  route_gate_topk<W><<<g.blocks, ROUTE_THREADS, 0, s>>>(h, gw, expert_bias, N, D, E, top_k, opts, g.tokens_per_block, \
+                                                        gate_slices(D), lg, topk_w, topk_idx, lse, w.block_hist,     \
+                                                        w.block_mass, w.block_z, src, rows_cap)
+      if (E <= 8) {
+        FFM_GATE_CASE(8);
+      } else if (E <= 16) {
+        FFM_GATE_CASE(16);
+      } else {
+        FFM_GATE_CASE(32);
+      }
+#undef FFM_GATE_CASE
+    } else if (E <= 64) {
+      FFM_ROUTE_CASE(2);
+    } else if (E <= 128) {
+      FFM_ROUTE_CASE(4);
+    } else {
+      FFM_ROUTE_CASE(8);
+    }
 #undef FFM_ROUTE_CASE
   }
   FFM_PREFER_MAX_SHARED(route_scan);
