@@ -36,6 +36,11 @@ int route_backward_losses(const float* gw, const float* topk_w, const int32_t* t
 int grouped_wgrad(const void* A, const void* B, int groups, const int32_t* tile_start, const int32_t* counts,
                   int64_t rows_cap, int M, int Nout, float scale, void* dW, int32_t* status, ffm_stream_t stream);
 
+// ffm_combine_forward_add2; with status_host (host memory the device can write) a non-zero *status is stored there.
+int combine_forward_status(const void* Y, const int32_t* pos, const float* w, const void* addend, const void* addend2,
+                           int64_t N, int top_k, int D, void* out, const int32_t* status, int32_t* status_host,
+                           ffm_stream_t stream);
+
 // out = a + b, bf16 values added in fp32 (n elements, a multiple of 8)
 int add_bf16(const void* a, const void* b, int64_t n, void* out, ffm_stream_t stream);
 

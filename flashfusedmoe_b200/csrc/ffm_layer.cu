@@ -13,17 +13,20 @@ namespace ffm {
 
 namespace {
 
-// An event for one fork or join. Destroying it with the record still pending is allowed (its resources go once it is
-// done), also while the stream is being captured.
+// An event for one fork or join, created when it is first recorded. Destroying it with the record still pending is
+// allowed (its resources go once it is done), also while the stream is being captured.
 class Event {
  public:
-  Event() { ok_ = cudaEventCreateWithFlags(&e_, cudaEventDisableTiming) == cudaSuccess; }
+  Event() = default;
   ~Event() {
     if (ok_) cudaEventDestroy(e_);
   }
   Event(const Event&) = delete;
   Event& operator=(const Event&) = delete;
-  bool record(ffm_stream_t s) { return ok_ && cudaEventRecord(e_, static_cast<cudaStream_t>(s)) == cudaSuccess; }
+  bool record(ffm_stream_t s) {
+    if (!ok_) ok_ = cudaEventCreateWithFlags(&e_, cudaEventDisableTiming) == cudaSuccess;
+    return ok_ && cudaEventRecord(e_, static_cast<cudaStream_t>(s)) == cudaSuccess;
+  }
   bool wait(ffm_stream_t s) { return ok_ && cudaStreamWaitEvent(static_cast<cudaStream_t>(s), e_, 0) == cudaSuccess; }
   // `to` goes on after what `from` holds now
   bool order(ffm_stream_t from, ffm_stream_t to) { return record(from) && wait(to); }
@@ -163,7 +166,9 @@ extern "C" int ffm_layer_forward(const ffm_layer_forward_args* args) {
   }
   if (Hs > 0 && sh != st) sites.require(shared_done.wait(st));
   const void* add = Hs > 0 ? a.s_out : a.addend;
-  sites.run(FFM_FWD_COMBINE, 1, st, [&] { return ffm_combine_forward(a.Y, a.pos, a.topk_w, add, a.N, k, D, a.out, st); });
+  sites.run(FFM_FWD_COMBINE, 1, st, [&] {
+    return combine_forward_status(a.Y, a.pos, a.topk_w, add, nullptr, a.N, k, D, a.out, a.status, a.status_host, st);
+  });
   return sites.rc();
 }
 

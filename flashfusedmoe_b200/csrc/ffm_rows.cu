@@ -61,7 +61,12 @@ __device__ __forceinline__ void add_rounded(float (&acc)[8], const uint4& piece)
 __global__ void __launch_bounds__(ROW_THREADS)
 combine_forward_kernel(const bf16* __restrict__ Y, const int32_t* __restrict__ pos, const float* __restrict__ w,
                        const bf16* __restrict__ addend, const bf16* __restrict__ addend2, long long N, int top_k, int D,
-                       bf16* __restrict__ out) {
+                       bf16* __restrict__ out, const int32_t* status, volatile int32_t* status_host) {
+  // last kernel of a forward pass: a failure that some kernel before it reported goes to the caller's mapped host word
+  if (status_host != nullptr && blockIdx.x == 0 && threadIdx.x == 0) {
+    const int32_t code = *status;
+    if (code != 0) *status_host = code;
+  }
   const int lane = threadIdx.x & 31;
   const int chunks = D >> 3;
   const int cblocks = (chunks + 31) >> 5;
@@ -215,9 +220,9 @@ extern "C" int ffm_permute_rows(const void* x, const int32_t* src, int64_t rows_
   return cudaGetLastError() == cudaSuccess ? FFM_OK : FFM_ERR_LAUNCH;
 }
 
-extern "C" int ffm_combine_forward_add2(const void* Y, const int32_t* pos, const float* w, const void* addend,
-                                        const void* addend2, int64_t N, int top_k, int D, void* out,
-                                        ffm_stream_t stream) {
+int ffm::combine_forward_status(const void* Y, const int32_t* pos, const float* w, const void* addend, const void* addend2,
+                                int64_t N, int top_k, int D, void* out, const int32_t* status, int32_t* status_host,
+                                ffm_stream_t stream) {
   if (!Y || !pos || !out) return FFM_ERR_BAD_ARG;
   if (N < 0 || top_k < 1 || D <= 0) return FFM_ERR_BAD_ARG;
   if (D % 8 != 0 || top_k > 32) return FFM_ERR_UNSUPPORTED;
@@ -225,8 +230,14 @@ extern "C" int ffm_combine_forward_add2(const void* Y, const int32_t* pos, const
   FFM_PREFER_MAX_SHARED(combine_forward_kernel);
   combine_forward_kernel<<<grid_for_rows(N * ((D / 8 + 31) / 32)), ROW_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const bf16*>(Y), pos, w, static_cast<const bf16*>(addend), static_cast<const bf16*>(addend2), N, top_k,
-      D, static_cast<bf16*>(out));
+      D, static_cast<bf16*>(out), status, status_host);
   return cudaGetLastError() == cudaSuccess ? FFM_OK : FFM_ERR_LAUNCH;
+}
+
+extern "C" int ffm_combine_forward_add2(const void* Y, const int32_t* pos, const float* w, const void* addend,
+                                        const void* addend2, int64_t N, int top_k, int D, void* out,
+                                        ffm_stream_t stream) {
+  return ffm::combine_forward_status(Y, pos, w, addend, addend2, N, top_k, D, out, nullptr, nullptr, stream);
 }
 
 extern "C" int ffm_combine_forward(const void* Y, const int32_t* pos, const float* w, const void* addend, int64_t N,

@@ -462,9 +462,8 @@ class _FusedMoEFunction(torch.autograd.Function):
         aux = torch.empty((), dtype=torch.float32, device=dev)
         z = torch.empty((), dtype=torch.float32, device=dev)
         dropped = torch.empty(1, dtype=torch.int32, device=dev)
-        # kept for the backward pass: tensors of their own; everything else shares one scratch allocation. All of it is
-        # allocated on the current stream, which the side streams are forked from and joined to inside the call.
-        arena = ops.Arena()
+        # Kept for the backward pass: tensors; everything else is scratch. All of it is allocated on the current stream,
+        # which the side streams are forked from and joined to inside the call.
         routing = Xg = pre = act = Y = s_act = s_pre = None
         if need_grad:
             routing = torch.empty(rt_bytes, dtype=torch.uint8, device=dev)
@@ -472,23 +471,16 @@ class _FusedMoEFunction(torch.autograd.Function):
             if has_shared:
                 s_act = torch.empty(N, Hs, dtype=dtype, device=dev)
                 s_pre = torch.empty(N, 2 * Hs, dtype=dtype, device=dev)
-        else:
-            o_rt, o_xg = arena.take(rt_bytes), arena.take(rows * D * 2)
-            if has_shared:
-                o_sact = arena.take(N * Hs * 2)
         if keep:
             pre = torch.empty(rows, 2 * H, dtype=dtype, device=dev)
             act = torch.empty(rows, H, dtype=dtype, device=dev)
             Y = torch.empty(rows, D, dtype=dtype, device=dev)
-        else:
-            o_act, o_y = arena.take(rows * H * 2), arena.take(rows * D * 2)
-        o_sout = arena.take(N * D * 2) if has_shared else 0
-        o_ws = arena.take(ws_bytes)
-        if fp8:
-            o_xq, o_xs, o_aq, o_as = (arena.take(n) for n in (rows * D, rows * 4, rows * H, rows * 4))
-        scratch = torch.empty(arena.size, dtype=torch.uint8, device=dev)
-        base = scratch.data_ptr()
-        rt = routing.data_ptr() if need_grad else base + o_rt
+        (rt, p_xg, p_sact, p_act, p_y, p_sout, p_ws, p_xq, p_xs, p_aq, p_as), scratch = ops.scratch_buffers(dev, (
+            0 if need_grad else rt_bytes, 0 if need_grad else rows * D * 2, 0 if need_grad else N * Hs * 2,
+            0 if keep else rows * H * 2, 0 if keep else rows * D * 2, N * D * 2 if has_shared else 0, ws_bytes,
+            *((rows * D, rows * 4, rows * H, rows * 4) if fp8 else (0, 0, 0, 0))))
+        if need_grad:
+            rt = routing.data_ptr()
         p = ops._ptr
         block = ops.LAYER_FORWARD_ARGS.pack(
             N, D, E, k, H, Hs, rows, _lib.GATING[cfg.gating], _lib.ACTIVATION[cfg.activation],
@@ -499,12 +491,9 @@ class _FusedMoEFunction(torch.autograd.Function):
             h.data_ptr(), h_route.data_ptr(), g.data_ptr(), wu.data_ptr(), wd.data_ptr(), p(bias), p(add), p(swg), p(swu),
             p(swd), *((p(wuq), p(wus), p(wdq), p(wds)) if fp8 else (0, 0, 0, 0)),
             rt + o_lg, rt + o_w, rt + o_idx, rt + o_lse, counts.data_ptr(), rt + o_ts, rt + o_pos, rt + o_src, rt + o_stats,
-            aux.data_ptr(), z.data_ptr(), dropped.data_ptr(), base + o_ws, ws_bytes,
-            Xg.data_ptr() if need_grad else base + o_xg, p(pre), act.data_ptr() if keep else base + o_act,
-            Y.data_ptr() if keep else base + o_y,
-            0 if not has_shared else (s_act.data_ptr() if need_grad else base + o_sact), p(s_pre), base + o_sout,
-            *((base + o_xq, base + o_xs, base + o_aq, base + o_as) if fp8 else (0, 0, 0, 0)), out.data_ptr(),
-            p(ops.status_tensor(dev)), ops._stream(), _side_handle("shared") if has_shared and _OVERLAP else 0,
+            aux.data_ptr(), z.data_ptr(), dropped.data_ptr(), p_ws, ws_bytes, p(Xg) or p_xg, p(pre), p(act) or p_act,
+            p(Y) or p_y, p(s_act) or p_sact, p(s_pre), p_sout, p_xq, p_xs, p_aq, p_as, out.data_ptr(),
+            p(ops.status_tensor(dev)), ops.reported_word(dev), ops._stream(), _side_handle("shared") if has_shared and _OVERLAP else 0,
             0 if add is None or cfg.addend_ready is None else cfg.addend_ready.cuda_event)
         ops.layer_call(_lib.load().ffm_layer_forward, block, ops.FORWARD_SITES)
         if add is not None and cfg.addend_ready is not None:
@@ -562,20 +551,11 @@ class _FusedMoEFunction(torch.autograd.Function):
         if shared:
             s_dw, s_dwd = empty(2 * Hs, D), empty(D, Hs)
         fused = 1 if _FUSED_GLU_BWD else 0
-        arena = ops.Arena()
-        take = arena.take
-        o_gyw, o_gw, o_gu = take(rows * D * 2), take(N * k * 4), take(rows * 4 * H)
-        o_dxg, o_dhr, o_ws = take(rows * D * 2), take(N * D * 2), take(ws_bytes)
-        o_dact = 0 if fused else take(rows * H * 2)
-        o_sgu = o_sdact = o_sdx = o_sparts = 0
-        if shared:
-            o_sgu, o_sdx = take(N * Hs * 4), take(N * D * 2)
-            o_sdact = 0 if fused else take(N * Hs * 2)
-            o_sparts = take(2 * D * Hs * 2) if split == 2 else 0
-        if not ctx.kept:
-            o_pre, o_act, o_y = take(rows * H * 4), take(rows * H * 2), take(rows * D * 2)
-        scratch = torch.empty(arena.size, dtype=torch.uint8, device=dev)
-        base = scratch.data_ptr()
+        (p_gyw, p_gw, p_gu, p_dxg, p_dhr, p_ws, p_dact, p_sgu, p_sdact, p_sdx, p_sparts, p_pre, p_act,
+         p_y), scratch = ops.scratch_buffers(dev, (
+             rows * D * 2, N * k * 4, rows * 4 * H, rows * D * 2, N * D * 2, ws_bytes, 0 if fused else rows * H * 2,
+             N * Hs * 4, 0 if fused else N * Hs * 2, N * D * 2 if shared else 0, 2 * D * Hs * 2 if split == 2 else 0,
+             *((0, 0, 0) if ctx.kept else (rows * H * 4, rows * H * 2, rows * D * 2))))
         rt = routing.data_ptr()
         p = ops._ptr
         names = ("shared", "backward_route", "backward_gemm", "small")
@@ -586,11 +566,9 @@ class _FusedMoEFunction(torch.autograd.Function):
             cfg.aux_loss_coeff * E / float(N), cfg.z_loss_coeff,
             go.data_ptr(), h.data_ptr(), g.data_ptr(), wu.data_ptr(), wd.data_ptr(), p(swg), p(swu), p(swd), p(grad_aux),
             p(grad_z), rt + o_w, rt + o_idx, rt + o_lg, rt + o_lse, counts.data_ptr(), rt + o_ts, rt + o_pos, rt + o_src,
-            Xg.data_ptr(), *((pre.data_ptr(), act.data_ptr(), Y.data_ptr()) if ctx.kept else
-                             (base + o_pre, base + o_act, base + o_y)), p(s_act), p(s_pre),
-            dH.data_ptr(), d_gate.data_ptr(), d_wu.data_ptr(), d_wd.data_ptr(), p(s_dw), p(s_dwd), base + o_gyw, base + o_gw,
-            base + o_gu, base + o_dxg, base + o_dhr, base + o_dact, base + o_sgu, base + o_sdact, base + o_sdx,
-            base + o_sparts, base + o_ws, ws_bytes,
+            Xg.data_ptr(), p(pre) or p_pre, p(act) or p_act, p(Y) or p_y, p(s_act), p(s_pre),
+            dH.data_ptr(), d_gate.data_ptr(), d_wu.data_ptr(), d_wd.data_ptr(), p(s_dw), p(s_dwd), p_gyw, p_gw, p_gu,
+            p_dxg, p_dhr, p_dact, p_sgu, p_sdact, p_sdx, p_sparts, p_ws, ws_bytes,
             p(ops.status_tensor(dev)), ops._stream(), *((_side_handle(n) if _OVERLAP else 0) for n in names))
         ops.layer_call(_lib.load().ffm_layer_backward, block, ops.BACKWARD_SITES, fused_glu=bool(fused))
 
@@ -1344,6 +1322,9 @@ def fused_moe(
             out, aux, z, counts, dropped = _FusedMoEEPFunction.apply(hidden_states, gate_weight, w_up, w_down, sw[0],
                                                                      sw[1], sw[2], lw[0], lw[1], cfg, dtype)
     else:
+        # a device-side failure of an earlier call (bounded wait that ran out, bad index) raises here; no GPU wait
+        if not torch.cuda.is_current_stream_capturing():
+            ops.raise_reported(hidden_states.device)
         sh = (None, None, None)
         if _shared is not None:
             sh = tuple(_shared[:3])
@@ -1360,8 +1341,9 @@ def fused_moe(
                     f"  1. Set max_tokens_per_expert={actual_max} (or higher) via calibration\n"
                     f"  2. Set allow_dropped_tokens=True to suppress this error")
 
-    # a device-side failure of an earlier call (bounded wait that ran out, bad index) raises here; no GPU wait
-    ops.poll_status(hidden_states.device)
+    if group is not None:
+        # the same for the expert-parallel path, whose kernels end on several streams: an asynchronous copy of the word
+        ops.poll_status(hidden_states.device)
 
     losses = {}
     if aux_loss_coeff > 0.0:

@@ -129,6 +129,8 @@ def check_status(device=None):
     # an asynchronous copy of the word queued by poll_status() carries the same information: drop it, so that a failure
     # reported here is not reported a second time by a later fused_moe() call
     key = dev.index if dev.index is not None else torch.cuda.current_device()
+    if code != 0 and key in _reported:
+        _reported[key][0][0] = 0
     entry = _status_host.get(key)
     if entry is not None and entry["pending"]:
         entry["done"].synchronize()
@@ -140,6 +142,33 @@ def check_status(device=None):
 
 
 _status_host = {}
+_reported = {}   # device index -> (numpy view, address) of the pinned word that the layer's last kernel stores a failure to
+
+
+def reported_word(device):
+    """Address of the pinned host word for failures on `device` (ffm_layer_forward's status_host); 0 while a first call is
+    being captured, which allows no allocation."""
+    entry = _reported.get(device.index)
+    if entry is None:
+        if torch.cuda.is_current_stream_capturing():
+            return 0
+        word = torch.zeros(1, dtype=torch.int32).pin_memory().numpy()
+        entry = _reported[device.index] = (word, word.ctypes.data)
+    return entry[1]
+
+
+def raise_reported(device):
+    """Raise if a kernel of an earlier call on `device` reported a failure, as far as the GPU has come: the last kernel of
+    a forward pass stores it to host memory, so there is nothing to enqueue and nothing to wait for."""
+    entry = _reported.get(device.index)
+    if entry is not None and entry[0][0] != 0:
+        word = entry[0]
+        torch.cuda.synchronize(device)   # no kernel that would store the old code again is left in flight
+        code = int(word[0])
+        word[0] = 0
+        status_tensor(device).zero_()
+        raise RuntimeError(f"libffmoe device status {code}: {_lib.error_string(code)} "
+                           "(reported by a kernel of an earlier call; its results are not valid)")
 
 
 def _status_entry(dev, key):
@@ -578,7 +607,7 @@ def route_backward(gw, routing, gaux, gz, hidden, gate_w, gating, dH=None):
 
 # argument blocks as include/ffmoe.h declares them (64-bit integers and pointers, doubles in between) without the last
 # two fields, timer and launched
-LAYER_FORWARD_ARGS = struct.Struct("=18q3d44q")
+LAYER_FORWARD_ARGS = struct.Struct("=18q3d45q")
 LAYER_BACKWARD_ARGS = struct.Struct("=15q2d48q")
 
 # (timer bucket, second bucket, C call) of every launch site, in the order of the FFM_FWD_* and FFM_BWD_* enumerations
@@ -622,16 +651,27 @@ def layer_call(fn, block, sites, fused_glu=True):
         _lib.check(rc, sites[site][2] if site >= 0 else "stream fork or join")
 
 
-class Arena:
-    """Byte offsets of buffers in one allocation, 256-byte aligned."""
+# Scratch buffers from this size on are allocations of their own: one block for all of them would be larger than anything
+# a program frees again, so that the allocator could not serve it from what it holds.
+_OWN_ALLOCATION = 16 << 20
 
-    def __init__(self):
-        self.size = 0
 
-    def take(self, nbytes):
-        offset = self.size
-        self.size += (int(nbytes) + 255) // 256 * 256
-        return offset
+def scratch_buffers(device, sizes):
+    """(device addresses, the tensors that hold them) of scratch buffers of the given byte sizes, 256-byte aligned; 0 for a
+    size of 0. Small ones share one allocation."""
+    keep, where, shared = [], [], 0
+    for n in sizes:
+        if n >= _OWN_ALLOCATION:
+            keep.append(torch.empty(n, dtype=torch.uint8, device=device))
+            where.append(-keep[-1].data_ptr())
+        else:
+            where.append(shared if n else None)
+            shared += (n + 255) // 256 * 256
+    base = 0
+    if shared:
+        keep.append(torch.empty(shared, dtype=torch.uint8, device=device))
+        base = keep[-1].data_ptr()
+    return [0 if w is None else (-w if w < 0 else base + w) for w in where], keep
 
 
 @lru_cache(maxsize=1024)
@@ -646,8 +686,9 @@ def layer_sizes(N, D, E, k):
 def routing_layout(N, E, k):
     """Offsets of the routing results kept for the backward pass in one buffer: (size, topk_w, topk_idx, logits, lse,
     tile_start, pos, src, stats)."""
-    a = Arena()
     T = N * k
-    offsets = [a.take(n) for n in (T * 4, T * 4, N * E * 2, N * 4, (E + 1) * 4, T * 4, max(rows_capacity(T, E), 1) * 4,
-                                   (E + 2) * 4)]
-    return (max(a.size, 256), *offsets)
+    offsets, size = [], 0
+    for n in (T * 4, T * 4, N * E * 2, N * 4, (E + 1) * 4, T * 4, max(rows_capacity(T, E), 1) * 4, (E + 2) * 4):
+        offsets.append(size)
+        size += (n + 255) // 256 * 256
+    return (max(size, 256), *offsets)

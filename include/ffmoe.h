@@ -336,6 +336,7 @@ int ffm_grouped_gemm_fp8(const void* Aq, const float* a_scale, const void* Bq, c
  * fused_glu: GLU backward inside the dAct GEMM; else d_act / s_d_act are scratch. shared_split: 1 or 2 ranges of the tokens
  * for the shared down-projection's gradient (2: s_parts [2, D, Hs]).
  *
+ * status_host (forward): null, or mapped host memory to which the combine stores a non-zero *status.
  * timer: null, or 2 cudaEvent_t per site (FFM_FWD_* / FFM_BWD_*), recorded around the launches of the sites that run.
  * launched [3] out: kernels enqueued, bit mask of the sites that ran, the site a non-zero return code comes from.
  * ------------------------------------------------------------------------------------------------- */
@@ -372,7 +373,7 @@ typedef struct {
   void *aq;
   float *a_scale;
   void *out;
-  int32_t *status;
+  int32_t *status, *status_host;
   ffm_stream_t stream, shared_stream;
   void *addend_ready;
   const int64_t *timer;
