@@ -50,10 +50,11 @@ SIGNATURES = {
                                        c_void_p, c_void_p, c_void_p]),
     "ffm_grouped_gemm_wgrad_rows": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int64, c_int, c_int, c_float,
                                             c_void_p, c_void_p, c_void_p]),
-    "ffm_decode_gemm_glu": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int, c_void_p, c_void_p, c_int64, c_int, c_int,
-                                    c_int, c_void_p, c_void_p, c_void_p]),
-    "ffm_decode_gemm": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int64, c_int, c_int, c_void_p, c_void_p,
-                                c_void_p]),
+    "ffm_decode_up": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_void_p, c_void_p, c_int64,
+                              c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p,
+                              c_void_p]),
+    "ffm_decode_down": (c_int, [c_void_p, c_int64, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p,
+                                c_void_p, c_int64, c_int, c_void_p, c_void_p, c_void_p, c_void_p]),
     "ffm_grouped_gemm_wgrad_glu_backward": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_int64, c_int, c_int, c_float,
                                                     c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_void_p,
                                                     c_void_p, c_void_p]),

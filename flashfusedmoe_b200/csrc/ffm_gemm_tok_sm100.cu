@@ -1,11 +1,14 @@
-// Grouped GEMM for decode: out[token, feature] = x[token, :] . W[feature, :] with a handful of tokens per expert.
+// The two projections of a decode-sized call: out[token, feature] = x[token, :] . W[feature, :] with a handful of tokens
+// per expert, the shared expert as one more group of the same launch.
 //
 // Such a call streams the weights of the experts that were hit; everything else should cost nothing. The weights are the
 // M operand (128 features per CTA), the tokens of one expert the N operand (up to 64), so a tile loads, computes and stores
-// only the 16- and 8-token boxes that hold tokens. With the tokens on the M side (ffm_gemm_sm100.cu) every tile loads a
-// 128-row box of mostly unused rows beside 256 rows of weights, and stores one.
+// only the 4-, 16- and 8-token boxes that hold tokens. With the tokens on the M side (ffm_gemm_sm100.cu) every tile loads
+// a 128-row box of mostly unused rows beside 256 rows of weights, and stores one.
 // Measured, 48 tokens on 64 experts, top-6, K = 2048, H = 1408 (0.74 + 0.37 GB of weights): up + GLU 131 -> 121 us (6.0
 // TB/s), down 75 -> 64 us (5.7 TB/s); a plain read of this card's memory reaches 7.3 TB/s.
+// The up-projection can gather the token rows itself (TMA gather4, four rows per instruction), which saves the permute
+// launch and costs more than it where experts have several rows: 120 -> 132 us at 48 tokens on 64 experts, 74 -> 76 at 8.
 //
 //   warp 0      TMA producer          warp 1   MMA issuer, TMEM owner
 //   warps 2..9  epilogue: two groups of four warps (one per TMEM lane quarter) take the 32-token steps of a tile in turn
@@ -20,6 +23,7 @@
 // GLU: the gate and up rows of a weight tile are staged interleaved by 16 (one 5-D tensor map), so that lanes 0..15 of a
 // quarter hold 16 gate features and lanes 16..31 the same up features: the activation stays inside a thread.
 #include "ffm_gemm_common.cuh"
+#include "ffm_internal.h"
 
 namespace ffm {
 
@@ -43,7 +47,7 @@ constexpr int RING_BYTES = STAGES * STAGE_BYTES;
 constexpr int CTRL_BYTES = 4096;
 constexpr int TMEM_COLS = NUM_ACC * NMAX;
 
-enum { EPI_PLAIN = 0, EPI_GLU = 1 };
+enum { EPI_PLAIN = 0, EPI_GLU = 1 };  // down-projection, up-projection
 
 template <int EPI>
 struct Shape {
@@ -53,16 +57,18 @@ struct Shape {
   static_assert(SMEM_BYTES <= 232448, "tile shape does not fit in shared memory");
 };
 
+// Index 1 of the pairs: the shared expert (rows 0 .. tokens - 1), present when feats[1] > 0.
 struct TokParams {
-  const int32_t* tile_start;  // [groups + 1] first 128-row tile of every group, or null: one group at row 0
-  const int32_t* counts;      // [groups] rows of every group, or null: `rows`
+  const int32_t* tile_start;  // [groups + 1] first 128-row tile of every group
+  const int32_t* counts;      // [groups] rows of every group
+  const int32_t* src;         // up: [rows] flat slot of a grouped row, or null: the rows lie grouped
   int groups;
-  int rows;
-  int k_blocks;      // 64-deep K blocks
-  int feats;         // output features per group
-  int a_group_rows;  // plain: rows of the weight map per group
-  int swap_gate;     // GLU: the interleaved weight map holds up rows before gate rows
-  int act;
+  int top_k;
+  int tokens;
+  int k_blocks[2];   // 64-deep K blocks
+  int feats[2];      // output features per group
+  int swap_gate[2];  // up: the interleaved weight map holds up rows before gate rows
+  int act[2];
   int32_t* status;
   long long wait_cycles;
 };
@@ -74,45 +80,63 @@ struct Ctrl {
   unsigned long long acc_empty_bar[NUM_ACC];
   uint32_t tmem_base;
   int abort_flag;
+  int4 token[NMAX / 4];       // up: token rows of the producer's tile
   int base[MAX_GROUPS];       // first row of a group
   int count[MAX_GROUPS];      // rows of a group
-  int items[MAX_GROUPS + 1];  // tiles before a group
+  int items[MAX_GROUPS + 1];  // routed tiles before a group
 };
 static_assert(sizeof(Ctrl) <= CTRL_BYTES, "control block too large");
 
 struct Tile {
   int group;
+  int shared;  // 1: a tile of the shared expert
   int f_tile;
-  int row0;    // first token row
+  int row0;    // first token row (grouped, or of the tokens)
   int tokens;  // valid tokens of this tile, 1..NMAX
 };
 
-// Tiles in launch order: expert, then feature tile, token tile fastest (the token tiles of an expert share its weights
-// through L2). CTA c takes tiles c, c + grid, ...
+// Tiles in launch order: the shared expert's, then by expert and feature tile, token tile fastest (the token tiles of an
+// expert share its weights through L2). CTA c takes tile G - 1 - c first and then c + G, c + 2 G, ...: the shared expert's
+// tiles, often the longest, go to the CTAs that have no tile in a partly filled last round.
 struct Walker {
   const Ctrl* c;
-  int groups, f_tiles, cur, g, total;
+  int groups, shared_tiles, shared_nt, tokens, cur, round, g, total;
 
-  __device__ Walker(const Ctrl* ctrl, int groups_, int f_tiles_) {
+  __device__ Walker(const Ctrl* ctrl, const TokParams& p, int feats_per_tile) {
     c = ctrl;
-    groups = groups_;
-    f_tiles = f_tiles_;
-    cur = blockIdx.x;
+    groups = p.groups;
+    tokens = p.tokens;
+    shared_nt = token_tiles(tokens);
+    shared_tiles = shared_nt * ((p.feats[1] + feats_per_tile - 1) / feats_per_tile);
+    cur = gridDim.x - 1 - blockIdx.x;
+    round = 0;
     g = 0;
-    total = ctrl->items[groups_];
+    total = shared_tiles + (groups > 0 ? ctrl->items[groups] : 0);
   }
   __device__ static int token_tiles(int count) { return (count + NMAX - 1) / NMAX; }
   __device__ bool next(Tile& t) {
     if (cur >= total) return false;
-    while (g < groups - 1 && cur >= c->items[g + 1]) ++g;
-    const int nt = token_tiles(c->count[g]);
-    const int r = cur - c->items[g];
-    t.group = g;
-    t.f_tile = r / nt;
-    const int first = (r % nt) * NMAX;
-    t.row0 = c->base[g] + first;
-    t.tokens = min(NMAX, c->count[g] - first);
-    cur += gridDim.x;
+    if (cur < shared_tiles) {
+      const int first = (cur % shared_nt) * NMAX;
+      t.group = 0;
+      t.shared = 1;
+      t.f_tile = cur / shared_nt;
+      t.row0 = first;
+      t.tokens = min(NMAX, tokens - first);
+    } else {
+      const int i = cur - shared_tiles;
+      while (g < groups - 1 && i >= c->items[g + 1]) ++g;
+      const int nt = token_tiles(c->count[g]);
+      const int r = i - c->items[g];
+      const int first = (r % nt) * NMAX;
+      t.group = g;
+      t.shared = 0;
+      t.f_tile = r / nt;
+      t.row0 = c->base[g] + first;
+      t.tokens = min(NMAX, c->count[g] - first);
+    }
+    ++round;
+    cur = round * gridDim.x + blockIdx.x;
     return true;
   }
 };
@@ -151,6 +175,15 @@ __device__ __forceinline__ bool group_all(int id, bool ok) {
   return r != 0;
 }
 
+// four rows y (any order) x 64 columns from x, stored as consecutive rows; the map's box is one row high
+__device__ __forceinline__ void tma_gather4(uint32_t dst, const void* map, uint32_t bar, int x, const int4& y) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes [%0], "
+      "[%1, {%3, %4, %5, %6, %7}], [%2];" ::"r"(dst),
+      "l"(map), "r"(bar), "r"(x), "r"(y.x), "r"(y.y), "r"(y.z), "r"(y.w)
+      : "memory");
+}
+
 __device__ __forceinline__ void tma_load_5d(uint32_t dst, const void* map, uint32_t bar, int c0, int c3, int c4) {
   asm volatile(
       "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %4, %5, %6}], [%2];"
@@ -183,7 +216,9 @@ __device__ __forceinline__ void glu_step(uint32_t tcol, uint32_t box, uint32_t o
 template <int EPI>
 __global__ void __launch_bounds__(THREADS, 1)
 ffm_gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                    const __grid_constant__ CUtensorMap tmC, const __grid_constant__ TokParams p) {
+                    const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmA1,
+                    const __grid_constant__ CUtensorMap tmB1, const __grid_constant__ CUtensorMap tmC1,
+                    const __grid_constant__ TokParams p) {
   using S = Shape<EPI>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
@@ -195,7 +230,7 @@ ffm_gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int f_tiles = (p.feats + S::FEATS - 1) / S::FEATS;
+  const int f_tiles = (p.feats[0] + S::FEATS - 1) / S::FEATS;
 
   // ---- set-up ------------------------------------------------------------------------------
   if (threadIdx.x == 0) {
@@ -223,9 +258,9 @@ ffm_gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       const int g = lane * PER + i;
       mine[i] = 0;
       if (g < p.groups) {
-        const int cnt = p.counts != nullptr ? __ldg(p.counts + g) : p.rows;
+        const int cnt = __ldg(p.counts + g);
         ctrl->count[g] = cnt;
-        ctrl->base[g] = p.tile_start != nullptr ? __ldg(p.tile_start + g) * 128 : 0;
+        ctrl->base[g] = __ldg(p.tile_start + g) * 128;
         mine[i] = Walker::token_tiles(cnt) * f_tiles;
       }
       sum += mine[i];
@@ -255,39 +290,56 @@ ffm_gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 
   const uint32_t tmem_base = ctrl->tmem_base;
   volatile int* abort_flag = &ctrl->abort_flag;
-  Walker walker(ctrl, p.groups, f_tiles);
+  Walker walker(ctrl, p, S::FEATS);
   Tile t;
 
   // ---- roles -------------------------------------------------------------------------------
   if (warp == 0) {
     // ================= TMA producer =================
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      while (ok && walker.next(t)) {
-        const int f0 = t.f_tile * S::FEATS;
-        const int nb = (t.tokens + 15) & ~15;  // token rows in 16-row boxes
-        for (int kb = 0; kb < p.k_blocks; ++kb) {
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    while (ok && walker.next(t)) {
+      const int f0 = t.f_tile * S::FEATS;
+      const CUtensorMap* mA = t.shared ? &tmA1 : &tmA;
+      const CUtensorMap* mB = t.shared ? &tmB1 : &tmB;
+      const int k_blocks = p.k_blocks[t.shared];
+      // token rows staged: gathered in fours (the last four repeat the last token), or in boxes of 16
+      const bool gather = EPI == EPI_GLU && p.src != nullptr && !t.shared;
+      const int nb = gather ? (t.tokens + 3) & ~3 : (t.tokens + 15) & ~15;
+      if (gather) {
+        for (int i = lane; i < nb; i += 32) {
+          reinterpret_cast<int*>(ctrl->token)[i] = __ldg(p.src + t.row0 + min(i, t.tokens - 1)) / p.top_k;
+        }
+        __syncwarp();
+      }
+      if (lane == 0) {
+        for (int kb = 0; kb < k_blocks; ++kb) {
           ok = mbar_wait_bounded(smem_u32(&ctrl->empty_bar[stage]), phase ^ 1u, abort_flag, p.status,
                                  FFM_STATUS_WAIT_PRODUCER, p.wait_cycles);
           if (!ok) break;
           const uint32_t full = smem_u32(&ctrl->full_bar[stage]);
           const uint32_t a_dst = smem_base + stage * STAGE_BYTES;
+          const uint32_t b_dst = a_dst + A_BYTES;
           mbar_expect_tx(full, A_BYTES + nb * 128);
           const int k0 = kb * BK;
           if (EPI == EPI_GLU) {
-            tma_load_5d(a_dst, &tmA, full, k0, f0 / 16, t.group);
+            tma_load_5d(a_dst, mA, full, k0, f0 / 16, t.group);
           } else {
-            tma_load_2d(a_dst, &tmA, full, k0, t.group * p.a_group_rows + f0);
+            tma_load_2d(a_dst, mA, full, k0, t.group * p.feats[0] + f0);
           }
-          for (int r = 0; r < nb; r += 16) tma_load_2d(a_dst + A_BYTES + r * 128, &tmB, full, k0, t.row0 + r);
+          if (gather) {
+            for (int r = 0; r < nb; r += 4) tma_gather4(b_dst + r * 128, mB, full, k0, ctrl->token[r >> 2]);
+          } else {
+            for (int r = 0; r < nb; r += 16) tma_load_2d(b_dst + r * 128, mB, full, k0, t.row0 + r);
+          }
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1u;
           }
         }
       }
+      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;  // also: the token list is overwritten only after its last use
     }
   } else if (warp == 1) {
     // ================= MMA issuer =================
@@ -304,7 +356,8 @@ ffm_gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * NMAX;
-        for (int kb = 0; kb < p.k_blocks; ++kb) {
+        const int k_blocks = p.k_blocks[t.shared];
+        for (int kb = 0; kb < k_blocks; ++kb) {
           ok = mbar_wait_bounded(smem_u32(&ctrl->full_bar[stage]), phase, abort_flag, p.status, FFM_STATUS_WAIT_MMA,
                                  p.wait_cycles);
           if (!ok) break;
@@ -356,8 +409,8 @@ ffm_gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * NMAX + c0;
         if (EPI == EPI_GLU) {
           const uint32_t o = box_offset(m_row, quarter * 2 + m_chunk);
-          const bool swap = p.swap_gate != 0;
-          switch (p.act) {
+          const bool swap = p.swap_gate[t.shared] != 0;
+          switch (p.act[t.shared]) {
             case FFM_ACT_SWIGLU: glu_step<FFM_ACT_SWIGLU>(taddr, buf, o, swap); break;
             case FFM_ACT_GEGLU_TANH: glu_step<FFM_ACT_GEGLU_TANH>(taddr, buf, o, swap); break;
             case FFM_ACT_RELU2: glu_step<FFM_ACT_RELU2>(taddr, buf, o, swap); break;
@@ -386,10 +439,11 @@ ffm_gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         group_sync(bar_id);
         if (storer) {
           const int rows = min(STEP_TOKENS, t.tokens - c0);
+          const CUtensorMap* mC = t.shared ? &tmC1 : &tmC;
           for (int r = 0; r < rows; r += STORE_ROWS) {
-            tma_store_3d(&tmC, buf + r * 128, f0, t.row0 + c0 + r, 0);
-            if (EPI == EPI_PLAIN && f0 + 64 < p.feats) {
-              tma_store_3d(&tmC, buf + BOX_BYTES + r * 128, f0 + 64, t.row0 + c0 + r, 0);
+            tma_store_3d(mC, buf + r * 128, f0, t.row0 + c0 + r, 0);
+            if (EPI == EPI_PLAIN && f0 + 64 < p.feats[t.shared]) {
+              tma_store_3d(mC, buf + BOX_BYTES + r * 128, f0 + 64, t.row0 + c0 + r, 0);
             }
           }
           bulk_commit();
@@ -451,13 +505,8 @@ int make_glu_weight_map(CUtensorMap* map, const void* lo, long long gap, int K, 
   return r == CUDA_SUCCESS ? FFM_OK : FFM_ERR_LAUNCH;
 }
 
-bool bad_groups(int groups, const int32_t* tile_start, const int32_t* counts, long long rows) {
-  if (groups < 1 || groups > MAX_GROUPS || rows < 0 || rows > (1LL << 30)) return true;
-  return (tile_start == nullptr) != (counts == nullptr) || (counts == nullptr && groups != 1);
-}
-
 template <int EPI>
-int launch_tok(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const TokParams& p, cudaStream_t stream) {
+int launch_tok(const CUtensorMap (&m)[6], const TokParams& p, long long rows, cudaStream_t stream) {
   using S = Shape<EPI>;
   static bool ready = false;
   auto kernel = ffm_gemm_tok_kernel<EPI>;
@@ -468,12 +517,41 @@ int launch_tok(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap
     }
     ready = true;
   }
-  // no more CTAs than there can be tiles: every group may end in a partly filled token tile
-  const long long f_tiles = (p.feats + S::FEATS - 1) / S::FEATS;
-  long long ctas = (p.rows / NMAX + p.groups) * f_tiles;
+  // no more CTAs than there can be tiles: every group may end in a partly filled token tile, and every routed row may be
+  // alone in its group
+  long long tiles = rows / NMAX + p.groups;
+  if (tiles > static_cast<long long>(p.tokens) * p.top_k) tiles = static_cast<long long>(p.tokens) * p.top_k;
+  long long ctas = tiles * ((p.feats[0] + S::FEATS - 1) / S::FEATS) +
+                   (p.tokens + NMAX - 1) / NMAX * ((p.feats[1] + S::FEATS - 1) / S::FEATS);
   if (ctas > num_sms()) ctas = num_sms();
-  kernel<<<static_cast<unsigned>(ctas), THREADS, S::SMEM_BYTES, stream>>>(tmA, tmB, tmC, p);
+  kernel<<<static_cast<unsigned>(ctas), THREADS, S::SMEM_BYTES, stream>>>(m[0], m[1], m[2], m[3], m[4], m[5], p);
   return cudaGetLastError() == cudaSuccess ? FFM_OK : FFM_ERR_LAUNCH;
+}
+
+// the maps of an absent part are never used, but the kernel prefetches their descriptors
+void fill_missing(CUtensorMap (&m)[6], bool routed, bool shared) {
+  for (int i = 0; i < 3; ++i) {
+    if (!routed) m[i] = m[i + 3];
+    if (!shared) m[i + 3] = m[i];
+  }
+}
+
+// weight map, output map and parameters of one GLU (routed or shared) of the up-projection
+int up_side(CUtensorMap* tmA, CUtensorMap* tmC, TokParams* p, int i, const void* w_gate, const void* w_up, int groups,
+            long long group_bytes, int D, int H, int activation, void* act, long long rows) {
+  const uint8_t* g = static_cast<const uint8_t*>(w_gate);
+  const uint8_t* u = static_cast<const uint8_t*>(w_up);
+  const bool up_low = reinterpret_cast<uintptr_t>(u) < reinterpret_cast<uintptr_t>(g);
+  const long long gap = static_cast<long long>(up_low ? reinterpret_cast<uintptr_t>(g) - reinterpret_cast<uintptr_t>(u)
+                                                      : reinterpret_cast<uintptr_t>(u) - reinterpret_cast<uintptr_t>(g));
+  // a tensor map's strides are multiples of 16 bytes below 2^40
+  if (H % 64 != 0 || gap == 0 || gap % 16 != 0 || gap >= (1LL << 40)) return FFM_ERR_UNSUPPORTED;
+  if (activation < 0 || activation > 3) return FFM_ERR_BAD_ARG;
+  p->feats[i] = H;
+  p->swap_gate[i] = up_low ? 1 : 0;
+  p->act[i] = activation;
+  const int rc = make_glu_weight_map(tmA, up_low ? u : g, gap, D, H, groups, group_bytes);
+  return rc != FFM_OK ? rc : make_store_map(tmC, act, rows, H);
 }
 
 }  // namespace
@@ -482,60 +560,82 @@ int launch_tok(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap
 
 using namespace ffm;
 
-extern "C" int ffm_decode_gemm_glu(const void* X, const void* w_gate, const void* w_up, int64_t group_rows, int groups,
-                                   const int32_t* tile_start, const int32_t* counts, int64_t rows, int K, int H,
-                                   int activation, void* act, int32_t* status, ffm_stream_t stream) {
-  if (!X || !w_gate || !w_up || !act || !status || bad_groups(groups, tile_start, counts, rows)) return FFM_ERR_BAD_ARG;
-  if (K <= 0 || H <= 0 || group_rows < H) return FFM_ERR_BAD_ARG;
-  if (activation < 0 || activation > 3) return FFM_ERR_BAD_ARG;
-  const uint8_t* g = static_cast<const uint8_t*>(w_gate);
-  const uint8_t* u = static_cast<const uint8_t*>(w_up);
-  const bool up_low = reinterpret_cast<uintptr_t>(u) < reinterpret_cast<uintptr_t>(g);
-  const long long gap = static_cast<long long>(up_low ? reinterpret_cast<uintptr_t>(g) - reinterpret_cast<uintptr_t>(u)
-                                                      : reinterpret_cast<uintptr_t>(u) - reinterpret_cast<uintptr_t>(g));
-  // a tensor map's strides are multiples of 16 bytes below 2^40
-  if (K % 64 != 0 || H % 64 != 0 || gap == 0 || gap % 16 != 0 || gap >= (1LL << 40)) return FFM_ERR_UNSUPPORTED;
-  if (rows == 0) return FFM_OK;
-  CUtensorMap tmA, tmB, tmC;
-  int rc;
-  if ((rc = make_glu_weight_map(&tmA, up_low ? u : g, gap, K, H, groups, group_rows * K * 2)) != FFM_OK) return rc;
-  if ((rc = make_map_2d(&tmB, X, rows, K, 64, 16)) != FFM_OK) return rc;
-  if ((rc = make_store_map(&tmC, act, rows, H)) != FFM_OK) return rc;
-  TokParams p = {};
-  p.tile_start = tile_start;
-  p.counts = counts;
-  p.groups = groups;
-  p.rows = static_cast<int>(rows);
-  p.k_blocks = K / BK;
-  p.feats = H;
-  p.swap_gate = up_low ? 1 : 0;
-  p.act = activation;
-  p.status = status;
-  p.wait_cycles = gemm_wait_cycles();
-  return launch_tok<EPI_GLU>(tmA, tmB, tmC, p, static_cast<cudaStream_t>(stream));
+// groups == 0: the shared expert alone
+static bool bad_decode(int64_t N, int D, int H, int Hs, int top_k, int groups, const int32_t* tile_start,
+                       const int32_t* counts, int64_t rows, const int32_t* status) {
+  if (!status || N < 1 || N > (1LL << 30) || D <= 0 || Hs < 0 || top_k < 1) return true;
+  if (groups < 0 || groups > MAX_GROUPS || rows < 0 || rows > (1LL << 30)) return true;
+  if (groups == 0) return Hs == 0;
+  return !tile_start || !counts || H <= 0 || rows < 1;
 }
 
-extern "C" int ffm_decode_gemm(const void* X, const void* W, int groups, const int32_t* tile_start, const int32_t* counts,
-                               int64_t rows, int K, int Nout, void* out, int32_t* status, ffm_stream_t stream) {
-  if (!X || !W || !out || !status || bad_groups(groups, tile_start, counts, rows)) return FFM_ERR_BAD_ARG;
-  if (K <= 0 || Nout <= 0) return FFM_ERR_BAD_ARG;
-  if (K % 64 != 0 || Nout % 32 != 0) return FFM_ERR_UNSUPPORTED;
-  if (static_cast<long long>(groups) * Nout > 0x7fffffffLL) return FFM_ERR_UNSUPPORTED;
-  if (rows == 0) return FFM_OK;
-  CUtensorMap tmA, tmB, tmC;
-  int rc;
-  if ((rc = make_map_2d(&tmA, W, static_cast<long long>(groups) * Nout, K, 64, 128)) != FFM_OK) return rc;
-  if ((rc = make_map_2d(&tmB, X, rows, K, 64, 16)) != FFM_OK) return rc;
-  if ((rc = make_store_map(&tmC, out, rows, Nout)) != FFM_OK) return rc;
+extern "C" int ffm_decode_up(const void* x, const int32_t* src, const void* hidden, int64_t N, int D, int top_k, int groups,
+                             const int32_t* tile_start, const int32_t* counts, int64_t rows, const void* w_up, int H,
+                             int activation, void* act, const void* sw_gate, const void* sw_up, int Hs,
+                             int shared_activation, void* s_act, int32_t* status, ffm_stream_t stream) {
+  if (bad_decode(N, D, H, Hs, top_k, groups, tile_start, counts, rows, status)) return FFM_ERR_BAD_ARG;
+  if (groups > 0 && (!x || !w_up || !act)) return FFM_ERR_BAD_ARG;
+  if (Hs > 0 && (!hidden || !sw_gate || !sw_up || !s_act)) return FFM_ERR_BAD_ARG;
+  if (D % 64 != 0) return FFM_ERR_UNSUPPORTED;
   TokParams p = {};
+  CUtensorMap m[6];
+  int rc;
+  if (groups > 0) {
+    const long long half = static_cast<long long>(H) * D * 2;
+    if ((rc = up_side(&m[0], &m[2], &p, 0, w_up, static_cast<const uint8_t*>(w_up) + half, groups, 2 * half, D, H,
+                      activation, act, rows)) != FFM_OK) return rc;
+    if ((rc = make_map_2d(&m[1], x, src != nullptr ? N : rows, D, 64, src != nullptr ? 1 : 16)) != FFM_OK) return rc;
+  }
+  if (Hs > 0) {
+    if ((rc = up_side(&m[3], &m[5], &p, 1, sw_gate, sw_up, 1, static_cast<long long>(Hs) * D * 2, D, Hs, shared_activation,
+                      s_act, N)) != FFM_OK) return rc;
+    if ((rc = make_map_2d(&m[4], hidden, N, D, 64, 16)) != FFM_OK) return rc;
+  }
+  fill_missing(m, groups > 0, Hs > 0);
+  p.tile_start = tile_start;
+  p.counts = counts;
+  p.src = src;
+  p.groups = groups;
+  p.top_k = top_k;
+  p.tokens = static_cast<int>(N);
+  p.k_blocks[0] = p.k_blocks[1] = D / BK;
+  p.status = status;
+  p.wait_cycles = gemm_wait_cycles();
+  return launch_tok<EPI_GLU>(m, p, rows, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int ffm_decode_down(const void* act, int64_t rows, int H, int groups, const int32_t* tile_start,
+                               const int32_t* counts, int top_k, const void* w_down, int D, void* Y, const void* s_act,
+                               int64_t N, int Hs, const void* sw_down, void* s_out, int32_t* status, ffm_stream_t stream) {
+  if (bad_decode(N, D, H, Hs, top_k, groups, tile_start, counts, rows, status)) return FFM_ERR_BAD_ARG;
+  if (groups > 0 && (!act || !w_down || !Y)) return FFM_ERR_BAD_ARG;
+  if (Hs > 0 && (!s_act || !sw_down || !s_out)) return FFM_ERR_BAD_ARG;
+  if ((groups > 0 && H % 64 != 0) || Hs % 64 != 0 || D % 32 != 0) return FFM_ERR_UNSUPPORTED;
+  if (static_cast<long long>(groups) * D > 0x7fffffffLL) return FFM_ERR_UNSUPPORTED;
+  TokParams p = {};
+  CUtensorMap m[6];
+  int rc;
+  if (groups > 0) {
+    if ((rc = make_map_2d(&m[0], w_down, static_cast<long long>(groups) * D, H, 64, 128)) != FFM_OK) return rc;
+    if ((rc = make_map_2d(&m[1], act, rows, H, 64, 16)) != FFM_OK) return rc;
+    if ((rc = make_store_map(&m[2], Y, rows, D)) != FFM_OK) return rc;
+    p.k_blocks[0] = H / BK;
+    p.feats[0] = D;
+  }
+  if (Hs > 0) {
+    if ((rc = make_map_2d(&m[3], sw_down, D, Hs, 64, 128)) != FFM_OK) return rc;
+    if ((rc = make_map_2d(&m[4], s_act, N, Hs, 64, 16)) != FFM_OK) return rc;
+    if ((rc = make_store_map(&m[5], s_out, N, D)) != FFM_OK) return rc;
+    p.k_blocks[1] = Hs / BK;
+    p.feats[1] = D;
+  }
+  fill_missing(m, groups > 0, Hs > 0);
   p.tile_start = tile_start;
   p.counts = counts;
   p.groups = groups;
-  p.rows = static_cast<int>(rows);
-  p.k_blocks = K / BK;
-  p.feats = Nout;
-  p.a_group_rows = Nout;
+  p.top_k = top_k;
+  p.tokens = static_cast<int>(N);
   p.status = status;
   p.wait_cycles = gemm_wait_cycles();
-  return launch_tok<EPI_PLAIN>(tmA, tmB, tmC, p, static_cast<cudaStream_t>(stream));
+  return launch_tok<EPI_PLAIN>(m, p, rows, static_cast<cudaStream_t>(stream));
 }

@@ -88,20 +88,25 @@ extern "C" int ffm_layer_forward(const ffm_layer_forward_args* args) {
   Sites sites(a.timer, a.launched);
   Event fork, shared_done;
 
-  // shared expert: beside the routing kernels, which leave the tensor cores idle
-  if (Hs > 0) {
+  // shared expert: beside the routing kernels, which leave the tensor cores idle; in a decode-sized call it is one more
+  // group of the expert GEMMs
+  const bool one_chain = (a.few_rows & FFM_FEW_ONE_CHAIN) != 0;
+  const bool shared_inside = Hs > 0 && one_chain;
+  const bool shared_beside = Hs > 0 && !shared_inside;
+  if (shared_beside) {
     if (sh != st) sites.require(fork.order(st, sh));
     sites.run(FFM_FWD_SHARED_UP, 1, sh, [&] {
       if (a.few_rows & FFM_FEW_DECODE_SHARED) {
-        return ffm_decode_gemm_glu(a.hidden, a.sw_gate, a.sw_up, Hs, 1, nullptr, nullptr, a.N, D, Hs,
-                                   static_cast<int>(a.shared_activation), a.s_act, a.status, sh);
+        return ffm_decode_up(nullptr, nullptr, a.hidden, a.N, D, k, 0, nullptr, nullptr, 0, nullptr, 0, 0, nullptr, a.sw_gate,
+                             a.sw_up, Hs, static_cast<int>(a.shared_activation), a.s_act, a.status, sh);
       }
       return ffm_grouped_gemm_glu(a.hidden, a.sw_gate, a.sw_up, Hs, 1, nullptr, a.N, D, Hs,
                                   static_cast<int>(a.shared_activation), a.s_act, a.s_preact, nullptr, 0, a.status, sh);
     });
     sites.run(FFM_FWD_SHARED_DOWN, 1, sh, [&] {
       if (a.few_rows & FFM_FEW_DECODE_SHARED) {
-        return ffm_decode_gemm(a.s_act, a.sw_down, 1, nullptr, nullptr, a.N, Hs, D, a.s_out, a.status, sh);
+        return ffm_decode_down(nullptr, 0, 0, 0, nullptr, nullptr, k, nullptr, D, nullptr, a.s_act, a.N, Hs, a.sw_down,
+                               a.s_out, a.status, sh);
       }
       return ffm_grouped_gemm(a.s_act, a.sw_down, FFM_B_KMAJOR, 1, nullptr, a.N, Hs, D, 1.0f, a.s_out, nullptr, 0,
                               a.status, sh);
@@ -126,9 +131,11 @@ extern "C" int ffm_layer_forward(const ffm_layer_forward_args* args) {
   // Without a backward pass nothing sums over the padding rows, so they are not zeroed -- except with capacity dropping: a
   // dropped slot keeps its grouped row (now a padding row) with weight 0, and 0 * (whatever the GEMMs make of
   // uninitialised memory, possibly NaN) would reach the output through the combine.
-  sites.run(FFM_FWD_PERMUTE, 1, st, [&] {
-    return ffm_permute_rows(a.hidden, a.src, a.rows_cap, k, D, a.need_grad || a.capacity >= 0 ? 1 : 0, a.Xg, st);
-  });
+  if (!one_chain) {
+    sites.run(FFM_FWD_PERMUTE, 1, st, [&] {
+      return ffm_permute_rows(a.hidden, a.src, a.rows_cap, k, D, a.need_grad || a.capacity >= 0 ? 1 : 0, a.Xg, st);
+    });
+  }
   const int32_t* valid = (a.few_rows & FFM_FEW_TILES) ? a.counts : nullptr;
   const int tile_rows = (a.few_rows & FFM_FEW_TILES) ? 128 : 0;
   if (a.fp8) {
@@ -146,15 +153,17 @@ extern "C" int ffm_layer_forward(const ffm_layer_forward_args* args) {
     const void* up_rows = static_cast<const char*>(a.w_up) + a.H * a.D * 2;
     sites.run(FFM_FWD_UP, 1, st, [&] {
       if (a.few_rows & FFM_FEW_DECODE_UP) {
-        return ffm_decode_gemm_glu(a.Xg, a.w_up, up_rows, 2 * a.H, E, a.tile_start, a.counts, a.rows_cap, D, H, act, a.act,
-                                   a.status, st);
+        return ffm_decode_up(one_chain ? a.hidden : a.Xg, one_chain ? a.src : nullptr, a.hidden, a.N, D, k, E, a.tile_start,
+                             a.counts, a.rows_cap, a.w_up, H, act, a.act, a.sw_gate, a.sw_up, shared_inside ? Hs : 0,
+                             static_cast<int>(a.shared_activation), a.s_act, a.status, st);
       }
       return ffm_grouped_gemm_glu(a.Xg, a.w_up, up_rows, 2 * a.H, E, a.tile_start, a.rows_cap, D, H, act, a.act, a.preact,
                                   valid, tile_rows, a.status, st);
     });
     sites.run(FFM_FWD_DOWN, 1, st, [&] {
       if (a.few_rows & FFM_FEW_DECODE_DOWN) {
-        return ffm_decode_gemm(a.act, a.w_down, E, a.tile_start, a.counts, a.rows_cap, H, D, a.Y, a.status, st);
+        return ffm_decode_down(a.act, a.rows_cap, H, E, a.tile_start, a.counts, k, a.w_down, D, a.Y, a.s_act, a.N,
+                               shared_inside ? Hs : 0, a.sw_down, a.s_out, a.status, st);
       }
       return ffm_grouped_gemm(a.act, a.w_down, FFM_B_KMAJOR, E, a.tile_start, a.rows_cap, H, D, 1.0f, a.Y, valid, tile_rows,
                               a.status, st);
@@ -164,7 +173,7 @@ extern "C" int ffm_layer_forward(const ffm_layer_forward_args* args) {
     sites.require(cudaStreamWaitEvent(static_cast<cudaStream_t>(st), static_cast<cudaEvent_t>(a.addend_ready), 0) ==
                   cudaSuccess);
   }
-  if (Hs > 0 && sh != st) sites.require(shared_done.wait(st));
+  if (shared_beside && sh != st) sites.require(shared_done.wait(st));
   const void* add = Hs > 0 ? a.s_out : a.addend;
   sites.run(FFM_FWD_COMBINE, 1, st, [&] {
     return combine_forward_status(a.Y, a.pos, a.topk_w, add, nullptr, a.N, k, D, a.out, a.status, a.status_host, st);

@@ -384,14 +384,20 @@ def _require_bf16(dtype):
 # Single-GPU layer
 # ----------------------------------------------------------------------------------------------
 
-# Decode-sized calls without gradients. The GEMMs that stream weights past a few tokens (ffm_decode_gemm*) take over up to
-# this many routed rows per expert. Measured at 64 experts, K = 2048, H = 1408, up + down in us against the 128-row tiles:
+# Decode-sized calls without gradients. The GEMMs that stream weights past a few tokens (ffm_decode_*) take over up to this
+# many routed rows per expert. Measured at 64 experts, K = 2048, H = 1408, up + down in us against the 128-row tiles:
 # 4 rows 131 + 75 -> 121 + 64, 32 rows 132 + 75 -> 126 + 67, 64 rows (many experts past one 64-token tile) 131 + 75 ->
 # 170 + 97.
 _DECODE_ROWS = 32
-# The shared expert as one dense group: up to one 64-token tile.
+# The shared expert runs in the same kernels up to one 64-token tile (14 + 17 us instead of 18 + 20 at 48 tokens, D = 2048,
+# Hs = 2816).
 _DECODE_SHARED_TOKENS = 64
-_FEW_TILES, _FEW_DECODE_UP, _FEW_DECODE_DOWN, _FEW_DECODE_SHARED = 1, 2, 4, 8   # FFM_FEW_*
+# Up to this many bytes of weights a call is over before the host has issued it: one chain of launches, with the token
+# rows gathered in the up-projection instead of a permute, and the shared expert inside the two GEMMs instead of beside
+# them. One token, 8 experts and a shared one (0.11 GB): 98 -> 86 us. Above, where the GPU is the slower side, both cost: 48
+# tokens on 64 experts and a shared one (1.15 GB) 212 -> 238 us.
+_ONE_CHAIN_BYTES = 256 << 20
+_FEW_TILES, _FEW_DECODE_UP, _FEW_DECODE_DOWN, _FEW_DECODE_SHARED, _FEW_ONE_CHAIN = 1, 2, 4, 8, 16   # FFM_FEW_*
 
 
 def _streams_weights(groups, K, n_out):
@@ -405,16 +411,21 @@ def _few_rows(N, D, E, k, H, capacity, w_gate, w_up):
     """FFM_FEW_* bits of a call without gradients: 128-row tiles that skip tiles without rows below 128 routed rows per
     expert, decode GEMMs for a handful. (With capacity dropping the counts do not bound the rows in use.)"""
     bits = 0
-    if w_gate is not None and N <= _DECODE_SHARED_TOKENS:
+    Hs = 0
+    if w_gate is not None and 0 < N <= _DECODE_SHARED_TOKENS:
+        Hs = w_gate.shape[0]
         gap = abs(w_gate.data_ptr() - w_up.data_ptr())   # one tensor map holds both matrices
         if 0 < gap < 1 << 40 and gap % 16 == 0:
             bits |= _FEW_DECODE_SHARED
     if capacity or N * k >= 128 * E:
         return bits
     bits |= _FEW_TILES
-    if N * k <= _DECODE_ROWS * E:
+    if 0 < N * k <= _DECODE_ROWS * E:
         bits |= _FEW_DECODE_UP if _streams_weights(E, D, 2 * H) else 0
         bits |= _FEW_DECODE_DOWN if _streams_weights(E, H, D) else 0
+        both = _FEW_DECODE_UP | _FEW_DECODE_DOWN
+        if bits & both == both and (w_gate is None or bits & _FEW_DECODE_SHARED):
+            bits |= _FEW_ONE_CHAIN if 6 * D * (E * H + Hs) <= _ONE_CHAIN_BYTES else 0
     return bits
 
 
@@ -493,7 +504,7 @@ class _FusedMoEFunction(torch.autograd.Function):
             rt + o_lg, rt + o_w, rt + o_idx, rt + o_lse, counts.data_ptr(), rt + o_ts, rt + o_pos, rt + o_src, rt + o_stats,
             aux.data_ptr(), z.data_ptr(), dropped.data_ptr(), p_ws, ws_bytes, p(Xg) or p_xg, p(pre), p(act) or p_act,
             p(Y) or p_y, p(s_act) or p_sact, p(s_pre), p_sout, p_xq, p_xs, p_aq, p_as, out.data_ptr(),
-            p(ops.status_tensor(dev)), ops.reported_word(dev), ops._stream(), _side_handle("shared") if has_shared and _OVERLAP else 0,
+            p(ops.status_tensor(dev)), ops.reported_word(dev), ops._stream(), _side_handle("shared") if has_shared and _OVERLAP and not few & _FEW_ONE_CHAIN else 0,
             0 if add is None or cfg.addend_ready is None else cfg.addend_ready.cuda_event)
         ops.layer_call(_lib.load().ffm_layer_forward, block, ops.FORWARD_SITES)
         if add is not None and cfg.addend_ready is not None:

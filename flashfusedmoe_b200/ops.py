@@ -398,33 +398,50 @@ def dense_gemm_two(A, B1, B2):
     return out
 
 
-def decode_gemm_glu(X, w_gate, w_up, group_rows_, groups, tile_start, counts, K, H, activation):
-    """act = glu(X Wg^T, X Wu^T) for a handful of rows per group (ffm_decode_gemm_glu); weights as in grouped_gemm_glu,
-    tile_start and counts None: one dense group."""
+def decode_up(x, src, top_k, tile_start, counts, rows, w_up, activation, shared=None):
+    """act [rows, H] of a decode-sized call (ffm_decode_up) from grouped rows x (src None) or from tokens x gathered through
+    src; shared = (hidden, gate, up, activation) adds a shared expert over all tokens. w_up None: the shared expert alone.
+    Returns (act, shared act), None where absent."""
     lib = _lib.load()
-    _req(X, torch.bfloat16, "X")
-    rows = X.shape[0]
-    act = torch.empty(rows, H, dtype=torch.bfloat16, device=X.device)
+    hidden, gate, up, s_activation = shared if shared is not None else (None, None, None, activation)
+    for name, t in (("x", x), ("w_up", w_up), ("hidden", hidden), ("gate", gate), ("up", up)):
+        if t is not None:
+            _req(t, torch.bfloat16, name)
+    some = x if x is not None else hidden
+    D = some.shape[1]
+    N = hidden.shape[0] if hidden is not None else (x.shape[0] if src is not None else max(rows // top_k, 1))
+    E, H = (w_up.shape[0], w_up.shape[1] // 2) if w_up is not None else (0, 0)
+    act = torch.empty(rows, H, dtype=torch.bfloat16, device=some.device) if E else None
+    Hs = 0 if gate is None else gate.shape[0]
+    s_act = torch.empty(N, Hs, dtype=torch.bfloat16, device=some.device) if Hs else None
     with _Launch("gemm_up_glu", 1):
-        rc = lib.ffm_decode_gemm_glu(_ptr(X), _ptr(w_gate), _ptr(w_up), group_rows_, groups, _ptr(tile_start),
-                                     _ptr(counts), rows, K, H, _lib.ACTIVATION[activation], _ptr(act),
-                                     _ptr(status_tensor(X.device)), _stream())
-    _lib.check(rc, "ffm_decode_gemm_glu")
-    return act
+        rc = lib.ffm_decode_up(_ptr(x), _ptr(src), _ptr(hidden), N, D, top_k, E, _ptr(tile_start), _ptr(counts), rows,
+                               _ptr(w_up), H, _lib.ACTIVATION[activation], _ptr(act), _ptr(gate), _ptr(up), Hs,
+                               _lib.ACTIVATION[s_activation], _ptr(s_act), _ptr(status_tensor(some.device)), _stream())
+    _lib.check(rc, "ffm_decode_up")
+    return act, s_act
 
 
-def decode_gemm(X, W, groups, tile_start, counts, K, n_out):
-    """X W^T for a handful of rows per group (ffm_decode_gemm); W [groups, n_out, K]."""
+def decode_down(act, tile_start, counts, top_k, N, w_down, shared=None):
+    """Y [rows, D] = act w_down^T per expert for a decode-sized call of N tokens (ffm_decode_down); shared = (act, weights)
+    of a shared expert. w_down None: the shared expert alone. Returns (Y, shared output), None where absent."""
     lib = _lib.load()
-    _req(X, torch.bfloat16, "X")
-    _req(W, torch.bfloat16, "W")
-    rows = X.shape[0]
-    out = torch.empty(rows, n_out, dtype=torch.bfloat16, device=X.device)
+    s_act, s_down = shared if shared is not None else (None, None)
+    for name, t in (("act", act), ("w_down", w_down), ("shared act", s_act), ("shared down", s_down)):
+        if t is not None:
+            _req(t, torch.bfloat16, name)
+    some = act if act is not None else s_act
+    rows, H = act.shape if act is not None else (0, 0)
+    E, D = w_down.shape[:2] if w_down is not None else (0, s_down.shape[0])
+    Y = torch.empty(rows, D, dtype=torch.bfloat16, device=some.device) if E else None
+    Hs = 0 if s_act is None else s_act.shape[1]
+    s_out = torch.empty(N, D, dtype=torch.bfloat16, device=some.device) if Hs else None
     with _Launch("gemm", 1):
-        rc = lib.ffm_decode_gemm(_ptr(X), _ptr(W), groups, _ptr(tile_start), _ptr(counts), rows, K, n_out, _ptr(out),
-                                 _ptr(status_tensor(X.device)), _stream())
-    _lib.check(rc, "ffm_decode_gemm")
-    return out
+        rc = lib.ffm_decode_down(_ptr(act), rows, H, E, _ptr(tile_start), _ptr(counts), top_k, _ptr(w_down), D, _ptr(Y),
+                                 _ptr(s_act), N, Hs, _ptr(s_down), _ptr(s_out), _ptr(status_tensor(some.device)),
+                                 _stream())
+    _lib.check(rc, "ffm_decode_down")
+    return Y, s_out
 
 
 def grouped_gemm_wgrad(A, B, groups, tile_start, scale=1.0, counts=None):

@@ -205,18 +205,22 @@ int ffm_grouped_gemm_wgrad_rows(const void* A, const void* B, int groups, const 
                                 const int32_t* counts, int64_t rows_cap, int M, int Nout, float scale, void* dW,
                                 int32_t* status, ffm_stream_t stream);
 
-/* Grouped GEMMs for a handful of rows per group (decode): the launch streams the weights of the groups that hold rows and
- * touches no others. Rows of group g are tile_start[g] * 128 ... + counts[g] (both null: one group of `rows`
- * rows); output rows beyond counts[g] rounded up to 8 are left untouched.
- *   _glu:     act [rows, H] = GLU(X Wg^T, X Wu^T), weights as ffm_grouped_gemm_glu; FFM_ERR_UNSUPPORTED also when w_gate and
- *             w_up lie 2^40 bytes or more apart
- *   (plain):  out [rows, Nout] = X W^T, W [groups, Nout, K]
- * K % 64 == 0, H % 64 == 0, Nout % 32 == 0. */
-int ffm_decode_gemm_glu(const void* X, const void* w_gate, const void* w_up, int64_t group_rows, int groups,
-                        const int32_t* tile_start, const int32_t* counts, int64_t rows, int K, int H, int activation,
-                        void* act, int32_t* status, ffm_stream_t stream);
-int ffm_decode_gemm(const void* X, const void* W, int groups, const int32_t* tile_start, const int32_t* counts,
-                    int64_t rows, int K, int Nout, void* out, int32_t* status, ffm_stream_t stream);
+/* The two projections of a decode-sized call (a handful of routed rows per group): the launch streams the weights of the
+ * groups that hold rows and touches no others. Rows of group g are tile_start[g] * 128 ... + counts[g]; output rows beyond
+ * counts[g] rounded up to 8 are left untouched. Hs > 0 adds a shared expert over all N tokens to the same launch.
+ *   ffm_decode_up:   act [rows, H] = GLU(x[r] W^T), w_up [groups, 2H, D] (gate rows, then up rows). src null: x [rows, D]
+ *                    holds the grouped rows; else x [N, D] the tokens, and row r is token src[r] / top_k (gathered, no
+ *                    permute needed). s_act [N, Hs] from hidden [N, D] and sw_gate, sw_up [Hs, D].
+ *   ffm_decode_down: Y [rows, D] = act W^T, w_down [groups, D, H]; s_out [N, D] = s_act sw_down^T, sw_down [D, Hs].
+ * groups == 0: the shared expert alone. D, H, Hs multiples of 64. FFM_ERR_UNSUPPORTED also when sw_gate and sw_up lie 2^40
+ * bytes or more apart. */
+int ffm_decode_up(const void* x, const int32_t* src, const void* hidden, int64_t N, int D, int top_k, int groups,
+                  const int32_t* tile_start, const int32_t* counts, int64_t rows, const void* w_up, int H, int activation,
+                  void* act, const void* sw_gate, const void* sw_up, int Hs, int shared_activation, void* s_act,
+                  int32_t* status, ffm_stream_t stream);
+int ffm_decode_down(const void* act, int64_t rows, int H, int groups, const int32_t* tile_start, const int32_t* counts,
+                    int top_k, const void* w_down, int D, void* Y, const void* s_act, int64_t N, int Hs,
+                    const void* sw_down, void* s_out, int32_t* status, ffm_stream_t stream);
 /* dAct GEMM with the GLU backward fused into its epilogue: gU [rows, 2H] = GLU backward of (gY Wd (N-major B, as
  * ffm_grouped_gemm with FFM_B_NMAJOR) rounded to bf16, preact [rows, 2H]), bit-identical to ffm_grouped_gemm followed by
  * ffm_glu_backward (reference: the bmm + activation_backward pair, fused_moe.py:520-531); dAct is never written. The
@@ -327,7 +331,9 @@ int ffm_grouped_gemm_fp8(const void* Aq, const float* a_scale, const void* Bq, c
  * Forward: routing (aux = aux_scale * stats[E + 1] and z = z_scale * stats[E] when not null), capacity >= 0: dropping,
  * permute, expert GEMMs, combine; Hs > 0: a shared expert (sw_*) beside the routing, its output added in the combine.
  * need_grad: zero the padding rows and store preact / s_preact where given. few_rows: FFM_FEW_* bits,
- * 128-row tiles that skip tiles without rows, and which GEMMs run as ffm_decode_gemm* (no preact then). fp8: e4m3 expert GEMMs (w_*_q, w_*_scale; xq, x_scale, aq, a_scale are scratch). addend_ready: a cudaEvent_t
+ * 128-row tiles that skip tiles without rows; which projections, and whether the shared expert, run as ffm_decode_up (no
+ * preact) and ffm_decode_down; ONE_CHAIN (with all of those): no permute, and the shared expert inside the two launches.
+ * fp8: e4m3 expert GEMMs (w_*_q, w_*_scale; xq, x_scale, aq, a_scale are scratch). addend_ready: a cudaEvent_t
  * the combine waits for, or null.
  *
  * Backward: go [N, D] and the forward pass's buffers (recompute: preact, act and Y are written here first) -> dH, d_gate,
@@ -349,6 +355,7 @@ enum { FFM_BWD_RE_UP, FFM_BWD_RE_DOWN, FFM_BWD_COMBINE, FFM_BWD_S_DACT, FFM_BWD_
 #define FFM_FEW_DECODE_UP 2
 #define FFM_FEW_DECODE_DOWN 4
 #define FFM_FEW_DECODE_SHARED 8
+#define FFM_FEW_ONE_CHAIN 16
 typedef struct {
   int64_t N, D, E, top_k, H, Hs, rows_cap, gating, activation, shared_activation, pre_softmax, n_group;
   int64_t topk_group, capacity, need_grad, few_rows, fp8, overlap;

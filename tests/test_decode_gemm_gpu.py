@@ -1,5 +1,5 @@
 """GEMMs of decode-sized calls and weight gradients that end at the last valid row, against torch in fp32, at the edges of
-their tiles: 8- and 16-row boxes, the 64-token tile, several token tiles per expert, features that do not fill a tile,
+their tiles: 4-, 8- and 16-row boxes, the 64-token tile, several token tiles per expert, features that do not fill a tile,
 empty experts.
 
 Bounds: products of bf16 values are exact in fp32, so an output differs from the fp32 evaluation by its own rounding to
@@ -78,48 +78,79 @@ def valid(starts):
     return [(e, slice(s, s + c)) for e, (c, s) in enumerate(zip(COUNTS, starts)) if c]
 
 
-@pytest.mark.parametrize("K,Nout", [(64, 32), (192, 128), (128, 288), (1024, 320)])
-def test_decode_gemm(K, Nout, monkeypatch):
-    g = torch.Generator(device=DEV).manual_seed(K + Nout)
+@pytest.mark.parametrize("H,D", [(64, 32), (192, 128), (128, 288), (1024, 320)])
+def test_decode_down(H, D, monkeypatch):
+    g = torch.Generator(device=DEV).manual_seed(H + D)
     ts, cn, starts, rows = layout(COUNTS)
-    x = grouped(COUNTS, starts, rows, K, g)
-    w = torch.randn(len(COUNTS), Nout, K, generator=g, device=DEV).bfloat16()
-    out = with_sentinel(monkeypatch, lambda: ops.decode_gemm(x, w, len(COUNTS), ts, cn, K, Nout))
+    N, k = sum(COUNTS), 1
+    x = grouped(COUNTS, starts, rows, H, g)
+    w = torch.randn(len(COUNTS), D, H, generator=g, device=DEV).bfloat16()
+    out, none = with_sentinel(monkeypatch, lambda: ops.decode_down(x, ts, cn, k, N, w))
+    assert none is None
     for e, r in valid(starts):
         check(out[r], x[r].float() @ w[e].float().T, x[r].float().abs() @ w[e].float().abs().T)
     untouched(out, starts)
 
 
 @pytest.mark.parametrize("activation", ["swiglu", "geglu", "relu_squared", "geglu_erf"])
-@pytest.mark.parametrize("K,H", [(64, 64), (192, 128), (576, 320)])
-def test_decode_gemm_glu(K, H, activation, monkeypatch):
-    g = torch.Generator(device=DEV).manual_seed(K + H)
+@pytest.mark.parametrize("D,H,k", [(64, 64, 1), (192, 128, 3), (576, 320, 2)])
+def test_decode_up(D, H, k, activation, monkeypatch):
+    """Token rows gathered through src, every token in several experts."""
+    g = torch.Generator(device=DEV).manual_seed(D + H)
     ts, cn, starts, rows = layout(COUNTS)
-    x = grouped(COUNTS, starts, rows, K, g)
-    w = (torch.randn(len(COUNTS), 2 * H, K, generator=g, device=DEV) * 0.2).bfloat16()
-    act = with_sentinel(monkeypatch, lambda: ops.decode_gemm_glu(x, w, w.view(-1, K)[H:], 2 * H, len(COUNTS), ts, cn, K,
-                                                                 H, activation))
+    T = sum(COUNTS)
+    N = -(-T // k)
+    slots = torch.randperm(N * k, generator=g, device=DEV)[:T].int()
+    src = torch.full((rows,), -1, dtype=torch.int32, device=DEV)
+    at = 0
+    for c, s in zip(COUNTS, starts):
+        src[s:s + c] = slots[at:at + c]
+        at += c
+    hidden = torch.randn(N, D, generator=g, device=DEV).bfloat16()
+    w = (torch.randn(len(COUNTS), 2 * H, D, generator=g, device=DEV) * 0.2).bfloat16()
+    act, none = with_sentinel(monkeypatch, lambda: ops.decode_up(hidden, src, k, ts, cn, rows, w, activation))
+    assert none is None
     for e, r in valid(starts):
-        check_glu(act[r], x[r].float() @ w[e].float().T, H, activation, x[r].float().abs() @ w[e].float().abs().T)
+        x = hidden[(src[r] // k).long()].float()
+        check_glu(act[r], x @ w[e].float().T, H, activation, x.abs() @ w[e].float().abs().T)
     untouched(act, starts)
-
-
-@pytest.mark.parametrize("rows", [1, 8, 33, 64, 100])
-@pytest.mark.parametrize("swap", [False, True])
-def test_dense(rows, swap):
-    """The shared expert: separate gate and up tensors in either address order, row counts that are no multiple of 8."""
-    g = torch.Generator(device=DEV).manual_seed(rows)
-    K, H = 128, 192
-    pair = (torch.randn(2, H, K, generator=g, device=DEV) * 0.2).bfloat16()
-    wg, wu = (pair[1], pair[0]) if swap else (pair[0], pair[1])
-    x = torch.randn(rows, K, generator=g, device=DEV).bfloat16()
-    act = ops.decode_gemm_glu(x, wg, wu, H, 1, None, None, K, H, "swiglu")
-    both = torch.cat([wg, wu]).float()
-    check_glu(act, x.float() @ both.T, H, "swiglu", x.float().abs() @ both.abs().T)
-    w = torch.randn(K, H, generator=g, device=DEV).bfloat16()
-    out = ops.decode_gemm(act, w, 1, None, None, H, K)
+    rows_grouped = torch.full((rows, D), float("nan"), device=DEV).bfloat16()
+    for _, r in valid(starts):
+        rows_grouped[r] = hidden[(src[r] // k).long()]
+    same, _ = ops.decode_up(rows_grouped, None, k, ts, cn, rows, w, activation)
     ops.check_status()
-    check(out, act.float() @ w.float().T, act.float().abs() @ w.float().abs().T)
+    for _, r in valid(starts):
+        assert torch.equal(same[r], act[r])
+
+
+@pytest.mark.parametrize("N", [1, 3, 17, 64, 100])
+@pytest.mark.parametrize("swap", [False, True])
+def test_shared_expert_inside(N, swap):
+    """Separate gate and up tensors in either address order, other widths than the routed experts, row counts that are no
+    multiple of 8; the routed outputs are those of a launch without it."""
+    g = torch.Generator(device=DEV).manual_seed(N)
+    D, H, Hs, E, k = 128, 64, 192, 5, 2
+    hidden = torch.randn(N, D, generator=g, device=DEV).bfloat16()
+    r = ops.route_forward(hidden, torch.randn(E, D, generator=g, device=DEV).bfloat16(), k)
+    wu = (torch.randn(E, 2 * H, D, generator=g, device=DEV) * 0.2).bfloat16()
+    wd = torch.randn(E, D, H, generator=g, device=DEV).bfloat16()
+    pair = (torch.randn(2, Hs, D, generator=g, device=DEV) * 0.2).bfloat16()
+    wg, wup = (pair[1], pair[0]) if swap else (pair[0], pair[1])
+    sd = torch.randn(D, Hs, generator=g, device=DEV).bfloat16()
+    act, s_act = ops.decode_up(hidden, r.src, k, r.tile_start, r.counts, r.rows_cap, wu, "swiglu",
+                               (hidden, wg, wup, "geglu_erf"))
+    alone, _ = ops.decode_up(hidden, r.src, k, r.tile_start, r.counts, r.rows_cap, wu, "swiglu")
+    Y, s_out = ops.decode_down(act, r.tile_start, r.counts, k, N, wd, (s_act, sd))
+    Y1, _ = ops.decode_down(act, r.tile_start, r.counts, k, N, wd)
+    _, s_alone = ops.decode_up(None, None, k, None, None, 0, None, "swiglu", (hidden, wg, wup, "geglu_erf"))
+    _, o_alone = ops.decode_down(None, None, None, k, N, None, (s_act, sd))
+    assert torch.equal(s_alone, s_act) and torch.equal(o_alone, s_out)
+    ops.check_status()
+    rows = r.pos.long()
+    assert torch.equal(act[rows], alone[rows]) and torch.equal(Y[rows], Y1[rows])
+    both = torch.cat([wg, wup]).float()
+    check_glu(s_act, hidden.float() @ both.T, Hs, "geglu_erf", hidden.float().abs() @ both.abs().T)
+    check(s_out, s_act.float() @ sd.float().T, s_act.float().abs() @ sd.float().abs().T)
 
 
 @pytest.mark.parametrize("M,Nout", [(64, 64), (192, 320)])
