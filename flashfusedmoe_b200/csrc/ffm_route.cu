@@ -256,7 +256,7 @@ __device__ __forceinline__ void route_token(const float (&logit)[NG], long long 
     v_pub = __shfl_sync(0xffffffffu, v_pub, best_e & (W - 1), W);
     if (lane == j) {
       my_val = v_pub;
-      my_idx = best_e;
+      my_idx = best_e < E ? best_e : -1;  // -1: nothing compares greater than -inf (NaN scores)
     }
   }
 
@@ -707,10 +707,7 @@ route_rank(const int32_t* __restrict__ ids, long long T, int E, int slots_per_bl
     const long long i = i0 + lane;
     const bool active = i < we;
     int e = active ? ids[i] : -1;
-    if (active && (e < 0 || e >= E)) {
-      atomicCAS(status, 0, FFM_STATUS_BAD_INDEX);
-      e = -1;
-    }
+    if (e < 0 || e >= E) e = -1;
     const unsigned same = __match_any_sync(0xffffffffu, e);
     const int leader = __ffs(same) - 1;
     const int rank = __popc(same & ((1u << lane) - 1u));
@@ -721,10 +718,11 @@ route_rank(const int32_t* __restrict__ ids, long long T, int E, int slots_per_bl
     }
     base = __shfl_sync(0xffffffffu, base, leader);
     __syncwarp();
-    if (e >= 0) {
+    if (active) {
       const long long r = static_cast<long long>(base) + rank;
-      if (r < rows_cap) {
-        pos[i] = static_cast<int32_t>(r);
+      const bool placed = e >= 0 && r < rows_cap;
+      pos[i] = placed ? static_cast<int32_t>(r) : -1;
+      if (placed) {
         src[r] = static_cast<int32_t>(i);
       } else {
         atomicCAS(status, 0, FFM_STATUS_BAD_INDEX);
@@ -906,10 +904,7 @@ route_finish_small(const bf16* __restrict__ logits, const float* __restrict__ bi
     const int i = i0 + lane;
     const bool active = i < we;
     int e = active ? __ldcg(topk_idx + i) : -1;
-    if (active && (e < 0 || e >= E)) {
-      atomicCAS(status, 0, FFM_STATUS_BAD_INDEX);
-      e = -1;
-    }
+    if (e < 0 || e >= E) e = -1;
     const unsigned same = __match_any_sync(0xffffffffu, e);
     const int leader = __ffs(same) - 1;
     const int rank = __popc(same & ((1u << lane) - 1u));
@@ -920,10 +915,11 @@ route_finish_small(const bf16* __restrict__ logits, const float* __restrict__ bi
     }
     base = __shfl_sync(0xffffffffu, base, leader);
     __syncwarp();
-    if (e >= 0) {
+    if (active) {
       const int r = base + rank;
-      if (r < rows_cap) {
-        pos[i] = r;
+      const bool placed = e >= 0 && r < rows_cap;
+      pos[i] = placed ? r : -1;
+      if (placed) {
         src[r] = i;
       } else {
         atomicCAS(status, 0, FFM_STATUS_BAD_INDEX);
@@ -1079,6 +1075,7 @@ int ffm::route_forward_losses(const void* hidden, const void* gate_w, const floa
   if (D % 8 != 0 || E > MAX_E || top_k > E || top_k > 32) return FFM_ERR_UNSUPPORTED;
   if (n_group < 0 || (n_group > 0 && (topk_group < 1 || topk_group > n_group))) return FFM_ERR_BAD_ARG;
   if (n_group > 32 || (n_group > 0 && E % n_group != 0)) return FFM_ERR_UNSUPPORTED;
+  if (n_group > 0 && topk_group * (E / n_group) < top_k) return FFM_ERR_BAD_ARG;  // the kept groups hold fewer experts
   if (rows_cap < ffm_rows_capacity(N * top_k, E)) return FFM_ERR_BAD_ARG;
   RouteOpts opts;
   opts.gating = gating;
@@ -1236,19 +1233,24 @@ compact_positions_kernel(const int32_t* __restrict__ pos, const int32_t* __restr
                          const int32_t* __restrict__ counts, const int32_t* __restrict__ tile_start, long long T, int E,
                          int32_t* __restrict__ cpos, int32_t* __restrict__ src_c) {
   __shared__ int s_shift[MAX_E];  // padded position minus compact position for rows of expert e
+  __shared__ int s_rows;          // slots with a row: all T unless some have no expert
   if (threadIdx.x == 0) {
     int before = 0;
     for (int e = 0; e < E; ++e) {
       s_shift[e] = tile_start[e] * 128 - before;
       before += counts[e];
     }
+    s_rows = before;
   }
   __syncthreads();
   const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i < T) {
-    const int c = pos[i] - s_shift[topk_idx[i]];
+    const int e = topk_idx[i];
+    const bool placed = e >= 0 && e < E && pos[i] >= 0;
+    const int c = placed ? pos[i] - s_shift[e] : -1;
     cpos[i] = c;
-    src_c[c] = static_cast<int32_t>(i);
+    if (placed) src_c[c] = static_cast<int32_t>(i);
+    if (i >= s_rows) src_c[i] = -1;
   }
 }
 

@@ -51,7 +51,10 @@ route_bwd_token(const float* __restrict__ gw, const float* __restrict__ topk_w, 
       g = gw[n * top_k + lane];
       s = topk_w[n * top_k + lane];
       idx = topk_idx[n * top_k + lane];
-      if (idx < 0 || idx >= E) idx = -1;
+      if (idx < 0 || idx >= E) {
+        idx = -1;
+        g = NAN;  // a slot without an expert has no row that gw could come from
+      }
     }
     float gtl;
     if (gating == FFM_GATING_SOFTMAX) {

@@ -677,6 +677,7 @@ class _EPPlan:
             return self.px.exchange(rows, cnt, region, dry=_EP_DRY_EXCHANGE), True
         in_splits = cnt[self.rank]
         out_splits = [cnt[s][self.rank] for s in range(self.ep)]
+        rows = rows[:sum(in_splits)]  # slots without an expert (NaN scores) have no row to send
         if _EP_DRY_EXCHANGE:
             return rows.new_zeros(sum(out_splits), rows.shape[1]), False
         ops.a2a_bytes_sent += (sum(in_splits) - in_splits[self.rank]) * rows.shape[1] * rows.element_size()
@@ -1305,6 +1306,8 @@ def fused_moe(
     use_groups = n_group is not None and topk_group is not None
     if use_groups:
         assert E % n_group == 0, f"E ({E}) must be divisible by n_group ({n_group})"
+        assert topk_group * (E // n_group) >= top_k, \
+            f"topk_group ({topk_group}) groups of {E // n_group} experts hold fewer than top_k ({top_k})"
     capacity = None
     if capacity_factor is not None and group is None:
         capacity = max(int((N / E) * capacity_factor), top_k)  # fused_moe.py:352-353

@@ -19,7 +19,10 @@
  *   expert's tokens and the next multiple of 256 are zero. Buffers hold ffm_rows_capacity(T, E) rows.
  *     tile_start[E + 1]  int32  cumulative count of 128-row tiles per expert, always even
  *                               (tile_start[E] = tiles in use)
- *     pos[T]             int32  grouped row of flat slot i = n * k + j          (reference: expand_to_batch)
+ *     pos[T]             int32  grouped row of flat slot i = n * k + j          (reference: expand_to_batch);
+ *                               -1 for a slot without an expert: topk_idx is -1 where no score is greater than
+ *                               -inf (NaN logits). Such a slot sets FFM_STATUS_BAD_INDEX, and every output and
+ *                               gradient row that sums over it is NaN
  *     src[rows_cap]      int32  flat slot held by a grouped row, -1 for padding (reference: sorted_order)
  */
 #ifndef FFMOE_H_
@@ -244,7 +247,8 @@ int ffm_grouped_gemm_wgrad_glu_backward(const void* A, const void* B, int groups
 /* -------------------------------------------------------------------------------------------------
  * Combine forward: out[n, :] = sum_j w[n, j] * Y[pos[n k + j], :] (+ addend[n, :]), fp32 accumulation.
  * w (f32) is rounded to bf16 before the multiply, as the reference does (fused_moe.py:412); w == NULL
- * means 1. Replaces fused_gather_reduce (kernels/moe_ops.py:166-241). Limits: D % 8 == 0, k <= 32.
+ * means 1. A negative pos makes the token's row NaN. Replaces fused_gather_reduce (kernels/moe_ops.py:166-241).
+ * Limits: D % 8 == 0, k <= 32.
  * ------------------------------------------------------------------------------------------------- */
 int ffm_combine_forward(const void* Y, const int32_t* pos, const float* w, const void* addend, int64_t N,
                         int top_k, int D, void* out, ffm_stream_t stream);
@@ -291,6 +295,7 @@ int ffm_route_backward(const float* gw, const float* topk_w, const int32_t* topk
 /* -------------------------------------------------------------------------------------------------
  * ffm_compact_positions: cpos[i] = position of flat slot i in the grouped order without the 256-row padding (the
  *   order in which an expert-parallel rank sends its rows, expert-major), src_c = the inverse map (int32 [T]).
+ *   Slots without an expert get cpos -1, and src_c ends with as many -1.
  *   Inputs are ffm_route_forward's pos, topk_idx, counts and tile_start. Replaces the stable sort by destination
  *   rank of the reference's dispatcher (expert_parallel.py:225-236). E <= 256.
  * ------------------------------------------------------------------------------------------------- */

@@ -56,6 +56,19 @@ def test_argument_validation_without_gpu():
     assert lib.ffm_combine_forward(0, 0, 0, 0, 4, 2, 64, 0, 0) == -1
 
 
+def test_groups_too_small_for_top_k_are_refused():
+    """A token cannot choose top_k experts from fewer: refused before any CUDA call (the workspace check comes after)."""
+    lib = _lib.load()
+
+    def route(topk_group, top_k):
+        E, N, D = 8, 4, 64
+        return lib.ffm_route_forward(1, 1, 0, N, D, E, top_k, 0, 1.0, 0, 4, topk_group, 1, 1, 1, 1, 1, 1, 1, 1,
+                                     lib.ffm_rows_capacity(N * top_k, E), 1, 1, 0, 1, 0)
+
+    assert route(1, 3) == -1 and route(2, 5) == -1
+    assert route(1, 2) == -4 and route(2, 4) == -4
+
+
 def test_product_path_has_no_cpu_fallback():
     import torch
     from flashfusedmoe_b200 import fused_moe
