@@ -124,21 +124,26 @@ def status_tensor(device):
 def check_status(device=None):
     """Synchronise and raise if any kernel reported a device-side failure since the last check."""
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
-    st = status_tensor(dev)
-    code = int(st.item())
-    # an asynchronous copy of the word queued by poll_status() carries the same information: drop it, so that a failure
-    # reported here is not reported a second time by a later fused_moe() call
+    code = int(status_tensor(dev).item())
+    if code != 0:
+        _clear_status(dev)
+        raise RuntimeError(f"libffmoe device status {code}: {_lib.error_string(code)}")
+
+
+def _clear_status(dev):
+    """Forget a failure that is about to be raised: the device word, the copy of it that poll_status() queued and the word
+    the layer's last kernel stores to carry the same code, and whichever stayed behind would blame a later call. The wait
+    is for kernels and copies in flight that would still hand the old code on."""
     key = dev.index if dev.index is not None else torch.cuda.current_device()
-    if code != 0 and key in _reported:
-        _reported[key][0][0] = 0
+    torch.cuda.synchronize(key)
     entry = _status_host.get(key)
-    if entry is not None and entry["pending"]:
-        entry["done"].synchronize()
+    if entry is not None:
         entry["pending"] = False
         entry["host"][0] = 0
-    if code != 0:
-        st.zero_()
-        raise RuntimeError(f"libffmoe device status {code}: {_lib.error_string(code)}")
+    if key in _reported:
+        _reported[key][0][0] = 0
+    status_tensor(dev).zero_()
+    torch.cuda.synchronize(key)   # the next call may run on another stream
 
 
 _status_host = {}
@@ -162,11 +167,8 @@ def raise_reported(device):
     a forward pass stores it to host memory, so there is nothing to enqueue and nothing to wait for."""
     entry = _reported.get(device.index)
     if entry is not None and entry[0][0] != 0:
-        word = entry[0]
-        torch.cuda.synchronize(device)   # no kernel that would store the old code again is left in flight
-        code = int(word[0])
-        word[0] = 0
-        status_tensor(device).zero_()
+        code = int(entry[0][0])
+        _clear_status(device)
         raise RuntimeError(f"libffmoe device status {code}: {_lib.error_string(code)} "
                            "(reported by a kernel of an earlier call; its results are not valid)")
 
@@ -205,8 +207,7 @@ def poll_status(device=None, enqueue=True):
         entry["pending"] = False
         code = int(entry["host"][0])
         if code != 0:
-            entry["host"][0] = 0
-            status_tensor(dev).zero_()
+            _clear_status(dev)
             raise RuntimeError(f"libffmoe device status {code}: {_lib.error_string(code)} "
                                "(reported by a kernel of an earlier call; its results are not valid)")
     if enqueue:
@@ -220,7 +221,7 @@ def raise_on_status(code, device):
     """Raise for a status code the caller already holds on the host (read together with other data)."""
     code = int(code)
     if code != 0:
-        status_tensor(device).zero_()
+        _clear_status(torch.device(device))
         raise RuntimeError(f"libffmoe device status {code}: {_lib.error_string(code)}")
 
 

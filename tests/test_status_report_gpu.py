@@ -61,3 +61,41 @@ def test_captured_call_reports_at_replay():
     with pytest.raises(RuntimeError, match="102"):
         _call()
     ops.check_status()
+
+
+@pytest.mark.parametrize("first", ["layer", "poll"])
+def test_both_channels_report_once(first):
+    """The expert-parallel path's copy of the word and the layer's own report carry one failure: it raises once, whichever
+    of the two is looked at first."""
+    _call()
+    ops.poll_status()
+    torch.cuda.synchronize()
+    ops.poll_status(enqueue=False)
+    ops.check_status()
+    ops.status_tensor(DEV).fill_(101)
+    _call()               # the layer's last kernel stores the code
+    ops.poll_status()     # and a copy of the word is queued
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError, match="101.*earlier call"):
+        _call() if first == "layer" else ops.poll_status()
+    _call()
+    ops.poll_status()
+    torch.cuda.synchronize()
+    _call()
+    ops.poll_status()
+    torch.cuda.synchronize()
+    ops.poll_status(enqueue=False)
+    ops.check_status()
+
+
+def test_code_read_with_other_data_clears_both_channels():
+    _call()
+    ops.status_tensor(DEV).fill_(103)
+    _call()
+    ops.poll_status()
+    with pytest.raises(RuntimeError, match="103"):
+        ops.raise_on_status(103, DEV)
+    torch.cuda.synchronize()
+    _call()
+    ops.poll_status(enqueue=False)
+    ops.check_status()
