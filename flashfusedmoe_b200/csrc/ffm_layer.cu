@@ -71,15 +71,41 @@ class Sites {
   int rc_ = FFM_OK;
 };
 
+// Callers pack the argument blocks by hand, eight bytes a field; tests/test_cabi_cpu.py compares the packing with the
+// header's field list and with these sizes.
+static_assert(sizeof(ffm_layer_forward_args) == 68 * 8, "a field was added or removed");
+static_assert(sizeof(ffm_layer_backward_args) == 67 * 8, "a field was added or removed");
+
+// Combinations of few_rows that would leave a buffer unwritten that a later launch reads: the decode GEMMs store no
+// pre-activations, and the one chain, which permutes nothing, needs both of them, the shared expert inside and every
+// routed row in use.
+bool bad_few_rows(const ffm_layer_forward_args& a) {
+  const int64_t both = FFM_FEW_DECODE_UP | FFM_FEW_DECODE_DOWN;
+  const bool decode = (a.few_rows & (both | FFM_FEW_DECODE_SHARED)) != 0;
+  if (a.few_rows & ~int64_t{FFM_FEW_TILES | both | FFM_FEW_DECODE_SHARED | FFM_FEW_ONE_CHAIN}) return true;
+  if (decode && (a.need_grad || a.preact != nullptr || a.s_preact != nullptr)) return true;
+  if ((a.few_rows & both) && a.fp8) return true;
+  if (!(a.few_rows & FFM_FEW_ONE_CHAIN)) return false;
+  return (a.few_rows & both) != both || a.capacity >= 0 || (a.Hs > 0 && !(a.few_rows & FFM_FEW_DECODE_SHARED));
+}
+
 }  // namespace
 
 }  // namespace ffm
 
 using namespace ffm;
 
+extern "C" int64_t ffm_layer_args_bytes(int backward) {
+  return backward ? sizeof(ffm_layer_backward_args) : sizeof(ffm_layer_forward_args);
+}
+
 extern "C" int ffm_layer_forward(const ffm_layer_forward_args* args) {
   if (args == nullptr || args->launched == nullptr) return FFM_ERR_BAD_ARG;
   const ffm_layer_forward_args& a = *args;
+  if (bad_few_rows(a)) {
+    for (int i = 0; i < 3; ++i) a.launched[i] = i == 2 ? FFM_FWD_UP : 0;
+    return FFM_ERR_BAD_ARG;
+  }
   const int D = static_cast<int>(a.D), E = static_cast<int>(a.E), H = static_cast<int>(a.H), k = static_cast<int>(a.top_k);
   const int Hs = static_cast<int>(a.Hs);
   const int act = static_cast<int>(a.activation);

@@ -336,8 +336,10 @@ int ffm_grouped_gemm_fp8(const void* Aq, const float* a_scale, const void* Bq, c
  * Forward: routing (aux = aux_scale * stats[E + 1] and z = z_scale * stats[E] when not null), capacity >= 0: dropping,
  * permute, expert GEMMs, combine; Hs > 0: a shared expert (sw_*) beside the routing, its output added in the combine.
  * need_grad: zero the padding rows and store preact / s_preact where given. few_rows: FFM_FEW_* bits,
- * 128-row tiles that skip tiles without rows; which projections, and whether the shared expert, run as ffm_decode_up (no
- * preact) and ffm_decode_down; ONE_CHAIN (with all of those): no permute, and the shared expert inside the two launches.
+ * 128-row tiles that skip tiles without rows; which projections, and whether the shared expert, run as ffm_decode_up and
+ * ffm_decode_down (neither with need_grad, preact or s_preact; projections not with fp8); ONE_CHAIN (with both of those,
+ * and SHARED where Hs > 0; not with capacity): no permute, and the shared expert inside the two launches. Any other
+ * combination is refused before anything is enqueued.
  * fp8: e4m3 expert GEMMs (w_*_q, w_*_scale; xq, x_scale, aq, a_scale are scratch). addend_ready: a cudaEvent_t
  * the combine waits for, or null.
  *
@@ -414,6 +416,8 @@ typedef struct {
 } ffm_layer_backward_args;
 int ffm_layer_forward(const ffm_layer_forward_args* args);
 int ffm_layer_backward(const ffm_layer_backward_args* args);
+/* Size of the two argument blocks (0: forward, 1: backward) in this build, for callers that pack them without this header. */
+int64_t ffm_layer_args_bytes(int backward);
 
 /* host[0] = *status by an asynchronous copy on side_stream, ordered after what `stream` holds: record `ready` on stream,
  * side_stream waits for it, copies, records `done` (cudaEvent_t handles; host is pinned memory). */

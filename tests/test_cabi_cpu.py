@@ -69,6 +69,65 @@ def test_groups_too_small_for_top_k_are_refused():
     assert route(1, 2) == -4 and route(2, 4) == -4
 
 
+def _block_fields(name):
+    """(field, "q" or "d") in the order in which include/ffmoe.h declares the fields of an argument block."""
+    text = open(os.path.join(ROOT, "include", "ffmoe.h")).read()
+    body = re.sub(r"/\*.*?\*/", "", text, flags=re.S).split("} " + name + ";")[0].rsplit("typedef struct {", 1)[1]
+    fields = []
+    for line in body.split(";"):
+        line = line.replace("const", " ").strip()
+        if line:
+            kind, names = line.split(None, 1)
+            for n in names.split(","):
+                value = n.strip()
+                assert kind in ("int64_t", "double") or value.startswith("*") or kind == "ffm_stream_t", (kind, value)
+                fields.append((value.lstrip("*"), "d" if kind == "double" and not value.startswith("*") else "q"))
+    return fields
+
+
+@pytest.mark.parametrize("name,backward", [("ffm_layer_forward_args", 0), ("ffm_layer_backward_args", 1)])
+def test_argument_block_is_packed_as_declared(name, backward):
+    """Eight bytes a field: the packing, the header and the compiled struct agree in number, kinds and size."""
+    from flashfusedmoe_b200 import ops
+    packing = ops.LAYER_BACKWARD_ARGS if backward else ops.LAYER_FORWARD_ARGS
+    fields = _block_fields(name)
+    assert [n for n, _ in fields[-2:]] == ["timer", "launched"]
+    packed = "".join(c * int(n) for n, c in re.findall(r"(\d+)([qd])", packing.format))
+    assert packed == "".join(k for _, k in fields[:-2])
+    assert _lib.load().ffm_layer_args_bytes(backward) == 8 * len(fields) == packing.size + 16
+
+
+def test_layer_forward_refuses_launches_that_read_unwritten_buffers():
+    """Every other field is zero: a combination that is let through fails on its null pointers, at another site."""
+    from flashfusedmoe_b200 import ops
+    lib = _lib.load()
+    names = [n for n, _ in _block_fields("ffm_layer_forward_args")]
+
+    def site(**values):
+        fields = dict.fromkeys(names, 0)
+        fields.update(dict(N=4, D=64, E=8, top_k=2, H=64, rows_cap=2048, capacity=-1), **values)
+        launched = (ctypes.c_int64 * 3)()
+        block = ops.LAYER_FORWARD_ARGS.pack(*[fields[n] for n in names[:-2]])
+        rc = lib.ffm_layer_forward(block + (0).to_bytes(8, "little") + ctypes.addressof(launched).to_bytes(8, "little"))
+        assert rc == -1
+        return launched[2]
+
+    tiles, up, down, shared, chain = 1, 2, 4, 8, 16
+    refused, route, shared_up = 6, 2, 0
+    for few in (chain, tiles | chain, up | chain, tiles | up | chain, down | chain, 32):
+        assert site(few_rows=few) == refused
+    assert site(few_rows=up | down | chain, capacity=4) == refused
+    assert site(few_rows=up | down | chain, Hs=64) == refused
+    for few in (up, down, shared):
+        assert site(few_rows=few, need_grad=1) == refused
+        assert site(few_rows=few, preact=16) == refused
+    assert site(few_rows=up, fp8=1) == refused
+    for few in (0, tiles, tiles | up, tiles | down, tiles | up | down, tiles | up | down | chain):
+        assert site(few_rows=few) == route
+    assert site(few_rows=tiles | up | down | shared | chain, Hs=64) == route
+    assert site(few_rows=shared, Hs=64) == shared_up
+
+
 def test_product_path_has_no_cpu_fallback():
     import torch
     from flashfusedmoe_b200 import fused_moe
