@@ -9,6 +9,7 @@
 #include <stdint.h>
 
 #include "../../include/ffmoe.h"
+#include "ffm_device.h"
 
 namespace ffm {
 
@@ -156,14 +157,14 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
 // registers, thread slots and few KiB of shared memory the GEMM leaves free) if it does not ask for a different one.
 #define FFM_PREFER_MAX_SHARED(kernel)                                                                              \
   do {                                                                                                             \
-    static bool ffm_carveout_set = false;                                                                          \
-    if (!ffm_carveout_set) {                                                                                       \
-      ffm_carveout_set = true;                                                                                     \
+    static ::ffm::PerDevice ffm_carveout_set;                                                                      \
+    ffm_carveout_set.get([&] {                                                                                     \
       if (cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,                             \
                                cudaSharedmemCarveoutMaxShared) != cudaSuccess) {                                   \
         cudaGetLastError();                                                                                        \
       }                                                                                                            \
-    }                                                                                                              \
+      return 1;                                                                                                    \
+    });                                                                                                            \
   } while (0)
 
 namespace ffm {

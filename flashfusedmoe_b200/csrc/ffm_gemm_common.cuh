@@ -208,14 +208,13 @@ inline int make_out_map(CUtensorMap* map, void* base, long long groups, long lon
 }
 
 inline int num_sms() {
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
+  static PerDevice sms;
+  return sms.get([] {
+    int dev = 0, n = 0;
     cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (sms <= 0) sms = 148;
-  }
-  return sms;
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    return n > 0 ? n : 148;
+  });
 }
 
 // Clock cycles after which a bounded wait inside a GEMM gives up (ffm_set_wait_cycles).

@@ -909,16 +909,16 @@ bool use_cta_pair() {
 template <int A_MN, int B_MN, int EPI, int GROUPK, int CTA2, int PASS = 0, int FP8 = 0>
 int launch_gemm_shape(const CUtensorMap& tmA, const CUtensorMap& tmB0, const CUtensorMap& tmB1, const CUtensorMap& tmC,
                       const CUtensorMap& tmC2, const GemmParams& p, long long max_units, cudaStream_t stream) {
-  static int max_ctas = 0;  // persistent grid size, found once per instantiation
+  static PerDevice persistent_grid;  // found once per instantiation and device
   auto kernel = ffm_gemm_kernel<A_MN, B_MN, EPI, GROUPK, CTA2, PASS, FP8>;
   constexpr int threads = gemm_threads(EPI, PASS);
   constexpr int smem_bytes = Shape<CTA2, EPI>::SMEM_BYTES;
-  if (max_ctas == 0) {
+  const int max_ctas = persistent_grid.get([&] {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) != cudaSuccess) {
       cudaGetLastError();
-      return FFM_ERR_LAUNCH;
+      return 0;
     }
-    max_ctas = num_sms();
+    int ctas = num_sms();
     if (CTA2) {
       // co-resident CTA pairs: a GPC with an odd number of usable SMs leaves one SM without a partner
       cudaLaunchConfig_t q = {};
@@ -937,9 +937,11 @@ int launch_gemm_shape(const CUtensorMap& tmA, const CUtensorMap& tmB0, const CUt
         cudaGetLastError();
         clusters = num_sms() / 2 - 4;
       }
-      max_ctas = 2 * clusters;
+      ctas = 2 * clusters;
     }
-  }
+    return ctas;
+  });
+  if (max_ctas <= 0) return FFM_ERR_LAUNCH;
   if (max_units <= 0 && !(PASS && p.pz_rows > 0)) return FFM_OK;
   long long ctas = CTA2 ? 2 * max_units : max_units;
   if (PASS && p.pz_rows > 0) ctas = max_ctas;  // the passenger job wants every SM, whatever the GEMM's tile count

@@ -508,15 +508,14 @@ int make_glu_weight_map(CUtensorMap* map, const void* lo, long long gap, int K, 
 template <int EPI>
 int launch_tok(const CUtensorMap (&m)[6], const TokParams& p, long long rows, cudaStream_t stream) {
   using S = Shape<EPI>;
-  static bool ready = false;
+  static PerDevice ready;
   auto kernel = ffm_gemm_tok_kernel<EPI>;
-  if (!ready) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM_BYTES) != cudaSuccess) {
-      cudaGetLastError();
-      return FFM_ERR_LAUNCH;
-    }
-    ready = true;
-  }
+  const bool ok = ready.get([&] {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM_BYTES) == cudaSuccess) return 1;
+    cudaGetLastError();
+    return 0;
+  }) > 0;
+  if (!ok) return FFM_ERR_LAUNCH;
   // no more CTAs than there can be tiles: every group may end in a partly filled token tile, and every routed row may be
   // alone in its group
   long long tiles = rows / NMAX + p.groups;
