@@ -77,6 +77,8 @@ SIGNATURES = {
                                       c_void_p]),
     "ffm_layer_forward": (c_int, [ctypes.c_char_p]),   # packed by ops.LAYER_FORWARD_ARGS / _BACKWARD_ARGS
     "ffm_layer_backward": (c_int, [ctypes.c_char_p]),
+    "ffm_route_forward_launches": (c_int, [c_int64, c_int, c_int, c_int, c_int]),
+    "ffm_route_backward_launches": (c_int, [c_int64, c_int, c_int, c_int, c_int, c_int, c_int]),
     "ffm_layer_args_bytes": (c_int64, [c_int]),
     "ffm_status_copy": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
     "ffm_p2p_push": (c_int, [c_int, c_void_p, c_void_p, c_void_p, c_void_p]),

@@ -1,6 +1,7 @@
 // Launch sequence of the single-GPU layer, forward and backward (host code only).
 //
-// One call enqueues a whole pass: its 9 to 20 launches and the events that fork and join the side streams. From Python,
+// One call enqueues a whole pass: 5 to 12 launches forward, 10 to 20 backward, and the events that fork and join the side
+// streams. From Python,
 // each launch cost a ctypes call with its argument checks, an output allocation and, at a fork, stream and event objects:
 // 230 us for a forward pass and 600 us for a backward pass however small, more than the GPU needed at up to a few
 // thousand tokens.
@@ -140,7 +141,7 @@ extern "C" int ffm_layer_forward(const ffm_layer_forward_args* args) {
     if (sh != st) sites.require(shared_done.record(sh));
   }
 
-  sites.run(FFM_FWD_ROUTE, 3, st, [&] {
+  sites.run(FFM_FWD_ROUTE, ffm_route_forward_launches(a.N, D, E, k, a.logits != nullptr), st, [&] {
     return route_forward_losses(a.hidden_route, a.gate, a.expert_bias, a.N, D, E, k, static_cast<int>(a.gating),
                                 static_cast<float>(a.weight_scale), static_cast<int>(a.pre_softmax),
                                 static_cast<int>(a.n_group), static_cast<int>(a.topk_group), a.logits, a.topk_w,
@@ -296,7 +297,9 @@ extern "C" int ffm_layer_backward(const ffm_layer_backward_args* args) {
   lg.aux_coef = static_cast<float>(a.aux_coef);
   lg.z_coef = static_cast<float>(a.z_coef);
   if (overlap) sites.require(rows_done.order(st, rt));
-  sites.run(FFM_BWD_ROUTE, 3, rt, [&] {
+  const int route_kernels = ffm_route_backward_launches(a.N, D, E, static_cast<int>(a.gating), a.grad_aux != nullptr,
+                                                        a.grad_z != nullptr, 0);
+  sites.run(FFM_BWD_ROUTE, route_kernels, rt, [&] {
     return route_backward_losses(a.gw, a.topk_w, a.topk_idx, a.logits, a.lse, lg, a.hidden, a.gate, a.N, D, E, k,
                                  static_cast<int>(a.gating), 0, a.dH_route, a.d_gate, a.workspace,
                                  static_cast<size_t>(a.workspace_bytes), a.status, rt);

@@ -1044,6 +1044,25 @@ int static_scratch_address(void** out) {
 
 using namespace ffm;
 
+// Few tokens: two launches. The line lies where the gate product on CUDA cores (N E D multiply-adds, 29 us at
+// N = 128, E = 256, D = 7168) stops being cheaper than the tensor-core GEMM, whose one CTA pair takes 46 us for that
+// contraction; 7 tokens, E = 8, D = 4096: 6 + 6 us against 72 + 3 + 3 with the kernels for many tokens.
+static bool route_few_tokens(int64_t N, int top_k, bool has_logits) {
+  return N > 0 && N <= SMALL_TOKENS && N * top_k <= SMALL_SLOTS && has_logits;
+}
+
+// Many experts: gate GEMM on the tensor cores (dense tcgen05 GEMM, fp32 accumulate, bf16 logits), then one
+// scoring kernel. Few experts: everything in one warp-level kernel.
+// (E = 32 included: one warp owning 32 experts keeps 64 accumulators per lane and ran at 0.12 TB/s)
+static bool route_tensor_gate(int D, int E, bool has_logits) {
+  return E >= 32 && D % 64 == 0 && E % 32 == 0 && has_logits;
+}
+
+extern "C" int ffm_route_forward_launches(int64_t N, int D, int E, int top_k, int has_logits) {
+  if (route_few_tokens(N, top_k, has_logits != 0)) return 2;
+  return N > 0 && route_tensor_gate(D, E, has_logits != 0) ? 4 : 3;
+}
+
 extern "C" int64_t ffm_rows_capacity(int64_t T, int E) {
   if (T < 0 || E < 1) return 0;
   return ((T + 255LL * E) / 256) * 256;
@@ -1088,10 +1107,7 @@ int ffm::route_forward_losses(const void* hidden, const void* gate_w, const floa
   const bf16* h = static_cast<const bf16*>(hidden);
   const bf16* gw = static_cast<const bf16*>(gate_w);
   bf16* lg = static_cast<bf16*>(logits);
-  // Few tokens: two launches. The line lies where the gate product on CUDA cores (N E D multiply-adds, 29 us at
-  // N = 128, E = 256, D = 7168) stops being cheaper than the tensor-core GEMM, whose one CTA pair takes 46 us for that
-  // contraction; 7 tokens, E = 8, D = 4096: 6 + 6 us against 72 + 3 + 3 with the kernels for many tokens.
-  if (N > 0 && N <= SMALL_TOKENS && N * top_k <= SMALL_SLOTS && lg != nullptr) {
+  if (route_few_tokens(N, top_k, lg != nullptr)) {
     const RouteWorkspace w = carve_workspace(workspace, FINISH_CLUSTER, E);
     const int n = static_cast<int>(N);
     const dim3 grid((n + SMALL_TG - 1) / SMALL_TG, (E + SMALL_EG - 1) / SMALL_EG, 1);
@@ -1106,10 +1122,7 @@ int ffm::route_forward_losses(const void* hidden, const void* gate_w, const floa
     return FFM_FINISH_CASE(8);
 #undef FFM_FINISH_CASE
   }
-  // Many experts: gate GEMM on the tensor cores (dense tcgen05 GEMM, fp32 accumulate, bf16 logits), then one
-  // scoring kernel. Few experts: everything in one warp-level kernel.
-  // (E = 32 included: one warp owning 32 experts keeps 64 accumulators per lane and ran at 0.12 TB/s)
-  const bool tensor_gate = E >= 32 && D % 64 == 0 && E % 32 == 0 && logits != nullptr;
+  const bool tensor_gate = route_tensor_gate(D, E, lg != nullptr);
   const RouteGrid g = route_grid(N > 0 ? N : 1, tensor_gate || E > 32 ? route_granule(E) : 32 / gate_slices(D));
   RouteWorkspace w = carve_workspace(workspace, g.blocks, E);
   if (tensor_gate) {

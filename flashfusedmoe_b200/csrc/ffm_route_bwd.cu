@@ -293,6 +293,19 @@ size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 
 using namespace ffm;
 
+// A z-loss, or an aux loss on sigmoid scores, makes every entry of gl non-zero: dH = gl gate_w is then a GEMM with
+// K = E, on the tensor cores where the shape allows (16384 tokens, E = 64, D = 2048: the token kernel ran 971 us beside
+// the layer's GEMMs, which it slowed down). Otherwise a row has top_k entries and the token kernel adds their rows.
+static bool dh_on_tensor_cores(int D, int E, int gating, bool has_aux, bool has_z, int accumulate) {
+  const bool dense = has_z || (gating == FFM_GATING_SIGMOID && has_aux);
+  return dense && accumulate == 0 && E % 64 == 0 && D % 64 == 0;
+}
+
+extern "C" int ffm_route_backward_launches(int64_t N, int D, int E, int gating, int has_aux, int has_z, int accumulate) {
+  if (N <= 0) return 1;
+  return dh_on_tensor_cores(D, E, gating, has_aux != 0, has_z != 0, accumulate) ? 4 : 3;
+}
+
 extern "C" size_t ffm_route_backward_workspace_bytes(int64_t N, int D, int E) {
   if (N < 0 || D <= 0 || E < 1) return 0;
   const int ldg_ = (E + 7) & ~7;
@@ -328,11 +341,7 @@ int ffm::route_backward_losses(const float* gw, const float* topk_w, const int32
     long long blocks = (N + RB_WARPS - 1) / RB_WARPS;
     if (blocks > 148LL * 16) blocks = 148LL * 16;
     FFM_PREFER_MAX_SHARED(route_bwd_token);
-    // A z-loss, or an aux loss on sigmoid scores, makes every entry of gl non-zero: dH = gl gate_w is then a GEMM with
-    // K = E, on the tensor cores where the shape allows (16384 tokens, E = 64, D = 2048: the token kernel ran 971 us beside
-    // the layer's GEMMs, which it slowed down). Otherwise a row has top_k entries and the token kernel adds their rows.
-    const bool dense = has_z || (gating == FFM_GATING_SIGMOID && has_aux);
-    const bool gemm_dh = dense && accumulate == 0 && E % 64 == 0 && D % 64 == 0;
+    const bool gemm_dh = dh_on_tensor_cores(D, E, gating, has_aux, has_z, accumulate);
     route_bwd_token<<<static_cast<int>(blocks), RB_THREADS, 0, s>>>(
         gw, topk_w, topk_idx, static_cast<const bf16*>(logits), lse, lg, static_cast<const bf16*>(gate_w), N, D,
         E, top_k, gating, accumulate, gl, gemm_dh ? nullptr : static_cast<bf16*>(dH));

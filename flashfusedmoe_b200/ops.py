@@ -281,7 +281,7 @@ def route_forward(hidden, gate_w, top_k, gating="softmax", expert_bias=None, wei
         rows_cap=rows_cap, top_k=top_k, num_experts=E)
     ws_bytes = int(lib.ffm_route_workspace_bytes(N, E, top_k))
     ws = _workspace(dev, ws_bytes, "route")
-    with _Launch("route_forward", 3):
+    with _Launch("route_forward", lib.ffm_route_forward_launches(N, D, E, top_k, 1)):
         rc = lib.ffm_route_forward(_ptr(hidden), _ptr(gate_w), _ptr(expert_bias), N, D, E, top_k,
                                    _lib.GATING[gating], float(weight_scale), 1 if pre_softmax else 0, int(n_group or 0),
                                    int(topk_group or 0), _ptr(r.logits), _ptr(r.topk_w),
@@ -610,7 +610,8 @@ def route_backward(gw, routing, gaux, gz, hidden, gate_w, gating, dH=None):
     dGate = torch.empty(E, D, dtype=torch.bfloat16, device=dev)
     ws_bytes = int(lib.ffm_route_backward_workspace_bytes(N, D, E))
     ws = _workspace(dev, ws_bytes, "route_bwd")
-    with _Launch("route_backward", 3):
+    kernels = lib.ffm_route_backward_launches(N, D, E, _lib.GATING[gating], gaux is not None, gz is not None, accumulate)
+    with _Launch("route_backward", kernels):
         rc = lib.ffm_route_backward(_ptr(gw), _ptr(routing.topk_w), _ptr(routing.topk_idx), _ptr(routing.logits),
                                     _ptr(routing.lse), _ptr(gaux), _ptr(gz), _ptr(hidden), _ptr(gate_w), N, D, E,
                                     routing.top_k, _lib.GATING[gating], 1 if accumulate else 0, _ptr(dH), _ptr(dGate),

@@ -109,6 +109,8 @@ int ffm_set_gemm_cta_pair(int enable);
  * Limits: D % 8 == 0, 1 <= k <= min(E, 32), E <= 256.
  * ------------------------------------------------------------------------------------------------- */
 size_t ffm_route_workspace_bytes(int64_t N, int E, int top_k);
+/* Kernels that ffm_route_forward enqueues (has_logits: a logits buffer is given). */
+int ffm_route_forward_launches(int64_t N, int D, int E, int top_k, int has_logits);
 int ffm_route_forward(const void* hidden, const void* gate_w, const float* expert_bias, int64_t N, int D, int E,
                       int top_k, int gating, float weight_scale, int pre_softmax, int n_group, int topk_group,
                       void* logits, float* topk_w, int32_t* topk_idx,
@@ -287,6 +289,8 @@ int ffm_glu_backward(const void* dAct, const void* preact, const int32_t* tile_s
  * D % 64 == 0 and N >= 1024 the dGate product runs as a tensor-core GEMM over the tokens, whose waits report there).
  * ------------------------------------------------------------------------------------------------- */
 size_t ffm_route_backward_workspace_bytes(int64_t N, int D, int E);
+/* Kernels that ffm_route_backward enqueues (has_aux / has_z: gaux / gz given). */
+int ffm_route_backward_launches(int64_t N, int D, int E, int gating, int has_aux, int has_z, int accumulate);
 int ffm_route_backward(const float* gw, const float* topk_w, const int32_t* topk_idx, const void* logits,
                        const float* lse, const float* gaux, const float* gz, const void* hidden, const void* gate_w,
                        int64_t N, int D, int E, int top_k, int gating, int accumulate, void* dH, void* dGate,
