@@ -150,6 +150,14 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
   return true;
 }
 
+// For a CTA that gives up: wait (about a tenth of a second at most) for what it still has in flight on this barrier.
+__device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity) {
+  const long long t0 = clock64();
+  while (!mbar_try_wait(bar, parity)) {
+    if (clock64() - t0 > 200000000LL) return;
+  }
+}
+
 }  // namespace ffm
 
 // Ask for the largest shared-memory carve-out for a kernel that itself needs little or none. The persistent GEMM

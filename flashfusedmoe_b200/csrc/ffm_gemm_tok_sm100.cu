@@ -78,8 +78,10 @@ struct Ctrl {
   unsigned long long empty_bar[STAGES];
   unsigned long long acc_full_bar[NUM_ACC];
   unsigned long long acc_empty_bar[NUM_ACC];
+  unsigned long long drain_bar;  // after an abort: the MMAs in flight
   uint32_t tmem_base;
   int abort_flag;
+  int filled;                 // stages the producer has filled in all
   int4 token[NMAX / 4];       // up: token rows of the producer's tile
   int base[MAX_GROUPS];       // first row of a group
   int count[MAX_GROUPS];      // rows of a group
@@ -242,6 +244,7 @@ ffm_gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       mbar_init(smem_u32(&ctrl->acc_full_bar[a]), 1);
       mbar_init(smem_u32(&ctrl->acc_empty_bar[a]), EPI_WARPS);
     }
+    mbar_init(smem_u32(&ctrl->drain_bar), 1);
     ctrl->abort_flag = 0;
     fence_barrier_init();
     tma_prefetch_desc(&tmA);
@@ -298,6 +301,7 @@ ffm_gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     // ================= TMA producer =================
     int stage = 0;
     uint32_t phase = 0;
+    int filled = 0;
     bool ok = true;
     while (ok && walker.next(t)) {
       const int f0 = t.f_tile * S::FEATS;
@@ -333,6 +337,7 @@ ffm_gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           } else {
             for (int r = 0; r < nb; r += 16) tma_load_2d(b_dst + r * 128, mB, full, k0, t.row0 + r);
           }
+          ++filled;
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1u;
@@ -341,6 +346,7 @@ ffm_gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       }
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;  // also: the token list is overwritten only after its last use
     }
+    if (lane == 0) ctrl->filled = filled;
   } else if (warp == 1) {
     // ================= MMA issuer =================
     if (lane == 0) {
@@ -463,6 +469,18 @@ ffm_gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   // ---- common exit: every role reaches this point, also after an abort ----------------------
   tc_fence_before();
   __syncthreads();
+  if (*abort_flag != 0) {
+    // loads and MMAs that nobody waited for must not land in shared memory or TMEM that the CTA has given back
+    if (threadIdx.x == 0) {
+      for (int f = max(ctrl->filled - STAGES, 0); f < ctrl->filled; ++f) {
+        mbar_drain(smem_u32(&ctrl->full_bar[f % STAGES]), (f / STAGES) & 1);
+      }
+    } else if (threadIdx.x == 32) {
+      umma_commit(smem_u32(&ctrl->drain_bar));
+      mbar_drain(smem_u32(&ctrl->drain_bar), 0);
+    }
+    __syncthreads();
+  }
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, TMEM_COLS);

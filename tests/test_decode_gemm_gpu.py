@@ -10,7 +10,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-from flashfusedmoe_b200 import ops  # noqa: E402
+from flashfusedmoe_b200 import _lib, ops  # noqa: E402
 from test_kernels_gpu import glu_ref  # noqa: E402
 
 DEV = "cuda"
@@ -163,3 +163,26 @@ def test_wgrad_up_to_the_last_valid_row(M, Nout):
     ref = ops.grouped_gemm_wgrad(torch.nan_to_num(a), torch.nan_to_num(b), len(COUNTS), ts)
     ops.check_status()
     assert torch.equal(got, ref)
+
+
+def test_a_wait_that_runs_out_ends_the_launch():
+    """With the shortest wait a CTA may give up: it reports that, takes its copies and MMAs in flight along, and the next
+    launch is right."""
+    torch.manual_seed(0)
+    x = torch.randn(64, 2048, device=DEV).bfloat16()
+    gate, up = (torch.randn(2816, 2048, device=DEV).bfloat16() for _ in range(2))
+    shared = (x, gate, up, "swiglu")
+    want = ops.decode_up(None, None, 1, None, None, 0, None, "swiglu", shared=shared)[1]
+    ops.check_status()
+    lib = _lib.load()
+    old = lib.ffm_set_wait_cycles(1)
+    try:
+        for _ in range(3):
+            ops.decode_up(None, None, 1, None, None, 0, None, "swiglu", shared=shared)
+        torch.cuda.synchronize()
+    finally:
+        lib.ffm_set_wait_cycles(old)
+    assert int(ops.status_tensor(x.device).item()) in (0, 101, 102, 103)
+    ops.status_tensor(x.device).zero_()
+    assert torch.equal(ops.decode_up(None, None, 1, None, None, 0, None, "swiglu", shared=shared)[1], want)
+    ops.check_status()
