@@ -178,7 +178,8 @@ struct TileCoord {
   int n_block;   // BN-column block (GLU: 128-column block of H)
   int k_row0;    // grouped-K: first K row; else 0
   int k_blocks;  // 64-deep K blocks to accumulate
-  int k_tail;    // 16-deep MMA steps of the last K block (4 unless grouped-K rows are given)
+  int k_full;    // grouped-K: blocks with all four MMA steps; at most one more is left,
+  int k_tail;    // which has this many
 };
 
 // Walks the tiles of this CTA (or CTA pair) in launch order. The unit is one MMA tile: 128 rows, or with CTA2
@@ -226,11 +227,13 @@ struct TileWalker {
       t.n_block = r / m_units_per_group;
       t.k_row0 = ts[t.group] * BM;
       t.k_blocks = (ts[t.group + 1] - ts[t.group]) * (BM / BK);
-      t.k_tail = BK / UMMA_K;
+      t.k_full = t.k_blocks;
+      t.k_tail = 0;
       if (k_rows != nullptr) {
         const int steps = (__ldg(k_rows + t.group) + UMMA_K - 1) / UMMA_K;
-        t.k_blocks = (steps + BK / UMMA_K - 1) / (BK / UMMA_K);
-        t.k_tail = steps - (t.k_blocks - 1) * (BK / UMMA_K);
+        t.k_full = steps / (BK / UMMA_K);
+        t.k_tail = steps % (BK / UMMA_K);
+        t.k_blocks = t.k_full + (t.k_tail > 0 ? 1 : 0);
       }
     } else {
       while (g < groups - 1 && cur >= static_cast<long long>(units(ts[g + 1])) * n_tiles) ++g;
@@ -594,7 +597,7 @@ ffm_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = 0; kb < t.k_blocks; ++kb) {
+        for (int kb = 0; kb < (GROUPK ? t.k_full : t.k_blocks); ++kb) {
           ok = mbar_wait_bounded(smem_u32(&ctrl->full_bar[stage]), phase, abort_flag, p.status, FFM_STATUS_WAIT_MMA,
                                  p.wait_cycles);
           if (!ok) break;
@@ -603,7 +606,6 @@ ffm_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           const uint32_t b_src = a_src + A_STAGE_BYTES;
 #pragma unroll
           for (int kk = 0; kk < BK / UMMA_K; ++kk) {
-            if (GROUPK && kb == t.k_blocks - 1 && kk >= t.k_tail) break;
             const uint64_t adesc = A_MN ? make_smem_desc_sw128(a_src + kk * 2048, 8192, 1024)
                                         : make_smem_desc_sw128(a_src + kk * 32, 16, 1024);
             const uint64_t bdesc = B_MN ? make_smem_desc_sw128(b_src + kk * 2048, 8192, 1024)
@@ -622,6 +624,41 @@ ffm_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             }
           }
           // free the stage (in both CTAs) once these MMAs retire
+          const uint32_t empty_local = smem_u32(&ctrl->empty_bar[stage]);
+          if (CTA2) {
+            umma_commit_pair(empty_local);
+            umma_commit_pair(map_to_cta(empty_local, 1));
+          } else {
+            umma_commit(empty_local);
+          }
+          if (++stage == STAGES) {
+            stage = 0;
+            phase ^= 1u;
+          }
+        }
+        if (GROUPK && ok && t.k_tail > 0) {
+          // The group's last K block, up to its last valid row. It stands apart because the issuing thread has no time to
+          // spare: with the test for the last step in the loop above every weight gradient was slower, also without
+          // padding (8 x 4096 rows, 4096 x 1024: 180 -> 203 us; 64 x 1536 rows, 2816 x 2048: 843 -> 972), and so were
+          // replayed training steps (16384 tokens, 8 experts and a shared one: 1966 -> 2037 us).
+          static_assert(!GROUPK || (A_MN && B_MN && !FP8), "both operands of a grouped-K GEMM are M/N-major bf16");
+          ok = mbar_wait_bounded(smem_u32(&ctrl->full_bar[stage]), phase, abort_flag, p.status, FFM_STATUS_WAIT_MMA,
+                                 p.wait_cycles);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t a_src = smem_base + stage * STAGE_BYTES;
+          const uint32_t b_src = a_src + A_STAGE_BYTES;
+#pragma unroll 1
+          for (int kk = 0; kk < t.k_tail; ++kk) {
+            const uint64_t adesc = make_smem_desc_sw128(a_src + kk * 2048, 8192, 1024);
+            const uint64_t bdesc = make_smem_desc_sw128(b_src + kk * 2048, 8192, 1024);
+            const uint32_t accumulate = (t.k_full > 0 || kk > 0) ? 1u : 0u;
+            if (CTA2) {
+              umma_bf16_pair(d_tmem, adesc, bdesc, idesc, accumulate);
+            } else {
+              umma_bf16(d_tmem, adesc, bdesc, idesc, accumulate);
+            }
+          }
           const uint32_t empty_local = smem_u32(&ctrl->empty_bar[stage]);
           if (CTA2) {
             umma_commit_pair(empty_local);
