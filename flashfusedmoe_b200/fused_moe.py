@@ -389,6 +389,13 @@ def _require_bf16(dtype):
 # 4 rows 131 + 75 -> 121 + 64, 32 rows 132 + 75 -> 126 + 67, 64 rows (many experts past one 64-token tile) 131 + 75 ->
 # 170 + 97.
 _DECODE_ROWS = 32
+# And up to this many tokens: rows per expert are an average, what bounds them under any load is the number of tokens, and
+# every 64 rows of an expert read its weights once more. The whole call, replayed, in us with 128-row tiles and with these
+# GEMMs, at the shape above, the load spread over all 64 experts / over 6 / over 12: 64 tokens 238 -> 219, 72 -> 59, 84 -> 84;
+# 128 tokens 240 -> 223, 74 -> 78, 84 -> 98; 160 tokens 244 -> 225, 78 -> 94, 90 -> 113; 341 tokens 254 -> 238, 100 -> 156 (over
+# 6). Up to 128 tokens no load was found that takes longer than these calls did when the host issued the launches one by one
+# and routing took three to five of them (94 and 104 us over 6 and 12); beyond, skewed loads do.
+_DECODE_TOKENS = 128
 # The shared expert runs in the same kernels up to one 64-token tile (14 + 17 us instead of 18 + 20 at 48 tokens, D = 2048,
 # Hs = 2816).
 _DECODE_SHARED_TOKENS = 64
@@ -420,7 +427,7 @@ def _few_rows(N, D, E, k, H, capacity, w_gate, w_up):
     if capacity or N * k >= 128 * E:
         return bits
     bits |= _FEW_TILES
-    if 0 < N * k <= _DECODE_ROWS * E:
+    if 0 < N * k <= _DECODE_ROWS * E and N <= _DECODE_TOKENS:
         bits |= _FEW_DECODE_UP if _streams_weights(E, D, 2 * H) else 0
         bits |= _FEW_DECODE_DOWN if _streams_weights(E, H, D) else 0
         both = _FEW_DECODE_UP | _FEW_DECODE_DOWN

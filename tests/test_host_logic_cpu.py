@@ -274,6 +274,22 @@ def test_backward_exchanges_alternate_receive_regions():
     assert all(r < p2p.NUM_REGIONS for r in seq1)
 
 
+def test_decode_gemms_end_where_a_skewed_load_makes_them_slow():
+    """Few rows per expert on average, but as many as there are tokens on one expert: the rule bounds both."""
+    import importlib
+    module = importlib.import_module("flashfusedmoe_b200.fused_moe")
+    up, down = module._FEW_DECODE_UP, module._FEW_DECODE_DOWN
+
+    def bits(N, E, k, capacity=False):
+        return module._few_rows(N, 1024, E, k, 512, capacity, None, None)
+
+    for N, E, k, wanted in ((1, 8, 2, True), (128, 8, 2, True), (129, 8, 2, False), (128, 64, 6, True), (129, 64, 6, False),
+                            (341, 64, 6, False), (1024, 256, 8, False), (128, 256, 8, True), (65, 8, 4, False)):
+        assert bool(bits(N, E, k) & up) == bool(bits(N, E, k) & down) == wanted, (N, E, k)
+        assert bool(bits(N, E, k) & module._FEW_TILES) == (N * k < 128 * E)
+        assert not bits(N, E, k, capacity=True)
+
+
 def test_expert_gemm_precision_switch():
     import flashfusedmoe_b200 as ffm
     assert ffm.set_expert_gemm_precision("fp8") == "bf16"
