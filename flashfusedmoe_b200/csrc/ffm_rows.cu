@@ -82,17 +82,18 @@ combine_forward_kernel(const bf16* __restrict__ Y, const int32_t* __restrict__ p
     if (lane < top_k) {
       my_pos = pos[n * top_k + lane];
       my_w = (w != nullptr) ? bf16_round(w[n * top_k + lane]) : 1.0f;
+      if (my_pos < 0) {
+        // a slot without an expert: NaN times any row (a test at every load: 33 -> 37 us, top-2 with an addend, 16384 tokens,
+        // D = 1024)
+        my_pos = 0;
+        my_w = NAN;
+      }
     }
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     for (int j = 0; j < top_k; ++j) {
       const int pj = __shfl_sync(0xffffffffu, my_pos, j);
       const float wj = __shfl_sync(0xffffffffu, my_w, j);
-      if (!active) continue;
-      if (pj >= 0) {
-        fma8(acc, __ldg(reinterpret_cast<const uint4*>(Y + static_cast<long long>(pj) * D) + c), wj);
-      } else {
-        acc[0] = acc[1] = acc[2] = acc[3] = acc[4] = acc[5] = acc[6] = acc[7] = NAN;  // a slot without an expert
-      }
+      if (active) fma8(acc, __ldg(reinterpret_cast<const uint4*>(Y + static_cast<long long>(pj) * D) + c), wj);
     }
     if (!active) continue;
     if (addend != nullptr) add_rounded(acc, __ldg(reinterpret_cast<const uint4*>(addend + n * D) + c));
