@@ -20,8 +20,7 @@ SCHEDULES = [(overlap, fused) for overlap in (True, False) for fused in (True, F
                                      dict(num_shared_experts=1, recompute_activations=True, gating="sigmoid",
                                           aux_loss_coeff=0.01), dict(capacity_factor=1.0, activation="geglu")])
 def test_schedules_agree(N, options, monkeypatch):
-    """Side streams change no bits. The GLU backward on its own reads dAct rounded to bf16, inside the GEMM unrounded: 2^-9
-    relative on each of the values that the gradients through it are sums of."""
+    """Neither the side streams nor the place where the GLU backward runs changes a bit."""
     D = 256
     torch.manual_seed(N)
     layer = MoELayer(D, 512, 8, 2, **options).to(DEV).bfloat16().train(True)
@@ -38,9 +37,6 @@ def test_schedules_agree(N, options, monkeypatch):
         ops.check_status()
         results[schedule] = dict(zip(names, grads), out=out.detach(), **{f"loss{i}": s.detach() for i, s in enumerate(scalars)})
     want = results[True, True]
-    for (overlap, fused), got in results.items():
-        same = want if fused else results[True, False]
+    for schedule, got in results.items():
         for name in got:
-            assert torch.equal(got[name], same[name]), (overlap, fused, name)
-            d = (got[name].float() - want[name].float()).norm() / want[name].float().norm().clamp_min(1e-20)
-            assert d <= 2.0 ** -8, (overlap, fused, name, float(d))
+            assert torch.equal(got[name], want[name]), (schedule, name)
