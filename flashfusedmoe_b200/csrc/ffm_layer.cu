@@ -1,8 +1,7 @@
 // Launch sequence of the single-GPU layer, forward and backward (host code only).
 //
-// One call enqueues a whole pass: 5 to 12 launches forward, 10 to 20 backward, and the events that fork and join the side
-// streams. From Python,
-// each launch cost a ctypes call with its argument checks, an output allocation and, at a fork, stream and event objects:
+// One call enqueues a whole pass: 5 to 13 launches forward, 9 to 19 backward, and the events that fork and join the side
+// streams. From Python, each launch cost a ctypes call with its argument checks, an output allocation and, at a fork, stream and event objects:
 // 230 us for a forward pass and 600 us for a backward pass however small, more than the GPU needed at up to a few
 // thousand tokens.
 #include <cuda_runtime.h>

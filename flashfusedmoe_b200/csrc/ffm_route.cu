@@ -618,7 +618,8 @@ __device__ __forceinline__ void finish_counts(const int* s_counts, const float* 
 // One block of 32 warps. block_off[e][b] = sum_{b' < b} hist[e][b']; counts; tile_start; stats.
 // One warp per expert, the lanes sweep its block histograms 32 at a time: the histograms are stored expert-major, so a
 // sweep reads one 128-byte line (block-major, each lane touched its own line: with eight warps the kernel took 73 us at
-// 512 blocks x 64 experts and 49 us at 64 x 256; now 15 us and, on the path for few tokens, part of route_finish_small). All sums keep a fixed order.
+// 512 blocks x 64 experts and 49 us at 64 x 256; now 15 us and, on the path for few tokens, part of route_finish_small). All
+// sums keep a fixed order.
 constexpr int SCAN_THREADS = 1024;
 __global__ void __launch_bounds__(SCAN_THREADS)
 route_scan(const int32_t* __restrict__ block_hist, const float* __restrict__ block_mass,
@@ -1044,9 +1045,11 @@ int static_scratch_address(void** out) {
 
 using namespace ffm;
 
-// Few tokens: two launches. The line lies where the gate product on CUDA cores (N E D multiply-adds, 29 us at
-// N = 128, E = 256, D = 7168) stops being cheaper than the tensor-core GEMM, whose one CTA pair takes 46 us for that
-// contraction; 7 tokens, E = 8, D = 4096: 6 + 6 us against 72 + 3 + 3 with the kernels for many tokens.
+// Few tokens: two launches. Whole routing, replayed, in us with two launches / with the kernels for many tokens: E = 256,
+// D = 7168: 33 / 64 at 64 tokens, 47 / 68 at 128, 61 / 72 at 192, 66 / 72 at 224, 74 / 72 at 256; E = 256, D = 2048: 35 / 45 at
+// 128, 51 / 49 at 256; E = 128, D = 7168: 49 / 61 at 256; E = 64, D = 2048: 27 / 31 at 256; E = 8, D = 1024: 16 / 16 at 256, D =
+// 4096 18 / 20. So the line at 256 tokens is on the slower side, by 3 %, only at its very end with 256 experts; what grows
+// beyond it is the gate product on CUDA cores, N E D multiply-adds.
 static bool route_few_tokens(int64_t N, int top_k, bool has_logits) {
   return N > 0 && N <= SMALL_TOKENS && N * top_k <= SMALL_SLOTS && has_logits;
 }

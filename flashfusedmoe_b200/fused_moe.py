@@ -397,7 +397,9 @@ _DECODE_ROWS = 32
 # and routing took three to five of them (94 and 104 us over 6 and 12); beyond, skewed loads do.
 _DECODE_TOKENS = 128
 # The shared expert runs in the same kernels up to one 64-token tile (14 + 17 us instead of 18 + 20 at 48 tokens, D = 2048,
-# Hs = 2816).
+# Hs = 2816). Whole calls of 16 and 64 tokens with 8 experts, replayed, dense tiles -> here, in us: D = 1024, Hs = 2048 65 ->
+# 61 and 66 -> 64; D = 4096, Hs = 2048 129 -> 123 and 129 -> 127; D = 4096, Hs = 8192 148 -> 141 and 152 to 154 -> 156 to 164
+# (over two allocations: the one point found on the slower side); D = 7168, Hs = 8192 230 -> 219 and 231 -> 223.
 _DECODE_SHARED_TOKENS = 64
 # Up to this many bytes of weights a call is over before the host has issued it: one chain of launches, with the token
 # rows gathered in the up-projection instead of a permute, and the shared expert inside the two GEMMs instead of beside
@@ -408,9 +410,10 @@ _FEW_TILES, _FEW_DECODE_UP, _FEW_DECODE_DOWN, _FEW_DECODE_SHARED, _FEW_ONE_CHAIN
 
 
 def _streams_weights(groups, K, n_out):
-    """Where the decode GEMM is the faster one: contractions up to 2304 and projections up to 1 GB. Beyond, its times
-    scatter with where the weights lie in memory (256 experts, 15.0 and 7.5 GB: 2415 and 1203 us with 128-row tiles, 2190 to
-    2760 and 1111 to 1600 here; 8 experts, K = 4096 and 14336: 333 and 156, here 300 to 375 and 155 to 205)."""
+    """Where the decode GEMM was measured to be the faster one: contractions up to 2304 and projections up to 1 GB. At the
+    larger ones measured its times scatter with where the weights lie in memory (256 experts, 15.0 and 7.5 GB: 2415 and 1203
+    us with 128-row tiles, 2190 to 2760 and 1111 to 1600 here; 8 experts, K = 4096 and 14336: 333 and 156, here 300 to 375 and
+    155 to 205). Contractions between 2304 and 4096 were not measured, and why the times scatter is open."""
     return K <= 2304 and groups * n_out * K * 2 <= 1 << 30
 
 
@@ -511,7 +514,8 @@ class _FusedMoEFunction(torch.autograd.Function):
             rt + o_lg, rt + o_w, rt + o_idx, rt + o_lse, counts.data_ptr(), rt + o_ts, rt + o_pos, rt + o_src, rt + o_stats,
             aux.data_ptr(), z.data_ptr(), dropped.data_ptr(), p_ws, ws_bytes, p(Xg) or p_xg, p(pre), p(act) or p_act,
             p(Y) or p_y, p(s_act) or p_sact, p(s_pre), p_sout, p_xq, p_xs, p_aq, p_as, out.data_ptr(),
-            p(ops.status_tensor(dev)), ops.reported_word(dev), ops._stream(), _side_handle("shared") if has_shared and _OVERLAP and not few & _FEW_ONE_CHAIN else 0,
+            p(ops.status_tensor(dev)), ops.reported_word(dev), ops._stream(),
+            _side_handle("shared") if has_shared and _OVERLAP and not few & _FEW_ONE_CHAIN else 0,
             0 if add is None or cfg.addend_ready is None else cfg.addend_ready.cuda_event)
         ops.layer_call(_lib.load().ffm_layer_forward, block, ops.FORWARD_SITES)
         if add is not None and cfg.addend_ready is not None:
