@@ -688,7 +688,6 @@ class _EPPlan:
             return self.px.exchange(rows, cnt, region, dry=_EP_DRY_EXCHANGE), True
         in_splits = cnt[self.rank]
         out_splits = [cnt[s][self.rank] for s in range(self.ep)]
-        rows = rows[:sum(in_splits)]  # slots without an expert (NaN scores) have no row to send
         if _EP_DRY_EXCHANGE:
             return rows.new_zeros(sum(out_splits), rows.shape[1]), False
         ops.a2a_bytes_sent += (sum(in_splits) - in_splits[self.rank]) * rows.shape[1] * rows.element_size()
