@@ -165,6 +165,7 @@ struct Ctrl {
   unsigned long long acc_empty_bar[NUM_ACC];
   uint32_t tmem_base;
   int abort_flag;
+  unsigned long long drain_bar;  // after an abort: the MMAs in flight
   unsigned long long pre_bar[EPI_WARPS][3];  // GLU-backward epilogue: "pre-activation boxes have landed", per warp and buffer
   unsigned long long help_bar[EPI_WARPS][3];  // ... and "the helper warp has written its half of the step"
   unsigned long long free_bar[EPI_WARPS][3];  // GLU epilogue with helpers: "the step's staging boxes may be overwritten"
@@ -451,6 +452,7 @@ ffm_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         }
       }
     }
+    mbar_init(smem_u32(&ctrl->drain_bar), 1);
     ctrl->abort_flag = 0;
     fence_barrier_init();
     tma_prefetch_desc(&tmA);
@@ -917,7 +919,28 @@ ffm_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   // ---- common exit: every role reaches this point, also after an abort ----------------------
   tc_fence_before();
   __syncthreads();
-  if (CTA2) cluster_sync_all();  // neither CTA leaves while its peer may still touch its barriers or operands
+  if (CTA2) {
+    if (*abort_flag != 0 && threadIdx.x == 0) st_shared_cluster(map_to_cta(smem_u32(&ctrl->abort_flag), rank ^ 1u), 1u);
+    cluster_sync_all();  // neither CTA leaves while its peer may still touch its barriers or operands
+  }
+  if (*abort_flag != 0) {
+    // MMAs and loads that nobody waited for must not land in TMEM or shared memory that has been given back. No role issues
+    // any more; which loads of a pair are out is known to neither of its CTAs, so they get time: a load takes a few
+    // microseconds, this is about half a millisecond.
+    if (threadIdx.x == 32 && leader) {
+      if (CTA2) {
+        umma_commit_pair(smem_u32(&ctrl->drain_bar));
+      } else {
+        umma_commit(smem_u32(&ctrl->drain_bar));
+      }
+      mbar_drain(smem_u32(&ctrl->drain_bar), 0);
+    }
+    const long long t0 = clock64();
+    while (clock64() - t0 < 1000000LL) {
+    }
+    __syncthreads();
+    if (CTA2) cluster_sync_all();
+  }
   if (warp == 1) {
     tc_fence_after();
     if (CTA2) {

@@ -575,3 +575,40 @@ def test_kernel_timer_merges_overlapping_launches():
     assert both < totals["a"][1] + totals["b"][1]          # the two sleeps ran at the same time
     assert abs(timer.union_ms(("a", "b"), exclude=("b",)) - totals["a"][1]) < 1e-3
     assert timer.union_ms(("missing",)) == 0.0
+
+
+@pytest.mark.parametrize("pair", [0, 1])
+def test_a_wait_that_runs_out_ends_the_gemm(pair):
+    """With the shortest wait a CTA (or a pair) may give up: it reports that, lets what it has in flight land, and the next
+    launch is right."""
+    torch.manual_seed(3)
+    lib = _lib.load()
+    A, B = (torch.randn(2048, 2048, device=DEV).bfloat16() for _ in range(2))
+    pre = torch.randn(2048, 4096, device=DEV).bfloat16()
+    ts = torch.tensor([0, 16], dtype=torch.int32, device=DEV)
+
+    def launches():
+        yield ops.grouped_gemm(A, B, _lib.B_KMAJOR, 1, None, 2048, 2048)
+        yield ops.grouped_gemm(A, B, _lib.B_NMAJOR, 1, None, 2048, 2048)
+        yield ops.grouped_gemm_glu(A, B, B, 2048, 1, None, 2048, 2048, "swiglu", want_preact=True)[0]
+        yield ops.grouped_gemm_dact_glu_backward(A, B, 1, None, 2048, 2048, pre, "swiglu")
+        yield ops.grouped_gemm_wgrad(A, B, 1, ts)
+
+    old_pair = lib.ffm_set_gemm_cta_pair(pair)
+    try:
+        want = list(launches())
+        ops.check_status()
+        old = lib.ffm_set_wait_cycles(1)
+        try:
+            for _ in range(2):
+                list(launches())
+            torch.cuda.synchronize()
+        finally:
+            lib.ffm_set_wait_cycles(old)
+        assert int(ops.status_tensor(A.device).item()) in (0, 101, 102, 103)
+        ops.status_tensor(A.device).zero_()
+        for got, ref in zip(launches(), want):
+            assert torch.equal(got, ref)
+        ops.check_status()
+    finally:
+        lib.ffm_set_gemm_cta_pair(old_pair)
