@@ -500,11 +500,12 @@ ffm_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 
   const uint32_t tmem_base = ctrl->tmem_base;
   volatile int* abort_flag = &ctrl->abort_flag;
+  bool issuer = false;  // the thread that issues this CTA's MMAs
 
   // ---- roles -------------------------------------------------------------------------------
   if (warp == 0) {
     // ================= TMA producer =================
-    if (lane == 0) {
+    if (elect_one()) {
       TileWalker<GROUPK, CTA2> walker(p, ctrl->tile_start, rank);
       TileCoord t;
       int stage = 0;
@@ -582,7 +583,11 @@ ffm_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     }
   } else if (warp == 1) {
     // ================= MMA issuer (with CTA2: only in the even CTA of the pair) =================
-    if (lane == 0 && leader) {
+    // Who issues decides how fast: with `lane == 0` instead of an elected lane every GEMM of a layer was slower (8 x 4096
+    // rows, D 1024, H 2048, in us, one card: up 226 -> 220, down 102 -> 97, dW_down 109 -> 103, dX 197 -> 191, dW_up 199 ->
+    // 190; dAct + GLU backward 164 either way, its epilogue is the slower side; 8192^3 774 -> 753).
+    if (leader && elect_one()) {
+      issuer = true;
       constexpr uint32_t idesc = FP8 ? make_idesc_e4m3(CTA2 ? 256 : 128, BN)
                                      : make_idesc_bf16(CTA2 ? 256 : 128, BN, A_MN, B_MN);
       TileWalker<GROUPK, CTA2> walker(p, ctrl->tile_start, rank);
@@ -927,7 +932,7 @@ ffm_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     // MMAs and loads that nobody waited for must not land in TMEM or shared memory that has been given back. No role issues
     // any more; which loads of a pair are out is known to neither of its CTAs, so they get time: a load takes a few
     // microseconds, this is about half a millisecond.
-    if (threadIdx.x == 32 && leader) {
+    if (issuer) {
       if (CTA2) {
         umma_commit_pair(smem_u32(&ctrl->drain_bar));
       } else {

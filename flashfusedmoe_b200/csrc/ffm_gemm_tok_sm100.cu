@@ -293,6 +293,7 @@ ffm_gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 
   const uint32_t tmem_base = ctrl->tmem_base;
   volatile int* abort_flag = &ctrl->abort_flag;
+  bool issuer = false;  // the thread that issues the MMAs
   Walker walker(ctrl, p, S::FEATS);
   Tile t;
 
@@ -303,6 +304,8 @@ ffm_gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     uint32_t phase = 0;
     int filled = 0;
     bool ok = true;
+    const bool producer = elect_one();
+    const int producer_lane = __ffs(__ballot_sync(0xffffffffu, producer)) - 1;
     while (ok && walker.next(t)) {
       const int f0 = t.f_tile * S::FEATS;
       const CUtensorMap* mA = t.shared ? &tmA1 : &tmA;
@@ -317,7 +320,7 @@ ffm_gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         }
         __syncwarp();
       }
-      if (lane == 0) {
+      if (producer) {
         for (int kb = 0; kb < k_blocks; ++kb) {
           ok = mbar_wait_bounded(smem_u32(&ctrl->empty_bar[stage]), phase ^ 1u, abort_flag, p.status,
                                  FFM_STATUS_WAIT_PRODUCER, p.wait_cycles);
@@ -344,12 +347,14 @@ ffm_gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           }
         }
       }
-      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;  // also: the token list is overwritten only after its last use
+      // also: the token list is overwritten only after its last use
+      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, producer_lane) != 0;
     }
-    if (lane == 0) ctrl->filled = filled;
+    if (producer) ctrl->filled = filled;
   } else if (warp == 1) {
     // ================= MMA issuer =================
-    if (lane == 0) {
+    if (elect_one()) {
+      issuer = true;
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
@@ -475,7 +480,7 @@ ffm_gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       for (int f = max(ctrl->filled - STAGES, 0); f < ctrl->filled; ++f) {
         mbar_drain(smem_u32(&ctrl->full_bar[f % STAGES]), (f / STAGES) & 1);
       }
-    } else if (threadIdx.x == 32) {
+    } else if (issuer) {
       umma_commit(smem_u32(&ctrl->drain_bar));
       mbar_drain(smem_u32(&ctrl->drain_bar), 0);
     }
