@@ -185,8 +185,19 @@ struct TileCoord {
 
 // Walks the tiles of this CTA (or CTA pair) in launch order. The unit is one MMA tile: 128 rows, or with CTA2
 // a pair of consecutive 128-row tiles (segments are aligned to 256 rows, so a pair never straddles experts).
-// Grouped-M order is expert-major, then N block, then M (M fastest), so CTAs running side by side share one
-// weight tile through L2.
+// Order: expert by expert, and inside an expert (grouped-K: inside its weight gradient) in bands of about BAND_UNITS
+// units, N block by N block, M fastest. The 74 pairs then work on about 9 x 8 tiles at a time and read 17 operand panels
+// (256 rows or columns x K) between them. Without bands, M fastest over the whole expert, they read 75 where an expert is
+// 74 units high: dW_up at 8 x ~2000 rows, 28672 x 4096, read its gradients again for each of its 16 N blocks, which cost
+// power above all (922 MHz under the cap): 2989 -> 2557 us, back to back 3644 -> 2956. 8192^3 753 -> 710 us, back to back
+// 908 -> 844 (cuBLAS 693 and 794). With few N blocks (8 x 4096 rows, K 4096, 1024 columns: 4) 191 -> 186 us. Bands of 5 or
+// 6, or of 11, are 0-2 % slower than 8 on these, of 3 up to 6 %.
+// One band where the expert's rows stay in L2 (a third of it) and its columns, more of them than rows, stream past once:
+// each band would read those again. 4096 x 14336, 8 x ~2000 rows deep: 1247 us, in bands 1280; up-projection of K 4096
+// to 2 x 14336: 3138 us back to back, in bands 3176.
+constexpr int BAND_UNITS = 8;
+constexpr long long BAND_L2_BYTES = 40ll << 20;
+
 template <int GROUPK, int CTA2>
 struct TileWalker {
   const int* ts;             // cumulative tiles to walk (shared memory)
@@ -217,17 +228,28 @@ struct TileWalker {
     g = 0;
   }
 
+  // unit and N block of the r-th tile of a group that is `cnt` units high and `depth` 64-deep K blocks deep
+  __device__ int place(int r, int cnt, int depth, int& n_block) const {
+    const long long panel = static_cast<long long>(CTA2 ? 2 * BM : BM) * BK * 2 * depth;
+    int bands = (cnt + BAND_UNITS / 2) / BAND_UNITS;
+    if (bands < 1 || (n_tiles > cnt && cnt * panel <= BAND_L2_BYTES)) bands = 1;
+    const int height = (cnt + bands - 1) / bands;
+    const int m0 = r / (height * n_tiles) * height;
+    const int h = min(height, cnt - m0);
+    const int q = r - m0 * n_tiles;
+    n_block = q / h;
+    return m0 + q % h;
+  }
+
   __device__ bool next(TileCoord& t) {
     if (cur >= total) return false;
     int unit;
     if (GROUPK) {
       const int per_group = m_units_per_group * n_tiles;
       t.group = static_cast<int>(cur / per_group);
-      const int r = static_cast<int>(cur % per_group);
-      unit = r % m_units_per_group;
-      t.n_block = r / m_units_per_group;
       t.k_row0 = ts[t.group] * BM;
       t.k_blocks = (ts[t.group + 1] - ts[t.group]) * (BM / BK);
+      unit = place(static_cast<int>(cur % per_group), m_units_per_group, t.k_blocks, t.n_block);
       t.k_full = t.k_blocks;
       t.k_tail = 0;
       if (k_rows != nullptr) {
@@ -242,8 +264,7 @@ struct TileWalker {
       const int cnt = units(ts[g + 1]) - u0;
       const int r = static_cast<int>(cur - static_cast<long long>(u0) * n_tiles);
       t.group = g;
-      t.n_block = r / cnt;
-      unit = (layout_ts != nullptr ? units(__ldg(layout_ts + g)) : u0) + r % cnt;
+      unit = (layout_ts != nullptr ? units(__ldg(layout_ts + g)) : u0) + place(r, cnt, k_blocks, t.n_block);
       t.k_row0 = 0;
       t.k_blocks = k_blocks;
     }
