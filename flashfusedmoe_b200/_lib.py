@@ -5,10 +5,12 @@ library raises, there is no fallback.
 """
 
 import ctypes
+import importlib.util
 import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libffmoe.so")
+NATIVE_PATH = os.path.join(_HERE, "_native.so")
 
 c_void_p = ctypes.c_void_p
 c_int = ctypes.c_int
@@ -98,6 +100,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_native = None
 
 
 def load():
@@ -116,6 +119,24 @@ def load():
         fn.argtypes = argtypes
     _lib = lib
     return lib
+
+
+def native():
+    """The torch side of the layer driver (csrc/ffm_torch.cpp, built beside libffmoe.so), bound to that library's functions."""
+    global _native
+    if _native is None:
+        lib = load()
+        if not os.path.exists(NATIVE_PATH):
+            raise RuntimeError(f"{NATIVE_PATH} is missing: build it with `python -m flashfusedmoe_b200.build`.")
+        import torch  # noqa: F401  (the extension links against its libraries)
+        spec = importlib.util.spec_from_file_location(__package__ + "._native", NATIVE_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        module.bind(*(ctypes.cast(getattr(lib, name), c_void_p).value for name in (
+            "ffm_layer_forward", "ffm_layer_backward", "ffm_rows_capacity", "ffm_route_workspace_bytes",
+            "ffm_route_backward_workspace_bytes")))
+        _native = module
+    return _native
 
 
 def error_string(code):

@@ -232,10 +232,6 @@ def _dense_ts(rows, device, split=1):
     return t
 
 
-def _device_tensor(t, name):
-    return ops._req(t, torch.bfloat16, name)
-
-
 def _side_handle(name):
     """cudaStream_t of a side stream. The shared expert's chain is the longest beside the routing kernels: its stream has
     priority."""
@@ -447,160 +443,66 @@ class _FusedMoEFunction(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, hidden_states, gate_weight, w_up, w_down, addend, sw_gate, sw_up, sw_down, cfg, dtype):
+        assert addend is None or sw_gate is None, "either an addend or shared expert weights"
         N, D = hidden_states.shape
-        E = gate_weight.shape[0]
-        H = w_up.shape[1] // 2
-        k = cfg.top_k
-        h = _device_tensor(_to(hidden_states, dtype), "hidden")
-        g = _to(gate_weight, dtype)
-        wu = _to(w_up, dtype)
-        wd = _to(w_down, dtype)
-        add = None if addend is None else _device_tensor(_to(addend, dtype), "addend")
+        E, H, k = gate_weight.shape[0], w_up.shape[1] // 2, cfg.top_k
         need_grad = cfg.wants_grad and any(ctx.needs_input_grad[:8])
-        keep = need_grad and not cfg.recompute
-        dev = h.device
-        has_shared = sw_gate is not None
-        Hs = 0
-        swg = swu = swd = None
-        if has_shared:
-            assert add is None, "either an addend or shared expert weights"
-            swg, swu, swd = (_device_tensor(_to(w, dtype), "shared expert weight") for w in (sw_gate, sw_up, sw_down))
-            Hs = swg.shape[0]
-        h_route = _jittered(h, cfg, hidden_states.requires_grad)
-        bias = cfg.expert_bias
-        if bias is not None:
-            bias = ops._req(bias.to(torch.float32).contiguous(), torch.float32, "expert_bias")
-        fp8 = _EXPERT_GEMM == "fp8" and D % 128 == 0 and H % 128 == 0
-        few = 0 if need_grad else _few_rows(N, D, E, k, H, cfg.capacity is not None, swg, swu)
-        fp8 = fp8 and not few & _FEW_TILES
-        if fp8:
-            (wuq, wus), (wdq, wds) = _quantized_weight(w_up, wu), _quantized_weight(w_down, wd)
-
-        rows, ws_bytes, _ = ops.layer_sizes(N, D, E, k)
-        rt_bytes, o_w, o_idx, o_lg, o_lse, o_ts, o_pos, o_src, o_stats = ops.routing_layout(N, E, k)
-        out = torch.empty(N, D, dtype=dtype, device=dev)
-        counts = torch.empty(E, dtype=torch.int32, device=dev)
-        aux = torch.empty((), dtype=torch.float32, device=dev)
-        z = torch.empty((), dtype=torch.float32, device=dev)
-        dropped = torch.empty(1, dtype=torch.int32, device=dev)
-        # Kept for the backward pass: tensors; everything else is scratch. All of it is allocated on the current stream,
-        # which the side streams are forked from and joined to inside the call.
-        routing = Xg = pre = act = Y = s_act = s_pre = None
-        if need_grad:
-            routing = torch.empty(rt_bytes, dtype=torch.uint8, device=dev)
-            Xg = torch.empty(rows, D, dtype=dtype, device=dev)
-            if has_shared:
-                s_act = torch.empty(N, Hs, dtype=dtype, device=dev)
-                s_pre = torch.empty(N, 2 * Hs, dtype=dtype, device=dev)
-        if keep:
-            pre = torch.empty(rows, 2 * H, dtype=dtype, device=dev)
-            act = torch.empty(rows, H, dtype=dtype, device=dev)
-            Y = torch.empty(rows, D, dtype=dtype, device=dev)
-        (rt, p_xg, p_sact, p_act, p_y, p_sout, p_ws, p_xq, p_xs, p_aq, p_as), scratch = ops.scratch_buffers(dev, (
-            0 if need_grad else rt_bytes, 0 if need_grad else rows * D * 2, 0 if need_grad else N * Hs * 2,
-            0 if keep else rows * H * 2, 0 if keep else rows * D * 2, N * D * 2 if has_shared else 0, ws_bytes,
-            *((rows * D, rows * 4, rows * H, rows * 4) if fp8 else (0, 0, 0, 0))))
-        if need_grad:
-            rt = routing.data_ptr()
-        p = ops._ptr
-        block = ops.LAYER_FORWARD_ARGS.pack(
-            N, D, E, k, H, Hs, rows, _lib.GATING[cfg.gating], _lib.ACTIVATION[cfg.activation],
-            _lib.ACTIVATION[cfg.shared_activation], 1 if cfg.pre_softmax else 0, cfg.n_group, cfg.topk_group,
-            -1 if cfg.capacity is None else cfg.capacity, 1 if need_grad else 0, few, 1 if fp8 else 0,
-            1 if _OVERLAP else 0,
-            cfg.weight_scale, cfg.aux_loss_coeff * E / (float(N) * float(N)), cfg.z_loss_coeff / float(N),
-            h.data_ptr(), h_route.data_ptr(), g.data_ptr(), wu.data_ptr(), wd.data_ptr(), p(bias), p(add), p(swg), p(swu),
-            p(swd), *((p(wuq), p(wus), p(wdq), p(wds)) if fp8 else (0, 0, 0, 0)),
-            rt + o_lg, rt + o_w, rt + o_idx, rt + o_lse, counts.data_ptr(), rt + o_ts, rt + o_pos, rt + o_src, rt + o_stats,
-            aux.data_ptr(), z.data_ptr(), dropped.data_ptr(), p_ws, ws_bytes, p(Xg) or p_xg, p(pre), p(act) or p_act,
-            p(Y) or p_y, p(s_act) or p_sact, p(s_pre), p_sout, p_xq, p_xs, p_aq, p_as, out.data_ptr(),
-            p(ops.status_tensor(dev)), ops.reported_word(dev), ops._stream(),
-            _side_handle("shared") if has_shared and _OVERLAP and not few & _FEW_ONE_CHAIN else 0,
-            0 if add is None or cfg.addend_ready is None else cfg.addend_ready.cuda_event)
-        ops.layer_call(_lib.load().ffm_layer_forward, block, ops.FORWARD_SITES)
-        if add is not None and cfg.addend_ready is not None:
-            add.record_stream(torch.cuda.current_stream())
+        weights = (w_up, w_down, sw_gate, sw_up, sw_down)
+        few, quantized = 0, (None, None, None, None)
+        if not need_grad:
+            if sw_gate is not None:   # cast here: which kernels run depends on where the copies lie
+                weights = (w_up, w_down, *(_to(w, dtype) for w in (sw_gate, sw_up, sw_down)))
+            few = _few_rows(N, D, E, k, H, cfg.capacity is not None, weights[2], weights[3])
+        if _EXPERT_GEMM == "fp8" and D % 128 == 0 and H % 128 == 0 and not few & _FEW_TILES:
+            weights = (_to(w_up, dtype), _to(w_down, dtype), *weights[2:])
+            quantized = _quantized_weight(w_up, weights[0]) + _quantized_weight(w_down, weights[1])
+        dev = hidden_states.device
+        pairs, timer = ops.timed(ops.FORWARD_SITES)
+        done, out, aux, z, counts, dropped, saved = _lib.native().layer_forward(
+            hidden_states, gate_weight, weights[0], weights[1], addend, *weights[2:], cfg.expert_bias, *quantized, k,
+            _lib.GATING[cfg.gating], _lib.ACTIVATION[cfg.activation], _lib.ACTIVATION[cfg.shared_activation],
+            cfg.pre_softmax, cfg.n_group, cfg.topk_group, -1 if cfg.capacity is None else cfg.capacity, need_grad,
+            cfg.recompute, few, _OVERLAP, cfg.input_jitter if hidden_states.requires_grad else 0.0, cfg.weight_scale,
+            cfg.aux_loss_coeff * E / (float(N) * float(N)), cfg.z_loss_coeff / float(N), ops.status_tensor(dev).data_ptr(),
+            ops.reported_word(dev), ops._stream(),
+            _side_handle("shared") if sw_gate is not None and _OVERLAP and not few & _FEW_ONE_CHAIN else 0,
+            0 if addend is None or cfg.addend_ready is None else cfg.addend_ready.cuda_event, timer)
+        ops.launched(done, pairs, ops.FORWARD_SITES)
+        if addend is not None and cfg.addend_ready is not None:
+            addend.record_stream(torch.cuda.current_stream())
 
         ctx.set_materialize_grads(False)
         ctx.cfg = cfg
-        ctx.shape = (N, D, E, H, Hs)
-        ctx.in_dtypes = (hidden_states.dtype, gate_weight.dtype, w_up.dtype, w_down.dtype,
-                         None if addend is None else addend.dtype) + tuple(
-                             None if w is None else w.dtype for w in (sw_gate, sw_up, sw_down))
-        ctx.kept = keep
-        ctx.has_shared = has_shared and need_grad
+        ctx.in_dtypes = tuple(None if t is None else t.dtype for t in (
+            hidden_states, gate_weight, w_up, w_down, addend, sw_gate, sw_up, sw_down))
         if need_grad:
-            ctx.save_for_backward(h, g, wu, wd, routing, counts, Xg, pre, act, Y, s_act, s_pre, swg, swu, swd)
+            ctx.save_for_backward(*saved)
         ctx.mark_non_differentiable(counts, dropped)
         return out, aux, z, counts, dropped
 
     @staticmethod
     def backward(ctx, grad_out, grad_aux, grad_z, _grad_counts, _grad_dropped):
         cfg = ctx.cfg
-        N, D, E, H, Hs = ctx.shape
-        k = cfg.top_k
-        (h, g, wu, wd, routing, counts, Xg, pre, act, Y, s_act, s_pre, swg, swu, swd) = ctx.saved_tensors
-        dev, dtype = h.device, h.dtype
-        # saved-tensor hooks may have handed back other tensors than were saved
-        for t in (h, g, wu, wd, Xg, pre, act, Y, s_act, s_pre, swg, swu, swd):
-            if t is not None:
-                _device_tensor(t, "saved tensor")
-        ops._req(routing, torch.uint8, "saved tensor")
-        ops._req(counts, torch.int32, "saved tensor")
-        shared = ctx.has_shared
-        if not shared:
-            Hs = 0
-        rows, _, ws_bytes = ops.layer_sizes(N, D, E, k)
-        _, o_w, o_idx, o_lg, o_lse, o_ts, o_pos, o_src, _ = ops.routing_layout(N, E, k)
-        if grad_out is None:
-            grad_out = torch.zeros(N, D, dtype=dtype, device=dev)
-        go = _device_tensor(_to(grad_out, dtype), "go")  # also densifies expanded (stride-0) gradients
+        saved = ctx.saved_tensors
+        dev, N, E = saved[0].device, saved[0].shape[0], saved[1].shape[0]
         # the softmax aux loss carries no gradient on the reference's fast path ("reference_cuda")
         if not (cfg.aux_loss_coeff > 0.0 and (cfg.aux_grad == "analytic" or cfg.gating == "sigmoid")):
             grad_aux = None
         if cfg.z_loss_coeff <= 0.0:
             grad_z = None
-        grad_aux, grad_z = (None if t is None else t.to(torch.float32) for t in (grad_aux, grad_z))
-        # [D, Hs] has few output tiles (32 CTA-pair tiles at D = 1024, Hs = 2048 for 74 pairs): split the token dimension
-        # in two halves, each accumulated in fp32, and add the two bf16 results
-        split = 2 if (N + 127) // 128 >= 64 and (D // 256) * ((Hs + 255) // 256) <= 40 else 1
-
-        def empty(*shape):
-            return torch.empty(*shape, dtype=dtype, device=dev)
-
-        dH, d_gate, d_wu, d_wd = empty(N, D), empty(E, D), empty(E, 2 * H, D), empty(E, D, H)
-        s_dw = s_dwd = None
-        if shared:
-            s_dw, s_dwd = empty(2 * Hs, D), empty(D, Hs)
-        fused = 1 if _FUSED_GLU_BWD else 0
-        (p_gyw, p_gw, p_gu, p_dxg, p_dhr, p_ws, p_dact, p_sgu, p_sdact, p_sdx, p_sparts, p_pre, p_act,
-         p_y), scratch = ops.scratch_buffers(dev, (
-             rows * D * 2, N * k * 4, rows * 4 * H, rows * D * 2, N * D * 2, ws_bytes, 0 if fused else rows * H * 2,
-             N * Hs * 4, 0 if fused else N * Hs * 2, N * D * 2 if shared else 0, 2 * D * Hs * 2 if split == 2 else 0,
-             *((0, 0, 0) if ctx.kept else (rows * H * 4, rows * H * 2, rows * D * 2))))
-        rt = routing.data_ptr()
-        p = ops._ptr
-        names = ("shared", "backward_route", "backward_gemm", "small")
-        block = ops.LAYER_BACKWARD_ARGS.pack(
-            N, D, E, k, H, Hs, rows, _lib.GATING[cfg.gating], _lib.ACTIVATION[cfg.activation],
-            _lib.ACTIVATION[cfg.shared_activation], 0 if ctx.kept else 1, 0 if cfg.capacity is None else 1, fused,
-            1 if _OVERLAP else 0, split,
-            cfg.aux_loss_coeff * E / float(N), cfg.z_loss_coeff,
-            go.data_ptr(), h.data_ptr(), g.data_ptr(), wu.data_ptr(), wd.data_ptr(), p(swg), p(swu), p(swd), p(grad_aux),
-            p(grad_z), rt + o_w, rt + o_idx, rt + o_lg, rt + o_lse, counts.data_ptr(), rt + o_ts, rt + o_pos, rt + o_src,
-            Xg.data_ptr(), p(pre) or p_pre, p(act) or p_act, p(Y) or p_y, p(s_act), p(s_pre),
-            dH.data_ptr(), d_gate.data_ptr(), d_wu.data_ptr(), d_wd.data_ptr(), p(s_dw), p(s_dwd), p_gyw, p_gw, p_gu,
-            p_dxg, p_dhr, p_dact, p_sgu, p_sdact, p_sdx, p_sparts, p_ws, ws_bytes,
-            p(ops.status_tensor(dev)), ops._stream(), *((_side_handle(n) if _OVERLAP else 0) for n in names))
-        ops.layer_call(_lib.load().ffm_layer_backward, block, ops.BACKWARD_SITES, fused_glu=bool(fused))
-
         dt = ctx.in_dtypes
-        d_add = None
-        if dt[4] is not None and ctx.needs_input_grad[4]:
-            d_add = go.to(dt[4])
+        pairs, timer = ops.timed(ops.BACKWARD_SITES)
+        done, dH, d_gate, d_wu, d_wd, s_gate, s_up, s_down, go = _lib.native().layer_backward(
+            grad_out, grad_aux, grad_z, *saved, cfg.top_k, _lib.GATING[cfg.gating], _lib.ACTIVATION[cfg.activation],
+            _lib.ACTIVATION[cfg.shared_activation], cfg.capacity is not None, _FUSED_GLU_BWD, _OVERLAP,
+            cfg.aux_loss_coeff * E / float(N), cfg.z_loss_coeff, ops.status_tensor(dev).data_ptr(), ops._stream(),
+            *((_side_handle(n) if _OVERLAP else 0) for n in ("shared", "backward_route", "backward_gemm", "small")), timer)
+        ops.launched(done, pairs, ops.BACKWARD_SITES, fused_glu=_FUSED_GLU_BWD)
+
+        d_add = go.to(dt[4]) if dt[4] is not None and ctx.needs_input_grad[4] else None
         s_grads = (None, None, None)
-        if shared:
-            s_grads = (s_dw[:Hs].to(dt[5]), s_dw[Hs:].to(dt[6]), s_dwd.to(dt[7]))
+        if s_gate is not None:
+            s_grads = (s_gate.to(dt[5]), s_up.to(dt[6]), s_down.to(dt[7]))
         return (dH.to(dt[0]), d_gate.to(dt[1]), d_wu.to(dt[2]), d_wd.to(dt[3]), d_add) + s_grads + (None, None)
 
 

@@ -8,7 +8,6 @@ or without the built library every call raises.
 import ctypes
 import struct
 from dataclasses import dataclass
-from functools import lru_cache
 
 import torch
 
@@ -625,7 +624,7 @@ def route_backward(gw, routing, gaux, gz, hidden, gate_w, gating, dH=None):
 # ----------------------------------------------------------------------------------------------
 
 # argument blocks as include/ffmoe.h declares them (64-bit integers and pointers, doubles in between) without the last
-# two fields, timer and launched
+# two fields, timer and launched, for callers that pack them by hand (csrc/ffm_torch.cpp fills the structs themselves)
 LAYER_FORWARD_ARGS = struct.Struct("=18q3d45q")
 LAYER_BACKWARD_ARGS = struct.Struct("=15q2d48q")
 
@@ -644,70 +643,30 @@ BACKWARD_SITES = (_GLU, _GEMM, ("combine_backward", None, "ffm_combine_backward"
                   _WGRAD, _GEMM, _WGRAD, ("combine_forward", None, "ffm_combine_forward"))
 
 
-def layer_call(fn, block, sites, fused_glu=True):
-    """Run ffm_layer_forward / ffm_layer_backward on a packed argument block (all fields but the last two, timer and
-    launched). Counts its launches and, with a timer installed, files an event pair per launch site."""
+def timed(sites):
+    """(event pairs and the array of their handles, its address) for a call of layer_forward / layer_backward whose launch
+    sites are `sites`; (None, 0) without a timer."""
+    if _timer is None:
+        return None, 0
+    pairs = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)) for _ in sites]
+    for a, b in pairs:
+        a.record()
+        b.record()
+    handles = (ctypes.c_int64 * (2 * len(sites)))(*(e.cuda_event for pair in pairs for e in pair))
+    return (pairs, handles), ctypes.addressof(handles)
+
+
+def launched(done, pairs, sites, fused_glu=True):
+    """Counts the launches of a finished call, files its event pairs and raises its error. `done`: return code, kernels
+    enqueued, bit mask of the sites that ran, site of the error; `pairs`: what timed() gave."""
     global launch_count
-    launched = (ctypes.c_int64 * 3)()
-    pairs = handles = None
-    if _timer is not None:
-        pairs = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)) for _ in sites]
-        for a, b in pairs:
-            a.record()
-            b.record()
-        handles = (ctypes.c_int64 * (2 * len(sites)))(*(e.cuda_event for pair in pairs for e in pair))
-    tail = struct.pack("=2q", 0 if handles is None else ctypes.addressof(handles), ctypes.addressof(launched))
-    rc = fn(block + tail)
-    launch_count += launched[0]
+    rc, kernels, ran, site = done
+    launch_count += kernels
     if pairs is not None:
-        for i, (pair, (name, also, _)) in enumerate(zip(pairs, sites)):
-            if launched[1] >> i & 1:
+        for i, (pair, (name, also, _)) in enumerate(zip(pairs[0], sites)):
+            if ran >> i & 1:
                 _timer.events.setdefault(name, []).append(pair)
                 if also is not None and fused_glu:
                     _timer.events.setdefault(also, []).append(pair)
     if rc != _lib.FFM_OK:
-        site = launched[2]
         _lib.check(rc, sites[site][2] if site >= 0 else "stream fork or join")
-
-
-# Scratch buffers from this size on are allocations of their own: one block for all of them would be larger than anything
-# a program frees again, so that the allocator could not serve it from what it holds.
-_OWN_ALLOCATION = 16 << 20
-
-
-def scratch_buffers(device, sizes):
-    """(device addresses, the tensors that hold them) of scratch buffers of the given byte sizes, 256-byte aligned; 0 for a
-    size of 0. Small ones share one allocation."""
-    keep, where, shared = [], [], 0
-    for n in sizes:
-        if n >= _OWN_ALLOCATION:
-            keep.append(torch.empty(n, dtype=torch.uint8, device=device))
-            where.append(-keep[-1].data_ptr())
-        else:
-            where.append(shared if n else None)
-            shared += (n + 255) // 256 * 256
-    base = 0
-    if shared:
-        keep.append(torch.empty(shared, dtype=torch.uint8, device=device))
-        base = keep[-1].data_ptr()
-    return [0 if w is None else (-w if w < 0 else base + w) for w in where], keep
-
-
-@lru_cache(maxsize=1024)
-def layer_sizes(N, D, E, k):
-    """(rows_cap, forward workspace bytes, backward workspace bytes)."""
-    lib = _lib.load()
-    return (rows_capacity(N * k, E), int(lib.ffm_route_workspace_bytes(N, E, k)),
-            int(lib.ffm_route_backward_workspace_bytes(N, D, E)))
-
-
-@lru_cache(maxsize=1024)
-def routing_layout(N, E, k):
-    """Offsets of the routing results kept for the backward pass in one buffer: (size, topk_w, topk_idx, logits, lse,
-    tile_start, pos, src, stats)."""
-    T = N * k
-    offsets, size = [], 0
-    for n in (T * 4, T * 4, N * E * 2, N * 4, (E + 1) * 4, T * 4, max(rows_capacity(T, E), 1) * 4, (E + 2) * 4):
-        offsets.append(size)
-        size += (n + 255) // 256 * 256
-    return (max(size, 256), *offsets)
