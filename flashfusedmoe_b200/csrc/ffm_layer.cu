@@ -43,12 +43,12 @@ class Sites {
   Sites(const int64_t* timer, int64_t* launched) : timer_(timer), launched_(launched) {
     for (int i = 0; i < 3; ++i) launched_[i] = 0;
   }
-  // chained: the launch directly follows a kernel of this library on `stream` (nothing but event records in between)
+  // chained: the launch directly follows a kernel of this library on `stream` (no event in between: with a timer there is)
   template <typename F>
   void run(int site, int kernels, ffm_stream_t stream, F&& launch, bool chained = false) {
     if (rc_ != FFM_OK) return;
     mark(2 * site, stream);
-    follows_kernel = chained;
+    follows_kernel = chained && timer_ == nullptr;
     rc_ = launch();
     follows_kernel = false;
     mark(2 * site + 1, stream);
@@ -237,9 +237,9 @@ extern "C" int ffm_layer_backward(const ffm_layer_backward_args* args) {
   Sites sites(a.timer, a.launched);
   Event start, sum_fork, sum_done, shared_done, rows_done, route_done, dx_done, join;
 
-  // Chained launches as in the forward pass, only without a shared expert: the CTAs of a GEMM placed early would take SMs
-  // from the shared expert's GEMMs while they wait.
-  const bool alone = Hs == 0;
+  // Launches of the backward pass are not chained (but for the recomputed projections): event records that other streams wait
+  // for lie between them, and with the expert GEMMs chained across one a loop of calls that filled the launch queue did not
+  // come to an end in two of six runs (3001 tokens on 16 experts), for a reason that was not found.
   if (a.recompute) {
     // recompute the three large tensors with the same kernels: bit-identical to the forward pass
     const void* up_rows = static_cast<const char*>(a.w_up) + a.H * a.D * 2;
@@ -258,7 +258,7 @@ extern "C" int ffm_layer_backward(const ffm_layer_backward_args* args) {
     if (a.zero_gw && cudaMemsetAsync(a.gw, 0, static_cast<size_t>(a.N) * k * 4, static_cast<cudaStream_t>(st)) != cudaSuccess)
       return FFM_ERR_LAUNCH;
     return ffm_combine_backward(a.go, a.Y, a.topk_w, a.src, a.rows_cap, k, D, a.gYw, a.gw, st);
-  }, alone && a.recompute && !a.zero_gw);
+  });
 
   if (Hs > 0) {
     if (overlap) sites.require(start.wait(sh));
@@ -319,10 +319,10 @@ extern "C" int ffm_layer_backward(const ffm_layer_backward_args* args) {
     sites.run(FFM_BWD_DACT, 1, st, [&] {
       return ffm_grouped_gemm_dact_glu_backward(a.gYw, a.w_down, E, a.tile_start, a.rows_cap, D, H, act, a.preact, a.gU, 0,
                                                 a.status, st);
-    }, alone && overlap);
+    });
     sites.run(FFM_BWD_WDOWN, 1, st, [&] {
       return grouped_wgrad(a.gYw, a.act, E, a.tile_start, a.counts, a.rows_cap, D, H, 1.0f, a.d_w_down, a.status, st);
-    }, alone);
+    });
   } else {
     sites.run(FFM_BWD_DACT, 1, st, [&] {
       return ffm_grouped_gemm(a.gYw, a.w_down, FFM_B_NMAJOR, E, a.tile_start, a.rows_cap, D, H, 1.0f, a.d_act, nullptr, 0,
@@ -346,7 +346,7 @@ extern "C" int ffm_layer_backward(const ffm_layer_backward_args* args) {
   sites.run(FFM_BWD_DX, 1, st, [&] {
     return ffm_grouped_gemm(a.gU, a.w_up, FFM_B_NMAJOR, E, a.tile_start, a.rows_cap, 2 * H, D, 1.0f, a.dXg, nullptr, 0,
                             a.status, st);
-  }, alone && a.fused_glu);
+  });
   if (overlap) sites.require(dx_done.order(st, gm));
   sites.run(FFM_BWD_WUP, 1, gm, [&] {
     return grouped_wgrad(a.gU, a.Xg, E, a.tile_start, a.counts, a.rows_cap, 2 * H, D, 1.0f, a.d_w_up, a.status, gm);
