@@ -77,6 +77,7 @@ SIGNATURES = {
     "ffm_glu_backward": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int64, c_int, c_int, c_void_p, c_void_p]),
     "ffm_compact_positions": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_void_p, c_void_p,
                                       c_void_p]),
+    "ffm_cast_many": (c_int, [c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p]),
     "ffm_layer_forward": (c_int, [ctypes.c_char_p]),   # packed by ops.LAYER_FORWARD_ARGS / _BACKWARD_ARGS
     "ffm_layer_backward": (c_int, [ctypes.c_char_p]),
     "ffm_route_forward_launches": (c_int, [c_int64, c_int, c_int, c_int, c_int]),
@@ -134,7 +135,7 @@ def native():
         spec.loader.exec_module(module)
         module.bind(*(ctypes.cast(getattr(lib, name), c_void_p).value for name in (
             "ffm_layer_forward", "ffm_layer_backward", "ffm_rows_capacity", "ffm_route_workspace_bytes",
-            "ffm_route_backward_workspace_bytes")))
+            "ffm_route_backward_workspace_bytes", "ffm_cast_many")))
         _native = module
     return _native
 

@@ -27,13 +27,16 @@ decltype(&ffm_layer_backward) backward_pass = nullptr;
 decltype(&ffm_rows_capacity) rows_capacity = nullptr;
 decltype(&ffm_route_workspace_bytes) forward_workspace = nullptr;
 decltype(&ffm_route_backward_workspace_bytes) backward_workspace = nullptr;
+decltype(&ffm_cast_many) cast_many = nullptr;
 
-void bind(uintptr_t forward, uintptr_t backward, uintptr_t capacity, uintptr_t forward_ws, uintptr_t backward_ws) {
+void bind(uintptr_t forward, uintptr_t backward, uintptr_t capacity, uintptr_t forward_ws, uintptr_t backward_ws,
+          uintptr_t cast) {
   forward_pass = reinterpret_cast<decltype(forward_pass)>(forward);
   backward_pass = reinterpret_cast<decltype(backward_pass)>(backward);
   rows_capacity = reinterpret_cast<decltype(rows_capacity)>(capacity);
   forward_workspace = reinterpret_cast<decltype(forward_workspace)>(forward_ws);
   backward_workspace = reinterpret_cast<decltype(backward_workspace)>(backward_ws);
+  cast_many = reinterpret_cast<decltype(cast_many)>(cast);
 }
 
 constexpr int64_t ALIGN = 256;
@@ -54,14 +57,49 @@ const Tensor& require(const Tensor& t, at::ScalarType dtype, const char* name) {
   return t;
 }
 
-// t in the compute type, contiguous
-Tensor computed(const Tensor& t, const char* name) {
+// Conversions between fp32 and bf16, collected and run in one launch.
+class Casts {
+ public:
+  static bool takes(const Tensor& t) {
+    return t.is_cuda() && t.layout() == at::kStrided && t.is_contiguous() && t.numel() > 0 &&
+           reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
+  }
+  void add(const void* src, void* dst, int64_t elements) {
+    if (count_ == FFM_CAST_MAX) throw std::logic_error("more tensors than one launch converts");
+    src_[count_] = src;
+    dst_[count_] = dst;
+    elements_[count_++] = elements;
+  }
+  // kernels enqueued
+  int64_t run(bool to_bf16, int64_t stream) {
+    if (count_ == 0) return 0;
+    const int rc = cast_many(count_, src_, dst_, elements_, to_bf16, reinterpret_cast<ffm_stream_t>(stream));
+    if (rc != FFM_OK) throw std::runtime_error("libffmoe ffm_cast_many failed: " + std::to_string(rc));
+    return 1;
+  }
+
+ private:
+  const void* src_[FFM_CAST_MAX];
+  void* dst_[FFM_CAST_MAX];
+  int64_t elements_[FFM_CAST_MAX];
+  int count_ = 0;
+};
+
+// t in the compute type, contiguous; an fp32 tensor's cast may only be entered in `casts`
+Tensor computed(const Tensor& t, const char* name, Casts* casts = nullptr) {
+  if (casts != nullptr && t.scalar_type() == at::kFloat && Casts::takes(t)) {
+    const Tensor c = at::empty(t.sizes(), t.options().dtype(at::kBFloat16));
+    casts->add(t.data_ptr(), c.data_ptr(), t.numel());
+    return c;
+  }
   Tensor c = t.scalar_type() == at::kBFloat16 ? t : t.to(at::kBFloat16);
   if (!c.is_contiguous()) c = c.contiguous();
   return require(c, at::kBFloat16, name);
 }
 
-Tensor computed(const OptTensor& t, const char* name) { return t.has_value() ? computed(*t, name) : Tensor(); }
+Tensor computed(const OptTensor& t, const char* name, Casts* casts) {
+  return t.has_value() ? computed(*t, name, casts) : Tensor();
+}
 
 template <typename T = void>
 T* ptr(const Tensor& t) {
@@ -148,10 +186,13 @@ py::tuple layer_forward(const Tensor& hidden, const Tensor& gate, const Tensor& 
                         int64_t capacity, bool need_grad, bool recompute, int64_t few, bool overlap, double jitter,
                         double weight_scale, double aux_scale, double z_scale, int64_t status, int64_t status_host,
                         int64_t stream, int64_t shared_stream, int64_t addend_ready, int64_t timer) {
-  const Tensor h = computed(hidden, "hidden"), g = computed(gate, "gate weight"), wu = computed(w_up, "w_up"),
-               wd = computed(w_down, "w_down"), add = computed(addend, "addend");
-  const Tensor swg = computed(sw_gate, "shared expert weight"), swu = computed(sw_up, "shared expert weight"),
-               swd = computed(sw_down, "shared expert weight");
+  Casts casts;
+  const Tensor h = computed(hidden, "hidden", &casts), g = computed(gate, "gate weight", &casts),
+               wu = computed(w_up, "w_up", &casts), wd = computed(w_down, "w_down", &casts),
+               add = computed(addend, "addend", &casts), swg = computed(sw_gate, "shared expert weight", &casts),
+               swu = computed(sw_up, "shared expert weight", &casts),
+               swd = computed(sw_down, "shared expert weight", &casts);
+  const int64_t cast_launches = casts.run(true, stream);
   const int64_t N = h.size(0), D = h.size(1), E = g.size(0), H = wu.size(1) / 2, Hs = swg.defined() ? swg.size(0) : 0;
   const bool keep = need_grad && !recompute, fp8 = w_up_q.has_value();
   // what the router sees; the noise is drawn as the reference draws it (fused_moe.py:329-332)
@@ -270,6 +311,7 @@ py::tuple layer_forward(const Tensor& hidden, const Tensor& gate, const Tensor& 
     py::gil_scoped_release released;
     rc = forward_pass(&a);
   }
+  launched[0] += cast_launches;
   py::list saved;
   if (need_grad) {
     for (const Tensor& t : {h, g, wu, wd, routing, counts, Xg, pre, act, Y, s_act, s_pre, swg, swu, swd}) {
@@ -279,7 +321,9 @@ py::tuple layer_forward(const Tensor& hidden, const Tensor& gate, const Tensor& 
   return py::make_tuple(outcome(rc, launched), out, aux, z, counts, dropped, saved);
 }
 
-// (outcome, dH, d_gate, d_w_up, d_w_down, shared gate, up and down gradients or None, grad_out as computed with)
+// (outcome, dH, d_gate, d_w_up, d_w_down, shared gate, up and down gradients or None, grad_out as computed with). Gradients
+// are in the compute type; with bit i of fp32_mask set the i-th of those four, of gate and up together (4) or of down (5) is
+// fp32.
 py::tuple layer_backward(const OptTensor& grad_out, const OptTensor& grad_aux, const OptTensor& grad_z, const Tensor& h,
                          const Tensor& g, const Tensor& wu, const Tensor& wd, const Tensor& routing, const Tensor& counts,
                          const Tensor& Xg, const OptTensor& pre, const OptTensor& act, const OptTensor& Y,
@@ -287,7 +331,7 @@ py::tuple layer_backward(const OptTensor& grad_out, const OptTensor& grad_aux, c
                          const OptTensor& swd, int64_t top_k, int64_t gating, int64_t activation, int64_t shared_activation,
                          bool capacity, bool fused, bool overlap, double aux_coef, double z_coef, int64_t status,
                          int64_t stream, int64_t shared_stream, int64_t route_stream, int64_t gemm_stream,
-                         int64_t small_stream, int64_t timer) {
+                         int64_t small_stream, int64_t timer, int64_t fp32_mask) {
   // saved-tensor hooks may have handed back other tensors than were saved
   for (const Tensor* t : {&h, &g, &wu, &wd, &Xg}) require(*t, at::kBFloat16, "saved tensor");
   for (const OptTensor* t : {&pre, &act, &Y, &s_act, &s_pre, &swg, &swu, &swd}) {
@@ -310,16 +354,36 @@ py::tuple layer_backward(const OptTensor& grad_out, const OptTensor& grad_aux, c
   // halves, each accumulated in fp32, and add the two bf16 results
   const int64_t split = (N + 127) / 128 >= 64 && (D / 256) * ((Hs + 255) / 256) <= 40 ? 2 : 1;
 
-  const Tensor dH = at::empty({N, D}, b16), d_gate = at::empty({E, D}, b16), d_wu = at::empty({E, 2 * H, D}, b16),
-               d_wd = at::empty({E, D, H}, b16);
-  Tensor s_dw, s_gate, s_up, s_dwd;
+  // Gradients of fp32 tensors are computed in bf16 like the others, in scratch, and converted in one launch at the end.
+  struct Grad {
+    Tensor t;             // as it is handed back
+    int64_t scratch = 0;  // bytes of the bf16 values where they are computed elsewhere
+  };
+  auto gradient = [&](int i, at::IntArrayRef shape) {
+    Grad gr;
+    const bool wide = (fp32_mask >> i & 1) != 0;
+    gr.t = at::empty(shape, wide ? b16.dtype(at::kFloat) : b16);
+    gr.scratch = wide ? gr.t.numel() * 2 : 0;
+    return gr;
+  };
+  const Grad dH = gradient(0, {N, D}), d_gate = gradient(1, {E, D}), d_wu = gradient(2, {E, 2 * H, D}),
+             d_wd = gradient(3, {E, D, H});
+  Grad s_dw, s_dwd;
+  Tensor s_gate, s_up;  // the halves of s_dw
   if (shared) {
-    s_dw = at::empty({2 * Hs, D}, b16);
-    s_gate = s_dw.narrow(0, 0, Hs);
-    s_up = s_dw.narrow(0, Hs, Hs);
-    s_dwd = at::empty({D, Hs}, b16);
+    if ((fp32_mask >> 4 & 1) != 0) {
+      s_dw.scratch = 2 * Hs * D * 2;
+      s_gate = at::empty({Hs, D}, b16.dtype(at::kFloat));
+      s_up = at::empty({Hs, D}, b16.dtype(at::kFloat));
+    } else {
+      s_dw.t = at::empty({2 * Hs, D}, b16);
+      s_gate = s_dw.t.narrow(0, 0, Hs);
+      s_up = s_dw.t.narrow(0, Hs, Hs);
+    }
+    s_dwd = gradient(5, {D, Hs});
   }
-  Scratch scratch(u8, {rows * D * 2, N * top_k * 4, rows * 4 * H, rows * D * 2, N * D * 2, ws_bytes,
+  Scratch scratch(u8, {dH.scratch, d_gate.scratch, d_wu.scratch, d_wd.scratch, s_dw.scratch, s_dwd.scratch,
+                       rows * D * 2, N * top_k * 4, rows * 4 * H, rows * D * 2, N * D * 2, ws_bytes,
                        fused ? 0 : rows * H * 2, N * Hs * 4, fused ? 0 : N * Hs * 2, shared ? N * D * 2 : 0,
                        split == 2 ? 2 * D * Hs * 2 : 0, kept ? 0 : rows * H * 4, kept ? 0 : rows * H * 2,
                        kept ? 0 : rows * D * 2});
@@ -367,12 +431,23 @@ py::tuple layer_backward(const OptTensor& grad_out, const OptTensor& grad_aux, c
   a.pos = reinterpret_cast<int32_t*>(rt + layout.pos);
   a.src = reinterpret_cast<int32_t*>(rt + layout.src);
   a.Xg = ptr(Xg);
-  a.dH = ptr(dH);
-  a.d_gate = ptr(d_gate);
-  a.d_w_up = ptr(d_wu);
-  a.d_w_down = ptr(d_wd);
-  a.s_d_gate_up = ptr(s_dw);
-  a.s_d_down = ptr(s_dwd);
+  Casts casts;
+  auto place = [&](const Grad& gr) {
+    void* narrow = scratch.take();
+    if (narrow == nullptr) return ptr(gr.t);
+    if (gr.t.defined()) casts.add(narrow, gr.t.data_ptr(), gr.t.numel());
+    return narrow;
+  };
+  a.dH = place(dH);
+  a.d_gate = place(d_gate);
+  a.d_w_up = place(d_wu);
+  a.d_w_down = place(d_wd);
+  a.s_d_gate_up = place(s_dw);
+  if (s_dw.scratch > 0) {
+    casts.add(a.s_d_gate_up, s_gate.data_ptr(), Hs * D);
+    casts.add(static_cast<char*>(a.s_d_gate_up) + Hs * D * 2, s_up.data_ptr(), Hs * D);
+  }
+  a.s_d_down = place(s_dwd);
   a.gYw = scratch.take();
   a.gw = scratch.take<float>();
   a.gU = scratch.take();
@@ -406,7 +481,9 @@ py::tuple layer_backward(const OptTensor& grad_out, const OptTensor& grad_aux, c
     py::gil_scoped_release released;
     rc = backward_pass(&a);
   }
-  return py::make_tuple(outcome(rc, launched), dH, d_gate, d_wu, d_wd, handed(s_gate), handed(s_up), handed(s_dwd), go);
+  if (rc == FFM_OK) launched[0] += casts.run(false, stream);
+  return py::make_tuple(outcome(rc, launched), dH.t, d_gate.t, d_wu.t, d_wd.t, handed(s_gate), handed(s_up),
+                        handed(s_dwd.t), go);
 }
 
 }  // namespace

@@ -496,7 +496,9 @@ class _FusedMoEFunction(torch.autograd.Function):
             grad_out, grad_aux, grad_z, *saved, cfg.top_k, _lib.GATING[cfg.gating], _lib.ACTIVATION[cfg.activation],
             _lib.ACTIVATION[cfg.shared_activation], cfg.capacity is not None, _FUSED_GLU_BWD, _OVERLAP,
             cfg.aux_loss_coeff * E / float(N), cfg.z_loss_coeff, ops.status_tensor(dev).data_ptr(), ops._stream(),
-            *((_side_handle(n) if _OVERLAP else 0) for n in ("shared", "backward_route", "backward_gemm", "small")), timer)
+            *((_side_handle(n) if _OVERLAP else 0) for n in ("shared", "backward_route", "backward_gemm", "small")), timer,
+            sum(1 << i for i, t in enumerate((dt[0], dt[1], dt[2], dt[3], dt[5] if dt[5] == dt[6] else None, dt[7]))
+                if t == torch.float32))
         ops.launched(done, pairs, ops.BACKWARD_SITES, fused_glu=_FUSED_GLU_BWD)
 
         d_add = go.to(dt[4]) if dt[4] is not None and ctx.needs_input_grad[4] else None

@@ -331,6 +331,12 @@ int ffm_grouped_gemm_fp8(const void* Aq, const float* a_scale, const void* Bq, c
                          const int32_t* tile_start, int64_t rows, int K, int Nout, void* out, int tile_rows,
                          int32_t* status, ffm_stream_t stream);
 
+/* dst[i] = src[i] for `count` <= FFM_CAST_MAX contiguous tensors of elements[i] values in one launch, fp32 -> bf16 (round to
+ * nearest even) with to_bf16 != 0, else bf16 -> fp32. Addresses are multiples of 16 bytes. */
+#define FFM_CAST_MAX 8
+int ffm_cast_many(int count, const void* const* src, void* const* dst, const int64_t* elements, int to_bf16,
+                  ffm_stream_t stream);
+
 /* -------------------------------------------------------------------------------------------------
  * The single-GPU layer in one call each way: the launches of the forward and of the backward pass (_FusedMoEFunction of
  * the reference, fused_moe.py:299-595) over caller-owned buffers, with the fork and join of the side streams. Nothing is
