@@ -405,12 +405,14 @@ _ONE_CHAIN_BYTES = 256 << 20
 _FEW_TILES, _FEW_DECODE_UP, _FEW_DECODE_DOWN, _FEW_DECODE_SHARED, _FEW_ONE_CHAIN = 1, 2, 4, 8, 16   # FFM_FEW_*
 
 
-def _streams_weights(groups, K, n_out):
-    """Where the decode GEMM was measured to be the faster one: contractions up to 2304 and projections up to 1 GB. At the
-    larger ones measured its times scatter with where the weights lie in memory (256 experts, 15.0 and 7.5 GB: 2415 and 1203
-    us with 128-row tiles, 2190 to 2760 and 1111 to 1600 here; 8 experts, K = 4096 and 14336: 333 and 156, here 300 to 375 and
-    155 to 205). Contractions between 2304 and 4096 were not measured, and why the times scatter is open."""
-    return K <= 2304 and groups * n_out * K * 2 <= 1 << 30
+def _streams_weights(N, K):
+    """Where the decode GEMM is the faster one for a contraction over K. Up + down in us with 128-row tiles and with it: 7 tokens
+    on 8 experts, D = 4096, H = 14336 341 + 170 -> 301 + 162; 128 tokens on 256 experts, D = 7168, H = 2048 2365 + 1182 -> 2110 +
+    1070; 8 tokens there 516 + 282 -> 475 + 252; 48 tokens on 64 experts, D = H = 3072 410 + 227 -> 365 + 199; 64 tokens, D = 7168,
+    8 experts, skewed 78 + 35 -> 56 + 35. (Its times had scattered with where the weights lie, up to 2760 + 1600 in the second
+    case, before an elected thread issued its loads.) With a second token tile it stays behind where a tile is long and
+    few: 128 tokens, 8 experts, skewed, K = 14336 168 -> 162 to 186; the same with K = 7168 and below is faster throughout."""
+    return N <= 64 or K <= 8192
 
 
 def _few_rows(N, D, E, k, H, capacity, w_gate, w_up):
@@ -427,8 +429,8 @@ def _few_rows(N, D, E, k, H, capacity, w_gate, w_up):
         return bits
     bits |= _FEW_TILES
     if 0 < N * k <= _DECODE_ROWS * E and N <= _DECODE_TOKENS:
-        bits |= _FEW_DECODE_UP if _streams_weights(E, D, 2 * H) else 0
-        bits |= _FEW_DECODE_DOWN if _streams_weights(E, H, D) else 0
+        bits |= _FEW_DECODE_UP if _streams_weights(N, D) else 0
+        bits |= _FEW_DECODE_DOWN if _streams_weights(N, H) else 0
         both = _FEW_DECODE_UP | _FEW_DECODE_DOWN
         if bits & both == both and (w_gate is None or bits & _FEW_DECODE_SHARED):
             bits |= _FEW_ONE_CHAIN if 6 * D * (E * H + Hs) <= _ONE_CHAIN_BYTES else 0
