@@ -672,7 +672,8 @@ ffm_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           // The group's last K block, up to its last valid row. It stands apart because the issuing thread has no time to
           // spare: with the test for the last step in the loop above every weight gradient was slower, also without
           // padding (8 x 4096 rows, 4096 x 1024: 180 -> 203 us; 64 x 1536 rows, 2816 x 2048: 843 -> 972), and so were
-          // replayed training steps (16384 tokens, 8 experts and a shared one: 1966 -> 2037 us).
+          // replayed training steps (16384 tokens, 8 experts and a shared one: 1966 -> 2037 us). (Measured before the
+          // issuing thread was elected.)
           static_assert(!GROUPK || (A_MN && B_MN && !FP8), "both operands of a grouped-K GEMM are M/N-major bf16");
           ok = mbar_wait_bounded(smem_u32(&ctrl->full_bar[stage]), phase, abort_flag, p.status, FFM_STATUS_WAIT_MMA,
                                  p.wait_cycles);

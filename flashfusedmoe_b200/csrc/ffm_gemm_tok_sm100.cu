@@ -5,8 +5,9 @@
 // M operand (128 features per CTA), the tokens of one expert the N operand (up to 64), so a tile loads, computes and stores
 // only the 4-, 16- and 8-token boxes that hold tokens. With the tokens on the M side (ffm_gemm_sm100.cu) every tile loads
 // a 128-row box of mostly unused rows beside 256 rows of weights, and stores one.
-// Measured, 48 tokens on 64 experts, top-6, K = 2048, H = 1408 (0.74 + 0.37 GB of weights): up + GLU 131 -> 121 us (6.0
-// TB/s), down 75 -> 64 us (5.7 TB/s); a plain read of this card's memory reaches 7.3 TB/s.
+// Measured, 48 tokens on 64 experts, top-6, K = 2048, H = 1408 (0.74 + 0.37 GB of weights): up + GLU 131 -> 121 us, down 75 ->
+// 64 us with loads issued under `lane == 0`; with an elected thread the whole call went from 214 to 205 us. 128 tokens on 256
+// experts, D = 7168, H = 2048: 2110 + 1070 us (7.0 and 6.9 TB/s, what a plain read of such tiles reaches) against 2365 + 1182.
 // The up-projection can gather the token rows itself (TMA gather4, four rows per instruction), which saves the permute
 // launch and costs more than it where experts have several rows: 120 -> 132 us at 48 tokens on 64 experts, 74 -> 76 at 8.
 //
@@ -14,7 +15,8 @@
 //   warps 2..9  epilogue: two groups of four warps (one per TMEM lane quarter) take the 32-token steps of a tile in turn
 //
 // Ring of 8 stages (16 KiB of weights + up to 8 KiB of tokens): 128 KiB of weights in flight per SM. Fewer stages are
-// slower (6: 122 / 65 us, 4: 132 / 71 us). As in the other GEMM: fp32 accumulators in TMEM, two of them, persistent CTAs,
+// slower (6: 122 / 65 us, 4: 132 / 71 us); stages twice as deep (128 rows x 256 bytes in one box, four of them) take the same
+// time within 1 %. As in the other GEMM: fp32 accumulators in TMEM, two of them, persistent CTAs,
 // bounded waits, TMA stores.
 //
 // The accumulator has features on TMEM lanes and tokens on columns, so the epilogue transposes: tcgen05.ld.16x256b hands
