@@ -122,16 +122,6 @@ __device__ __forceinline__ bool elect_one() {
   return r != 0;
 }
 
-// Chained launches. A kernel launched ahead of the end of the one before it (launch_kernel, chained) must not touch memory
-// before chain_wait(): it returns once that kernel has ended and its stores are visible, and every thread calls it, so that
-// the end of one kernel of a chain still means the end of all before it. chain_next() lets the next one be placed (once all
-// CTAs of this kernel have called it or ended); a no-op in a kernel that nothing is chained to.
-// Between kernels that follow the ordinary way 1.5-3.5 us pass, in which the GPU drains, launches and sets up. Whole calls,
-// without and with: prefill of 1999 tokens, D 1024, 8 experts and a shared one 117 -> 111 us; training of 3001 tokens on 16
-// experts 584 -> 564; decode of 7 tokens on 8 wide experts 412 -> 397, of 48 on 64 experts 204 -> 202.
-__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }

@@ -23,8 +23,6 @@ __device__ __forceinline__ uint32_t pack_e4m3x4(float a, float b, float c, float
 __global__ void __launch_bounds__(Q_THREADS)
 quantize_rows_e4m3_kernel(const bf16* __restrict__ x, long long rows, int K, uint8_t* __restrict__ q,
                           float* __restrict__ scale) {
-  chain_wait();
-  chain_next();
   const int lane = threadIdx.x & 31;
   const int chunks = K >> 3;
   for (long long r = static_cast<long long>(blockIdx.x) * Q_WARPS + (threadIdx.x >> 5); r < rows;
@@ -90,10 +88,9 @@ extern "C" int ffm_quantize_rows_e4m3(const void* x, int64_t rows, int K, void* 
   if (rows == 0) return FFM_OK;
   long long blocks = (rows + Q_WARPS - 1) / Q_WARPS;
   if (blocks > 148LL * 16) blocks = 148LL * 16;
-  const bool ok = launch_kernel(quantize_rows_e4m3_kernel, dim3(static_cast<unsigned>(blocks)), Q_THREADS, 0,
-                                static_cast<cudaStream_t>(stream), follows_kernel, 0, static_cast<const bf16*>(x), rows, K,
-                                static_cast<uint8_t*>(q), scale);
-  return ok ? FFM_OK : FFM_ERR_LAUNCH;
+  quantize_rows_e4m3_kernel<<<static_cast<int>(blocks), Q_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<const bf16*>(x), rows, K, static_cast<uint8_t*>(q), scale);
+  return cudaGetLastError() == cudaSuccess ? FFM_OK : FFM_ERR_LAUNCH;
 }
 
 extern "C" int ffm_quantize_rows_given_scale_e4m3(const void* x, int64_t rows, int K, int64_t rows_per_scale,

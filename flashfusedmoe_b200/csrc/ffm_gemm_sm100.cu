@@ -482,16 +482,6 @@ ffm_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     tma_prefetch_desc(&tmC);
     tma_prefetch_desc(&tmC2);
   }
-  if (warp == 1) {
-    if (CTA2) {
-      tmem_alloc2(smem_u32(&ctrl->tmem_base), TMEM_COLS);
-      tmem_relinquish2();
-    } else {
-      tmem_alloc(smem_u32(&ctrl->tmem_base), TMEM_COLS);
-      tmem_relinquish();
-    }
-  }
-  chain_wait();
   if (!GROUPK && p.group_rows != nullptr) {
     // walk only the tiles that hold valid rows: per group ceil(rows / 128), rounded up to a pair with CTA2
     for (int i = threadIdx.x; i < p.groups; i += blockDim.x) {
@@ -513,6 +503,15 @@ ffm_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     // dense: one group, or (grouped-K) equal ranges of the rows
     for (int i = threadIdx.x; i <= p.groups; i += blockDim.x) {
       ctrl->tile_start[i] = static_cast<int>(static_cast<long long>(p.dense_m_tiles) * i / p.groups);
+    }
+  }
+  if (warp == 1) {
+    if (CTA2) {
+      tmem_alloc2(smem_u32(&ctrl->tmem_base), TMEM_COLS);
+      tmem_relinquish2();
+    } else {
+      tmem_alloc(smem_u32(&ctrl->tmem_base), TMEM_COLS);
+      tmem_relinquish();
     }
   }
   tc_fence_before();
@@ -602,9 +601,6 @@ ffm_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           }
         }
       }
-      // Every load of this CTA is on its way. Not earlier: the next kernel's CTAs take the SMs of CTAs that end, and
-      // would hold them from another stream's GEMM while they wait.
-      chain_next();
     }
   } else if (warp == 1) {
     // ================= MMA issuer (with CTA2: only in the even CTA of the pair) =================
@@ -1037,10 +1033,23 @@ int launch_gemm_shape(const CUtensorMap& tmA, const CUtensorMap& tmB0, const CUt
   long long ctas = CTA2 ? 2 * max_units : max_units;
   if (PASS && p.pz_rows > 0) ctas = max_ctas;  // the passenger job wants every SM, whatever the GEMM's tile count
   if (ctas > max_ctas) ctas = max_ctas;
-  return launch_kernel(kernel, dim3(static_cast<unsigned>(ctas)), threads, smem_bytes, stream, follows_kernel, CTA2 ? 2 : 0,
-                       tmA, tmB0, tmB1, tmC, tmC2, p)
-             ? FFM_OK
-             : FFM_ERR_LAUNCH;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(ctas), 1, 1);
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.dynamicSmemBytes = smem_bytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = CTA2 ? 2 : 1;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = CTA2 ? 1 : 0;  // the one-CTA shape is an ordinary launch
+  if (cudaLaunchKernelEx(&cfg, kernel, tmA, tmB0, tmB1, tmC, tmC2, p) != cudaSuccess) {
+    cudaGetLastError();
+    return FFM_ERR_LAUNCH;
+  }
+  return FFM_OK;
 }
 
 // max_m_tiles: upper bound on the 128-row tiles of M the walker can see (per group for grouped-K);

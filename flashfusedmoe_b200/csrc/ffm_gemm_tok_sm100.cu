@@ -253,11 +253,6 @@ ffm_gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     tma_prefetch_desc(&tmB);
     tma_prefetch_desc(&tmC);
   }
-  if (warp == 1) {
-    tmem_alloc(smem_u32(&ctrl->tmem_base), TMEM_COLS);
-    tmem_relinquish();
-  }
-  chain_wait();
   if (warp == 2) {
     // tiles before every group: eight consecutive groups per lane
     constexpr int PER = MAX_GROUPS / 32;
@@ -289,6 +284,10 @@ ffm_gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       run += mine[i];
       if (g + 1 == p.groups) ctrl->items[p.groups] = run;
     }
+  }
+  if (warp == 1) {
+    tmem_alloc(smem_u32(&ctrl->tmem_base), TMEM_COLS);
+    tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
@@ -353,10 +352,7 @@ ffm_gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       // also: the token list is overwritten only after its last use
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, producer_lane) != 0;
     }
-    if (producer) {
-      ctrl->filled = filled;
-      chain_next();
-    }
+    if (producer) ctrl->filled = filled;
   } else if (warp == 1) {
     // ================= MMA issuer =================
     if (elect_one()) {
@@ -552,10 +548,8 @@ int launch_tok(const CUtensorMap (&m)[6], const TokParams& p, long long rows, cu
   long long ctas = tiles * ((p.feats[0] + S::FEATS - 1) / S::FEATS) +
                    (p.tokens + NMAX - 1) / NMAX * ((p.feats[1] + S::FEATS - 1) / S::FEATS);
   if (ctas > num_sms()) ctas = num_sms();
-  return launch_kernel(kernel, dim3(static_cast<unsigned>(ctas)), THREADS, S::SMEM_BYTES, stream, follows_kernel, 0, m[0],
-                       m[1], m[2], m[3], m[4], m[5], p)
-             ? FFM_OK
-             : FFM_ERR_LAUNCH;
+  kernel<<<static_cast<unsigned>(ctas), THREADS, S::SMEM_BYTES, stream>>>(m[0], m[1], m[2], m[3], m[4], m[5], p);
+  return cudaGetLastError() == cudaSuccess ? FFM_OK : FFM_ERR_LAUNCH;
 }
 
 // the maps of an absent part are never used, but the kernel prefetches their descriptors

@@ -4,10 +4,15 @@
 // streams. From Python, each launch cost a ctypes call with its argument checks, an output allocation and, at a fork, stream and event objects:
 // 230 us for a forward pass and 600 us for a backward pass however small, more than the GPU needed at up to a few
 // thousand tokens.
+//
+// Every launch waits for the end of the one before it on its stream. Placed ahead of that end (programmatic stream
+// serialization) a forward pass is a few us faster: prefill of 1999 tokens 117 -> 111. But in loops of training
+// calls that filled the launch queue (3001 tokens on 16 experts) two of six runs did not come to an end, with events that other
+// streams wait for between such launches. No cause was found in the kernels, and a library cannot keep events from between its
+// launches: the calls release the interpreter's lock, and the allocator records events of its own.
 #include <cuda_runtime.h>
 
 #include "../../include/ffmoe.h"
-#include "ffm_device.h"
 #include "ffm_internal.h"
 
 namespace ffm {
@@ -43,14 +48,11 @@ class Sites {
   Sites(const int64_t* timer, int64_t* launched) : timer_(timer), launched_(launched) {
     for (int i = 0; i < 3; ++i) launched_[i] = 0;
   }
-  // chained: the launch directly follows a kernel of this library on `stream` (no event in between: with a timer there is)
   template <typename F>
-  void run(int site, int kernels, ffm_stream_t stream, F&& launch, bool chained = false) {
+  void run(int site, int kernels, ffm_stream_t stream, F&& launch) {
     if (rc_ != FFM_OK) return;
     mark(2 * site, stream);
-    follows_kernel = chained && timer_ == nullptr;
     rc_ = launch();
-    follows_kernel = false;
     mark(2 * site + 1, stream);
     launched_[0] += kernels;
     launched_[1] |= int64_t{1} << site;
@@ -118,9 +120,6 @@ extern "C" int ffm_layer_forward(const ffm_layer_forward_args* args) {
   Sites sites(a.timer, a.launched);
   Event fork, shared_done;
 
-  // Which launches are chained (see chain_wait): those that directly follow a kernel on their stream, except the expert
-  // GEMM where the shared expert runs beside it: its CTAs would take SMs as the shared expert's first GEMM ends, and hold
-  // them from its second one until the routing and permute kernels are through.
   // shared expert: beside the routing kernels, which leave the tensor cores idle; in a decode-sized call it is one more
   // group of the expert GEMMs
   const bool one_chain = (a.few_rows & FFM_FEW_ONE_CHAIN) != 0;
@@ -143,7 +142,7 @@ extern "C" int ffm_layer_forward(const ffm_layer_forward_args* args) {
       }
       return ffm_grouped_gemm(a.s_act, a.sw_down, FFM_B_KMAJOR, 1, nullptr, a.N, Hs, D, 1.0f, a.s_out, nullptr, 0,
                               a.status, sh);
-    }, true);
+    });
     if (sh != st) sites.require(shared_done.record(sh));
   }
 
@@ -167,21 +166,21 @@ extern "C" int ffm_layer_forward(const ffm_layer_forward_args* args) {
   if (!one_chain) {
     sites.run(FFM_FWD_PERMUTE, 1, st, [&] {
       return ffm_permute_rows(a.hidden, a.src, a.rows_cap, k, D, a.need_grad || a.capacity >= 0 ? 1 : 0, a.Xg, st);
-    }, a.capacity < 0);
+    });
   }
   const int32_t* valid = (a.few_rows & FFM_FEW_TILES) ? a.counts : nullptr;
   const int tile_rows = (a.few_rows & FFM_FEW_TILES) ? 128 : 0;
   if (a.fp8) {
-    sites.run(FFM_FWD_QUANT_X, 1, st, [&] { return ffm_quantize_rows_e4m3(a.Xg, a.rows_cap, D, a.xq, a.x_scale, st); }, true);
+    sites.run(FFM_FWD_QUANT_X, 1, st, [&] { return ffm_quantize_rows_e4m3(a.Xg, a.rows_cap, D, a.xq, a.x_scale, st); });
     sites.run(FFM_FWD_UP, 1, st, [&] {
       return ffm_grouped_gemm_glu_fp8(a.xq, a.x_scale, a.w_up_q, static_cast<const float*>(a.w_up_scale), E, a.tile_start,
                                       a.rows_cap, D, H, act, a.act, a.preact, 0, a.status, st);
-    }, !shared_beside);
-    sites.run(FFM_FWD_QUANT_ACT, 1, st, [&] { return ffm_quantize_rows_e4m3(a.act, a.rows_cap, H, a.aq, a.a_scale, st); }, true);
+    });
+    sites.run(FFM_FWD_QUANT_ACT, 1, st, [&] { return ffm_quantize_rows_e4m3(a.act, a.rows_cap, H, a.aq, a.a_scale, st); });
     sites.run(FFM_FWD_DOWN, 1, st, [&] {
       return ffm_grouped_gemm_fp8(a.aq, a.a_scale, a.w_down_q, static_cast<const float*>(a.w_down_scale), E, a.tile_start,
                                   a.rows_cap, H, D, a.Y, 0, a.status, st);
-    }, true);
+    });
   } else {
     const void* up_rows = static_cast<const char*>(a.w_up) + a.H * a.D * 2;
     sites.run(FFM_FWD_UP, 1, st, [&] {
@@ -192,7 +191,7 @@ extern "C" int ffm_layer_forward(const ffm_layer_forward_args* args) {
       }
       return ffm_grouped_gemm_glu(a.Xg, a.w_up, up_rows, 2 * a.H, E, a.tile_start, a.rows_cap, D, H, act, a.act, a.preact,
                                   valid, tile_rows, a.status, st);
-    }, !shared_beside);
+    });
     sites.run(FFM_FWD_DOWN, 1, st, [&] {
       if (a.few_rows & FFM_FEW_DECODE_DOWN) {
         return ffm_decode_down(a.act, a.rows_cap, H, E, a.tile_start, a.counts, k, a.w_down, D, a.Y, a.s_act, a.N,
@@ -200,7 +199,7 @@ extern "C" int ffm_layer_forward(const ffm_layer_forward_args* args) {
       }
       return ffm_grouped_gemm(a.act, a.w_down, FFM_B_KMAJOR, E, a.tile_start, a.rows_cap, H, D, 1.0f, a.Y, valid, tile_rows,
                               a.status, st);
-    }, true);
+    });
   }
   if (a.addend_ready != nullptr) {
     sites.require(cudaStreamWaitEvent(static_cast<cudaStream_t>(st), static_cast<cudaEvent_t>(a.addend_ready), 0) ==
@@ -210,7 +209,7 @@ extern "C" int ffm_layer_forward(const ffm_layer_forward_args* args) {
   const void* add = Hs > 0 ? a.s_out : a.addend;
   sites.run(FFM_FWD_COMBINE, 1, st, [&] {
     return combine_forward_status(a.Y, a.pos, a.topk_w, add, nullptr, a.N, k, D, a.out, a.status, a.status_host, st);
-  }, a.addend_ready == nullptr && !shared_beside);
+  });
   return sites.rc();
 }
 
@@ -237,9 +236,6 @@ extern "C" int ffm_layer_backward(const ffm_layer_backward_args* args) {
   Sites sites(a.timer, a.launched);
   Event start, sum_fork, sum_done, shared_done, rows_done, route_done, dx_done, join;
 
-  // Launches of the backward pass are not chained (but for the recomputed projections): event records that other streams wait
-  // for lie between them, and with the expert GEMMs chained across one a loop of calls that filled the launch queue did not
-  // come to an end in two of six runs (3001 tokens on 16 experts), for a reason that was not found.
   if (a.recompute) {
     // recompute the three large tensors with the same kernels: bit-identical to the forward pass
     const void* up_rows = static_cast<const char*>(a.w_up) + a.H * a.D * 2;
@@ -250,7 +246,7 @@ extern "C" int ffm_layer_backward(const ffm_layer_backward_args* args) {
     sites.run(FFM_BWD_RE_DOWN, 1, st, [&] {
       return ffm_grouped_gemm(a.act, a.w_down, FFM_B_KMAJOR, E, a.tile_start, a.rows_cap, H, D, 1.0f, a.Y, nullptr, 0,
                               a.status, st);
-    }, true);
+    });
   }
   if (Hs > 0 && overlap) sites.require(start.record(st));
   // first in launch order: the routed GEMMs wait for it, the shared expert's do not

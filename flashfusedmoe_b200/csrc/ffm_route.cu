@@ -350,8 +350,6 @@ route_gate_topk(const bf16* __restrict__ hidden, const bf16* __restrict__ gate_w
                 bf16* __restrict__ logits_out, float* __restrict__ topk_w, int32_t* __restrict__ topk_idx,
                 float* __restrict__ lse_out, int32_t* __restrict__ block_hist, float* __restrict__ block_mass,
                 float* __restrict__ block_z, int32_t* __restrict__ src, long long rows_cap) {
-  chain_wait();
-  chain_next();
   __shared__ float s_mass[ROUTE_WARPS][32];
   __shared__ int s_cnt[ROUTE_WARPS][32];
   __shared__ float s_z[ROUTE_WARPS];
@@ -447,8 +445,6 @@ route_gate_topk_many(const bf16* __restrict__ hidden, const bf16* __restrict__ g
                      bf16* __restrict__ logits_out, float* __restrict__ topk_w, int32_t* __restrict__ topk_idx,
                      float* __restrict__ lse_out, int32_t* __restrict__ block_hist, float* __restrict__ block_mass,
                      float* __restrict__ block_z, int32_t* __restrict__ src, long long rows_cap) {
-  chain_wait();
-  chain_next();
   __shared__ float s_mass[ROUTE_WARPS][NG * 32];
   __shared__ int s_cnt[ROUTE_WARPS][NG * 32];
   __shared__ float s_z[ROUTE_WARPS];
@@ -525,8 +521,6 @@ route_from_logits(const bf16* __restrict__ logits, const float* __restrict__ bia
                   RouteOpts opts, int tokens_per_block, float* __restrict__ topk_w, int32_t* __restrict__ topk_idx,
                   float* __restrict__ lse_out, int32_t* __restrict__ block_hist, float* __restrict__ block_mass,
                   float* __restrict__ block_z, int32_t* __restrict__ src, long long rows_cap) {
-  chain_wait();
-  chain_next();
   __shared__ float s_mass[ROUTE_WARPS][NG * 32];
   __shared__ int s_cnt[ROUTE_WARPS][NG * 32];
   __shared__ float s_z[ROUTE_WARPS];
@@ -631,8 +625,6 @@ __global__ void __launch_bounds__(SCAN_THREADS)
 route_scan(const int32_t* __restrict__ block_hist, const float* __restrict__ block_mass,
            const float* __restrict__ block_z, int blocks, int E, int32_t* __restrict__ block_off,
            int32_t* __restrict__ counts, int32_t* __restrict__ tile_start, float* __restrict__ stats, LossOut lo) {
-  chain_wait();
-  chain_next();
   __shared__ int s_counts[MAX_E];
   __shared__ float s_mass[MAX_E];
   __shared__ float s_zsum;
@@ -681,8 +673,6 @@ __global__ void __launch_bounds__(ROUTE_THREADS)
 route_rank(const int32_t* __restrict__ ids, long long T, int E, int slots_per_block,
            const int32_t* __restrict__ block_off, const int32_t* __restrict__ tile_start, long long rows_cap,
            int32_t* __restrict__ pos, int32_t* __restrict__ src, int32_t* __restrict__ status) {
-  chain_wait();
-  chain_next();
   __shared__ int s_run[ROUTE_WARPS][MAX_E];
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -761,8 +751,6 @@ constexpr int FINISH_CLUSTER = 8;
 __global__ void __launch_bounds__(ROUTE_THREADS, 2)
 route_gate_small(const bf16* __restrict__ hidden, const bf16* __restrict__ gate_w, int N, int D, int E,
                  bf16* __restrict__ logits, int32_t* __restrict__ src, long long rows_cap) {
-  chain_wait();
-  chain_next();
   constexpr int EG = SMALL_EG;
   constexpr int ACC = EG * SMALL_TG;
   __shared__ float s_part[ROUTE_WARPS][ACC];
@@ -817,8 +805,6 @@ route_finish_small(const bf16* __restrict__ logits, const float* __restrict__ bi
                    int32_t* block_hist, float* block_mass, float* block_z, int32_t* __restrict__ counts,
                    int32_t* __restrict__ tile_start, float* __restrict__ stats, long long rows_cap,
                    int32_t* __restrict__ pos, int32_t* __restrict__ src, int32_t* __restrict__ status, LossOut lo) {
-  chain_wait();
-  chain_next();
   __shared__ float s_mass[FINISH_WARPS][NG * 32];
   __shared__ int s_cnt[FINISH_WARPS][NG * 32];
   __shared__ float s_z[FINISH_WARPS];
@@ -975,13 +961,25 @@ int launch_finish_small(const bf16* logits, const float* bias, int N, int E, int
                         float* topk_w, int32_t* topk_idx, float* lse, const RouteWorkspace& w, int32_t* counts,
                         int32_t* tile_start, float* stats, long long rows_cap, int32_t* pos, int32_t* src,
                         int32_t* status, const LossOut& lo, cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
   // up to one token per warp, a single block is enough; beyond, the tokens are spread over a cluster
-  const int blocks = N <= FINISH_WARPS ? 1 : FINISH_CLUSTER;
-  return launch_kernel(route_finish_small<NG>, dim3(blocks), FINISH_THREADS, 0, s, true, blocks, logits, bias, N, E, top_k,
-                       opts, topk_w, topk_idx, lse, w.block_hist, w.block_mass, w.block_z, counts, tile_start, stats,
-                       rows_cap, pos, src, status, lo)
-             ? FFM_OK
-             : FFM_ERR_LAUNCH;
+  cfg.gridDim = dim3(N <= FINISH_WARPS ? 1 : FINISH_CLUSTER, 1, 1);
+  cfg.blockDim = dim3(FINISH_THREADS, 1, 1);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cfg.gridDim.x;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, route_finish_small<NG>, logits, bias, N, E, top_k, opts, topk_w, topk_idx, lse,
+                         w.block_hist, w.block_mass, w.block_z, counts, tile_start, stats, rows_cap, pos, src,
+                         status, lo) != cudaSuccess) {
+    cudaGetLastError();
+    return FFM_ERR_LAUNCH;
+  }
+  return FFM_OK;
 }
 
 // Expert capacity: a routed slot whose rank inside its expert segment is >= capacity is dropped. One thread
@@ -1134,11 +1132,10 @@ int ffm::route_forward_losses(const void* hidden, const void* gate_w, const floa
     const int rc = ffm_grouped_gemm(hidden, gate_w, FFM_B_KMAJOR, 1, nullptr, N, D, E, 1.0f, logits, nullptr, 0, status,
                                     stream);
     if (rc != FFM_OK) return rc;
-#define FFM_LOGIT_CASE(NG)                                                                                            \
-  if (!launch_kernel(route_from_logits<NG>, dim3(g.blocks), ROUTE_THREADS, 0, s, true, 0, lg, expert_bias, N, E, top_k, \
-                     opts, g.tokens_per_block, topk_w, topk_idx, lse, w.block_hist, w.block_mass, w.block_z, src,        \
-                     rows_cap))                                                                                          \
-  return FFM_ERR_LAUNCH
+#define FFM_LOGIT_CASE(NG)                                                                                      \
+  route_from_logits<NG><<<g.blocks, ROUTE_THREADS, 0, s>>>(lg, expert_bias, N, E, top_k, opts, g.tokens_per_block, \
+                                                           topk_w, topk_idx, lse, w.block_hist, w.block_mass, w.block_z,  \
+                                                           src, rows_cap)
     if (E <= 64) {
       FFM_LOGIT_CASE(2);
     } else if (E <= 128) {
@@ -1176,12 +1173,11 @@ int ffm::route_forward_losses(const void* hidden, const void* gate_w, const floa
 #undef FFM_ROUTE_CASE
   }
   FFM_PREFER_MAX_SHARED(route_scan);
-  if (cudaGetLastError() != cudaSuccess) return FFM_ERR_LAUNCH;
-  const bool ok = launch_kernel(route_scan, dim3(1), SCAN_THREADS, 0, s, true, 0, w.block_hist, w.block_mass, w.block_z,
-                                g.blocks, E, w.block_off, counts, tile_start, stats, lo) &&
-                  launch_kernel(route_rank, dim3(g.blocks), ROUTE_THREADS, 0, s, true, 0, topk_idx, N * top_k, E,
-                                g.tokens_per_block * top_k, w.block_off, tile_start, rows_cap, pos, src, status);
-  return ok ? FFM_OK : FFM_ERR_LAUNCH;
+  route_scan<<<1, SCAN_THREADS, 0, s>>>(w.block_hist, w.block_mass, w.block_z, g.blocks, E, w.block_off, counts,
+                                         tile_start, stats, lo);
+  route_rank<<<g.blocks, ROUTE_THREADS, 0, s>>>(topk_idx, N * top_k, E, g.tokens_per_block * top_k, w.block_off,
+                                                tile_start, rows_cap, pos, src, status);
+  return cudaGetLastError() == cudaSuccess ? FFM_OK : FFM_ERR_LAUNCH;
 }
 
 extern "C" int ffm_route_forward(const void* hidden, const void* gate_w, const float* expert_bias, int64_t N, int D,

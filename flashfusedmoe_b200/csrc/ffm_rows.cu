@@ -13,8 +13,6 @@ constexpr int ROW_WARPS = ROW_THREADS / 32;
 __global__ void __launch_bounds__(ROW_THREADS)
 permute_rows_kernel(const bf16* __restrict__ x, const int32_t* __restrict__ src, long long rows, int top_k, int D,
                     int zero_padding, bf16* __restrict__ grouped) {
-  chain_wait();
-  chain_next();
   const int lane = threadIdx.x & 31;
   const int chunks = D >> 3;
   for (long long r = static_cast<long long>(blockIdx.x) * ROW_WARPS + (threadIdx.x >> 5); r < rows;
@@ -64,8 +62,6 @@ __global__ void __launch_bounds__(ROW_THREADS)
 combine_forward_kernel(const bf16* __restrict__ Y, const int32_t* __restrict__ pos, const float* __restrict__ w,
                        const bf16* __restrict__ addend, const bf16* __restrict__ addend2, long long N, int top_k, int D,
                        bf16* __restrict__ out, const int32_t* status, volatile int32_t* status_host) {
-  chain_wait();
-  chain_next();
   // last kernel of a forward pass: a failure that some kernel before it reported goes to the caller's mapped host word
   if (status_host != nullptr && blockIdx.x == 0 && threadIdx.x == 0) {
     const int32_t code = *status;
@@ -110,8 +106,6 @@ __global__ void __launch_bounds__(ROW_THREADS)
 combine_backward_kernel(const bf16* __restrict__ go, const bf16* __restrict__ Y, const float* __restrict__ w,
                         const int32_t* __restrict__ src, long long rows, int top_k, int D, bf16* __restrict__ gYw,
                         float* __restrict__ gw) {
-  chain_wait();
-  chain_next();
   const int lane = threadIdx.x & 31;
   const int chunks = D >> 3;
   for (long long r = static_cast<long long>(blockIdx.x) * ROW_WARPS + (threadIdx.x >> 5); r < rows;
@@ -296,10 +290,9 @@ extern "C" int ffm_permute_rows(const void* x, const int32_t* src, int64_t rows_
   if (D % 8 != 0) return FFM_ERR_UNSUPPORTED;
   if (rows_cap == 0) return FFM_OK;
   FFM_PREFER_MAX_SHARED(permute_rows_kernel);
-  const bool ok = launch_kernel(permute_rows_kernel, dim3(grid_for_rows(rows_cap)), ROW_THREADS, 0,
-                                static_cast<cudaStream_t>(stream), follows_kernel, 0, static_cast<const bf16*>(x), src,
-                                rows_cap, top_k, D, zero_padding, static_cast<bf16*>(grouped));
-  return ok ? FFM_OK : FFM_ERR_LAUNCH;
+  permute_rows_kernel<<<grid_for_rows(rows_cap), ROW_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<const bf16*>(x), src, rows_cap, top_k, D, zero_padding, static_cast<bf16*>(grouped));
+  return cudaGetLastError() == cudaSuccess ? FFM_OK : FFM_ERR_LAUNCH;
 }
 
 int ffm::combine_forward_status(const void* Y, const int32_t* pos, const float* w, const void* addend, const void* addend2,
@@ -310,11 +303,10 @@ int ffm::combine_forward_status(const void* Y, const int32_t* pos, const float* 
   if (D % 8 != 0 || top_k > 32) return FFM_ERR_UNSUPPORTED;
   if (N == 0) return FFM_OK;
   FFM_PREFER_MAX_SHARED(combine_forward_kernel);
-  const bool ok = launch_kernel(combine_forward_kernel, dim3(grid_for_rows(N * ((D / 8 + 31) / 32))), ROW_THREADS, 0,
-                                static_cast<cudaStream_t>(stream), follows_kernel, 0, static_cast<const bf16*>(Y), pos, w,
-                                static_cast<const bf16*>(addend), static_cast<const bf16*>(addend2), N, top_k, D,
-                                static_cast<bf16*>(out), status, status_host);
-  return ok ? FFM_OK : FFM_ERR_LAUNCH;
+  combine_forward_kernel<<<grid_for_rows(N * ((D / 8 + 31) / 32)), ROW_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<const bf16*>(Y), pos, w, static_cast<const bf16*>(addend), static_cast<const bf16*>(addend2), N, top_k,
+      D, static_cast<bf16*>(out), status, status_host);
+  return cudaGetLastError() == cudaSuccess ? FFM_OK : FFM_ERR_LAUNCH;
 }
 
 extern "C" int ffm_combine_forward_add2(const void* Y, const int32_t* pos, const float* w, const void* addend,
@@ -335,10 +327,10 @@ extern "C" int ffm_combine_backward(const void* go, const void* Y, const float* 
   if (D % 8 != 0) return FFM_ERR_UNSUPPORTED;
   if (rows_cap == 0) return FFM_OK;
   FFM_PREFER_MAX_SHARED(combine_backward_kernel);
-  const bool ok = launch_kernel(combine_backward_kernel, dim3(grid_for_rows(rows_cap)), ROW_THREADS, 0,
-                                static_cast<cudaStream_t>(stream), follows_kernel, 0, static_cast<const bf16*>(go),
-                                static_cast<const bf16*>(Y), w, src, rows_cap, top_k, D, static_cast<bf16*>(gYw), gw);
-  return ok ? FFM_OK : FFM_ERR_LAUNCH;
+  combine_backward_kernel<<<grid_for_rows(rows_cap), ROW_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<const bf16*>(go), static_cast<const bf16*>(Y), w, src, rows_cap, top_k, D,
+      static_cast<bf16*>(gYw), gw);
+  return cudaGetLastError() == cudaSuccess ? FFM_OK : FFM_ERR_LAUNCH;
 }
 
 extern "C" int ffm_glu_backward(const void* dAct, const void* preact, const int32_t* tile_start, int groups,

@@ -128,6 +128,17 @@ def test_layer_forward_refuses_launches_that_read_unwritten_buffers():
     assert site(few_rows=shared, Hs=64) == shared_up
 
 
+def test_no_kernel_is_launched_ahead_of_the_one_before_it():
+    """Programmatic stream serialization is ordered with the kernel right before on the stream, and this library does not know
+    what that is: another thread's event, or the allocator's, may lie between two launches of a call. Kernels here also read
+    what the one before wrote through the read-only path, which holds only if that kernel has ended."""
+    csrc = os.path.join(os.path.dirname(_lib.LIB_PATH), "csrc")
+    for name in sorted(os.listdir(csrc)):
+        if name.endswith((".cu", ".cuh", ".h", ".cpp")):
+            text = open(os.path.join(csrc, name)).read()
+            assert not re.search(r"griddepcontrol|cudaGridDependency|cudaTriggerProgrammatic|LaunchAttributeProgrammatic", text), name
+
+
 def test_product_path_has_no_cpu_fallback():
     import torch
     from flashfusedmoe_b200 import fused_moe
