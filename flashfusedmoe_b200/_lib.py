@@ -7,10 +7,10 @@ library raises, there is no fallback.
 import ctypes
 import importlib.util
 import os
+import sysconfig
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libffmoe.so")
-NATIVE_PATH = os.path.join(_HERE, "_native.so")
 
 c_void_p = ctypes.c_void_p
 c_int = ctypes.c_int
@@ -122,15 +122,23 @@ def load():
     return lib
 
 
+def native_path():
+    """File of the torch extension. Its layout of tensors and its Python interface are those of the torch and the Python that it
+    was built against, so the name carries both: with another one installed the file is missing, not loaded."""
+    import torch
+    abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)
+    return os.path.join(_HERE, f"_native.torch{torch.__version__}-abi{abi}{sysconfig.get_config_var('EXT_SUFFIX')}")
+
+
 def native():
     """The torch side of the layer driver (csrc/ffm_torch.cpp, built beside libffmoe.so), bound to that library's functions."""
     global _native
     if _native is None:
-        lib = load()
-        if not os.path.exists(NATIVE_PATH):
-            raise RuntimeError(f"{NATIVE_PATH} is missing: build it with `python -m flashfusedmoe_b200.build`.")
-        import torch  # noqa: F401  (the extension links against its libraries)
-        spec = importlib.util.spec_from_file_location(__package__ + "._native", NATIVE_PATH)
+        lib, path = load(), native_path()
+        if not os.path.exists(path):
+            raise RuntimeError(f"{path} is missing: the package was not built for this torch and Python. Build it with "
+                               "`python -m flashfusedmoe_b200.build`.")
+        spec = importlib.util.spec_from_file_location(__package__ + "._native", path)
         module = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(module)
         module.bind(*(ctypes.cast(getattr(lib, name), c_void_p).value for name in (

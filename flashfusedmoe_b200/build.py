@@ -1,4 +1,4 @@
-"""Build libffmoe.so (sm_100a only, nvcc) and _native.so (its torch side, g++) in-tree.
+"""Build libffmoe.so (sm_100a only, nvcc) and its torch side (g++; _lib.native_path) in-tree.
 
 Usage: python -m flashfusedmoe_b200.build [--force]
 The shared libraries land next to this file so that they travel with the source tree.
@@ -8,11 +8,13 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
+
+from ._lib import native_path
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libffmoe.so")
-NATIVE = os.path.join(HERE, "_native.so")
 NATIVE_SOURCE = os.path.join(CSRC, "ffm_torch.cpp")
 PTXAS_LOG = os.path.join(HERE, "libffmoe.ptxas.txt")
 SOURCES = ["ffm_api.cu", "ffm_route.cu", "ffm_rows.cu", "ffm_route_bwd.cu", "ffm_gemm_sm100.cu", "ffm_gemm_tok_sm100.cu",
@@ -29,9 +31,8 @@ def _newest_source_mtime():
     return max(os.path.getmtime(p) for p in paths)
 
 
-def _native_command():
+def _native_command(target):
     """g++ command of the torch extension: host code only, against the installed torch's headers and libraries."""
-    import sysconfig
     import torch
     root = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(shutil.which(os.environ.get("NVCC", "nvcc")) or "/usr/local/cuda/bin/nvcc"))
@@ -39,17 +40,17 @@ def _native_command():
                sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
     return (["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_native",
              f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"] + ["-I" + d for d in include] +
-            [NATIVE_SOURCE, "-o", NATIVE, "-L" + os.path.join(root, "lib"), "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10"])
+            [NATIVE_SOURCE, "-o", target, "-L" + os.path.join(root, "lib"), "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10"])
 
 
 def build(force=False, verbose=False):
-    """Compile every .cu under csrc/ into libffmoe.so and ffm_torch.cpp into _native.so. Returns the first one's path."""
-    newest = _newest_source_mtime()
-    if not force and all(os.path.exists(f) and os.path.getmtime(f) >= newest for f in (LIB, NATIVE)):
+    """Compile every .cu under csrc/ into libffmoe.so and ffm_torch.cpp into the torch extension. Returns the first one's path."""
+    newest, native = _newest_source_mtime(), native_path()
+    if not force and all(os.path.exists(f) and os.path.getmtime(f) >= newest for f in (LIB, native)):
         return LIB
     nvcc = os.environ.get("NVCC", "nvcc")
     objs = []
-    procs = [("ffm_torch.cpp", subprocess.Popen(_native_command(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT,
+    procs = [("ffm_torch.cpp", subprocess.Popen(_native_command(native), stdout=subprocess.PIPE, stderr=subprocess.STDOUT,
                                                 text=True))]
     for src in SOURCES:
         obj = os.path.join(CSRC, src.replace(".cu", ".o"))

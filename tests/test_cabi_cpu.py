@@ -139,6 +139,33 @@ def test_no_kernel_is_launched_ahead_of_the_one_before_it():
             assert not re.search(r"griddepcontrol|cudaGridDependency|cudaTriggerProgrammatic|LaunchAttributeProgrammatic", text), name
 
 
+def test_extension_of_another_torch_is_built_again(monkeypatch):
+    """The torch extension belongs to one torch and one Python: after a change build() compiles, and nothing loads the old file."""
+    import torch
+    from flashfusedmoe_b200 import build
+
+    class Compiled(Exception):
+        pass
+
+    def compiler(*args, **kwargs):
+        raise Compiled
+
+    assert build.build(force=False) == build.LIB
+    monkeypatch.setattr(build.subprocess, "Popen", compiler)
+    assert build.build(force=False) == build.LIB
+    monkeypatch.setattr(_lib, "_native", None)
+    monkeypatch.setattr(torch, "__version__", "0.0.0+other")
+    with pytest.raises(Compiled):
+        build.build(force=False)
+    with pytest.raises(RuntimeError, match="not built for this torch.*flashfusedmoe_b200.build"):
+        _lib.native()
+    monkeypatch.undo()
+    monkeypatch.setattr(build.subprocess, "Popen", compiler)
+    monkeypatch.setattr(build.sysconfig, "get_config_var", lambda name: ".cpython-399-x86_64-linux-gnu.so")
+    with pytest.raises(Compiled):
+        build.build(force=False)
+
+
 def test_product_path_has_no_cpu_fallback():
     import torch
     from flashfusedmoe_b200 import fused_moe
