@@ -61,8 +61,8 @@ const Tensor& require(const Tensor& t, at::ScalarType dtype, const char* name) {
 class Casts {
  public:
   static bool takes(const Tensor& t) {
-    return t.is_cuda() && t.layout() == at::kStrided && t.is_contiguous() && t.numel() > 0 &&
-           reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
+    return t.is_cuda() && t.layout() == at::kStrided && t.is_contiguous() && !t.is_neg() && !t._is_zerotensor() &&
+           t.numel() > 0 && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
   }
   void add(const void* src, void* dst, int64_t elements) {
     if (count_ == FFM_CAST_MAX) throw std::logic_error("more tensors than one launch converts");
@@ -85,7 +85,8 @@ class Casts {
   int count_ = 0;
 };
 
-// t in the compute type, contiguous; an fp32 tensor's cast may only be entered in `casts`
+// t in the compute type, contiguous, with its values in memory (no negation pending); an fp32 tensor's cast may only be entered
+// in `casts`
 Tensor computed(const Tensor& t, const char* name, Casts* casts = nullptr) {
   if (casts != nullptr && t.scalar_type() == at::kFloat && Casts::takes(t)) {
     const Tensor c = at::empty(t.sizes(), t.options().dtype(at::kBFloat16));
@@ -94,6 +95,7 @@ Tensor computed(const Tensor& t, const char* name, Casts* casts = nullptr) {
   }
   Tensor c = t.scalar_type() == at::kBFloat16 ? t : t.to(at::kBFloat16);
   if (!c.is_contiguous()) c = c.contiguous();
+  if (c.is_neg()) c = c.resolve_neg();
   return require(c, at::kBFloat16, name);
 }
 

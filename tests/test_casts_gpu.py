@@ -73,3 +73,14 @@ def test_fp32_parameters_under_autocast(shared, offset):
         wide[:, :128] = x
         out2, grads2, _ = step(layer, wide[:, :128])
         assert torch.equal(out2, ref) and torch.equal(grads2[0], grads[0])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_tokens_whose_negation_is_pending(dtype):
+    """A view may carry a negation that its memory does not hold (the imaginary part of a conjugate): it is carried out."""
+    torch.manual_seed(4)
+    layer = MoELayer(128, 256, 8, 2).to(DEV).to(dtype).eval()
+    x = torch.randn(300, 128, device=DEV).to(dtype)
+    with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+        want, got = layer(-x)[0], layer(torch._neg_view(x))[0]
+    assert torch.equal(got, want)
