@@ -6,6 +6,7 @@
 #include <cuda_fp8.h>
 
 #include "ffm_common.cuh"
+#include "ffm_internal.h"
 
 namespace ffm {
 
@@ -86,6 +87,7 @@ extern "C" int ffm_quantize_rows_e4m3(const void* x, int64_t rows, int K, void* 
   if (rows < 0 || K <= 0) return FFM_ERR_BAD_ARG;
   if (K % 16 != 0) return FFM_ERR_UNSUPPORTED;
   if (rows == 0) return FFM_OK;
+  if (off_16_bytes(x) || (reinterpret_cast<uintptr_t>(q) & 7u) != 0) return FFM_ERR_UNSUPPORTED;
   long long blocks = (rows + Q_WARPS - 1) / Q_WARPS;
   if (blocks > 148LL * 16) blocks = 148LL * 16;
   quantize_rows_e4m3_kernel<<<static_cast<int>(blocks), Q_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
@@ -99,6 +101,7 @@ extern "C" int ffm_quantize_rows_given_scale_e4m3(const void* x, int64_t rows, i
   if (rows < 0 || K <= 0 || rows_per_scale < 1) return FFM_ERR_BAD_ARG;
   if (K % 16 != 0) return FFM_ERR_UNSUPPORTED;
   if (rows == 0) return FFM_OK;
+  if (off_16_bytes(x) || (reinterpret_cast<uintptr_t>(q) & 7u) != 0) return FFM_ERR_UNSUPPORTED;
   long long blocks = (rows + Q_WARPS - 1) / Q_WARPS;
   if (blocks > 148LL * 16) blocks = 148LL * 16;
   quantize_rows_given_scale_kernel<<<static_cast<int>(blocks), Q_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(

@@ -1247,6 +1247,7 @@ extern "C" int ffm_grouped_gemm_wgrad_glu_backward(const void* A, const void* B,
   if (!A || !B || !dW || !status || !tile_start) return FFM_ERR_BAD_ARG;
   if (groups < 1 || groups > MAX_GROUPS || rows_cap <= 0 || M <= 0 || Nout <= 0) return FFM_ERR_BAD_ARG;
   if (M % 64 != 0 || Nout % 64 != 0) return FFM_ERR_UNSUPPORTED;
+  if (off_16_bytes(dAct, preact, gU)) return FFM_ERR_UNSUPPORTED;
   CUtensorMap tmA, tmB, tmC;
   int rc;
   if ((rc = make_map_2d(&tmA, A, rows_cap, M, 64, 64)) != FFM_OK) return rc;

@@ -6,6 +6,13 @@
 
 namespace ffm {
 
+// True where an address does not lie on a 16-byte boundary. The row and routing kernels load and store 16 bytes at a time, and an
+// access off that boundary ends the context; the GEMMs' tensor maps refuse such operands themselves.
+template <typename... P>
+bool off_16_bytes(const P*... p) {
+  return ((reinterpret_cast<uintptr_t>(p) | ...) & 15u) != 0;
+}
+
 // ffm_route_forward; aux = aux_scale * stats[E + 1], z = z_scale * stats[E], *zero = 0 (each skipped when null).
 int route_forward_losses(const void* hidden, const void* gate_w, const float* expert_bias, int64_t N, int D, int E,
                          int top_k, int gating, float weight_scale, int pre_softmax, int n_group, int topk_group,

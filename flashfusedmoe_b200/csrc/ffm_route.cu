@@ -1106,6 +1106,7 @@ int ffm::route_forward_losses(const void* hidden, const void* gate_w, const floa
   opts.n_group = n_group;
   opts.topk_group = topk_group;
   if (workspace_bytes < ffm_route_workspace_bytes(N, E, top_k)) return FFM_ERR_WORKSPACE;
+  if (N > 0 && off_16_bytes(hidden, gate_w)) return FFM_ERR_UNSUPPORTED;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bf16* h = static_cast<const bf16*>(hidden);
   const bf16* gw = static_cast<const bf16*>(gate_w);

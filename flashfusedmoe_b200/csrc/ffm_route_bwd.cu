@@ -332,6 +332,7 @@ int ffm::route_backward_losses(const float* gw, const float* topk_w, const int32
   if (need_logits && (!logits || (has_z && !lse))) return FFM_ERR_BAD_ARG;
   if (D % 8 != 0 || E > MAX_E || top_k > 32 || top_k > E) return FFM_ERR_UNSUPPORTED;
   if (workspace_bytes < ffm_route_backward_workspace_bytes(N, D, E)) return FFM_ERR_WORKSPACE;
+  if (N > 0 && off_16_bytes(hidden, gate_w, dH, workspace)) return FFM_ERR_UNSUPPORTED;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int ldg_ = (E + 7) & ~7;
   bf16* gl = static_cast<bf16*>(workspace);

@@ -256,6 +256,7 @@ using namespace ffm;
 int ffm::add_bf16(const void* a, const void* b, int64_t n, void* out, ffm_stream_t stream) {
   if (n % 8 != 0) return FFM_ERR_UNSUPPORTED;
   if (n == 0) return FFM_OK;
+  if (off_16_bytes(a, b, out)) return FFM_ERR_UNSUPPORTED;
   add_bf16_kernel<<<grid_for_rows(n / 256 + 1), ROW_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const uint4*>(a), static_cast<const uint4*>(b), n / 8, static_cast<uint4*>(out));
   return cudaGetLastError() == cudaSuccess ? FFM_OK : FFM_ERR_LAUNCH;
@@ -270,7 +271,7 @@ extern "C" int ffm_cast_many(int count, const void* const* src, void* const* dst
     if (elements[i] < 0) return FFM_ERR_BAD_ARG;
     if (elements[i] == 0) continue;
     if (!src[i] || !dst[i]) return FFM_ERR_BAD_ARG;
-    if (((reinterpret_cast<uintptr_t>(src[i]) | reinterpret_cast<uintptr_t>(dst[i])) & 15u) != 0) return FFM_ERR_UNSUPPORTED;
+    if (off_16_bytes(src[i], dst[i])) return FFM_ERR_UNSUPPORTED;
     chunks += (elements[i] + 7) / 8;
     job.src[job.count] = src[i];
     job.dst[job.count] = dst[i];
@@ -289,6 +290,7 @@ extern "C" int ffm_permute_rows(const void* x, const int32_t* src, int64_t rows_
   if (rows_cap < 0 || top_k < 1 || D <= 0) return FFM_ERR_BAD_ARG;
   if (D % 8 != 0) return FFM_ERR_UNSUPPORTED;
   if (rows_cap == 0) return FFM_OK;
+  if (off_16_bytes(x, grouped)) return FFM_ERR_UNSUPPORTED;
   FFM_PREFER_MAX_SHARED(permute_rows_kernel);
   permute_rows_kernel<<<grid_for_rows(rows_cap), ROW_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const bf16*>(x), src, rows_cap, top_k, D, zero_padding, static_cast<bf16*>(grouped));
@@ -302,6 +304,7 @@ int ffm::combine_forward_status(const void* Y, const int32_t* pos, const float* 
   if (N < 0 || top_k < 1 || D <= 0) return FFM_ERR_BAD_ARG;
   if (D % 8 != 0 || top_k > 32) return FFM_ERR_UNSUPPORTED;
   if (N == 0) return FFM_OK;
+  if (off_16_bytes(Y, addend, addend2, out)) return FFM_ERR_UNSUPPORTED;
   FFM_PREFER_MAX_SHARED(combine_forward_kernel);
   combine_forward_kernel<<<grid_for_rows(N * ((D / 8 + 31) / 32)), ROW_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const bf16*>(Y), pos, w, static_cast<const bf16*>(addend), static_cast<const bf16*>(addend2), N, top_k,
@@ -326,6 +329,7 @@ extern "C" int ffm_combine_backward(const void* go, const void* Y, const float* 
   if (rows_cap < 0 || top_k < 1 || D <= 0) return FFM_ERR_BAD_ARG;
   if (D % 8 != 0) return FFM_ERR_UNSUPPORTED;
   if (rows_cap == 0) return FFM_OK;
+  if (off_16_bytes(go, Y, gYw)) return FFM_ERR_UNSUPPORTED;
   FFM_PREFER_MAX_SHARED(combine_backward_kernel);
   combine_backward_kernel<<<grid_for_rows(rows_cap), ROW_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const bf16*>(go), static_cast<const bf16*>(Y), w, src, rows_cap, top_k, D,
@@ -340,6 +344,7 @@ extern "C" int ffm_glu_backward(const void* dAct, const void* preact, const int3
   if (tile_start != nullptr && groups < 1) return FFM_ERR_BAD_ARG;
   if (H % 8 != 0) return FFM_ERR_UNSUPPORTED;
   if (rows == 0) return FFM_OK;
+  if (off_16_bytes(dAct, preact, gU)) return FFM_ERR_UNSUPPORTED;
   long long work = rows * (H / 8);
   long long blocks = (work + ROW_THREADS - 1) / ROW_THREADS;
   const long long cap = 148LL * 32;

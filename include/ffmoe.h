@@ -13,7 +13,8 @@
  * Data layout shared by all entry points
  * --------------------------------------
  *   N tokens, D model width, H = ffn_dim / 2, E experts (E_local with expert parallelism), k = top_k,
- *   T = N * k routed rows. All activations and weights are bf16, row-major, contiguous.
+ *   T = N * k routed rows. All activations and weights are bf16, row-major, contiguous,
+ *   from 16-byte boundaries on.
  *   "Grouped rows": routed rows sorted by expert, stable in (token, slot) order, each expert's segment
  *   starting on a multiple of 256 rows (the height of the two-CTA MMA tile). Rows between the end of an
  *   expert's tokens and the next multiple of 256 are zero. Buffers hold ffm_rows_capacity(T, E) rows.
@@ -40,7 +41,7 @@ extern "C" {
 /* Return codes */
 #define FFM_OK 0
 #define FFM_ERR_BAD_ARG (-1)      /* null pointer, negative size, unknown enum */
-#define FFM_ERR_UNSUPPORTED (-2)  /* shape outside what the kernels handle (see each function) */
+#define FFM_ERR_UNSUPPORTED (-2)  /* shape outside what the kernels handle (see each function), or an address off 16 bytes */
 #define FFM_ERR_LAUNCH (-3)       /* cudaGetLastError() after a launch, or a driver call failed */
 #define FFM_ERR_WORKSPACE (-4)    /* workspace too small */
 #define FFM_ERR_NO_DRIVER (-5)    /* cuTensorMapEncodeTiled could not be resolved */

@@ -2,6 +2,8 @@
 answer without a GPU. No compute kernel is launched here."""
 
 import ctypes
+import inspect
+import multiprocessing
 import os
 import re
 
@@ -67,6 +69,41 @@ def test_groups_too_small_for_top_k_are_refused():
 
     assert route(1, 3) == -1 and route(2, 5) == -1
     assert route(1, 2) == -4 and route(2, 4) == -4
+
+
+def _check_operand_addresses():
+    """Each operand in turn off its boundary; with fitting addresses a call gets as far as its launch, which fails without a device."""
+    lib = _lib.load()
+    a, off = 256, 260
+    N, D, E, k = 512, 64, 8, 2
+    cap, big = lib.ffm_rows_capacity(N * k, E), 1 << 30
+    for call in (
+            lambda hidden, gate: lib.ffm_route_forward(hidden, gate, 0, N, D, E, k, 0, 1.0, 0, 0, 0, a, a, a, a, a, a, a, a, cap, a,
+                                                       a, big, a, 0),
+            lambda hidden, gate, dH, workspace: lib.ffm_route_backward(a, a, a, a, a, 0, 0, hidden, gate, N, D, E, k, 0, 0, dH, a,
+                                                                       workspace, big, a, 0),
+            lambda x, grouped: lib.ffm_permute_rows(x, a, cap, k, D, 1, grouped, 0),
+            lambda Y, add, add2, out: lib.ffm_combine_forward_add2(Y, a, a, add, add2, N, k, D, out, 0),
+            lambda go, Y, gYw: lib.ffm_combine_backward(go, Y, a, a, cap, k, D, gYw, a, 0),
+            lambda d_act, preact, gU: lib.ffm_glu_backward(d_act, preact, a, E, cap, D, 0, gU, 0),
+            lambda x, q: lib.ffm_quantize_rows_e4m3(x, cap, D, q, a, 0),
+            lambda x, q: lib.ffm_quantize_rows_given_scale_e4m3(x, cap, D, 128, a, q, 0),
+            lambda d_act, preact, gU: lib.ffm_grouped_gemm_wgrad_glu_backward(a, a, E, a, cap, D, D, 1.0, a, d_act, preact, cap, D, 0,
+                                                                              gU, a, 0)):
+        names = inspect.signature(call).parameters
+        fitting = dict.fromkeys(names, a)
+        assert call(**fitting) not in (0, -1, -2)
+        for name in names:
+            assert call(**{**fitting, name: off}) == -2, (inspect.getsource(call), name)
+
+
+def test_operands_off_a_16_byte_boundary_are_refused(monkeypatch):
+    """Kernels that load and store 16 bytes at a time would end the context on such an address. In a process that sees no device."""
+    monkeypatch.setenv("CUDA_VISIBLE_DEVICES", "")
+    child = multiprocessing.get_context("spawn").Process(target=_check_operand_addresses)
+    child.start()
+    child.join()
+    assert child.exitcode == 0
 
 
 def _block_fields(name):
