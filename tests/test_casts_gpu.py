@@ -84,3 +84,37 @@ def test_tokens_whose_negation_is_pending(dtype):
     with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
         want, got = layer(-x)[0], layer(torch._neg_view(x))[0]
     assert torch.equal(got, want)
+
+
+# router alone; one half of the shared expert's gate and up; everything but that half and the router
+@pytest.mark.parametrize("wide", [("gate.weight",), ("shared_expert.w_gate.weight",),
+                                  ("w_up", "w_down", "shared_expert.w_up.weight", "shared_expert.w_down.weight")])
+def test_layer_of_mixed_types(wide):
+    """Some parameters fp32, the others bf16, on a stream that is not the default one: the bf16 layer's bits, each gradient in the
+    type of its parameter."""
+    torch.manual_seed(5)
+    layer = MoELayer(128, 256, 8, 2, num_shared_experts=1, aux_loss_coeff=0.01).to(DEV).bfloat16().train(True)
+    mixed = MoELayer(128, 256, 8, 2, num_shared_experts=1, aux_loss_coeff=0.01).to(DEV).bfloat16().train(True)
+    mixed.load_state_dict(layer.state_dict())
+    parameters = dict(mixed.named_parameters())
+    for name in wide:
+        parameters[name].data = parameters[name].data.float()
+    x = torch.randn(300, 128, device=DEV).bfloat16()
+    go = torch.randn(300, 128, device=DEV).bfloat16()
+
+    def step(m):
+        tokens = x.detach().requires_grad_(True)
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            out, losses = m(tokens)
+        leaves = [tokens, *m.parameters()]
+        return out, torch.autograd.grad([out, losses["aux_loss"]], leaves, [go, torch.ones((), device=DEV)]), leaves
+
+    ref, ref_grads, _ = step(layer)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        out, grads, leaves = step(mixed)
+    torch.cuda.current_stream().wait_stream(side)
+    assert torch.equal(out, ref)
+    for got, want, leaf in zip(grads, ref_grads, leaves):
+        assert got.dtype == leaf.dtype and torch.equal(got.float(), want.float())
