@@ -201,7 +201,7 @@ py::tuple layer_forward(const Tensor& hidden, const Tensor& gate, const Tensor& 
   Tensor h_route = h;
   if (jitter > 0.0) h_route = h * at::empty_like(h).uniform_(1.0 - jitter, 1.0 + jitter);
   Tensor bias;
-  if (expert_bias.has_value()) bias = require(expert_bias->to(at::kFloat).contiguous(), at::kFloat, "expert_bias");
+  if (expert_bias.has_value()) bias = require(expert_bias->to(at::kFloat).contiguous().resolve_neg(), at::kFloat, "expert_bias");
 
   const int64_t rows = rows_capacity(N * top_k, static_cast<int>(E));
   const int64_t ws_bytes = static_cast<int64_t>(forward_workspace(N, static_cast<int>(E), static_cast<int>(top_k)));
@@ -350,8 +350,8 @@ py::tuple layer_backward(const OptTensor& grad_out, const OptTensor& grad_aux, c
   // computed() also densifies expanded (stride-0) gradients
   const Tensor go = grad_out.has_value() ? computed(*grad_out, "go") : at::zeros({N, D}, b16);
   Tensor gaux, gz;
-  if (grad_aux.has_value()) gaux = grad_aux->to(at::kFloat);
-  if (grad_z.has_value()) gz = grad_z->to(at::kFloat);
+  if (grad_aux.has_value()) gaux = grad_aux->to(at::kFloat).resolve_neg();
+  if (grad_z.has_value()) gz = grad_z->to(at::kFloat).resolve_neg();
   // [D, Hs] has few output tiles (32 CTA-pair tiles at D = 1024, Hs = 2048 for 74 pairs): split the token dimension in two
   // halves, each accumulated in fp32, and add the two bf16 results
   const int64_t split = (N + 127) / 128 >= 64 && (D / 256) * ((Hs + 255) / 256) <= 40 ? 2 : 1;

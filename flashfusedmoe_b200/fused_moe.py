@@ -217,7 +217,7 @@ class _Cfg:
 
 def _to(t, dtype):
     t = t if t.dtype == dtype else t.to(dtype)
-    return t if t.is_contiguous() else t.contiguous()
+    return (t if t.is_contiguous() else t.contiguous()).resolve_neg()   # kernels read memory, which holds no pending negation
 
 
 def _dense_ts(rows, device, split=1):

@@ -266,7 +266,7 @@ def route_forward(hidden, gate_w, top_k, gating="softmax", expert_bias=None, wei
     T = N * top_k
     rows_cap = rows_capacity(T, E)
     if expert_bias is not None:
-        expert_bias = _req(expert_bias.to(torch.float32).contiguous(), torch.float32, "expert_bias")
+        expert_bias = _req(expert_bias.to(torch.float32).contiguous().resolve_neg(), torch.float32, "expert_bias")
     r = Routing(
         topk_w=torch.empty(N, top_k, dtype=torch.float32, device=dev),
         topk_idx=torch.empty(N, top_k, dtype=torch.int32, device=dev),

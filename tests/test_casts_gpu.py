@@ -7,7 +7,8 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-from flashfusedmoe_b200 import MoELayer, _lib  # noqa: E402
+from flashfusedmoe_b200 import MoELayer, _lib, fused_moe, set_expert_gemm_precision  # noqa: E402
+from flashfusedmoe_b200.fused_moe import glu_ffn  # noqa: E402
 
 DEV = "cuda"
 
@@ -118,3 +119,41 @@ def test_layer_of_mixed_types(wide):
     assert torch.equal(out, ref)
     for got, want, leaf in zip(grads, ref_grads, leaves):
         assert got.dtype == leaf.dtype and torch.equal(got.float(), want.float())
+
+
+def _negated(t):
+    return torch._neg_view(t.neg())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_other_operands_whose_negation_is_pending(dtype):
+    """The selection bias, the weights of the e4m3 projections, the gradients of the losses and a plain GLU block's operands."""
+    torch.manual_seed(7)
+    x = torch.randn(600, 128, device=DEV).bfloat16()
+    g, wu, wd = (torch.randn(*s, device=DEV).mul_(0.05).to(dtype) for s in ((8, 128), (8, 512, 128), (8, 128, 256)))
+    bias = torch.randn(8, device=DEV).to(dtype)
+
+    def moe(*weights, expert_bias=None):
+        with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+            return fused_moe(x, *weights, top_k=2, expert_bias=expert_bias)[0]
+
+    assert torch.equal(moe(g, wu, wd, expert_bias=_negated(bias)), moe(g, wu, wd, expert_bias=bias))
+    set_expert_gemm_precision("fp8")
+    try:
+        want = moe(g, wu.bfloat16(), wd.bfloat16())
+        assert torch.equal(moe(g, _negated(wu), _negated(wd)), want)
+    finally:
+        set_expert_gemm_precision("bf16")
+
+    gate, up, down = (torch.randn(*s, device=DEV).mul_(0.05).to(dtype) for s in ((256, 128), (256, 128), (128, 256)))
+    with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+        want = glu_ffn(x, gate, up, down, "swiglu")
+        assert torch.equal(glu_ffn(_negated(x), _negated(gate), _negated(up), _negated(down), "swiglu"), want)
+
+    def gate_gradient(of_loss):
+        weight = g.detach().requires_grad_(True)
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            losses = fused_moe(x, weight, wu, wd, top_k=2, gating="sigmoid", aux_loss_coeff=0.01, z_loss_coeff=0.01)[1]
+        return torch.autograd.grad([losses["aux_loss"], losses["z_loss"]], weight, [of_loss, of_loss])[0]
+
+    assert torch.equal(gate_gradient(_negated(torch.ones((), device=DEV))), gate_gradient(torch.ones((), device=DEV)))
