@@ -9,13 +9,14 @@
 // 64 us with loads issued under `lane == 0`; with an elected thread the whole call went from 214 to 205 us. 128 tokens on 256
 // experts, D = 7168, H = 2048: 2110 + 1070 us (7.0 and 6.9 TB/s, what a plain read of such tiles reaches) against 2365 + 1182.
 // The up-projection can gather the token rows itself (TMA gather4, four rows per instruction), which saves the permute
-// launch and costs more than it where experts have several rows: 120 -> 132 us at 48 tokens on 64 experts, 74 -> 76 at 8.
+// launch and costs about as much where experts have several rows (48 tokens on 64 experts and a shared one, whole call, replayed:
+// 201 us with the permute, 197 without).
 //
 //   warp 0      TMA producer          warp 1   MMA issuer, TMEM owner
 //   warps 2..9  epilogue: two groups of four warps (one per TMEM lane quarter) take the 32-token steps of a tile in turn
 //
-// Ring of 8 stages (16 KiB of weights + up to 8 KiB of tokens): 128 KiB of weights in flight per SM. Fewer stages are
-// slower (6: 122 / 65 us, 4: 132 / 71 us); stages twice as deep (128 rows x 256 bytes in one box, four of them) take the same
+// Ring of 8 stages (16 KiB of weights + up to 8 KiB of tokens): 128 KiB of weights in flight per SM. Fewer stages were
+// slower (8: 121 / 64 us, 6: 122 / 65, 4: 132 / 71, with loads issued under `lane == 0`); stages twice as deep (128 rows x 256 bytes in one box, four of them) take the same
 // time within 1 %. As in the other GEMM: fp32 accumulators in TMEM, two of them, persistent CTAs,
 // bounded waits, TMA stores.
 //

@@ -6,7 +6,7 @@
 // thousand tokens.
 //
 // Every launch waits for the end of the one before it on its stream. Placed ahead of that end (programmatic stream
-// serialization) a forward pass is a few us faster: prefill of 1999 tokens 117 -> 111. But in loops of training
+// serialization) a forward pass is up to 3 % faster (4096 tokens on 64 experts 663 us instead of 681). But in loops of training
 // calls that filled the launch queue (3001 tokens on 16 experts) two of six runs did not come to an end, with events that other
 // streams wait for between such launches. No cause was found in the kernels, and a library cannot keep events from between its
 // launches: the calls release the interpreter's lock, and the allocator records events of its own.

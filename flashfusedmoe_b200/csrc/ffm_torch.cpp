@@ -1,9 +1,9 @@
 // The single-GPU layer's passes for torch tensors: operand checks and casts, output and scratch allocations and the
 // argument block of ffm_layer_forward / ffm_layer_backward, in one call from Python each way.
 //
-// From Python these cost more host time than the GPU needed for a small call: a decode step of one token (8 experts and a
-// shared one) took 91 us of host time, 15 of them in the library with its five launches, and the GPU 46; now 68. See
-// fused_moe.py for what stays there (validation, losses, the autograd function).
+// From Python these cost more host time than the GPU needs for a small call: a decode step of one token (8 experts and a shared
+// one) took 91 us of host time, 15 of them in the library with its five launches; now 62 to 70, while the GPU needs 31
+// (replayed from a graph). See fused_moe.py for what stays there (validation, losses, the autograd function).
 #include <torch/extension.h>
 
 #include <initializer_list>

@@ -381,26 +381,24 @@ def _require_bf16(dtype):
 # ----------------------------------------------------------------------------------------------
 
 # Decode-sized calls without gradients. The GEMMs that stream weights past a few tokens (ffm_decode_*) take over up to this
-# many routed rows per expert. Measured at 64 experts, K = 2048, H = 1408, up + down in us against the 128-row tiles:
-# 4 rows 131 + 75 -> 121 + 64, 32 rows 132 + 75 -> 126 + 67, 64 rows (many experts past one 64-token tile) 131 + 75 ->
-# 170 + 97.
+# many routed rows per expert. Whole calls, replayed, in us with the 128-row tiles and with these GEMMs at 32 / 48 / 64 rows per
+# expert: 4 experts, D = 2048, H = 1408 49 -> 37 / 49 -> 38 / 49 -> 43; 4 experts, D = H = 4096 109 -> 95 / 109 -> 97 / 109 -> 117; 8
+# experts, D = H = 4096 172 -> 161 / 172 -> 162 / 172 -> 180. At 64 rows it depends on the size.
 _DECODE_ROWS = 32
 # And up to this many tokens: rows per expert are an average, what bounds them under any load is the number of tokens, and
-# every 64 rows of an expert read its weights once more. The whole call, replayed, in us with 128-row tiles and with these
-# GEMMs, at the shape above, the load spread over all 64 experts / over 6 / over 12: 64 tokens 238 -> 219, 72 -> 59, 84 -> 84;
-# 128 tokens 240 -> 223, 74 -> 78, 84 -> 98; 160 tokens 244 -> 225, 78 -> 94, 90 -> 113; 341 tokens 254 -> 238, 100 -> 156 (over
-# 6). Up to 128 tokens no load was found that takes longer than these calls did when the host issued the launches one by one
-# and routing took three to five of them (94 and 104 us over 6 and 12); beyond, skewed loads do.
+# every 64 rows of an expert read its weights once more. The same at 64 experts, top-6, D = 2048, H = 1408, with the load spread over
+# all 64 experts / over 12 / over 6: 48 tokens 222 -> 193, 73 -> 66, 60 -> 47; 128 tokens 227 -> 200, 75 -> 74, 63 -> 57; 160 tokens
+# 231 -> 205, 79 -> 81, 68 -> 68; 341 tokens 242 -> 221, 110 -> 113, 92 -> 110.
 _DECODE_TOKENS = 128
-# The shared expert runs in the same kernels up to one 64-token tile (14 + 17 us instead of 18 + 20 at 48 tokens, D = 2048,
-# Hs = 2816). Whole calls of 16 and 64 tokens with 8 experts, replayed, dense tiles -> here, in us: D = 1024, Hs = 2048 65 ->
-# 61 and 66 -> 64; D = 4096, Hs = 2048 129 -> 123 and 129 -> 127; D = 4096, Hs = 8192 148 -> 141 and 152 to 154 -> 156 to 164
-# (over two allocations: the one point found on the slower side); D = 7168, Hs = 8192 230 -> 219 and 231 -> 223.
+# The shared expert runs in the same kernels up to one 64-token tile. Whole calls of 16 and 64 tokens with 8 experts, replayed,
+# dense tiles -> here, in us: D = 1024, Hs = 2048 50 -> 42 and 54 -> 43; D = 4096, Hs = 2048 100 -> 98 and 101 -> 101; D = 4096, Hs =
+# 8192 127 -> 112 and 144 -> 128; D = 7168, Hs = 8192 189 -> 182 and 221 -> 189.
 _DECODE_SHARED_TOKENS = 64
 # Up to this many bytes of weights a call is over before the host has issued it: one chain of launches, with the token
 # rows gathered in the up-projection instead of a permute, and the shared expert inside the two GEMMs instead of beside
-# them. One token, 8 experts and a shared one (0.11 GB): 98 -> 86 us. Above, where the GPU is the slower side, both cost: 48
-# tokens on 64 experts and a shared one (1.15 GB) 212 -> 238 us.
+# them. One token, 8 experts and a shared one (0.11 GB): 96 -> 62 us queued (all of it host time), 34 -> 31 replayed; 7 tokens
+# 76 -> 63 and 48 -> 41. Above, the GPU is the slower side and the two ways are level: 48 tokens on 64 experts and a shared one
+# (1.15 GB) 208 and 207 us queued, 201 and 197 replayed.
 _ONE_CHAIN_BYTES = 256 << 20
 _FEW_TILES, _FEW_DECODE_UP, _FEW_DECODE_DOWN, _FEW_DECODE_SHARED, _FEW_ONE_CHAIN = 1, 2, 4, 8, 16   # FFM_FEW_*
 
@@ -408,10 +406,13 @@ _FEW_TILES, _FEW_DECODE_UP, _FEW_DECODE_DOWN, _FEW_DECODE_SHARED, _FEW_ONE_CHAIN
 def _streams_weights(N, K):
     """Where the decode GEMM is the faster one for a contraction over K. Up + down in us with 128-row tiles and with it: 7 tokens
     on 8 experts, D = 4096, H = 14336 341 + 170 -> 301 + 162; 128 tokens on 256 experts, D = 7168, H = 2048 2365 + 1182 -> 2110 +
-    1070; 8 tokens there 516 + 282 -> 475 + 252; 48 tokens on 64 experts, D = H = 3072 410 + 227 -> 365 + 199; 64 tokens, D = 7168,
-    8 experts, skewed 78 + 35 -> 56 + 35. (Its times had scattered with where the weights lie, up to 2760 + 1600 in the second
-    case, before an elected thread issued its loads.) With a second token tile it stays behind where a tile is long and
-    few: 128 tokens, 8 experts, skewed, K = 14336 168 -> 162 to 186; the same with K = 7168 and below is faster throughout."""
+    1070; 8 tokens there 516 + 282 -> 475 + 252; 48 tokens on 64 experts, D = H = 3072 410 + 227 -> 365 + 199.
+    With a second token tile it depends on the load, which the host does not know. Whole calls of 65 to 128 tokens, replayed, up /
+    down alone exchanged: all 8 experts hit, K from 2560 to 7168 -52 to 0 / -18 to +4 us of 68 to 486; 64 experts hit, D = H = 3072
+    -50 / -36 of 657. Where all tokens choose the same few experts an up-projection loses when its tiles end in a nearly empty wave:
+    2 of 8 experts hit, D = H = 7168 +25 of 155, D = 4096, H = 14336 +14 of 205 (H = 7168 +14 of 119, its down-projection -22); 12 of
+    64, D = H = 3072 +6 / +7 of 150. Most such loads gain too (2 of 8, D = 7168, H = 2048 -30 of 104). At K = 14336 a down-projection
+    is -45 to +21 of 205 to 330: that one keeps the 128-row tiles."""
     return N <= 64 or K <= 8192
 
 
